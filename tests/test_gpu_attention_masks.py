@@ -1,0 +1,96 @@
+"""Attention of few queries and attention under boolean masks against the plain statement in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchtune_b200 import ops
+from torchtune_b200.ops import reference as ref
+from torchtune_b200.ops.mask import AttentionMask
+
+
+@pytest.fixture(autouse=True)
+def _check_device_errors():
+    yield
+    from torchtune_b200.ops._lib import check_device_errors
+
+    torch.cuda.synchronize()
+    check_device_errors()
+
+
+def _qkv(b, s, sk, hq, hkv, d, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn(b, n, h, d, generator=g, device="cuda").to(torch.bfloat16) for n, h in ((s, hq), (sk, hkv), (sk, hkv))]
+
+
+def _check(q, k, v, mask, dense):
+    with torch.no_grad():
+        got = ops.attention(q, k, v, mask)
+    want = ref.span_attention(q.double(), k.double(), v.double(), dense, q.shape[-1] ** -0.5).double()
+    # probabilities are rounded to 8 bits once (2^-9 relative, weights sum to 1) and so is the result
+    bound = 2.0**-8 * (want.abs() + v.double().abs().amax())
+    assert ((got.double() - want).abs() <= bound).all(), float(((got.double() - want).abs() - bound).max())
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,s,sk,hq,hkv", [(1, 1, 1, 4, 4), (1, 1, 61, 32, 8), (3, 1, 64, 8, 8), (2, 1, 65, 16, 1), (1, 4, 129, 8, 2), (40, 1, 200, 32, 8), (1, 1, 4097, 8, 1), (2, 16, 333, 2, 2),
+                                           (1, 1, 65536, 1, 1)])
+def test_few_queries(b, s, sk, hq, hkv, d):
+    """Tile edges, cluster sizes, one to sixteen rows per key head; boolean masks (also views of wider ones), causal ends and row starts."""
+    q, k, v = _qkv(b, s, sk, hq, hkv, d, seed=sk)
+    at = torch.arange(sk, device="cuda")
+    used = max(s, sk - 3)
+    own = torch.arange(used - s, used, device="cuda")
+    wide = torch.zeros(1, s, sk + 5, dtype=torch.bool, device="cuda")
+    wide[..., :sk] = at[None, None, :] <= own[None, :, None]
+    k[:, used:], v[:, used:] = float("nan"), float("nan")  # slots that no query sees don't enter the result
+    kk, vv = k.nan_to_num(), v.nan_to_num()
+    with torch.no_grad():
+        torch.testing.assert_close(ops.attention(q, k, v, AttentionMask(causal=False, bool_mask=wide[..., :sk])), ops.attention(q, kk, vv, AttentionMask(causal=False, bool_mask=wide[..., :sk])), rtol=0, atol=0)
+    _check(q, kk, vv, AttentionMask(causal=False, bool_mask=wide[..., :sk]), wide[..., :sk].expand(b, s, sk))
+    _check(q, kk, vv, AttentionMask(causal=True), (at[None, None, :] <= (sk - s + torch.arange(s, device="cuda"))[None, :, None]).expand(b, s, sk))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    m = torch.rand(b, s, sk, generator=g, device="cuda") < 0.4
+    m[0, 0] = False  # a query that sees nothing gives zeros
+    _check(q, kk, vv, AttentionMask(causal=False, bool_mask=m), m)
+    start = torch.randint(0, max(1, sk - s), (b,), generator=g, device="cuda", dtype=torch.int32)
+    slots = AttentionMask(causal=True, key_start=start, query_start=sk - s)
+    _check(q, kk, vv, slots, slots.dense(b, s, sk, "cuda"))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,s,sk", [(2, 300, 300), (1, 513, 700), (3, 130, 257)])
+def test_boolean_masks(b, s, sk, d):
+    """Causal masks over a wider cache (shared by all rows), left padding, masks with gaps, ranges that jump and rows that see nothing."""
+    q, k, v = _qkv(b, s, sk, 8, 2, d, seed=s)
+    at, own = torch.arange(sk, device="cuda"), torch.arange(s, device="cuda")
+    causal = (at[None, :] <= own[:, None])[None]
+    _check(q, k, v, AttentionMask(causal=False, bool_mask=causal), causal.expand(b, s, sk))
+    pad = torch.randint(0, s // 2, (b,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    left = (causal & (at >= pad[:, None, None])) | (at[None, :] == own[:, None])
+    _check(q, k, v, AttentionMask(causal=False, bool_mask=left.unsqueeze(1)), left)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    gaps = torch.rand(b, s, sk, generator=g, device="cuda") < 0.2
+    gaps[:, 5] = False
+    _check(q, k, v, AttentionMask(causal=False, bool_mask=gaps), gaps)
+    jump = torch.zeros(b, s, sk, dtype=torch.bool, device="cuda")  # the two query tiles of a CTA see far ranges, in either order
+    jump[:, :128, sk - 20 :], jump[:, 128:, :9] = True, True
+    _check(q, k, v, AttentionMask(causal=False, bool_mask=jump), jump)
+    jump = jump.flip(2).contiguous()
+    _check(q, k, v, AttentionMask(causal=False, bool_mask=jump), jump)
+
+
+def test_mask_bounds_on_the_device_are_the_plain_ones():
+    from torchtune_b200.ops._cuda_attention import dense_mask_bounds, mask_row_bounds
+
+    g = torch.Generator().manual_seed(0)
+    for sk in (1, 15, 16, 17, 47, 400):
+        m = torch.rand(3, 7, sk + 3, generator=g) < 0.5
+        m[1, 2] = False
+        m[2, 3] = True
+        for view in (m[..., :sk], m[..., 3:], m[:1, :, 1 : sk + 1].expand(3, 7, sk)):
+            _, lo, hi = dense_mask_bounds(view, 3, 7, sk)
+            count = view.sum(-1)
+            lo2, hi2, solid = mask_row_bounds(view.cuda() if view.stride(0) else view[:1].cuda().expand(3, 7, sk))
+            assert (lo2.cpu() == lo).all() and (hi2.cpu() == hi).all()
+            assert (solid.cpu().bool() == ((count == 0) | (count == hi - lo + 1))).all()

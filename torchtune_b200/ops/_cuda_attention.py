@@ -4,8 +4,6 @@ from __future__ import annotations
 import math
 from typing import Optional, Tuple
 
-import os
-
 import torch
 
 from ._lib import check, err_word, lib, stream_ptr
@@ -42,15 +40,22 @@ def lower_bounds(mask: AttentionMask, b: int, s: int, device) -> Optional[torch.
     return lo
 
 
-def dense_mask_bounds(m: torch.Tensor, b: int, s: int, sk: int) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """Boolean mask (``[b, s, sk]``, ``[b, 1, s, sk]`` or anything that broadcasts to the first) → the kernel's
-    ``(kmask uint8 [b, s, sk], lo, hi)`` with ``lo`` / ``hi`` the first / last visible key of every row (``sk`` / ``-1`` for
-    rows that see nothing), which lets the kernel skip key blocks outside every row's range."""
+def _mask_rows(m: torch.Tensor, b: int, s: int, sk: int) -> torch.Tensor:
+    """A boolean mask in any of its forms as ``[b, s, sk]`` (a view where the given one allows it)."""
     if m.dim() == 4:
         if m.shape[1] != 1:
             raise ValueError("per-head boolean attention masks are not supported")
         m = m[:, 0]
-    m = m.to(torch.bool).expand(b, s, sk).contiguous()
+    return m.to(torch.bool).expand(b, s, sk)
+
+
+def dense_mask_bounds(m: torch.Tensor, b: int, s: int, sk: int) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Boolean mask (``[b, s, sk]``, ``[b, 1, s, sk]`` or anything that broadcasts to the first) → the kernel's
+    ``(kmask uint8 [b, s, sk], lo, hi)`` with ``lo`` / ``hi`` the first / last visible key of every row (``sk`` / ``-1`` for
+    rows that see nothing), which lets the kernel skip key blocks outside every row's range."""
+    m = _mask_rows(m, b, s, sk).contiguous()
+    if m.is_cuda:
+        return m.view(torch.uint8), *mask_row_bounds(m)[:2]
     seen = m.any(-1)
     as_int = m.to(torch.int8)
     first = as_int.argmax(-1)
@@ -60,34 +65,71 @@ def dense_mask_bounds(m: torch.Tensor, b: int, s: int, sk: int) -> Tuple[torch.T
     return m.view(torch.uint8), lo, hi
 
 
+def mask_row_bounds(m: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """``(lo, hi, solid)`` of a CUDA boolean mask ``[b, s, sk]`` with unit inner stride: first and last visible key of every row and whether all
+    keys between them are visible, each ``[b, s]`` (``[1, s]`` for a mask that is one batch row expanded); one pass over the mask."""
+    b = m.shape[0] if m.stride(0) or m.shape[0] == 1 else 1
+    s, sk = m.shape[1:]
+    lo = torch.empty(b, s, dtype=torch.int32, device=m.device)
+    hi = torch.empty_like(lo)
+    solid = torch.empty(b, s, dtype=torch.uint8, device=m.device)
+    if m.numel():
+        check(lib().ttb_mask_bounds(m.data_ptr(), m.stride(0), m.stride(1), b, s, sk, lo.data_ptr(), hi.data_ptr(), solid.data_ptr(), stream_ptr()), "mask bounds")
+    return lo, hi, solid
+
+
 def _p(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+def decodes(s: int, sk: int, hq: int, hkv: int) -> bool:
+    """Whether a gradient-free call runs on the decoding kernel: its query rows per key head fit one 16-row tile and the visibility words of a
+    CTA fit their share of shared memory (one query: up to 65 536 keys).  One query row of 128 is real on the tile kernels at these sizes."""
+    return s * (hq // hkv) <= 16 and -(-sk // 64) * (s + 1) * 8 <= 16384
+
+
 class _FlashAttention(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, lo, hi, kmask, monotone, scale, causal, softcap):
+    def forward(ctx, q, k, v, lo, hi, kmask, monotone, scale, causal, softcap, mask=None):
+        """``mask``: a boolean mask ``[b, s, sk]`` (bool, unit inner stride); for backward and for soft-capped scores it comes as ``kmask`` and its bounds too."""
         b, s, hq, d = q.shape
         sk, hkv = k.shape[1], k.shape[2]
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         o = torch.empty_like(q)
-        lse = torch.empty(b, hq, s, dtype=torch.float32, device=q.device)
-        # head dim 128 with structured (monotone) bounds: two query tiles per CTA, probabilities kept in tensor memory
-        two_tile = d == 128 and kmask is None and softcap == 0.0 and (monotone or (lo is None and hi is None)) and os.environ.get("TTB_ATTN_TWO_TILE", "1") != "0"
-        if two_tile:
+        grads = any(ctx.needs_input_grad)
+        if not grads and softcap == 0.0 and decodes(s, sk, hq, hkv):
+            if causal and hi is None:  # as many keys as queries here
+                hi = torch.arange(s, device=q.device, dtype=torch.int32).view(1, s).expand(b, s).contiguous()
             check(
-                lib().ttb_attn_fwd2(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(lo), _p(hi), b, s, sk, hq, hkv, float(scale), int(causal),
+                lib().ttb_attn_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), _p(mask), 0 if mask is None else mask.stride(0), 0 if mask is None else mask.stride(1),
+                                      _p(lo), _p(hi), b, s, sk, hq, hkv, d, float(scale), stream_ptr()),
+                "attention of few queries",
+            )
+            return o
+        lse = torch.empty(b, hq, s, dtype=torch.float32, device=q.device)
+        if mask is not None:
+            lo, hi, solid = mask_row_bounds(mask)
+            check(
+                lib().ttb_attn_fwd2_masked(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(), solid.data_ptr(),
+                                           s if lo.shape[0] > 1 else 0, mask.data_ptr(), mask.stride(0), mask.stride(1), b, s, sk, hq, hkv, d, float(scale),
+                                           err_word(q.device).data_ptr(), stream_ptr()),
+                "attention forward (boolean mask)",
+            )
+        elif softcap == 0.0:  # structured (monotone) bounds
+            check(
+                lib().ttb_attn_fwd2(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(lo), _p(hi), b, s, sk, hq, hkv, d, float(scale), int(causal),
                                     err_word(q.device).data_ptr(), stream_ptr()),
-                "attention forward (two query tiles)",
+                "attention forward",
             )
         else:
             check(
                 lib().ttb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(lo), _p(hi), _p(kmask), int(monotone), b, s, sk, hq, hkv, d,
                                    float(scale), int(causal), float(softcap), err_word(q.device).data_ptr(), stream_ptr()),
-                "attention forward",
+                "attention forward (soft-capped scores)",
             )
-        ctx.save_for_backward(q, k, v, o, lse, lo, hi, kmask)
-        ctx.meta = (scale, causal, softcap, monotone)
+        if grads:
+            ctx.save_for_backward(q, k, v, o, lse, lo, hi, kmask)
+            ctx.meta = (scale, causal, softcap, monotone)
         return o
 
     @staticmethod
@@ -106,7 +148,7 @@ class _FlashAttention(torch.autograd.Function):
                                _p(lo), _p(hi), _p(kmask), int(monotone), b, s, sk, hq, hkv, d, float(scale), int(causal), float(softcap), err_word(q.device).data_ptr(), stream_ptr()),
             "attention backward",
         )
-        return dq_acc.to(q.dtype), dk, dv, None, None, None, None, None, None, None
+        return dq_acc.to(q.dtype), dk, dv, None, None, None, None, None, None, None, None
 
 
 def unsupported_reason(q: torch.Tensor, k: torch.Tensor, mask: AttentionMask) -> Optional[str]:
@@ -130,7 +172,7 @@ def attention(q, k, v, mask: AttentionMask, scale: Optional[float], softcap: flo
     b, s, hq, d = q.shape
     sk = k.shape[1]
     scale = (1.0 / math.sqrt(d)) if scale is None else scale
-    lo = hi = kmask = None
+    lo = hi = kmask = dense = None
     monotone, causal = 1, bool(mask.causal)
     if mask.key_start is not None:
         if mask.key_start.numel() != b or mask.query_start + s > sk:
@@ -138,6 +180,10 @@ def attention(q, k, v, mask: AttentionMask, scale: Optional[float], softcap: flo
         lo = mask.key_start.to(device=q.device, dtype=torch.int32).view(b, 1).expand(b, s).contiguous()
         hi = (torch.arange(s, device=q.device, dtype=torch.int32) + mask.query_start).view(1, s).expand(b, s).contiguous()
         causal = False
+    elif mask.bool_mask is not None and softcap == 0.0 and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)):
+        dense = _mask_rows(mask.bool_mask.to(q.device), b, s, sk)
+        dense = dense if dense.stride(2) == 1 or sk == 1 else dense.contiguous()
+        monotone, causal = 0, False
     elif mask.bool_mask is not None:
         cached = getattr(mask, "_dense_cache", None)
         if cached is not None and cached[0] == (b, s, sk, mask.bool_mask.data_ptr()):
@@ -148,9 +194,10 @@ def attention(q, k, v, mask: AttentionMask, scale: Optional[float], softcap: flo
                 mask._dense_cache = ((b, s, sk, mask.bool_mask.data_ptr()), (kmask, lo, hi))
             except Exception:
                 pass
+        dense = kmask.view(torch.bool) if softcap == 0.0 else None
         monotone, causal = 0, False
     else:
         lo = lower_bounds(mask, b, s, q.device)
         if causal and s != sk:  # queries are the last s positions of the key sequence (bottom-right aligned causal mask)
             hi = (torch.arange(s, device=q.device, dtype=torch.int32) + (sk - s)).view(1, s).expand(b, s).contiguous()
-    return _FlashAttention.apply(q, k, v, lo, hi, kmask, monotone, scale, causal, float(softcap or 0.0))
+    return _FlashAttention.apply(q, k, v, lo, hi, kmask, monotone, scale, causal, float(softcap or 0.0), dense)

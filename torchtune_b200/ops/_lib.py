@@ -63,8 +63,14 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_attn_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, f32, vp, vp]
     L.ttb_attn_bwd.restype = i32
     L.ttb_attn_fwd.restype = i32
-    L.ttb_attn_fwd2.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp]
+    L.ttb_attn_fwd2.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp, vp]
     L.ttb_attn_fwd2.restype = i32
+    L.ttb_attn_fwd2_masked.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i64, vp, i64, i64, i32, i32, i32, i32, i32, i32, f32, vp, vp]
+    L.ttb_attn_fwd2_masked.restype = i32
+    L.ttb_attn_decode.argtypes = [vp, vp, vp, vp, vp, i64, i64, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp]
+    L.ttb_attn_decode.restype = i32
+    L.ttb_mask_bounds.argtypes = [vp, i64, i64, i32, i32, i32, vp, vp, vp, vp]
+    L.ttb_mask_bounds.restype = i32
     L.ttb_gemm_bf16_2sm.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i64, i64, i64, i32, vp, f32, vp, vp]
     L.ttb_gemm_bf16_2sm.restype = i32
     L.ttb_ensure_device.argtypes = [i32]

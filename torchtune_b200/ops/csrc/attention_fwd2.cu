@@ -9,8 +9,11 @@
 // for long.  S_X(j+1) may overwrite P_X(j) because MMAs of one thread execute in issue order.
 //
 // Masks: per-query bounds lo / hi that do not decrease along the sequence (causal, packed documents, sliding windows, chunks), or
-// none.  Each tile visits only its own range of key blocks.  Element-wise masks, soft-capping and head dims other than 128 stay on
-// the one-tile kernel in attention.cu.  Every wait is bounded and reports through the error word.
+// none; each tile visits only its own range of key blocks.  A boolean mask comes with the bounds of its rows in any order (the MASKED
+// form takes a tile's range from all its rows) and a flag per row that says whether everything between its bounds is visible: then the
+// bounds are the whole mask, as for the causal masks of cached generation, and only the other rows read mask bytes.
+// Causal forward, head dim 64 (one-tile kernel before): 8 x 2048 tokens 788 -> 374 us, 1 x 16384 tokens 5079 -> 2042 us; exponentials bound it.
+// Soft-capped scores stay on the one-tile kernel in attention.cu.  Every wait is bounded and reports through the error word.
 #include "common/attn_math.cuh"
 #include "common/ptx.cuh"
 #include "common/tmap.h"
@@ -19,10 +22,11 @@ namespace ttb {
 namespace fa2 {
 
 using namespace attn;
-static constexpr int D = 128;
-static constexpr int kTileBytes = kBlk * D * 2;
 static constexpr int kThreads = 384;
-static constexpr int kSmemBytes = 6 * kTileBytes + 1024 + 256;
+template <int D>
+static constexpr int kTileBytesOf = kBlk * D * 2;
+template <int D>
+static constexpr int kSmemBytes = 6 * kTileBytesOf<D> + 1024 + 256;
 
 struct Params {
   int b, s, sk, hq, hkv;
@@ -30,13 +34,21 @@ struct Params {
   int causal;
   const int* lo;  // [b, s] or nullptr
   const int* hi;  // [b, s] or nullptr (causal: q, else sk - 1)
+  // MASKED: bounds of every mask row (both given; bound_b elements from one batch row to the next, 0 = shared), the rows' flags laid out
+  // like the bounds, and the mask bytes of row (b, i) at mask + b * mask_b + i * mask_r
+  long long bound_b;
+  const uint8_t* solid;
+  const uint8_t* mask;
+  long long mask_b, mask_r;
   __nv_bfloat16* o;
   float* lse;
   int* err;
 };
 
+template <int D, bool MASKED>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, Params p) {
+  constexpr int kTileBytes = kTileBytesOf<D>, kPanels = D / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ[2] = {smem, smem + kTileBytes};
@@ -53,6 +65,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* o_done = bars + 13;   // [2] per tile
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* ranges = reinterpret_cast<int*>(tmem_slot + 2);  // MASKED, per tile: smallest lo, largest lo, smallest hi, largest hi, rows that read mask bytes
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, bi = blockIdx.z;
@@ -60,6 +73,24 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int q0 = blockIdx.x * 2 * kBlk;
   const int row_base = bi * p.s;
   const int krow_base = bi * p.sk;
+  const long long bound_base = MASKED ? bi * p.bound_b : row_base;
+  if (MASKED) {
+    if (threadIdx.x < 10) {
+      const int f = threadIdx.x % 5;
+      ranges[threadIdx.x] = f == 0 || f == 2 ? 0x7fffffff : (f == 4 ? 0 : -1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kBlk && q0 + static_cast<int>(threadIdx.x) < p.s) {
+      int* t = ranges + 5 * (threadIdx.x / kBlk);
+      const int lo = p.lo[bound_base + q0 + threadIdx.x], hi = p.hi[bound_base + q0 + threadIdx.x];
+      atomicMin(t, lo);
+      atomicMax(t + 1, lo);
+      atomicMin(t + 2, hi);
+      atomicMax(t + 3, hi);
+      if (!p.solid[bound_base + q0 + threadIdx.x]) atomicOr(t + 4, 1);
+    }
+    __syncthreads();
+  }
 
   // Key-block range of each tile: [begin, begin + count).  The bounds are monotone, so first and last row give them.
   int begin[2], count[2];
@@ -71,11 +102,16 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       continue;
     }
     const int qz = min(qa + kBlk, p.s) - 1;
-    const int lo_first = p.lo != nullptr ? max(p.lo[row_base + qa], 0) : 0;
-    const int hi_last = p.hi != nullptr ? p.hi[row_base + qz] : (p.causal ? qz : p.sk - 1);
+    const int lo_first = MASKED ? max(ranges[5 * x], 0) : (p.lo != nullptr ? max(p.lo[row_base + qa], 0) : 0);
+    const int hi_last = MASKED ? ranges[5 * x + 3] : (p.hi != nullptr ? p.hi[row_base + qz] : (p.causal ? qz : p.sk - 1));
     const int end_tok = min(p.sk, hi_last + 1);
     begin[x] = lo_first / kBlk;
     count[x] = max((end_tok + kBlk - 1) / kBlk - begin[x], 0);
+  }
+  if (MASKED && count[0] > 0 && count[1] > 0) {
+    // the stages are handed on block by block, so no block between the two ranges may be without a reader: the later range grows downwards
+    const int late = begin[0] > begin[1] ? 0 : 1, end = begin[1 - late] + count[1 - late];
+    if (begin[late] > end) count[late] += begin[late] - end, begin[late] = end;
   }
   int u_begin, u_end;  // union of the two ranges
   if (count[0] > 0 && count[1] > 0) {
@@ -118,7 +154,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (lane == 0 && n_union > 0) {
       mbar_arrive_expect_tx(q_full, 2 * kTileBytes);
       for (int x = 0; x < 2; ++x)
-        for (int j = 0; j < 2; ++j) tma_load_2d(sQ[x] + j * kPanelBytes, &tmQ, q_full, h * D + j * 64, row_base + q0 + x * kBlk);
+        for (int j = 0; j < kPanels; ++j) tma_load_2d(sQ[x] + j * kPanelBytes, &tmQ, q_full, h * D + j * 64, row_base + q0 + x * kBlk);
     }
     uint32_t phase = 0;
     for (int i = 0; i < n_union && !*abort_flag; ++i) {
@@ -130,7 +166,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       if (lane == 0) {
         mbar_arrive_expect_tx(&k_full[st], kTileBytes);
-        for (int j = 0; j < 2; ++j) tma_load_2d(sK[st] + j * kPanelBytes, &tmK, &k_full[st], hk * D + j * 64, krow_base + kv0);
+        for (int j = 0; j < kPanels; ++j) tma_load_2d(sK[st] + j * kPanelBytes, &tmK, &k_full[st], hk * D + j * 64, krow_base + kv0);
       }
       __syncwarp();
       if (!mbar_wait(&v_empty[st], phase ^ 1)) {
@@ -139,7 +175,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       if (lane == 0) {
         mbar_arrive_expect_tx(&v_full[st], kTileBytes);
-        for (int j = 0; j < 2; ++j) tma_load_2d(sV[st] + j * kPanelBytes, &tmV, &v_full[st], hk * D + j * 64, krow_base + kv0);
+        for (int j = 0; j < kPanels; ++j) tma_load_2d(sV[st] + j * kPanelBytes, &tmV, &v_full[st], hk * D + j * 64, krow_base + kv0);
       }
       __syncwarp();
       if (st == 1) phase ^= 1;
@@ -215,10 +251,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
     const bool row_valid = q_idx < p.s;
     const bool tile_valid = qa < p.s;
-    const int lo_row = (p.lo != nullptr && row_valid) ? p.lo[row_base + q_idx] : 0;
-    const int hi_row = (p.hi != nullptr) ? (row_valid ? p.hi[row_base + q_idx] : -1) : (p.causal ? (row_valid ? q_idx : -1) : (row_valid ? p.sk - 1 : -1));
-    const int lo_max = (p.lo == nullptr || !tile_valid) ? 0 : p.lo[row_base + q_last];
-    const int hi_min = !tile_valid ? -1 : ((p.hi != nullptr) ? p.hi[row_base + qa] : (p.causal ? qa : p.sk - 1));
+    const int lo_row = (p.lo != nullptr && row_valid) ? p.lo[bound_base + q_idx] : 0;
+    const int hi_row = (p.hi != nullptr) ? (row_valid ? p.hi[bound_base + q_idx] : -1) : (p.causal ? (row_valid ? q_idx : -1) : (row_valid ? p.sk - 1 : -1));
+    const int lo_max = (p.lo == nullptr || !tile_valid) ? 0 : (MASKED ? ranges[5 * x + 1] : p.lo[row_base + q_last]);
+    const int hi_min = !tile_valid ? -1 : (MASKED ? ranges[5 * x + 2] : ((p.hi != nullptr) ? p.hi[row_base + qa] : (p.causal ? qa : p.sk - 1)));
+    const bool bytes = MASKED && ranges[5 * x + 4] != 0;  // the same for all rows of the tile
+    const uint8_t* mrow = (bytes && row_valid && !p.solid[bound_base + q_idx]) ? p.mask + bi * p.mask_b + q_idx * p.mask_r : nullptr;
     const bool ragged_rows = qa + kBlk > p.s;  // rows past the end of the sequence must be masked in every block
     const float c = p.scale * kLog2e;
     float m_used = -INFINITY, l = 0.f;
@@ -245,6 +283,15 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int i = 0; i < 32; ++i) {
             const int j = kv0 + ch * 32 + i;
             if (j < lo_row || j > hi_row || j >= p.sk) sv[ch][i] = 0xff800000u;  // -inf
+          }
+        }
+      }
+      if (MASKED && bytes && mrow != nullptr) {
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            if (mrow[min(kv0 + ch * 32 + i, p.sk - 1)] == 0) sv[ch][i] = 0xff800000u;
           }
         }
       }
@@ -347,36 +394,56 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 2) tmem_dealloc(tmem_base, 512);
 }
 
+template <int D>
 static int make_head_map(CUtensorMap* m, const void* base, int b, int s, int heads) {
   return make_tmap_2d(m, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, static_cast<uint64_t>(b) * s, static_cast<uint64_t>(heads) * D,
                       static_cast<uint64_t>(heads) * D, kBlk, 64, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+template <int D, bool MASKED>
+static int launch(const void* q, const void* k, const void* v, const Params& p, cudaStream_t st) {
+  CUtensorMap tq, tk, tv;
+  int rc;
+  if ((rc = make_head_map<D>(&tq, q, p.b, p.s, p.hq)) != kOk) return rc;
+  if ((rc = make_head_map<D>(&tk, k, p.b, p.sk, p.hkv)) != kOk) return rc;
+  if ((rc = make_head_map<D>(&tv, v, p.b, p.sk, p.hkv)) != kOk) return rc;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(attn_fwd2_kernel<D, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<D>) != cudaSuccess) return kErrDriver;
+    attr = true;
+  }
+  dim3 grid((p.s + 2 * kBlk - 1) / (2 * kBlk), p.hq, p.b);
+  TTB_COUNT_LAUNCH(1);
+  attn_fwd2_kernel<D, MASKED><<<grid, kThreads, kSmemBytes<D>, st>>>(tq, tk, tv, p);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
+}
+
 }  // namespace fa2
 }  // namespace ttb
 
-// Forward attention for head dim 128 with monotone per-query bounds (or none): q [b, s, hq, 128], k / v [b, sk, hkv, 128], o like q,
-// lse [b, hq, s] (log2 domain).  lo / hi as in ttb_attn_fwd; they must not decrease along the sequence.
+// Forward attention with monotone per-query bounds (or none): q [b, s, hq, d], k / v [b, sk, hkv, d], o like q, lse [b, hq, s] (log2 domain), d 64 or
+// 128.  lo / hi as in ttb_attn_fwd; they must not decrease along the sequence.
 extern "C" int ttb_attn_fwd2(const void* q, const void* k, const void* v, void* o, float* lse, const int* lo, const int* hi, int b, int s, int sk,
-                             int hq, int hkv, float scale, int causal, int* err, void* stream) {
+                             int hq, int hkv, int d, float scale, int causal, int* err, void* stream) {
   using namespace ttb;
-  if (hq % hkv || s <= 0 || sk <= 0 || b <= 0) return kErrBadShape;
+  if ((d != 64 && d != 128) || hq % hkv || s <= 0 || sk <= 0 || b <= 0) return kErrBadShape;
   if (causal && hi == nullptr && s != sk) return kErrBadShape;
   fa2::Params p{};
   p.b = b, p.s = s, p.sk = sk, p.hq = hq, p.hkv = hkv, p.scale = scale, p.causal = causal, p.lo = lo, p.hi = hi;
   p.o = static_cast<__nv_bfloat16*>(o), p.lse = lse, p.err = err;
-  CUtensorMap tq, tk, tv;
-  int rc;
-  if ((rc = fa2::make_head_map(&tq, q, b, s, hq)) != kOk) return rc;
-  if ((rc = fa2::make_head_map(&tk, k, b, sk, hkv)) != kOk) return rc;
-  if ((rc = fa2::make_head_map(&tv, v, b, sk, hkv)) != kOk) return rc;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(fa2::attn_fwd2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fa2::kSmemBytes) != cudaSuccess) return kErrDriver;
-    attr = true;
-  }
-  dim3 grid((s + 2 * fa2::kBlk - 1) / (2 * fa2::kBlk), hq, b);
-  TTB_COUNT_LAUNCH(1);
-  fa2::attn_fwd2_kernel<<<grid, fa2::kThreads, fa2::kSmemBytes, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, p);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
+  auto st = static_cast<cudaStream_t>(stream);
+  return d == 128 ? fa2::launch<128, false>(q, k, v, p, st) : fa2::launch<64, false>(q, k, v, p, st);
+}
+
+// The same under a boolean mask: lo, hi, solid as ttb_mask_bounds gives them (bound_b elements per batch row, 0 = one set for all), the mask as there.
+extern "C" int ttb_attn_fwd2_masked(const void* q, const void* k, const void* v, void* o, float* lse, const int* lo, const int* hi, const void* solid, long long bound_b,
+                                    const void* mask, long long mask_b, long long mask_r, int b, int s, int sk, int hq, int hkv, int d, float scale, int* err, void* stream) {
+  using namespace ttb;
+  if ((d != 64 && d != 128) || hq % hkv || s <= 0 || sk <= 0 || b <= 0 || lo == nullptr || hi == nullptr || solid == nullptr || mask == nullptr) return kErrBadShape;
+  fa2::Params p{};
+  p.b = b, p.s = s, p.sk = sk, p.hq = hq, p.hkv = hkv, p.scale = scale, p.lo = lo, p.hi = hi;
+  p.solid = static_cast<const uint8_t*>(solid), p.bound_b = bound_b, p.mask = static_cast<const uint8_t*>(mask), p.mask_b = mask_b, p.mask_r = mask_r;
+  p.o = static_cast<__nv_bfloat16*>(o), p.lse = lse, p.err = err;
+  auto st = static_cast<cudaStream_t>(stream);
+  return d == 128 ? fa2::launch<128, true>(q, k, v, p, st) : fa2::launch<64, true>(q, k, v, p, st);
 }
