@@ -1,0 +1,86 @@
+"""Linear layers of a few tokens, and sampling, against plain statements in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchtune_b200 import ops
+
+
+def _rand(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda").to(torch.bfloat16)
+
+
+def _check(got, want, x, w, extra=0.0):
+    # one rounding to bf16 (2^-9 of the value, twice that for ties and the bias), and fp32 sums of K terms in any order
+    bound = 2.0**-8 * (want.abs() + extra) + 2.0**-19 * (x.double().abs() @ w.double().abs().t())
+    assert got.shape == want.shape and ((got.double() - want).abs() <= bound).all(), float(((got.double() - want).abs() - bound).max())
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(8, 8), (40, 136), (512, 2048), (1000, 1032), (4096, 1024), (20000, 264)])
+def test_products(M, N, K):
+    """Edges of the token tiles, rows and contractions that end inside a tile, one to eight CTAs per tile; pitched operands and outputs."""
+    from torchtune_b200.ops._cuda import _gemm_rows, gemm
+
+    x = _rand(M, K + 16, seed=M)[:, 8 : K + 8]
+    w = _rand(N, K + 8, seed=N)[:, :K]
+    bias = _rand(N, seed=3)
+    want = x.double() @ w.double().t()
+    _check(gemm(x, w), want, x, w)
+    _check(gemm(x, w, bias=bias, alpha=0.5), 0.5 * want + bias.double(), x, w, 1.0)
+    out = torch.full((M, N + 24), float("nan"), dtype=torch.float32, device="cuda")
+    _gemm_rows(x, [w], [out[:, :N]])
+    assert ((out[:, :N].double() - want).abs() <= 2.0**-19 * (x.double().abs() @ w.double().abs().t())).all() and out[:, N:].isnan().all()
+
+
+@pytest.mark.parametrize("M", [1, 16, 40, 64])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 264), (8192, 2048), (1032, 14336)])
+def test_residual_gate_and_groups(M, N, K):
+    from torchtune_b200.ops._cuda import _gemm_rows, gate_up_swiglu
+
+    x, w, w3 = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(N, K, seed=3)
+    r = _rand(M, N, seed=4)
+    a, b = x.double() @ w.double().t(), x.double() @ w3.double().t()
+    with torch.no_grad():
+        y = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        _gemm_rows(x, [w], [y], residual=r)
+        _check(y, a + r.double(), x, w)
+        _check(ops.linear_residual(x, w, None, r), a + r.double(), x, w, a.abs())  # other kernels round the product first
+        x, scale = x / K**0.5, K**-0.5
+        a, b = (x.double() @ t.double().t() for t in (w, w3))
+        for clamp in (None, (0.7, 1.702)):
+            got = gate_up_swiglu(x, w, w3, clamp)
+            if got is None:  # left to the separate operators
+                assert M > 32 and N > 4096
+                continue
+            got = got.double()
+            ca, cb = (a, b) if clamp is None else (a.clamp(max=clamp[0]), b.clamp(-clamp[0], clamp[0]) + 1)
+            want = ca * torch.sigmoid(ca * (1.0 if clamp is None else clamp[1])) * cb
+            # both pre-activations are rounded to bf16 first: 2^-8 of each, with |gate'| <= 1.1, then the result once more
+            bound = 2.0**-8 * (want.abs() + 1.2 * a.abs() * cb.abs() + ca.abs() * b.abs()) + 1e-4
+            assert ((got - want).abs() <= bound).all()
+        ws = [w, w3[: max(8, N // 4)], w3]
+        bias = _rand(N, seed=5)
+        for got, wi, bi in zip(ops.linear_group(x, ws, [None, None, bias]), ws, (None, None, bias)):
+            _check(got, x.double() @ wi.double().t() + (0 if bi is None else bi.double()), x, wi, 0 if bi is None else bi.double().abs())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V,top_k", [(1, 1), (7, 3), (4099, 50), (128256, 300), (128256, 128255), (128256, 0), (400000, 20)])
+def test_sampling(V, top_k, dtype):
+    """Rows shorter than their eight parts, parts that don't fit shared memory, ties at the threshold, infinities."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = (torch.randn(3, V, generator=g, device="cuda") * 3).to(dtype)
+    if V > 8:
+        logits[1] = logits[1].round()  # many ties
+        logits[2, : V // 2] = float("-inf")
+    q = -torch.log(torch.rand(3, V, generator=g, device="cuda").clamp_min(1e-7)) + 1e-7
+    got = ops.sample_tokens(logits, q, 0.6, top_k or None)
+    t = (logits / 0.6).float()
+    if 0 < top_k < V:
+        t = torch.where(t < torch.topk(t, top_k).values[:, -1:], float("-inf"), t)
+    race = t.double() - q.double().log()
+    picked = race.gather(1, got.long())
+    # logarithms and one subtraction in fp32: a few units of 2^-21 at logits below 32
+    assert (picked >= race.amax(1, keepdim=True) - 1e-5).all()

@@ -10,6 +10,7 @@ from torch import nn
 from .. import ops
 from ..ops.mask import AttentionMask
 from .kv_cache import KVCache
+from .linear import is_plain_linear
 
 logger = logging.getLogger(__name__)
 
@@ -114,7 +115,13 @@ class MultiHeadAttention(nn.Module):
         """``residual``: a tensor of the output's shape that is added to the result; with a plain output projection the addition
         happens in that projection's GEMM epilogue (a decoder layer passes its residual stream)."""
         b, s_x, _ = x.shape
-        q = self.q_proj(x).view(b, s_x, self.num_heads, self.head_dim)
+        k = v = None
+        projections = (self.q_proj, self.k_proj, self.v_proj)
+        if y is x and all(is_plain_linear(m) for m in projections):
+            q, k, v = ops.linear_group(x, [m.weight for m in projections], [m.bias for m in projections])
+        else:
+            q = self.q_proj(x)
+        q = q.view(b, s_x, self.num_heads, self.head_dim)
         if self.q_norm is not None and self.qk_norm_before_rope:
             q = self.q_norm(q)
         if self.pos_embeddings is not None:
@@ -128,8 +135,10 @@ class MultiHeadAttention(nn.Module):
             k, v = self.kv_cache.k_cache[:b], self.kv_cache.v_cache[:b]
         else:
             s_y = y.shape[1]
-            k = self.k_proj(y).view(b, s_y, self.num_kv_heads, self.head_dim)
-            v = self.v_proj(y).view(b, s_y, self.num_kv_heads, self.head_dim)
+            if k is None:
+                k, v = self.k_proj(y), self.v_proj(y)
+            k = k.view(b, s_y, self.num_kv_heads, self.head_dim)
+            v = v.view(b, s_y, self.num_kv_heads, self.head_dim)
             if self.k_norm is not None and self.qk_norm_before_rope:
                 k = self.k_norm(k)
             if self.pos_embeddings is not None:
@@ -158,6 +167,6 @@ class MultiHeadAttention(nn.Module):
         out = out.reshape(b, s_x, self.num_heads * self.head_dim)
         if residual is None:
             return self.output_proj(out)
-        if type(self.output_proj) is nn.Linear:
+        if is_plain_linear(self.output_proj):
             return ops.linear_residual(out, self.output_proj.weight, self.output_proj.bias, residual)
         return self.output_proj(out) + residual

@@ -7,6 +7,7 @@ import torch
 from torch import nn
 
 from .. import ops
+from .linear import is_plain_linear
 
 
 class ClampedGLU(nn.Module):
@@ -53,7 +54,7 @@ class FeedForward(nn.Module):
         """Down projection; with ``residual`` the block's input stream is added in the projection's GEMM epilogue."""
         if residual is None:
             return self.w2(h)
-        if type(self.w2) is nn.Linear:
+        if is_plain_linear(self.w2):
             return ops.linear_residual(h, self.w2.weight, self.w2.bias, residual)
         return self.w2(h) + residual
 

@@ -13,3 +13,9 @@ class Linear(nn.Linear):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         return ops.linear(x, self.weight, self.bias)
+
+
+def is_plain_linear(module: nn.Module) -> bool:
+    """Whether calling ``module`` is nothing but ``x @ weight.T (+ bias)``: no derived class, no hooks.  Callers may then take the weight and
+    join the product with what surrounds it."""
+    return type(module) in (nn.Linear, Linear) and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)

@@ -13,7 +13,7 @@ from __future__ import annotations
 
 import os
 import warnings
-from typing import Dict, Optional, Tuple
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 import torch.nn.functional as F
@@ -29,6 +29,7 @@ __all__ = [
     "mxfp8_linear",
     "matmul",
     "linear",
+    "linear_group",
     "linear_residual",
     "linear_wide",
     "residual_norm",
@@ -93,6 +94,11 @@ def _native(t: torch.Tensor, dtypes=(torch.bfloat16,)) -> bool:
     return t.is_cuda and not _FORCE_REFERENCE and t.dtype in dtypes
 
 
+def _differentiated(*tensors: Optional[torch.Tensor]) -> bool:
+    """Whether a call on these tensors may have to be differentiated, in either mode; kernels without an autograd function then don't apply."""
+    return (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)) or torch.autograd.forward_ad._current_level >= 0
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x @ weight.T (+ bias)``; bf16 CUDA inputs run the tcgen05 GEMM (fwd, dgrad, wgrad)."""
     if _native(x) and weight.dtype == torch.bfloat16:
@@ -112,6 +118,17 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         pad = (-x.shape[-1]) % 8
         return linear(F.pad(x, (0, pad)), F.pad(weight, (0, pad)), bias)
     return F.linear(x, weight, bias)
+
+
+def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Sequence[Optional[torch.Tensor]]) -> List[torch.Tensor]:
+    """``[linear(x, w, b) for w, b in zip(weights, biases)]``; a few bf16 CUDA tokens outside autograd take all of them in one launch."""
+    if _native(x) and not _differentiated(x, *weights, *biases):
+        from . import _cuda
+
+        ys = _cuda.linear_group(x, weights, biases)
+        if ys is not None:
+            return ys
+    return [linear(x, w, b) for w, b in zip(weights, biases)]
 
 
 def linear_wide(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:

@@ -36,6 +36,46 @@ def _use_pair_kernel(M: int, N: int, K: int, out: torch.Tensor) -> bool:
     return K >= 128 and (-(-M // 256)) * (-(-N // 256)) >= _SM_PAIRS
 
 
+ROWS_LIMIT = 64  # most tokens csrc/gemm_rows.cu takes
+
+
+def _runs_rows(M: int, N: int, K: int) -> bool:
+    """Whether a linear layer streams its weights through registers (``csrc/gemm_rows.cu``) instead of running on a tile kernel.  The lines lie
+    where the two met on a B200 (us here / on the tile kernels, weights from HBM): 64 x 4096 x 4096 17.4 / 18.5 and 64 x 6144 x 4096 29 / 19, since the tile
+    kernels leave most SMs idle below about 4096 weight rows; 32 x 6144 x 4096 19.1 / 18.5 and gated 32 x 14336 x 4096 55 / 88; with a
+    vocabulary of rows the CTA-pair kernel streams as well: 16 x 128256 x 2048 100 / 116, x 4096 191 / 179, 8 x 128256 x 4096 185 / 203."""
+    most = ROWS_LIMIT if N <= 4096 else 32 if N <= 32768 else 16 if K < 4096 else 8
+    return 0 < M <= most and K > 0 and K % 8 == 0
+
+
+def _gemm_rows(x: torch.Tensor, weights: Sequence[torch.Tensor], outs: Sequence[torch.Tensor], biases: Optional[Sequence[Optional[torch.Tensor]]] = None,
+               residual: Optional[torch.Tensor] = None, alpha: float = 1.0) -> None:
+    """``outs[i] = alpha · x · weights[i]ᵀ (+ biases[i]) (+ residual)`` for up to :data:`ROWS_LIMIT` tokens and three weights; rows 16-byte aligned."""
+    n = len(weights)
+    vps, lls = ctypes.c_void_p * n, ctypes.c_longlong * n
+    rc = lib().ttb_gemm_rows(x.data_ptr(), x.stride(0), x.shape[0], x.shape[1], n, vps(*[w.data_ptr() for w in weights]), lls(*[w.stride(0) for w in weights]),
+                             (ctypes.c_int * n)(*[w.shape[0] for w in weights]), vps(*[o.data_ptr() for o in outs]), lls(*[o.stride(0) for o in outs]),
+                             None if biases is None else vps(*[_ptr(b) for b in biases]), _ptr(residual), 0 if residual is None else residual.stride(0),
+                             int(outs[0].dtype == torch.float32), float(alpha), stream_ptr())
+    check(rc, f"gemm of few rows M={x.shape[0]} K={x.shape[1]}")
+
+
+def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Sequence[Optional[torch.Tensor]]) -> Optional[List[torch.Tensor]]:
+    """The linear layers ``weights[i]`` of one input in one launch, outside autograd; ``None`` where the kernel for few tokens does not apply."""
+    K = x.shape[-1]
+    M = x.numel() // K if K else 0
+    if len(weights) > 3 or not all(_runs_rows(M, w.shape[0], K) for w in weights) or any(w.dtype != _BF16 or w.stride(1) != 1 or w.stride(0) % 8 or w.data_ptr() % 16 for w in weights):
+        return None
+    if any(b is not None and (b.dtype != _BF16 or not b.is_contiguous()) for b in biases):
+        return None
+    x2 = x.reshape(M, K)
+    if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+        x2 = x2.contiguous()
+    outs = [torch.empty(M, w.shape[0], dtype=_BF16, device=x.device) for w in weights]
+    _gemm_rows(x2, weights, outs, None if all(b is None for b in biases) else biases)
+    return [o.view(*x.shape[:-1], o.shape[1]) for o in outs]
+
+
 def gemm(
     a: torch.Tensor,
     b: torch.Tensor,
@@ -73,6 +113,9 @@ def gemm(
         return out
     if K == 0:
         return out if accumulate else out.zero_()
+    if not (a_mn or b_mn or accumulate) and _runs_rows(M, N, K) and (bias is None or (bias.dtype == _BF16 and bias.is_contiguous())):
+        _gemm_rows(a, [b], [out], None if bias is None else [bias], alpha=alpha)
+        return out
     if _use_pair_kernel(M, N, K, out):
         rc = lib().ttb_gemm_bf16_2sm(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, int(a_mn), int(b_mn), a.stride(0), b.stride(0), out.stride(0), int(accumulate),
                                      _ptr(bias), float(alpha), err_word(a.device).data_ptr(), stream_ptr())
@@ -131,8 +174,8 @@ def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: b
 
 
 def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``a[M, K] · b[N, K]ᵀ (+ bias) + residual[M, N]`` with the addition in the GEMM epilogue (CTA-pair kernel); problems too small for that
-    kernel run the plain GEMM followed by an add."""
+    """``a[M, K] · b[N, K]ᵀ (+ bias) + residual[M, N]`` with the addition in the GEMM epilogue (CTA-pair kernel and the one for few
+    tokens); problems between the two run the plain GEMM followed by an add."""
     def ok(t):
         return t if (t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0) else t.contiguous()
 
@@ -140,6 +183,9 @@ def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias
     M, K = a.shape
     N = b.shape[0]
     out = torch.empty(M, N, dtype=_BF16, device=a.device)
+    if _runs_rows(M, N, K) and (bias is None or (bias.dtype == _BF16 and bias.is_contiguous())):
+        _gemm_rows(a, [b], [out], None if bias is None else [bias], residual=residual)
+        return out
     if K % 8 == 0 and _use_pair_kernel(M, N, K, out):
         rc = lib().ttb_gemm_bf16_2sm_residual(a.data_ptr(), b.data_ptr(), out.data_ptr(), residual.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), residual.stride(0),
                                               _ptr(bias), err_word(a.device).data_ptr(), stream_ptr())
@@ -1140,7 +1186,9 @@ class _GateUpSwiGLU(torch.autograd.Function):
 def gate_up_swiglu(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, clamp: Optional[Tuple[float, float]] = None) -> Optional[torch.Tensor]:
     """Fused gate / up projections + SwiGLU (``clamp`` ``(limit, alpha)``: the clamped gate, outside autograd), or ``None`` when the shapes do not suit the CTA-pair kernel (the caller then runs the three
     separate operators)."""
-    if not _PAIR_KERNEL or os.environ.get("TTB_FUSE_SWIGLU", "1") == "0":
+    from . import _differentiated
+
+    if not _PAIR_KERNEL or os.environ.get("TTB_FUSE_SWIGLU", "1") == "0" or x.numel() == 0:
         return None
     K, N = x.shape[-1], w1.shape[0]
     M = x.numel() // K
@@ -1150,6 +1198,14 @@ def gate_up_swiglu(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, clamp: O
         return None
     if clamp is not None and (clamp[0] <= 0.0 or (torch.is_grad_enabled() and (x.requires_grad or w1.requires_grad or w3.requires_grad))):
         return None
+    if _runs_rows(M, N, K) and not _differentiated(x, w1, w3):
+        x2 = x.reshape(M, K)
+        if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+            x2 = x2.contiguous()
+        h = torch.empty(M, N, dtype=_BF16, device=x.device)
+        check(lib().ttb_gemm_rows_gated(x2.data_ptr(), x2.stride(0), w1.data_ptr(), w3.data_ptr(), K, h.data_ptr(), N, M, N, K, *(clamp or (0.0, 0.0)), stream_ptr()),
+              f"gate/up GEMM of few rows M={M} N={N} K={K}")
+        return h.view(*x.shape[:-1], N)
     global _SM_PAIRS
     if _SM_PAIRS is None:
         _SM_PAIRS = max(1, torch.cuda.get_device_properties(x.device).multi_processor_count // 2)
