@@ -84,3 +84,54 @@ def test_sampling(V, top_k, dtype):
     picked = race.gather(1, got.long())
     # logarithms and one subtraction in fp32: a few units of 2^-21 at logits below 32
     assert (picked >= race.amax(1, keepdim=True) - 1e-5).all()
+
+
+@pytest.mark.parametrize("interleaved", [True, False])
+@pytest.mark.parametrize("b,s,hq,hkv,d", [(1, 1, 4, 4, 64), (3, 5, 8, 2, 128), (2, 70, 32, 8, 64), (2, 3, 3, 1, 16)])
+def test_rotation_into_a_cache(b, s, hq, hkv, d, interleaved):
+    """The same bits as two rotations and two copies, and not a byte of the cache beside the named slots."""
+    q, k, v = _rand(b, s, hq, d, seed=1), _rand(b, s, hkv, d, seed=2), _rand(b, s, hkv, d, seed=3)
+    ang = torch.rand(97, d // 2, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda") * 6
+    table = torch.stack([ang.cos(), ang.sin()], -1)
+    kc, vc = _rand(b, s + 9, hkv, d, seed=5), _rand(b, s + 9, hkv, d, seed=6)
+    want_k, want_v = kc.clone(), vc.clone()
+    slots = torch.arange(4, 4 + s, device="cuda")
+    for pos in (None, torch.arange(s, device="cuda") + 20, torch.randint(0, 97, (b, s), device="cuda")):
+        want_k[:, 4 : 4 + s], want_v[:, 4 : 4 + s] = ops.rope(k, table, pos, interleaved), v
+        with torch.no_grad():
+            got = ops.rope_append(q, k, v, table, pos, interleaved, kc, vc, slots)
+        assert torch.equal(got, ops.rope(q, table, pos, interleaved)) and torch.equal(kc, want_k) and torch.equal(vc, want_v)
+
+
+def test_recorded_steps_are_the_plain_ones():
+    """Generation with recorded steps, on used and on fresh caches, against a loop of plain calls; full caches are still refused."""
+    import copy
+
+    from torchtune_b200 import generation, training
+    from torchtune_b200.generation._step_graph import StepGraph
+    from torchtune_b200.models.llama3_1 import llama3_1
+
+    torch.manual_seed(0)
+    with training.set_default_dtype(torch.bfloat16), torch.device("cuda"):
+        model = llama3_1(vocab_size=1024, num_layers=3, num_heads=8, num_kv_heads=2, embed_dim=512, max_seq_len=512, intermediate_dim=1024).eval()
+        model.setup_caches(batch_size=3, dtype=torch.bfloat16, decoder_max_seq_len=60)
+
+    def run(prompt, n, **kw):
+        model.reset_caches()
+        rng = torch.Generator(device="cuda").manual_seed(1)
+        return generation.generate(model, prompt, max_generated_tokens=n, temperature=0.8, top_k=50, rng=rng, **kw)
+
+    for b, s, n in ((3, 20, 12), (1, 7, 40), (3, 48, 12), (2, 30, 4)):
+        prompt = torch.randint(1, 1024, (b, s), device="cuda")
+        assert StepGraph.suits(model, prompt)
+        tokens, logits = run(prompt, n)
+        plain_tokens, plain_logits = run(prompt, n, custom_generate_next_token=generation.generate_next_token)
+        assert torch.equal(tokens, plain_tokens) and torch.equal(logits, plain_logits)
+        assert model.layers[1].attn.kv_cache.size == s + n - 1 and int(model.layers[1].attn.kv_cache.cache_pos[0]) == s + n - 1
+        again, _ = run(prompt, n)
+        assert torch.equal(again, tokens)
+    copy.deepcopy(model)
+    with pytest.raises(AssertionError, match="full"):
+        run(torch.randint(1, 1024, (2, 55), device="cuda"), 8)
+    model.layers[0].register_forward_hook(lambda *a: None)
+    assert not StepGraph.suits(model, prompt)

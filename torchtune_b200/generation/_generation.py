@@ -8,6 +8,7 @@ import torch
 from ..modules import TransformerDecoder
 from ..modules.attention import MaskLike
 from ._rows import DecodeGraph, RowLayout, hidden_states
+from ._step_graph import StepGraph
 
 
 def multinomial_sample_one(probs: torch.Tensor, q: torch.Tensor) -> torch.Tensor:
@@ -158,6 +159,13 @@ def generate(
 
         def step_fn(model, input_pos, x, q=None, *, mask=None, temperature=1.0, top_k=None):
             logits = model.unembed_normed(graph(x))[:, -1]
+            return sample(logits, temperature=temperature, top_k=top_k, q=q), logits.unsqueeze(1)
+
+    elif incremental and custom_generate_next_token is None and max_generated_tokens > 3 and StepGraph.suits(model, prompt):
+        graph_step = StepGraph(model, bsz)
+
+        def step_fn(model, input_pos, x, q=None, *, mask=None, temperature=1.0, top_k=None):
+            logits = graph_step(x, input_pos, mask)
             return sample(logits, temperature=temperature, top_k=top_k, q=q), logits.unsqueeze(1)
 
     for _ in range(max_generated_tokens - 1):

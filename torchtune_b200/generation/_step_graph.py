@@ -1,0 +1,110 @@
+"""The one-token step of a plain decoder on its KV caches as a CUDA graph.
+
+A step of a small model is a few hundred launches of a few microseconds each, and the host needs longer to issue one than the GPU to run it."""
+from __future__ import annotations
+
+from typing import Optional
+
+import torch
+from torch import nn
+
+from ..modules import FeedForward, KVCache, MultiHeadAttention, RMSNorm, TransformerDecoder, TransformerSelfAttentionLayer
+from ..modules.linear import Linear
+from ..modules.position_embeddings import RotaryPositionalEmbeddings
+from ..modules.tied_linear import TiedLinear
+
+# Modules whose forward pass of one token is the same sequence of launches in every step and needs no look at the device.
+_PLAIN = (TransformerDecoder, TransformerSelfAttentionLayer, MultiHeadAttention, FeedForward, KVCache, RMSNorm, Linear, nn.Linear, nn.Embedding, nn.ModuleList, nn.Identity,
+          nn.SiLU, nn.GELU, nn.ReLU)
+
+
+class _LastGraph:
+    """The graph that last ran on a cache.  The next one shares its memory pool, so that any number of generations on one set of caches
+    hold one pool, which goes with the caches.  Copies and pickles of the cache come without it."""
+
+    def __init__(self) -> None:
+        self.graph: Optional[torch.cuda.CUDAGraph] = None
+
+    def __deepcopy__(self, memo) -> "_LastGraph":
+        return _LastGraph()
+
+    def __reduce__(self):
+        return _LastGraph, ()
+
+
+class StepGraph:
+    """``model(x, input_pos, mask)[:, -1]`` for one token per row: the first call runs as it is, the second is recorded, and it and all later
+    ones replay the recording on the inputs that they are given."""
+
+    @staticmethod
+    def suits(model: nn.Module, like: torch.Tensor) -> bool:
+        if type(model) is not TransformerDecoder or not like.is_cuda or model.tok_embeddings.weight.dtype != torch.bfloat16 or model.loop is not None:
+            return False
+        if model.num_output_chunks or model.output_hidden_states or model.skip_output_layer or model.pos_embeddings is not None:
+            return False
+        if type(model.output) not in (Linear, nn.Linear, TiedLinear):
+            return False
+        if torch.is_inference_mode_enabled() or torch.cuda.is_current_stream_capturing() or torch.autograd.forward_ad._current_level >= 0:
+            return False
+        for m in model.modules():
+            rotary = isinstance(m, RotaryPositionalEmbeddings) and type(m).forward is RotaryPositionalEmbeddings.forward
+            if not (rotary or type(m) in _PLAIN) or m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+                return False
+        for layer in model.layers:
+            if type(layer) is not TransformerSelfAttentionLayer or layer.mask_mod is not None or type(layer.attn) is not MultiHeadAttention:
+                return False
+            attn = layer.attn
+            if type(attn.kv_cache) is not KVCache or not attn.cache_enabled or attn.kv_cache.cache_pos.is_inference() or getattr(attn, "context_parallel", None) is not None:
+                return False
+            if attn.training and attn.attn_dropout:
+                return False
+        return all(p.device == like.device and p.dtype == torch.bfloat16 for p in model.parameters())
+
+    def __init__(self, model: TransformerDecoder, batch: int) -> None:
+        self.model, self.batch = model, batch
+        self.caches = [layer.attn.kv_cache for layer in model.layers]
+        self.graph: Optional[torch.cuda.CUDAGraph] = None
+        self.calls = 0
+
+    def __call__(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
+        self.calls += 1
+        if self.calls == 2:
+            self._record(x, input_pos, mask)
+        if self.graph is None:
+            return self.model(x, input_pos=input_pos, mask=mask)[:, -1]
+        for cache in self.caches:
+            cache.reserve(self.batch, 1)  # raises when the cache is full
+        self.x.copy_(x)
+        self.pos.copy_(input_pos.view(-1, 1))
+        self.mask.copy_(mask)
+        self.graph.replay()
+        for cache in self.caches:
+            cache._note(cache.size + 1)
+        return self.logits.clone()
+
+    def _record(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> None:
+        device = x.device
+        for cache in self.caches:
+            cache.reserve(self.batch, 1)
+        used = [cache.size for cache in self.caches]
+        self.x, self.mask = torch.empty_like(x), torch.empty_like(mask)
+        self.pos = torch.empty(self.batch, 1, dtype=torch.int32, device=device)
+        home = self.caches[0].__dict__.setdefault("last_graph", _LastGraph())
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=device)
+        stream.wait_stream(torch.cuda.current_stream(device))
+        for cache in self.caches:
+            cache.recording = True
+        try:
+            with torch.cuda.stream(stream):
+                graph.capture_begin(**({} if home.graph is None else {"pool": home.graph.pool()}), capture_error_mode="thread_local")
+                try:
+                    self.logits = self.model(self.x, input_pos=self.pos, mask=self.mask)[:, -1]
+                    torch._foreach_add_([cache.cache_pos for cache in self.caches], 1)
+                finally:
+                    graph.capture_end()
+        finally:
+            for cache, n in zip(self.caches, used):
+                cache.recording = False
+                cache._note(n)  # nothing has run yet
+        torch.cuda.current_stream(device).wait_stream(stream)
+        self.graph = home.graph = graph

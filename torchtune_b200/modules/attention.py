@@ -11,6 +11,7 @@ from .. import ops
 from ..ops.mask import AttentionMask
 from .kv_cache import KVCache
 from .linear import is_plain_linear
+from .position_embeddings import RotaryPositionalEmbeddings
 
 logger = logging.getLogger(__name__)
 
@@ -103,6 +104,20 @@ class MultiHeadAttention(nn.Module):
             raise RuntimeError("Key value caches are not setup. Call ``setup_caches()`` first.")
         self.kv_cache.reset()
 
+    def _rotate_into_cache(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, input_pos: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+        """Rotary embedding of ``q`` (returned) and of ``k``, the latter and ``v`` going straight to their slots of the cache; ``None``, with nothing
+        done, for anything but a plain rotation in front of a plain cache."""
+        cache, pe = self.kv_cache, self.pos_embeddings
+        if not self.cache_enabled or type(cache) is not KVCache or self.q_norm is not None or not isinstance(pe, RotaryPositionalEmbeddings):
+            return None
+        if type(pe).forward is not RotaryPositionalEmbeddings.forward or pe._forward_hooks or pe._forward_pre_hooks:
+            return None
+        b, s = q.shape[:2]
+        out = ops.rope_append(q, k, v, pe.cache, input_pos, pe.interleaved, cache.k_cache[:b], cache.v_cache[:b], cache.reserve(b, s))
+        if out is not None:
+            cache.advance(s)
+        return out
+
     def forward(
         self,
         x: torch.Tensor,
@@ -122,31 +137,36 @@ class MultiHeadAttention(nn.Module):
         else:
             q = self.q_proj(x)
         q = q.view(b, s_x, self.num_heads, self.head_dim)
-        if self.q_norm is not None and self.qk_norm_before_rope:
-            q = self.q_norm(q)
-        if self.pos_embeddings is not None:
-            q = self.pos_embeddings(q, input_pos=input_pos)
-        if self.q_norm is not None and not self.qk_norm_before_rope:
-            q = self.q_norm(q)
-
-        if y is None:
-            if self.kv_cache is None or not self.cache_enabled:
-                raise ValueError("Must provide y input or use kv_cache to enable streaming decoding")
-            k, v = self.kv_cache.k_cache[:b], self.kv_cache.v_cache[:b]
+        rotated = None
+        if k is not None:
+            k, v = (t.view(b, s_x, self.num_kv_heads, self.head_dim) for t in (k, v))
+            rotated = self._rotate_into_cache(q, k, v, input_pos)
+        if rotated is not None:
+            q, k, v = rotated, self.kv_cache.k_cache[:b], self.kv_cache.v_cache[:b]
         else:
-            s_y = y.shape[1]
-            if k is None:
-                k, v = self.k_proj(y), self.v_proj(y)
-            k = k.view(b, s_y, self.num_kv_heads, self.head_dim)
-            v = v.view(b, s_y, self.num_kv_heads, self.head_dim)
-            if self.k_norm is not None and self.qk_norm_before_rope:
-                k = self.k_norm(k)
+            if self.q_norm is not None and self.qk_norm_before_rope:
+                q = self.q_norm(q)
             if self.pos_embeddings is not None:
-                k = self.pos_embeddings(k, input_pos=input_pos)
-            if self.k_norm is not None and not self.qk_norm_before_rope:
-                k = self.k_norm(k)
-            if self.kv_cache is not None and self.cache_enabled:
-                k, v = self.kv_cache.update(k, v)
+                q = self.pos_embeddings(q, input_pos=input_pos)
+            if self.q_norm is not None and not self.qk_norm_before_rope:
+                q = self.q_norm(q)
+            if y is None:
+                if self.kv_cache is None or not self.cache_enabled:
+                    raise ValueError("Must provide y input or use kv_cache to enable streaming decoding")
+                k, v = self.kv_cache.k_cache[:b], self.kv_cache.v_cache[:b]
+            else:
+                s_y = y.shape[1]
+                if k is None:
+                    k = self.k_proj(y).view(b, s_y, self.num_kv_heads, self.head_dim)
+                    v = self.v_proj(y).view(b, s_y, self.num_kv_heads, self.head_dim)
+                if self.k_norm is not None and self.qk_norm_before_rope:
+                    k = self.k_norm(k)
+                if self.pos_embeddings is not None:
+                    k = self.pos_embeddings(k, input_pos=input_pos)
+                if self.k_norm is not None and not self.qk_norm_before_rope:
+                    k = self.k_norm(k)
+                if self.kv_cache is not None and self.cache_enabled:
+                    k, v = self.kv_cache.update(k, v)
 
         plain = self.kv_cache is None or not self.cache_enabled
         attn_mask = _as_mask(mask, default_causal=self.is_causal and plain and mask is None)

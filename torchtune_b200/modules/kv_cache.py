@@ -12,6 +12,11 @@ from torch import nn
 
 
 class KVCache(nn.Module):
+    # (cache_pos, its version, number of tokens at that version): spares the host a look at the device as long as nobody else wrote to it
+    _known: Optional[Tuple[torch.Tensor, int, int]] = None
+    # True while a decode step is recorded: the recorded step moves cache_pos on for all layers at once
+    recording = False
+
     def __init__(self, batch_size: int, max_seq_len: int, num_kv_heads: int, head_dim: int, dtype: torch.dtype) -> None:
         super().__init__()
         shape = (batch_size, max_seq_len, num_kv_heads, head_dim)
@@ -25,26 +30,45 @@ class KVCache(nn.Module):
     def reset(self) -> None:
         self.k_cache.zero_()
         self.v_cache.zero_()
-        self.cache_pos -= self.size
+        self.cache_pos -= self.cache_pos[0].clone()
+        self._note(0)
+
+    def _note(self, used: int) -> None:
+        self._known = None if self.cache_pos.is_inference() else (self.cache_pos, self.cache_pos._version, used)
 
     @property
     def size(self) -> int:
-        return int(self.cache_pos[0].item())
+        known, pos = self._known, self.cache_pos
+        if known is None or known[0] is not pos or known[1] != pos._version:
+            self._note(int(pos[0].item()))
+            if self._known is None:
+                return int(pos[0].item())
+        return self._known[2]
 
-    def update(self, k_val: torch.Tensor, v_val: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
-        """Append ``[b, s, n_kv, d]`` keys/values and return the full buffers."""
-        bsz, seq_len = k_val.shape[0], k_val.shape[1]
+    def reserve(self, bsz: int, seq_len: int) -> torch.Tensor:
+        """Slots of the next ``seq_len`` tokens of ``bsz`` rows; :meth:`advance` follows once they are written."""
         if bsz > self.k_cache.shape[0]:
             raise ValueError(
                 f"The current cache has been setup with a batch size of {self.k_cache.shape[0]}"
                 f", but found new key tensors with batch size {bsz}!"
             )
-        if self.cache_pos[0] + seq_len > self.max_seq_len:
+        if self.size + seq_len > self.max_seq_len:
             raise AssertionError("KV cache is full: cannot write past max_seq_len")
-        where = self.cache_pos[:seq_len]
+        return self.cache_pos[:seq_len]
+
+    def advance(self, seq_len: int) -> None:
+        used = self.size + seq_len
+        if not self.recording:
+            self.cache_pos.add_(seq_len)
+        self._note(used)
+
+    def update(self, k_val: torch.Tensor, v_val: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+        """Append ``[b, s, n_kv, d]`` keys/values and return the full buffers."""
+        bsz, seq_len = k_val.shape[0], k_val.shape[1]
+        where = self.reserve(bsz, seq_len)
         self.k_cache[:bsz].index_copy_(1, where, k_val)
         self.v_cache[:bsz].index_copy_(1, where, v_val)
-        self.cache_pos.add_(seq_len)
+        self.advance(seq_len)
         return self.k_cache[:bsz], self.v_cache[:bsz]
 
 

@@ -39,6 +39,7 @@ __all__ = [
     "softcap",
     "rms_norm",
     "rope",
+    "rope_append",
     "swiglu",
     "attention",
     "linear_cross_entropy",
@@ -310,6 +311,26 @@ def rope(
         return _cuda.rope(x, cache, input_pos, interleaved)
     fn = reference.rope_interleaved if interleaved else reference.rope_half
     return fn(x, cache, input_pos)
+
+
+def rope_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: torch.Tensor, input_pos: Optional[torch.Tensor], interleaved: bool, k_cache: torch.Tensor,
+                v_cache: torch.Tensor, slots: torch.Tensor) -> Optional[torch.Tensor]:
+    """:func:`rope` of ``q`` (returned) and of ``k``, the latter and ``v`` written to ``k_cache`` / ``v_cache`` ``[b, max_seq, heads, d]`` at ``slots`` (int64 ``[s]``), in one launch
+    outside autograd; ``None``, with nothing written, where that does not apply."""
+    same = (torch.bfloat16,)
+    if not (_native(q, same) and all(_native(t, same) for t in (k, v, k_cache, v_cache))) or _differentiated(q, k, v, k_cache, v_cache) or q.numel() == 0:
+        return None
+    if q.shape[-1] % 16 or cache.dtype != torch.float32 or not cache.is_contiguous() or cache.device != q.device or cache.shape[-2] * 2 != q.shape[-1]:
+        return None
+    if k.shape != v.shape or k.shape[:2] != q.shape[:2] or k_cache.shape != v_cache.shape or k_cache.shape[0] != k.shape[0] or k_cache.shape[2:] != k.shape[2:] or k.shape[3] != q.shape[3]:
+        return None
+    if not (k_cache.is_contiguous() and v_cache.is_contiguous()) or slots.dtype != torch.int64 or not slots.is_contiguous() or slots.numel() != k.shape[1]:
+        return None
+    if any(t.data_ptr() % 16 for t in (cache, k_cache, v_cache)):
+        return None
+    from . import _cuda
+
+    return _cuda.rope_append(q, k, v, cache, input_pos, interleaved, k_cache, v_cache, slots)
 
 
 def swiglu(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:

@@ -1096,11 +1096,24 @@ def rope(x: torch.Tensor, cache: torch.Tensor, input_pos: Optional[torch.Tensor]
         from . import reference
 
         return (reference.rope_interleaved if interleaved else reference.rope_half)(x, cache, input_pos)
-    pos = None
-    if input_pos is not None:
-        pos = input_pos.to(device=x.device, dtype=torch.int32)
-        pos = pos.expand(b, s).contiguous() if pos.dim() == 2 else pos.view(1, s).expand(b, s).contiguous()
-    return _RoPE.apply(x, cache, pos, interleaved)
+    return _RoPE.apply(x, cache, _positions(input_pos, b, s, x.device), interleaved)
+
+
+def _positions(input_pos: Optional[torch.Tensor], b: int, s: int, device) -> Optional[torch.Tensor]:
+    if input_pos is None:
+        return None
+    pos = input_pos.to(device=device, dtype=torch.int32)
+    return pos.expand(b, s).contiguous() if pos.dim() == 2 else pos.view(1, s).expand(b, s).contiguous()
+
+
+def rope_append(q, k, v, cache: torch.Tensor, input_pos: Optional[torch.Tensor], interleaved: bool, k_cache: torch.Tensor, v_cache: torch.Tensor, slots: torch.Tensor) -> torch.Tensor:
+    b, s, hq, d = q.shape
+    q, k, v = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in (q, k, v))
+    out = torch.empty_like(q)
+    pos = _positions(input_pos, b, s, q.device)
+    check(lib().ttb_rope_append(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cache.data_ptr(), _ptr(pos), slots.data_ptr(), b * s, hq,
+                                k.shape[2], d, s, k_cache.shape[1], int(interleaved), int(cache.shape[0]), stream_ptr()), "rope + cache append")
+    return out
 
 
 # ======================================================================= SwiGLU

@@ -73,6 +73,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_mask_bounds.restype = i32
     L.ttb_gemm_bf16_2sm.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i64, i64, i64, i32, vp, f32, vp, vp]
     L.ttb_gemm_bf16_2sm.restype = i32
+    L.ttb_rope_append.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, i32, vp]
+    L.ttb_rope_append.restype = i32
     L.ttb_gemm_rows.argtypes = [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, vp]
     L.ttb_gemm_rows.restype = i32
     L.ttb_gemm_rows_gated.argtypes = [vp, i64, vp, vp, i64, vp, i64, i32, i32, i32, f32, f32, vp]
