@@ -33,8 +33,8 @@ class _LastGraph:
 
 
 class StepGraph:
-    """``model(x, input_pos, mask)[:, -1]`` for one token per row: the first call runs as it is, the second is recorded, and it and all later
-    ones replay the recording on the inputs that they are given."""
+    """``model(x, input_pos, mask)[:, -1]`` for one token per row: a call is recorded, and it and all later ones replay the recording on the inputs
+    that they are given.  On caches that have not been stepped yet the first call runs as it is, so that one-time set-up stays out of the recording."""
 
     @staticmethod
     def suits(model: nn.Module, like: torch.Tensor) -> bool:
@@ -64,13 +64,14 @@ class StepGraph:
         self.model, self.batch = model, batch
         self.caches = [layer.attn.kv_cache for layer in model.layers]
         self.graph: Optional[torch.cuda.CUDAGraph] = None
-        self.calls = 0
+        self.home: _LastGraph = self.caches[0].__dict__.setdefault("last_graph", _LastGraph())
+        self.ready = self.home.graph is not None
 
     def __call__(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
-        self.calls += 1
-        if self.calls == 2:
+        if self.graph is None and self.ready:
             self._record(x, input_pos, mask)
         if self.graph is None:
+            self.ready = True
             return self.model(x, input_pos=input_pos, mask=mask)[:, -1]
         for cache in self.caches:
             cache.reserve(self.batch, 1)  # raises when the cache is full
@@ -89,14 +90,13 @@ class StepGraph:
         used = [cache.size for cache in self.caches]
         self.x, self.mask = torch.empty_like(x), torch.empty_like(mask)
         self.pos = torch.empty(self.batch, 1, dtype=torch.int32, device=device)
-        home = self.caches[0].__dict__.setdefault("last_graph", _LastGraph())
         graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=device)
         stream.wait_stream(torch.cuda.current_stream(device))
         for cache in self.caches:
             cache.recording = True
         try:
             with torch.cuda.stream(stream):
-                graph.capture_begin(**({} if home.graph is None else {"pool": home.graph.pool()}), capture_error_mode="thread_local")
+                graph.capture_begin(**({} if self.home.graph is None else {"pool": self.home.graph.pool()}), capture_error_mode="thread_local")
                 try:
                     self.logits = self.model(self.x, input_pos=self.pos, mask=self.mask)[:, -1]
                     torch._foreach_add_([cache.cache_pos for cache in self.caches], 1)
@@ -107,4 +107,4 @@ class StepGraph:
                 cache.recording = False
                 cache._note(n)  # nothing has run yet
         torch.cuda.current_stream(device).wait_stream(stream)
-        self.graph = home.graph = graph
+        self.graph = self.home.graph = graph
