@@ -1,0 +1,44 @@
+"""Log-probabilities from fp32 logits and scaled gradients against plain statements in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchtune_b200 import rlhf
+
+
+def _logits(rows, V, dtype, seed=0):
+    x = torch.randn(rows, V, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * 4
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("temperature", [1.0, 0.7])
+@pytest.mark.parametrize("b,s,V", [(1, 1, 4), (2, 3, 2048), (3, 5, 8188), (2, 4, 128256), (2, 3, 1001)])
+def test_log_probabilities(b, s, V, temperature):
+    """Slices of a batch, widths that end inside a load, one that the kernel does not take; infinities."""
+    x = _logits(b * (s + 2), V, torch.float32, V).view(b, s + 2, V)
+    x[0, 1, 1:] = float("-inf")
+    tokens = torch.randint(0, V, (b, s), device="cuda")
+    tokens[0, 0] = 0
+    with torch.no_grad():
+        got = rlhf.logits_to_logprobs(x[:, 1:-1], tokens, temperature)
+    want = torch.log_softmax((x[:, 1:-1] / temperature).double(), -1).gather(2, tokens[..., None])[..., 0]
+    assert got.dtype == torch.float32 and ((got.double() - want).abs() <= 2.0**-20 * (1 + want.abs())).all()
+    x[0, 1] = float("-inf")
+    with torch.no_grad():
+        assert rlhf.logits_to_logprobs(x[:, 1:-1], tokens, temperature)[0, 0].isnan()
+    x[0, 1], x[0, 1, 1] = 0.0, float("nan")
+    with torch.no_grad():
+        assert rlhf.logits_to_logprobs(x[:, 1:-1], tokens, temperature)[0, 0].isnan()
+    x.requires_grad_()
+    rlhf.logits_to_logprobs(x, torch.zeros(b, s + 2, dtype=torch.int64, device="cuda")).nansum().backward()
+    assert x.grad is not None
+
+
+@pytest.mark.parametrize("n", [8, 8 * 255, 8 * 1025, 8 * 1_000_003])
+def test_scaled_gradients(n):
+    from torchtune_b200.ops._cuda import _scaled
+
+    x = _logits(1, n, torch.bfloat16)[0]
+    f = torch.tensor(1 / 3, device="cuda")
+    assert torch.equal(_scaled(x, f), (x.float() * f).to(torch.bfloat16))

@@ -421,13 +421,15 @@ def logit_softcap_of(model) -> float:
 
 
 def logits_logprobs(logits: torch.Tensor, tokens: torch.Tensor, temperature: float = 1.0) -> Optional[torch.Tensor]:
-    """``log_softmax(logits / T)`` gathered at ``tokens`` (fp32, shape of ``tokens``) for bf16 CUDA logits whose vocabulary width is a
-    multiple of 8, without an fp32 ``[..., V]`` intermediate; ``None`` otherwise."""
-    if not (_native(logits) and logits.shape[-1] % 8 == 0 and tokens.is_cuda and tokens.dtype == torch.int64 and logits.shape[:-1] == tokens.shape and logits.numel() > 0):
+    """``log_softmax(logits / T)`` gathered at ``tokens`` (fp32, shape of ``tokens``) without a further ``[..., V]`` intermediate: bf16 CUDA logits whose vocabulary
+    width is a multiple of 8, and outside autograd fp32 ones; ``None`` otherwise."""
+    if not (_native(logits, (torch.bfloat16, torch.float32)) and tokens.is_cuda and tokens.dtype == torch.int64 and logits.shape[:-1] == tokens.shape and logits.numel() > 0):
         return None
     from . import _cuda
 
-    return _cuda.logits_logprobs(logits, tokens, temperature)
+    if logits.dtype == torch.float32:
+        return None if _differentiated(logits) or isinstance(temperature, torch.Tensor) else _cuda.logits_logprobs_f32(logits, tokens, temperature)
+    return _cuda.logits_logprobs(logits, tokens, temperature) if logits.shape[-1] % 8 == 0 else None
 
 
 def sample_tokens(logits: torch.Tensor, q: torch.Tensor, temperature: float, top_k: Optional[int]) -> Optional[torch.Tensor]:

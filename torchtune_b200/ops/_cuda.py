@@ -1025,6 +1025,20 @@ def logits_logprobs(logits: torch.Tensor, tokens: torch.Tensor, temperature: flo
     return out.view(tokens.shape)
 
 
+def logits_logprobs_f32(logits: torch.Tensor, tokens: torch.Tensor, temperature: float) -> Optional[torch.Tensor]:
+    """``log_softmax(logits / T)`` at ``tokens`` from fp32 logits ``[..., V]`` in one pass, outside autograd; rows may be a slice of a batch.  ``None`` for layouts that it does not cover."""
+    V = logits.shape[-1]
+    if logits.dim() == 2:
+        logits = logits.unsqueeze(0)
+    if logits.dim() != 3 or logits.stride(2) != 1 or V % 4 or logits.stride(0) % 4 or logits.stride(1) % 4 or logits.data_ptr() % 16 or logits.numel() // V >= 2**31:
+        return None
+    out = torch.empty(tokens.shape, dtype=torch.float32, device=logits.device)
+    tokens = tokens.contiguous()
+    check(lib().ttb_token_logprobs_f32(logits.data_ptr(), logits.stride(0), logits.stride(1), logits.shape[1], tokens.data_ptr(), out.data_ptr(), tokens.numel(), V, float(temperature),
+                                       stream_ptr()), "log-probabilities")
+    return out
+
+
 # ======================================================================= sampling
 def sample(logits: torch.Tensor, q: torch.Tensor, temperature: float, top_k: Optional[int]) -> torch.Tensor:
     """One token per row of ``logits`` (``[rows, V]``, bf16 or fp32): temperature, optional top-k and the exponential-race draw
@@ -1247,6 +1261,15 @@ def _ce_chunk_rows(T: int, num_chunks: int) -> int:
     return max(1, -(-T // max(1, num_chunks)))
 
 
+def _scaled(t: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
+    """``t · factor`` for a contiguous gradient and a 0-dim fp32 tensor; one vector pass for bf16, with the factor unrounded."""
+    if t.dtype != _BF16 or factor.dtype != torch.float32 or t.numel() % 8 or t.data_ptr() % 16:
+        return t * factor.to(t.dtype)
+    out = torch.empty_like(t)
+    check(lib().ttb_scale_bf16(t.data_ptr(), out.data_ptr(), t.numel(), factor.data_ptr(), stream_ptr()), "scale")
+    return out
+
+
 # Above this many bytes of bf16 logits the token dimension is processed in chunks; below it the
 # whole batch is one pass (one logits GEMM, one dgrad, one wgrad written once in bf16).
 _CE_SINGLE_PASS_BYTES = 6 * 2**30
@@ -1313,8 +1336,8 @@ class _LinearCE(torch.autograd.Function):
         # The gradients were formed for d(loss_sum) = 1; an upstream factor multiplies them.
         # With direct delivery the weight gradient already sits in the flat buffer, which is
         # only valid for an upstream factor of one (the recipes back-propagate the sum itself).
-        gh = (dh * g_loss.to(dh.dtype)).view(ctx.h_shape) if dh is not None else None
-        gw = (dw * g_loss).to(ctx.w_dtype) if dw is not None else None
+        gh = _scaled(dh, g_loss).view(ctx.h_shape) if dh is not None else None
+        gw = _scaled(dw, g_loss).to(ctx.w_dtype) if dw is not None else None
         return gh, gw, None, None, None, None
 
 

@@ -75,6 +75,10 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_gemm_bf16_2sm.restype = i32
     L.ttb_rope_append.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, i32, vp]
     L.ttb_rope_append.restype = i32
+    L.ttb_token_logprobs_f32.argtypes = [vp, i64, i64, i32, vp, vp, i32, i32, f32, vp]
+    L.ttb_token_logprobs_f32.restype = i32
+    L.ttb_scale_bf16.argtypes = [vp, vp, i64, vp, vp]
+    L.ttb_scale_bf16.restype = i32
     L.ttb_gemm_rows.argtypes = [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, vp]
     L.ttb_gemm_rows.restype = i32
     L.ttb_gemm_rows_gated.argtypes = [vp, i64, vp, vp, i64, vp, i64, i32, i32, i32, f32, f32, vp]

@@ -21,7 +21,7 @@ def truncate_sequence_at_first_stop_token(sequences: torch.Tensor, stop_tokens: 
 
 
 def logits_to_logprobs(logits: torch.Tensor, sequences: torch.Tensor, temperature: float = 1.0) -> torch.Tensor:
-    """``log_softmax(logits / T)`` gathered at ``sequences`` → ``[b, s]`` (bf16 CUDA logits: fused kernel, fp32 result)."""
+    """``log_softmax(logits / T)`` gathered at ``sequences`` → ``[b, s]`` (CUDA logits: fused kernels, fp32 result)."""
     from .. import ops
 
     fused = ops.logits_logprobs(logits, sequences, temperature)
