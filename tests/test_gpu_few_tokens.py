@@ -135,3 +135,25 @@ def test_recorded_steps_are_the_plain_ones():
         run(torch.randint(1, 1024, (2, 55), device="cuda"), 8)
     model.layers[0].register_forward_hook(lambda *a: None)
     assert not StepGraph.suits(model, prompt)
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N,K,splits", [(8, 8, 16, 2), (72, 264, 1000, 3), (136, 520, 4104, 8), (8, 4096, 2048, 9), (304, 2048, 8192, 4), (128, 64, 200, 64)])
+def test_split_contraction(M, N, K, splits, a_mn, b_mn):
+    """More ranges than blocks of the contraction, ragged tiles and ends, every epilogue; the same bits every time."""
+    from torchtune_b200.ops._cuda import _gemm_split
+
+    a, b = _rand(M, K, seed=1), _rand(N, K, seed=2)
+    want = a.double() @ b.double().t()
+    x = a.t().contiguous() if a_mn else a
+    w = b.t().contiguous() if b_mn else b
+    new = lambda: torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    bias, r = _rand(N, seed=3), _rand(M, N, seed=4)
+    got = _gemm_split(x, w, new(), splits, a_mn=a_mn, b_mn=b_mn)
+    _check(got, want, a, b)
+    assert torch.equal(got, _gemm_split(x, w, new(), splits, a_mn=a_mn, b_mn=b_mn))
+    _check(_gemm_split(x, w, new(), splits, a_mn=a_mn, b_mn=b_mn, bias=bias, residual=r, alpha=0.5), 0.5 * want + bias.double() + r.double(), a, b)
+    _check(_gemm_split(x, w, r.clone(), splits, a_mn=a_mn, b_mn=b_mn, accumulate=True), want + r.double(), a, b)
+    wide = torch.ones(M, N + 8, dtype=torch.float32, device="cuda")
+    _gemm_split(x, w, wide[:, :N], splits, a_mn=a_mn, b_mn=b_mn, accumulate=True)
+    assert ((wide[:, :N].double() - want - 1).abs() <= 2.0**-19 * (a.double().abs() @ b.double().abs().t() + 1)).all() and (wide[:, N:] == 1).all()

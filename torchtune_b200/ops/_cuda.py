@@ -27,13 +27,16 @@ _SM_PAIRS = None
 
 def _use_pair_kernel(M: int, N: int, K: int, out: torch.Tensor) -> bool:
     """The CTA-pair kernel (``tcgen05.mma.cta_group::2``, 256 × 256 tiles, ``csrc/gemm2sm.cu``) takes bf16-output problems with
-    at least one 256 × 256 tile per SM pair; smaller ones keep 128-row tiles, which spread over more SMs."""
+    at least one 256 × 256 tile per SM pair; smaller ones keep 128-row tiles, which spread over more SMs, unless the contraction is so long that the
+    pairs' faster products outweigh half of the SMs (us with 128-row tiles / with pairs: 1024 x 4096 x 4096 25.3 / 27.4, x 14336 92.6 / 86.7, and
+    666 x 4096 x 14336 86.6 / 74.3)."""
     global _SM_PAIRS
     if not _PAIR_KERNEL or out.dtype != _BF16:
         return False
     if _SM_PAIRS is None:
         _SM_PAIRS = max(1, torch.cuda.get_device_properties(out.device).multi_processor_count // 2)
-    return K >= 128 and (-(-M // 256)) * (-(-N // 256)) >= _SM_PAIRS
+    tiles = (-(-M // 256)) * (-(-N // 256))
+    return K >= 128 and (tiles >= _SM_PAIRS or (K >= 8192 and 2 * tiles > _SM_PAIRS and M > 128 and N > 128))
 
 
 ROWS_LIMIT = 64  # most tokens csrc/gemm_rows.cu takes
@@ -116,6 +119,9 @@ def gemm(
     if not (a_mn or b_mn or accumulate) and _runs_rows(M, N, K) and (bias is None or (bias.dtype == _BF16 and bias.is_contiguous())):
         _gemm_rows(a, [b], [out], None if bias is None else [bias], alpha=alpha)
         return out
+    splits = _splits(M, N, K) if out.data_ptr() % 16 == 0 and (bias is None or bias.dtype == _BF16) else 1
+    if splits > 1:
+        return _gemm_split(a, b, out, splits, a_mn=a_mn, b_mn=b_mn, accumulate=accumulate, bias=bias, alpha=alpha)
     if _use_pair_kernel(M, N, K, out):
         rc = lib().ttb_gemm_bf16_2sm(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, int(a_mn), int(b_mn), a.stride(0), b.stride(0), out.stride(0), int(accumulate),
                                      _ptr(bias), float(alpha), err_word(a.device).data_ptr(), stream_ptr())
@@ -161,16 +167,36 @@ def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: b
     a, b = ok(a), ok(b)
     M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
     N = b.shape[1] if b_mn else b.shape[0]
-    bn = 256 if N > 128 else (128 if N > 64 else 64)
-    tiles = -(-M // 128) * -(-N // bn)
-    splits = min(64, 148 // tiles, -(-K // 256)) if tiles else 1
+    out = torch.empty(M, N, dtype=_BF16, device=a.device)
+    splits = min(64, 148 // _tiles(M, N), -(-K // 256)) if M and N else 1
     if splits <= 1:
         return gemm(a, b, a_mn=a_mn, b_mn=b_mn, alpha=alpha)
-    out = torch.zeros(M, N, dtype=torch.float32, device=a.device)
-    rc = lib().ttb_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, int(a_mn), int(b_mn), a.stride(0), b.stride(0), out.stride(0), splits,
-                                    float(alpha), err_word(a.device).data_ptr(), stream_ptr())
-    check(rc, f"gemm_splitk M={M} N={N} K={K} splits={splits}")
-    return out.to(_BF16)
+    return _gemm_split(a, b, out, splits, a_mn=a_mn, b_mn=b_mn, alpha=alpha)
+
+
+def _tiles(M: int, N: int) -> int:
+    """Output tiles of the single-CTA kernel."""
+    return -(-M // 128) * -(-N // (256 if N > 128 else 128 if N > 64 else 64))
+
+
+def _splits(M: int, N: int, K: int) -> int:
+    """In how many ranges to cut the contraction of an ordinary product; 1: not at all.  Worth it where at least two ranges find free SMs and the
+    contraction is long enough to pay for the second launch (us whole / in ranges: 300 x 2048 x 2048 14.0 / 14.0, 100 x 4096 x 4096 18.6 / 14.1,
+    512 x 2048 x 8192 40.7 / 22.4, 512 x 4096 x 14336 85.9 / 59.0, and 666 x 2048 x 128256 718 / 292)."""
+    return max(1, min(16, 148 // _tiles(M, N), K // 512)) if K >= 4096 else 1
+
+
+def _gemm_split(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, splits: int, *, a_mn: bool = False, b_mn: bool = False, accumulate: bool = False, bias: Optional[torch.Tensor] = None,
+                residual: Optional[torch.Tensor] = None, alpha: float = 1.0) -> torch.Tensor:
+    """:func:`gemm` with the contraction cut into ``splits`` ranges, each the work of its own CTAs; their fp32 partial sums are added in a fixed order."""
+    M, N = out.shape
+    K = a.shape[0] if a_mn else a.shape[1]
+    work = torch.empty(splits * M * N, dtype=torch.float32, device=a.device)
+    rc = lib().ttb_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), work.data_ptr(), out.data_ptr(), M, N, K, int(a_mn), int(b_mn), a.stride(0), b.stride(0), out.stride(0),
+                                    int(out.dtype == torch.float32), int(accumulate), _ptr(bias), _ptr(residual), 0 if residual is None else residual.stride(0), splits, float(alpha),
+                                    err_word(a.device).data_ptr(), stream_ptr())
+    check(rc, f"gemm in {splits} ranges M={M} N={N} K={K} a_mn={a_mn} b_mn={b_mn}")
+    return out
 
 
 def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -186,6 +212,9 @@ def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias
     if _runs_rows(M, N, K) and (bias is None or (bias.dtype == _BF16 and bias.is_contiguous())):
         _gemm_rows(a, [b], [out], None if bias is None else [bias], residual=residual)
         return out
+    splits = _splits(M, N, K) if K % 8 == 0 and (bias is None or bias.dtype == _BF16) else 1
+    if splits > 1:
+        return _gemm_split(a, b, out, splits, bias=bias, residual=residual)
     if K % 8 == 0 and _use_pair_kernel(M, N, K, out):
         rc = lib().ttb_gemm_bf16_2sm_residual(a.data_ptr(), b.data_ptr(), out.data_ptr(), residual.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), residual.stride(0),
                                               _ptr(bias), err_word(a.device).data_ptr(), stream_ptr())

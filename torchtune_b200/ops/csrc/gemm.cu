@@ -37,9 +37,8 @@ struct GemmParams {
   int* err;        // device error word (0 = ok)
   int K2 = 0;         // plain kernel: extent of a second operand pair whose product is accumulated into the same tile
                       // (C = A·op(B) + A2·op(B2), e.g. base weight + low-rank adapter); 0 = none
-  int splits = 1;     // plain kernel, fp32 output: the contraction is cut into `splits` ranges, one tile per (m, n, range), partial
-                      // sums added with vector atomics into a zero-initialised (or accumulated-into) C — for skinny outputs
-                      // whose few tiles would otherwise leave most SMs idle (adapter weight gradients)
+  int splits = 1;     // plain kernel, fp32 output: the contraction is cut into `splits` ranges, one tile per (m, n, range), and C is
+                      // [splits, M, N] partial sums — for outputs whose few tiles would otherwise leave most SMs idle
   int tma_store = 0;  // 1: bf16 output without accumulation leaves through shared memory + TMA stores (plain kernel)
 };
 
@@ -543,10 +542,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
               if (col0 + i < p.N) v[i] += __bfloat162float(__ldg(p.bias + col0 + i));
           }
           if (TP == 0 && splits > 1) {
-            float* dst = reinterpret_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
+            float* dst = reinterpret_cast<float*>(p.C) + (static_cast<long long>(split) * p.M + row) * p.ldc + col0;
 #pragma unroll
             for (int g = 0; g < 8; ++g)
-              if (col0 + g * 4 + 4 <= p.N) atomicAdd(reinterpret_cast<float4*>(dst + g * 4), make_float4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]));
+              if (col0 + g * 4 + 4 <= p.N) *reinterpret_cast<float4*>(dst + g * 4) = make_float4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
           } else if (p.out_fp32) {
             float* dst = reinterpret_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
 #pragma unroll
@@ -1210,20 +1209,63 @@ extern "C" int ttb_gemm_bf16_dual(const void* A, const void* B, const void* A2, 
   return dispatch_bn<true, false>(A, B, p, lda, ldb, s, sp);
 }
 
-// Split-K form of ttb_gemm_bf16 for skinny outputs: fp32 C (zero-initialised by the caller, or holding a value to add to), the
-// contraction cut into `splits` ranges whose partial tiles are added with 16-byte float atomics.
-extern "C" int ttb_gemm_bf16_splitk(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, long long lda,
-                                    long long ldb, long long ldc, int splits, float alpha, int* err, void* stream) {
+// The partial sums of a split contraction, added in the order of the ranges (the same result every time), with what the epilogue would have done.  Four columns
+// per thread; the partials come from L2.
+namespace ttb {
+__global__ void __launch_bounds__(256)
+splitk_sum_kernel(const float4* __restrict__ part, int splits, int M, int N, void* __restrict__ C, long long ldc, int out_fp32, int accumulate, const __nv_bfloat16* __restrict__ bias,
+                  const __nv_bfloat16* __restrict__ residual, long long ldr) {
+  const int vecs = N >> 2;
+  const long long total = static_cast<long long>(M) * vecs;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
+    const long long row = i / vecs;
+    const int col = static_cast<int>(i % vecs) * 4;
+    float4 v = part[i];
+#pragma unroll 4
+    for (int s = 1; s < splits; ++s) {
+      const float4 t = part[s * total + i];
+      v.x += t.x, v.y += t.y, v.z += t.z, v.w += t.w;
+    }
+    auto add4 = [&](const __nv_bfloat16* from) {
+      const uint2 u = *reinterpret_cast<const uint2*>(from);
+      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+      v.x += lo.x, v.y += lo.y, v.z += hi.x, v.w += hi.y;
+    };
+    if (bias != nullptr) v.x += __bfloat162float(bias[col]), v.y += __bfloat162float(bias[col + 1]), v.z += __bfloat162float(bias[col + 2]), v.w += __bfloat162float(bias[col + 3]);
+    if (residual != nullptr) add4(residual + row * ldr + col);
+    if (out_fp32) {
+      float4* dst = reinterpret_cast<float4*>(static_cast<float*>(C) + row * ldc + col);
+      if (accumulate) v.x += dst->x, v.y += dst->y, v.z += dst->z, v.w += dst->w;
+      *dst = v;
+    } else {
+      __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(C) + row * ldc + col;
+      if (accumulate) add4(dst);
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+    }
+  }
+}
+}  // namespace ttb
+
+// ttb_gemm_bf16 with the contraction cut into `splits` ranges (2 ... 64): `work` takes splits * M * N fp32 partial sums, which a second kernel adds up.
+// residual (nullable): bf16 [M, N] with pitch ldr (a multiple of 8), added to the result.
+extern "C" int ttb_gemm_bf16_splitk(const void* A, const void* B, float* work, void* C, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int out_fp32,
+                                    int accumulate, const void* bias, const void* residual, long long ldr, int splits, float alpha, int* err, void* stream) {
   using namespace ttb;
-  if (M <= 0 || N <= 0 || K <= 0 || splits < 1 || splits > 64) return kErrBadShape;
-  if ((lda & 7) || (ldb & 7) || (ldc & 3) || (N & 7)) return kErrBadShape;
+  if (M <= 0 || N <= 0 || K <= 0 || splits < 2 || splits > 64) return kErrBadShape;
+  if ((lda & 7) || (ldb & 7) || (ldc & (out_fp32 ? 3 : 7)) || (N & 7) || (residual != nullptr && (ldr & 7))) return kErrBadShape;
   if ((a_mn ? (M & 7) : (K & 7)) || (b_mn ? (N & 7) : (K & 7))) return kErrBadShape;
+  for (const void* t : {static_cast<const void*>(work), static_cast<const void*>(C), residual})
+    if (reinterpret_cast<uintptr_t>(t) & (t == residual ? 7 : 15)) return kErrBadShape;
   GemmParams p;
-  p.M = M, p.N = N, p.K = K, p.C = C, p.ldc = ldc;
+  p.M = M, p.N = N, p.K = K, p.C = work, p.ldc = N;
   p.bias = nullptr, p.alpha = alpha, p.out_fp32 = 1, p.accumulate = 0, p.err = err, p.splits = splits;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!a_mn && !b_mn) return dispatch_bn<false, false>(A, B, p, lda, ldb, s);
-  if (!a_mn && b_mn) return dispatch_bn<false, true>(A, B, p, lda, ldb, s);
-  if (a_mn && b_mn) return dispatch_bn<true, true>(A, B, p, lda, ldb, s);
-  return dispatch_bn<true, false>(A, B, p, lda, ldb, s);
+  const int rc = !a_mn && !b_mn ? dispatch_bn<false, false>(A, B, p, lda, ldb, s) : !a_mn ? dispatch_bn<false, true>(A, B, p, lda, ldb, s)
+               : b_mn ? dispatch_bn<true, true>(A, B, p, lda, ldb, s) : dispatch_bn<true, false>(A, B, p, lda, ldb, s);
+  if (rc != kOk) return rc;
+  const long long blocks = (static_cast<long long>(M) * (N / 4) + 255) / 256;
+  TTB_COUNT_LAUNCH(1);
+  splitk_sum_kernel<<<static_cast<int>(blocks < 8ll * sm_count() ? blocks : 8ll * sm_count()), 256, 0, s>>>(reinterpret_cast<const float4*>(work), splits, M, N, C, ldc, out_fp32, accumulate,
+                                                                                                static_cast<const __nv_bfloat16*>(bias), static_cast<const __nv_bfloat16*>(residual), ldr);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
 }
