@@ -94,3 +94,42 @@ def test_mask_bounds_on_the_device_are_the_plain_ones():
             lo2, hi2, solid = mask_row_bounds(view.cuda() if view.stride(0) else view[:1].cuda().expand(3, 7, sk))
             assert (lo2.cpu() == lo).all() and (hi2.cpu() == hi).all()
             assert (solid.cpu().bool() == ((count == 0) | (count == hi - lo + 1))).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,s,sk,hq,hkv,kind", [(1, 1, 1, 1, 1, "full"), (2, 130, 70, 4, 2, "full"), (3, 257, 257, 6, 2, "causal"), (1, 640, 640, 8, 1, "causal"), (2, 100, 333, 4, 4, "causal"),
+                                                (2, 500, 500, 4, 2, "documents"), (1, 700, 700, 4, 1, "window"), (2, 150, 500, 4, 2, "slots"), (2, 129, 300, 2, 1, "slots")])
+def test_gradients(b, s, sk, hq, hkv, kind, d):
+    """One to many query blocks per key block, ragged ends beside another batch row, keys and queries that nothing reaches."""
+    q, k, v = _qkv(b, s, sk, hq, hkv, d, seed=s + d)
+    do = _qkv(b, s, sk, hq, hkv, d, seed=5)[0]
+    at, own = torch.arange(sk, device="cuda"), torch.arange(sk - s, sk, device="cuda")
+    dense = (at[None, :] <= own[:, None])[None].expand(b, s, sk)
+    mask = AttentionMask(causal=True)
+    if kind == "full":
+        mask, dense = AttentionMask(causal=False), torch.ones(b, s, sk, dtype=torch.bool, device="cuda")
+    elif kind == "documents":
+        mask = AttentionMask.from_seq_lens([[3, 250, 1, 246], [128, 372]]).to("cuda")
+        ids = mask.doc_ids
+        dense = dense & (ids[:, :, None] == ids[:, None, :])
+    elif kind == "window":
+        mask = AttentionMask(causal=True, window=90)
+        dense = dense & (own[:, None] - at[None, :] < 90)
+    elif kind == "slots":
+        start = torch.randint(0, 60, (b,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1), dtype=torch.int32)
+        mask = AttentionMask(causal=True, key_start=start, query_start=40)  # the first queries of a row see nothing, nor does anything see the last keys
+        dense = mask.dense(b, s, sk, "cuda")
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    ops.attention(*leaves, mask).backward(do)
+    want = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    with torch.no_grad():
+        seen = dense.any(-1)
+    group = hq // hkv
+    kk, vv = (t.repeat_interleave(group, 2) for t in want[1:])
+    score = torch.einsum("bqhd,bkhd->bhqk", want[0], kk) * d**-0.5
+    prob = torch.softmax(score.masked_fill(~dense[:, None], float("-inf")).masked_fill(~seen[:, None, :, None], 0.0), -1) * dense[:, None]
+    torch.einsum("bhqk,bkhd->bqhd", prob, vv).backward(do.double())
+    for got, ref64, name in zip(leaves, want, "qkv"):
+        # probabilities, their gradients and the results are rounded to 8 bits; so are the output and dO that delta is the sum of
+        err = (got.grad.double() - ref64.grad).norm() / ref64.grad.norm().clamp_min(1e-3)
+        assert err < 0.01 and (got.grad.double() - ref64.grad).abs().max() < 0.03 * max(1.0, ref64.grad.abs().max().item()), (name, float(err))

@@ -68,36 +68,6 @@ __device__ __forceinline__ float fast_tanh(float x) {
   return y;
 }
 
-// two-wide fp32 arithmetic (one instruction per pair of values held in a 64-bit register)
-__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ uint64_t pack_u32x2(uint32_t lo, uint32_t hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
-  return d;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 __device__ __forceinline__ void fail(volatile int* abort_flag, int* err, int code) {
   *abort_flag = 1;
   atomicExch(err, code);
@@ -423,8 +393,8 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
   }
 }
 
-// EXTRA compiles in soft-capping and the element-wise boolean mask; the plain instantiation keeps the hot loop free of both.
-template <int D, bool EXTRA>
+// Soft-capped scores and element-wise boolean masks; all other calls run on attention_bwd2.cu.
+template <int D>
 __global__ void __launch_bounds__(256, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, AttnParams p) {
@@ -586,56 +556,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const float dlt = row_ok ? p.delta[stat] : 0.f;
       const int lo_row = (p.lo != nullptr && row_ok) ? p.lo[row_base + q_idx] : 0;
       const int hi_row = (p.hi != nullptr) ? (row_ok ? p.hi[row_base + q_idx] : -1) : (p.causal ? q_idx : p.sk - 1);
-      const uint8_t* mrow = (EXTRA && p.kmask != nullptr && row_ok) ? p.kmask + static_cast<long long>(row_base + q_idx) * p.sk : nullptr;
+      const uint8_t* mrow = (p.kmask != nullptr && row_ok) ? p.kmask + static_cast<long long>(row_base + q_idx) * p.sk : nullptr;
       if (!mbar_wait(sdp_full, ph)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      // A block every row of which sees every key (the interior of a causal or packed mask) needs no per-element test: the bounds
-      // are monotone, so the tile's largest lo and smallest hi decide.  Such blocks take the two-wide fp32 path below.
-      bool interior = !EXTRA && (p.monotone || (p.lo == nullptr && p.hi == nullptr)) && q0 + kBlk <= p.s && kv0 + kBlk <= p.sk;
-      if (interior) {
-        const int lo_max = p.lo != nullptr ? p.lo[row_base + q0 + kBlk - 1] : 0;
-        const int hi_min = p.hi != nullptr ? p.hi[row_base + q0] : (p.causal ? q0 : p.sk - 1);
-        interior = lo_max <= kv0 && hi_min >= kv0 + kBlk - 1;
-      }
 #pragma unroll 1
       for (int ch = 0; ch < 4; ++ch) {
         uint32_t sv[32], dv[32];
         tmem_ld_32x32(tS + lane_sel + ch * 32, sv);
         tmem_ld_32x32(tdP + lane_sel + ch * 32, dv);
         tmem_ld_wait();
-        if (interior) {
-          // p = exp2(s·c − lse),  dS = p · (dP − delta) · scale, two elements per instruction
-          const uint64_t c2 = pack_f32x2(c, c), nl2 = pack_f32x2(-lse, -lse), nd2 = pack_f32x2(-dlt, -dlt), sc2 = pack_f32x2(p.scale, p.scale);
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint32_t pu[4], du[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int e = g * 8 + 2 * i;
-              float t0, t1;
-              unpack_f32x2(fma_f32x2(pack_u32x2(sv[e], sv[e + 1]), c2, nl2), t0, t1);
-              const float p0 = fast_exp2(t0), p1 = fast_exp2(t1);
-              const uint64_t p2 = pack_f32x2(p0, p1);
-              float d0, d1;
-              unpack_f32x2(mul_f32x2(mul_f32x2(p2, sc2), add_f32x2(pack_u32x2(dv[e], dv[e + 1]), nd2)), d0, d1);
-              pu[i] = pack_bf16x2(p0, p1);
-              du[i] = pack_bf16x2(d0, d1);
-            }
-            const uint32_t off = swz_offset(r, ch * 32 + g * 8);
-            *reinterpret_cast<uint4*>(sP + off) = make_uint4(pu[0], pu[1], pu[2], pu[3]);
-            *reinterpret_cast<uint4*>(sdS + off) = make_uint4(du[0], du[1], du[2], du[3]);
-          }
-          continue;
-        }
         float pr[32], ds[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const int j = kv0 + ch * 32 + i;
           const bool vis = row_ok && j >= lo_row && j <= hi_row && j < p.sk && lse != -INFINITY && (mrow == nullptr || mrow[min(j, p.sk - 1)]);
-          if (EXTRA && p.softcap > 0.f) {  // logit = softcap · tanh(score / softcap): the chain rule adds the factor 1 − tanh²
+          if (p.softcap > 0.f) {  // logit = softcap · tanh(score / softcap): the chain rule adds the factor 1 − tanh²
             const float th = fast_tanh(__uint_as_float(sv[i]) * cap_in);
             pr[i] = vis ? fast_exp2(th * cap_out - lse) : 0.f;
             ds[i] = pr[i] * (__uint_as_float(dv[i]) - dlt) * p.scale * (1.f - th * th);
@@ -774,12 +712,11 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   if ((rc = make_head_map(&tk, k, p.b, p.sk, p.hkv, D)) != kOk) return rc;
   if ((rc = make_head_map(&tv, v, p.b, p.sk, p.hkv, D)) != kOk) return rc;
   if ((rc = make_head_map(&tdo, d_o, p.b, p.s, p.hq, D)) != kOk) return rc;
-  const bool extra = p.softcap > 0.f || p.kmask != nullptr;
-  auto kern = extra ? attn_bwd_kernel<D, true> : attn_bwd_kernel<D, false>;
-  static bool attr[2] = {false, false};
-  if (!attr[extra]) {
+  auto kern = attn_bwd_kernel<D>;
+  static bool attr = false;
+  if (!attr) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem_bytes<D>()) != cudaSuccess) return kErrDriver;
-    attr[extra] = true;
+    attr = true;
   }
   dim3 grid((p.sk + kBlk - 1) / kBlk, p.hkv, p.b);
   TTB_COUNT_LAUNCH(1);
@@ -810,6 +747,10 @@ extern "C" int ttb_attn_fwd(const void* q, const void* k, const void* v, void* o
   return d == 128 ? launch_fwd<128>(q, k, v, p, st) : launch_fwd<64>(q, k, v, p, st);
 }
 
+// attention_bwd2.cu
+int ttb_attn_bwd2(const void* q, const void* k, const void* v, const void* d_o, const float* lse, const float* delta, float* dq, void* dk, void* dv, const int* lo, const int* hi,
+                  int monotone, int b, int s, int sk, int hq, int hkv, int d, float scale, int causal, int* err, cudaStream_t stream);
+
 // delta: [b, hq, s] fp32 scratch, dq_accum: [b, s, hq, d] fp32 zero-filled by the caller; dk, dv: [b, sk, hkv, d].
 extern "C" int ttb_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                             const float* lse, float* delta, float* dq_accum, void* dk, void* dv, const int* lo, const int* hi,
@@ -827,5 +768,6 @@ extern "C" int ttb_attn_bwd(const void* q, const void* k, const void* v, const v
   p.kmask = static_cast<const uint8_t*>(kmask), p.monotone = monotone, p.softcap = softcap;
   p.lse = const_cast<float*>(lse), p.delta = delta, p.dq_accum = dq_accum;
   p.dk = static_cast<__nv_bfloat16*>(dk), p.dv = static_cast<__nv_bfloat16*>(dv), p.err = err;
+  if (!(softcap > 0.f) && kmask == nullptr) return ttb_attn_bwd2(q, k, v, d_o, lse, delta, dq_accum, dk, dv, lo, hi, monotone, b, s, sk, hq, hkv, d, scale, causal, err, st);
   return d == 128 ? launch_bwd<128>(q, k, v, d_o, p, st) : launch_bwd<64>(q, k, v, d_o, p, st);
 }
