@@ -42,3 +42,14 @@ def test_scaled_gradients(n):
     x = _logits(1, n, torch.bfloat16)[0]
     f = torch.tensor(1 / 3, device="cuda")
     assert torch.equal(_scaled(x, f), (x.float() * f).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("n", [2**20, 2**20 + 8, 8 * 1_000_003])
+def test_widened_logits(n):
+    from torchtune_b200 import ops
+
+    x = _logits(1, n, torch.bfloat16, n)
+    x[0, :3] = torch.tensor([float("nan"), float("inf"), -0.0])
+    with torch.no_grad():
+        got = ops.widen(x)
+    assert got.dtype == torch.float32 and torch.equal(got.view(torch.int32)[:, 1:], x.float().view(torch.int32)[:, 1:]) and got[0, 0].isnan()

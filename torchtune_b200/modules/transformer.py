@@ -426,7 +426,7 @@ class TransformerDecoder(nn.Module):
     def unembed_normed(self, h: torch.Tensor) -> torch.Tensor:
         if self.wide_logits and type(self.output).__name__ == "Linear" and self.output.bias is None:
             return self._cap(ops.linear_wide(h, self.output.weight))
-        return self._cap(self.output(h).float())
+        return self._cap(ops.widen(self.output(h)))
 
     def unembed(self, h: torch.Tensor) -> torch.Tensor:
         """Final norm + output projection of a hidden state (fp32 logits)."""

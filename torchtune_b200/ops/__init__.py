@@ -37,6 +37,7 @@ __all__ = [
     "embed_positions",
     "clamped_glu",
     "softcap",
+    "widen",
     "rms_norm",
     "rope",
     "rope_append",
@@ -143,6 +144,17 @@ def linear_wide(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         y = _cuda.gemm(x.reshape(-1, x.shape[-1]), weight, out_dtype=torch.float32)
         return y[:, :n].reshape(*x.shape[:-1], n)
     return linear(x, weight).float()
+
+
+def widen(x: torch.Tensor) -> torch.Tensor:
+    """``x.float()``; large contiguous bf16 CUDA tensors outside autograd in one vector pass."""
+    if _native(x) and x.numel() >= 2**20 and x.numel() % 8 == 0 and x.is_contiguous() and not _differentiated(x) and x.data_ptr() % 16 == 0:
+        from ._lib import check, lib, stream_ptr
+
+        y = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+        check(lib().ttb_widen(x.data_ptr(), y.data_ptr(), x.numel(), stream_ptr()), "widen")
+        return y
+    return x.float()
 
 
 def softcap(logits: torch.Tensor, cap: float) -> torch.Tensor:

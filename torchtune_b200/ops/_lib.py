@@ -79,6 +79,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_token_logprobs_f32.restype = i32
     L.ttb_scale_bf16.argtypes = [vp, vp, i64, vp, vp]
     L.ttb_scale_bf16.restype = i32
+    L.ttb_widen.argtypes = [vp, vp, i64, vp]
+    L.ttb_widen.restype = i32
     L.ttb_gemm_rows.argtypes = [vp, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, vp]
     L.ttb_gemm_rows.restype = i32
     L.ttb_gemm_rows_gated.argtypes = [vp, i64, vp, vp, i64, vp, i64, i32, i32, i32, f32, f32, vp]
