@@ -117,13 +117,14 @@ struct GroupArgs {
   // TP == 4 (grouped weight gradient): dW[e][M, N] = A_eᵀ · B_e where A is [rows, M] and B is [rows, N] (both MN-major operands)
   // and expert e owns `counts[e]` consecutive rows — the *reduction* dimension is the ragged one.  Tiles are (expert, m, n);
   // every CTA derives the experts' row ranges from `counts` itself (no host read).  The last 64-row block of an expert also
-  // brings in rows of the next expert: the MMA warp zeroes those rows in shared memory (whole 128-byte rows, which the swizzle
-  // keeps intact) before issuing.  Experts without rows get a zero gradient.
+  // brings in rows of the next expert: the MMA warp leaves out the steps that lie in them and zeroes the rest in shared memory (whole
+  // 128-byte rows, which the swizzle keeps intact) before issuing.  Experts without rows get a zero gradient.
   const long long* counts;
   int num_experts;
   long long c_expert_stride;
 };
 static constexpr int kMaxGroupedExperts = 1024;
+static constexpr int kStagedExperts = 128;  // as many as fit beside the staging tiles of the output
 
 template <int TP>
 __device__ __forceinline__ int tp_rotate_m(int m_blk, int num_m, const TpArgs* tp) {
@@ -192,9 +193,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
   const int num_tiles = TP == 4 ? ga->num_experts * num_m * num_n : num_m * num_n * splits;
   const int num_kb = (p.K + BK - 1) / BK;
   const int num_kb2 = TP == 0 ? (p.K2 + BK - 1) / BK : 0;  // k-blocks of the second operand pair (same accumulator)
-  // TP 4: first row and row count of every expert, after the barrier region
-  int* g_row0 = reinterpret_cast<int*>(smem + Cfg::kStages * Cfg::kStageBytes + 256);
-  int* g_cnt = g_row0 + kMaxGroupedExperts;
+  // TP 4: first row and row count of every expert, after the barrier region (and the staging tiles, where the output leaves through them)
+  int* g_row0 = reinterpret_cast<int*>(smem + Cfg::kStages * Cfg::kStageBytes + (TP == 4 && p.tma_store ? 1024 + kRsStageBytes : 256));
+  int* g_cnt = g_row0 + (TP == 4 && p.tma_store ? kStagedExperts : kMaxGroupedExperts);
   if (TP == 4 && threadIdx.x == 32) {
     int run = 0;
     for (int e = 0; e < ga->num_experts; ++e) {
@@ -380,14 +381,15 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
           ok = false;
           break;
         }
+        int steps = BK / 16;
         if (TP == 4 && tail_rows != 0 && kb == kb_count - 1) {
-          // rows [tail_rows, 64) of every 64-column box belong to the next expert: zero them (16 bytes per lane and step)
-          uint8_t* st = smem + stage * Cfg::kStageBytes;
-          constexpr int kBoxes = BM / 64 + BN / 64;
-          const int chunks = (BK - tail_rows) * 8;  // 16-byte chunks per box
-          for (int i = lane; i < chunks * kBoxes; i += 32) {
-            const int box = i / chunks, c = i - box * chunks;
-            *reinterpret_cast<uint4*>(st + box * 8192 + tail_rows * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+          // Rows [tail_rows, 64) of every 64-column box belong to the next expert: steps of 16 rows that hold nothing else are left out, and what is left of the
+          // last one is zeroed (16 bytes per lane, four rows at a time).
+          uint8_t* st = smem + stage * Cfg::kStageBytes + (lane & 7) * 16;
+          steps = (tail_rows + 15) / 16;
+          for (int r = tail_rows + (lane >> 3); r < steps * 16; r += 4) {
+#pragma unroll
+            for (int box = 0; box < BM / 64 + BN / 64; ++box) *reinterpret_cast<uint4*>(st + box * 8192 + r * 128) = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async_smem();
           __syncwarp();
@@ -398,6 +400,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
           const uint32_t sb = sa + Cfg::kABytes;
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
+            if (TP == 4 && k >= steps) break;
             // K-major: 32 bytes per K=16 step inside the swizzled row; SBO = 8 rows * 128 B.
             // MN-major: 16 k-rows = 2 swizzle atoms of 1024 B; LBO = one 64-wide box of BK rows.
             const uint64_t da = A_MN ? make_smem_desc_sw128(sa + k * 2048, 8192, 1024)
@@ -465,7 +468,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
         row_ok = (quarter * 32 + lane) < ga->tile_rows[m_blk];
       }
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
-      if (TP == 2 || ((TP == 0 || TP == 1 || TP == 5) && p.tma_store)) {
+      if (TP == 2 || ((TP == 0 || TP == 1 || TP == 4 || TP == 5) && p.tma_store)) {
         // this warp's 32 rows leave through the TMA store unit, 64 columns at a time (TP 2: into the owner's staging slot)
         uint8_t* stage_base = smem + Cfg::kStages * Cfg::kStageBytes + 1024;  // 1024-byte aligned: after the barrier block
         uint8_t* my_stage = stage_base + quarter * 8192;
@@ -493,7 +496,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
             for (int j = 0; j < 4; ++j) {  // four 16-byte chunks of this half, 128-byte swizzle (chunk ^ row mod 8)
               float f[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[j * 8 + i]) * p.alpha;
+              for (int i = 0; i < 8; ++i) f[i] = (TP == 4 && empty_expert) ? 0.f : __uint_as_float(r[j * 8 + i]) * p.alpha;
               if (TP != 2 && p.bias != nullptr) {
                 const int cb = col0 + h * 32 + j * 8;
 #pragma unroll
@@ -512,7 +515,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_2d(mapC, buf, col0, slot_row0);
+            if (TP == 4)
+              tma_store_3d(mapC, buf, col0, slot_row0, expert);
+            else
+              tma_store_2d(mapC, buf, col0, slot_row0);
             tma_store_commit();
           }
           ++rs_buf;
@@ -604,7 +610,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmA_ptr, const CUte
     }
   }
 
-  if ((TP == 2 || TP == 0 || TP == 1 || TP == 5) && warp >= 4 && warp < 8 && lane == 0) tma_store_wait<0>();  // every staged sub-tile has left shared memory and landed
+  if ((TP == 2 || TP == 0 || TP == 1 || TP == 4 || TP == 5) && warp >= 4 && warp < 8 && lane == 0) tma_store_wait<0>();  // every staged sub-tile has left shared memory and landed
 
   if (TP == 5 && warp >= 8) {
     // ------------------------------------------------------------------ copier warps (weight all-gather over peer memory)
@@ -720,8 +726,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p, GroupArgs ga) {
-  gemm_body<BN, true, true, 4>(&tmA, &tmB, p, nullptr, &ga);
+gemm_grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC, GemmParams p, GroupArgs ga) {
+  gemm_body<BN, true, true, 4>(&tmA, &tmB, p, nullptr, &ga, &tmC);
 }
 
 // One block: exclusive scan of the per-expert row counts, then one m-tile entry per 128 rows of every expert.
@@ -1091,8 +1097,19 @@ static int launch_grouped_wgrad(const void* A, const void* B, const GemmParams& 
   if (rc != kOk) return rc;
   rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, p.N, ldb, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != kOk) return rc;
+  // An expert has few rows and each of its tiles few products, so the launch is bound by what the epilogue can write: without accumulation the tiles
+  // leave through shared memory and TMA stores.  16 experts, 4096 rows, 5120 x 8192 each: 856 us with a row per lane and store, 668 us so, and 421 us with the
+  // tail of the contraction left out instead of zeroed as a whole by the warp that issues the products (3.2 TB/s written; eight epilogue warps gave nothing).
+  GemmParams q = p;
+  CUtensorMap tmC;
+  memset(&tmC, 0, sizeof(tmC));
+  q.tma_store = !p.accumulate && ga.num_experts <= kStagedExperts && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 &&
+                make_tmap_3d(&tmC, p.C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, p.N, p.M, ga.num_experts, p.ldc * 2, ga.c_expert_stride * 2, 64, 32, 1, CU_TENSOR_MAP_SWIZZLE_128B) == kOk;
   auto kern = gemm_grouped_wgrad_kernel<BN>;
-  constexpr int smem = Cfg::kSmemBytes + 2 * kMaxGroupedExperts * static_cast<int>(sizeof(int));
+  constexpr int plain = Cfg::kSmemBytes + 2 * kMaxGroupedExperts * static_cast<int>(sizeof(int));
+  constexpr int staged = Cfg::kSmemBytes + 768 + kRsStageBytes + 2 * kStagedExperts * static_cast<int>(sizeof(int));
+  constexpr int smem = plain > staged ? plain : staged;
+  static_assert(smem <= 232448, "shared memory budget of one CTA");
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kErrDriver;
@@ -1101,7 +1118,7 @@ static int launch_grouped_wgrad(const void* A, const void* B, const GemmParams& 
   const long long tiles = static_cast<long long>(ga.num_experts) * ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
   TTB_COUNT_LAUNCH(1);
-  kern<<<grid, kThreads, smem, stream>>>(tmA, tmB, p, ga);
+  kern<<<grid, kThreads, smem, stream>>>(tmA, tmB, tmC, q, ga);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
 }
 }  // namespace ttb
