@@ -19,11 +19,13 @@ _PLAIN = (TransformerDecoder, TransformerSelfAttentionLayer, MultiHeadAttention,
 
 
 class _LastGraph:
-    """The graph that last ran on a cache.  The next one shares its memory pool, so that any number of generations on one set of caches
-    hold one pool, which goes with the caches.  Copies and pickles of the cache come without it."""
+    """The graph that last ran on a cache and the stream it was recorded on.  The next one shares both and with them the memory pool (its blocks belong to a
+    stream), so that any number of generations on one set of caches hold one pool, which goes with the caches.  Copies and pickles of the cache
+    come without it."""
 
     def __init__(self) -> None:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
+        self.stream: Optional[torch.cuda.Stream] = None
 
     def __deepcopy__(self, memo) -> "_LastGraph":
         return _LastGraph()
@@ -90,7 +92,9 @@ class StepGraph:
         used = [cache.size for cache in self.caches]
         self.x, self.mask = torch.empty_like(x), torch.empty_like(mask)
         self.pos = torch.empty(self.batch, 1, dtype=torch.int32, device=device)
-        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device=device)
+        if self.home.stream is None or self.home.stream.device != device:
+            self.home.stream = torch.cuda.Stream(device=device)
+        graph, stream = torch.cuda.CUDAGraph(), self.home.stream
         stream.wait_stream(torch.cuda.current_stream(device))
         for cache in self.caches:
             cache.recording = True
