@@ -11,9 +11,10 @@
 // Forward: one CTA per (128-query block, query head, batch).  S = Q·Kᵀ and O += P·V run on
 // tcgen05 with S double-buffered in TMEM so the next block's scores are computed while the
 // softmax warps work; O stays in TMEM and is rescaled lazily (only when a row maximum grows
-// by more than 2^8).  Backward: one CTA per (128-key block, KV head, batch) loops over the
-// query heads of its group and the query blocks that can see it, accumulating dK/dV in TMEM
-// and adding dQ partial tiles into an fp32 buffer.
+// by more than 2^8).  It serves soft-capped scores; all others run on attention_fwd2.cu.  Backward: one CTA
+// per (128-key block, KV head, batch) loops over the query heads of its group and the query blocks
+// that can see it, accumulating dK/dV in TMEM and adding dQ partial tiles into an fp32 buffer; it
+// serves soft-capped scores and boolean masks, all others run on attention_bwd2.cu.
 #include "common/ptx.cuh"
 #include "common/tmap.h"
 
