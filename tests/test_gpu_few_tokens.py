@@ -157,3 +157,21 @@ def test_split_contraction(M, N, K, splits, a_mn, b_mn):
     wide = torch.ones(M, N + 8, dtype=torch.float32, device="cuda")
     _gemm_split(x, w, wide[:, :N], splits, a_mn=a_mn, b_mn=b_mn, accumulate=True)
     assert ((wide[:, :N].double() - want - 1).abs() <= 2.0**-19 * (a.double().abs() @ b.double().abs().t() + 1)).all() and (wide[:, N:] == 1).all()
+
+
+def test_observed_modules_are_called():
+    """Hooks on every module are seen by each call of each layer: projections are not joined and steps are not recorded."""
+    from torchtune_b200 import generation, training
+    from torchtune_b200.models.llama3_1 import llama3_1
+
+    with training.set_default_dtype(torch.bfloat16), torch.device("cuda"):
+        model = llama3_1(vocab_size=256, num_layers=1, num_heads=4, num_kv_heads=2, embed_dim=256, max_seq_len=128, intermediate_dim=256).eval()
+        model.setup_caches(batch_size=1, dtype=torch.bfloat16, decoder_max_seq_len=32)
+    seen = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda m, args, out: seen.append(m))
+    try:
+        generation.generate(model, torch.randint(1, 256, (1, 9), device="cuda"), max_generated_tokens=8)
+    finally:
+        handle.remove()
+    for m in (model.layers[0].attn.k_proj, model.layers[0].attn.output_proj, model.layers[0].mlp.w2, model.norm):
+        assert sum(x is m for x in seen) == 8

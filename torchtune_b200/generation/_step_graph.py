@@ -7,9 +7,11 @@ from typing import Optional
 
 import torch
 from torch import nn
+from torch.utils._device import DeviceContext
 
+from .. import ops
 from ..modules import FeedForward, KVCache, MultiHeadAttention, RMSNorm, TransformerDecoder, TransformerSelfAttentionLayer
-from ..modules.linear import Linear
+from ..modules.linear import Linear, has_hooks
 from ..modules.position_embeddings import RotaryPositionalEmbeddings
 from ..modules.tied_linear import TiedLinear
 
@@ -46,11 +48,14 @@ class StepGraph:
             return False
         if type(model.output) not in (Linear, nn.Linear, TiedLinear):
             return False
+        modes = torch.overrides._get_current_function_mode_stack()
+        if not ops.cuda_ops_enabled(like) or torch._C._len_torch_dispatch_stack() or any(type(m) is not DeviceContext for m in modes):  # somebody wants to see every operation
+            return False
         if torch.is_inference_mode_enabled() or torch.cuda.is_current_stream_capturing() or torch.autograd.forward_ad._current_level >= 0:
             return False
         for m in model.modules():
             rotary = isinstance(m, RotaryPositionalEmbeddings) and type(m).forward is RotaryPositionalEmbeddings.forward
-            if not (rotary or type(m) in _PLAIN) or m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+            if not (rotary or type(m) in _PLAIN) or has_hooks(m):
                 return False
         for layer in model.layers:
             if type(layer) is not TransformerSelfAttentionLayer or layer.mask_mod is not None or type(layer.attn) is not MultiHeadAttention:

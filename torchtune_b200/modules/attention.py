@@ -10,7 +10,7 @@ from torch import nn
 from .. import ops
 from ..ops.mask import AttentionMask
 from .kv_cache import KVCache
-from .linear import is_plain_linear
+from .linear import has_hooks, is_plain_linear
 from .position_embeddings import RotaryPositionalEmbeddings
 
 logger = logging.getLogger(__name__)
@@ -110,7 +110,7 @@ class MultiHeadAttention(nn.Module):
         cache, pe = self.kv_cache, self.pos_embeddings
         if not self.cache_enabled or type(cache) is not KVCache or self.q_norm is not None or not isinstance(pe, RotaryPositionalEmbeddings):
             return None
-        if type(pe).forward is not RotaryPositionalEmbeddings.forward or pe._forward_hooks or pe._forward_pre_hooks:
+        if type(pe).forward is not RotaryPositionalEmbeddings.forward or has_hooks(pe) or has_hooks(cache):
             return None
         b, s = q.shape[:2]
         out = ops.rope_append(q, k, v, pe.cache, input_pos, pe.interleaved, cache.k_cache[:b], cache.v_cache[:b], cache.reserve(b, s))

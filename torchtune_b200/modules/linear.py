@@ -15,7 +15,14 @@ class Linear(nn.Linear):
         return ops.linear(x, self.weight, self.bias)
 
 
+def has_hooks(module: nn.Module) -> bool:
+    """Whether calling ``module`` runs anything beside its class's ``forward``: hooks of its own, hooks on all modules, or a replaced ``forward``."""
+    everywhere = nn.modules.module
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks or "forward" in module.__dict__
+                or everywhere._global_forward_hooks or everywhere._global_forward_pre_hooks or everywhere._global_backward_hooks or everywhere._global_backward_pre_hooks)
+
+
 def is_plain_linear(module: nn.Module) -> bool:
     """Whether calling ``module`` is nothing but ``x @ weight.T (+ bias)``: no derived class, no hooks.  Callers may then take the weight and
     join the product with what surrounds it."""
-    return type(module) in (nn.Linear, Linear) and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
+    return type(module) in (nn.Linear, Linear) and not has_hooks(module)
