@@ -1,0 +1,63 @@
+"""Which calls the CUDA wrappers take, pass on or refuse, with the kernel library replaced by a recorder (no GPU)."""
+import pytest
+import torch
+
+from torchtune_b200 import ops
+from torchtune_b200.ops import _cuda
+
+
+class _Recorder:
+    """Stands for the kernel library: notes the entry points that are called and does nothing."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def entry(*args):
+            self.calls.append(name)
+            return 0
+
+        return entry
+
+
+@pytest.fixture
+def library(monkeypatch):
+    rec = _Recorder()
+    monkeypatch.setattr(_cuda, "lib", lambda: rec)
+    monkeypatch.setattr(_cuda, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(_cuda, "err_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(_cuda, "_SM_PAIRS", 74)
+    return rec
+
+
+def _zeros(*shape):
+    return torch.zeros(*shape, dtype=torch.bfloat16)
+
+
+@pytest.mark.parametrize("tokens", [4, 300, 20000])
+@pytest.mark.parametrize("width,weight_width", [(4096, 2048), (8192, 4096), (2048, 4096)])
+def test_contraction_widths_have_to_agree(library, tokens, width, weight_width):
+    """An input of another width than the weight is refused, whichever kernel the sizes would choose."""
+    x, w, r = _zeros(1, width).expand(tokens, width), _zeros(4096, weight_width), _zeros(1, 4096).expand(tokens, 4096)
+    with pytest.raises(ValueError, match="contraction mismatch"):
+        _cuda.gemm_residual(x, w, r)
+    with torch.no_grad():
+        assert _cuda.linear_group(x, [_zeros(4096, width), w], [None, None]) is None
+        assert _cuda.gate_up_swiglu(x, w, w) is None
+    assert library.calls == []
+
+
+def test_agreeing_widths_are_taken(library):
+    x, w = _zeros(4, 2048), _zeros(512, 2048)
+    with torch.no_grad():
+        assert _cuda.gemm_residual(x, w, _zeros(4, 512)).shape == (4, 512)
+        assert [y.shape for y in _cuda.linear_group(x, [w, w], [None, None])] == [(4, 512)] * 2
+        assert _cuda.gate_up_swiglu(x, w, w).shape == (4, 512)
+    assert library.calls == ["ttb_gemm_rows", "ttb_gemm_rows", "ttb_gemm_rows_gated"]
+
+
+def test_a_bias_of_another_length_is_left_to_the_general_path(library):
+    x, w = _zeros(4, 2048), _zeros(512, 2048)
+    with torch.no_grad():
+        assert _cuda.linear_group(x, [w, w], [None, _zeros(256)]) is None
+    assert library.calls == []

@@ -67,9 +67,11 @@ def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Seque
     """The linear layers ``weights[i]`` of one input in one launch, outside autograd; ``None`` where the kernel for few tokens does not apply."""
     K = x.shape[-1]
     M = x.numel() // K if K else 0
-    if len(weights) > 3 or not all(_runs_rows(M, w.shape[0], K) for w in weights) or any(w.dtype != _BF16 or w.stride(1) != 1 or w.stride(0) % 8 or w.data_ptr() % 16 for w in weights):
+    if len(weights) > 3 or not all(_runs_rows(M, w.shape[0], K) for w in weights):
         return None
-    if any(b is not None and (b.dtype != _BF16 or not b.is_contiguous()) for b in biases):
+    if any(w.shape[1] != K or w.dtype != _BF16 or w.stride(1) != 1 or w.stride(0) % 8 or w.data_ptr() % 16 for w in weights):
+        return None
+    if any(b is not None and (b.shape != w.shape[:1] or b.dtype != _BF16 or not b.is_contiguous()) for w, b in zip(weights, biases)):
         return None
     x2 = x.reshape(M, K)
     if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
@@ -77,6 +79,12 @@ def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Seque
     outs = [torch.empty(M, w.shape[0], dtype=_BF16, device=x.device) for w in weights]
     _gemm_rows(x2, weights, outs, None if all(b is None for b in biases) else biases)
     return [o.view(*x.shape[:-1], o.shape[1]) for o in outs]
+
+
+def _check_contraction(K: int, Kb: int) -> None:
+    """No kernel sees more of the second operand than its address, pitch and rows: one of another width would be read past its end."""
+    if K != Kb:
+        raise ValueError(f"gemm contraction mismatch: {K} vs {Kb}")
 
 
 def gemm(
@@ -104,8 +112,7 @@ def gemm(
         b = b.contiguous()
     M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
     N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
-    if K != Kb:
-        raise ValueError(f"gemm contraction mismatch: {K} vs {Kb}")
+    _check_contraction(K, Kb)
     if out is None:
         if accumulate:
             raise ValueError("accumulate=True needs an existing `out`")
@@ -166,7 +173,8 @@ def gemm_skinny(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: b
 
     a, b = ok(a), ok(b)
     M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
-    N = b.shape[1] if b_mn else b.shape[0]
+    N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
+    _check_contraction(K, Kb)
     out = torch.empty(M, N, dtype=_BF16, device=a.device)
     splits = min(64, 148 // _tiles(M, N), -(-K // 256)) if M and N else 1
     if splits <= 1:
@@ -208,6 +216,7 @@ def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias
     a, b, residual = ok(a), ok(b), ok(residual)
     M, K = a.shape
     N = b.shape[0]
+    _check_contraction(K, b.shape[1])
     out = torch.empty(M, N, dtype=_BF16, device=a.device)
     if _runs_rows(M, N, K) and (bias is None or (bias.dtype == _BF16 and bias.is_contiguous())):
         _gemm_rows(a, [b], [out], None if bias is None else [bias], residual=residual)
@@ -1248,7 +1257,7 @@ def gate_up_swiglu(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, clamp: O
         return None
     K, N = x.shape[-1], w1.shape[0]
     M = x.numel() // K
-    if w1.shape != w3.shape or w1.dtype != _BF16 or w3.dtype != _BF16 or K % 8 or N % 8 or not (w1.is_contiguous() and w3.is_contiguous()):
+    if w1.shape != w3.shape or w1.shape[1] != K or w1.dtype != _BF16 or w3.dtype != _BF16 or K % 8 or N % 8 or not (w1.is_contiguous() and w3.is_contiguous()):
         return None
     if w1.data_ptr() % 16 or w3.data_ptr() % 16:
         return None
