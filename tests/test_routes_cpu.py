@@ -61,3 +61,15 @@ def test_a_bias_of_another_length_is_left_to_the_general_path(library):
     with torch.no_grad():
         assert _cuda.linear_group(x, [w, w], [None, _zeros(256)]) is None
     assert library.calls == []
+
+
+@pytest.mark.parametrize("width", [2048, 4096, 8192])
+def test_residual_product_of_no_tokens(library, width):
+    """Nothing to multiply: an empty result, and gradients of zeros, at widths that would be cut into ranges too."""
+    x, w, r = (_zeros(*s).requires_grad_() for s in ((0, width), (512, width), (0, 512)))
+    y = _cuda.linear_residual(x, w, None, r)
+    assert y.shape == (0, 512)
+    y.sum().backward()
+    assert x.grad.shape == (0, width) and r.grad.shape == (0, 512) and w.grad.shape == (512, width) and not w.grad.any()
+    assert _cuda.gemm_residual(_zeros(5, width), _zeros(0, width), _zeros(5, 0)).shape == (5, 0)
+    assert library.calls == []

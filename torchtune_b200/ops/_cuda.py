@@ -191,7 +191,7 @@ def _splits(M: int, N: int, K: int) -> int:
     """In how many ranges to cut the contraction of an ordinary product; 1: not at all.  Worth it where at least two ranges find free SMs and the
     contraction is long enough to pay for the second launch (us whole / in ranges: 300 x 2048 x 2048 14.0 / 14.0, 100 x 4096 x 4096 18.6 / 14.1,
     512 x 2048 x 8192 40.7 / 22.4, 512 x 4096 x 14336 85.9 / 59.0, and 666 x 2048 x 128256 718 / 292)."""
-    return max(1, min(16, 148 // _tiles(M, N), K // 512)) if K >= 4096 else 1
+    return max(1, min(16, 148 // _tiles(M, N), K // 512)) if K >= 4096 and M and N else 1
 
 
 def _gemm_split(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, splits: int, *, a_mn: bool = False, b_mn: bool = False, accumulate: bool = False, bias: Optional[torch.Tensor] = None,
@@ -218,6 +218,8 @@ def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias
     N = b.shape[0]
     _check_contraction(K, b.shape[1])
     out = torch.empty(M, N, dtype=_BF16, device=a.device)
+    if M == 0 or N == 0:
+        return out
     if _runs_rows(M, N, K) and (bias is None or (bias.dtype == _BF16 and bias.is_contiguous())):
         _gemm_rows(a, [b], [out], None if bias is None else [bias], residual=residual)
         return out
