@@ -133,3 +133,31 @@ def test_gradients(b, s, sk, hq, hkv, kind, d):
         # probabilities, their gradients and the results are rounded to 8 bits; so are the output and dO that delta is the sum of
         err = (got.grad.double() - ref64.grad).norm() / ref64.grad.norm().clamp_min(1e-3)
         assert err < 0.01 and (got.grad.double() - ref64.grad).abs().max() < 0.03 * max(1.0, ref64.grad.abs().max().item()), (name, float(err))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("scale", [-0.2, 0.0, 0.05])
+@pytest.mark.parametrize("s,sk", [(1, 77), (200, 200), (140, 300)])
+def test_scales_of_any_sign(s, sk, scale, d):
+    """Scores times a negative scale or 0, without a mask, causal and under a boolean mask with gaps: results and gradients of all kernels."""
+    q, k, v = _qkv(2, s, sk, 4, 2, d, seed=sk)
+    do = _qkv(2, s, sk, 4, 2, d, seed=5)[0]
+    at, own = torch.arange(sk, device="cuda"), torch.arange(sk - s, sk, device="cuda")
+    causal = (at[None, :] <= own[:, None])[None].expand(2, s, sk)
+    gaps = (torch.rand(2, s, sk, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)) < 0.3) | (at[None, None, :] == own[None, :, None])
+    for mask, dense in ((AttentionMask(causal=False), torch.ones_like(causal)), (AttentionMask(causal=True), causal), (AttentionMask(causal=False, bool_mask=gaps), gaps)):
+        leaves = [t.detach().clone().requires_grad_() for t in (q, k, v)]
+        got = ops.attention(*leaves, mask, scale=scale)
+        got.backward(do)
+        with torch.no_grad():
+            alone = ops.attention(q, k, v, mask, scale=scale)
+        want = [t.detach().double().requires_grad_() for t in (q, k, v)]
+        kk, vv = (t.repeat_interleave(2, 2) for t in want[1:])
+        prob = torch.softmax((torch.einsum("bqhd,bkhd->bhqk", want[0], kk) * scale).masked_fill(~dense[:, None], float("-inf")), -1)
+        out = torch.einsum("bhqk,bkhd->bqhd", prob, vv)
+        out.backward(do.double())
+        # probabilities and results are rounded to 8 bits, as in the tests above
+        bound = 2.0**-8 * (out.abs() + torch.einsum("bhqk,bkhd->bqhd", prob, vv.abs()))
+        assert ((got.double() - out).abs() <= bound).all() and ((alone.double() - out).abs() <= bound).all()
+        for leaf, ref64 in zip(leaves, want):
+            assert (leaf.grad.double() - ref64.grad).norm() <= 0.01 * ref64.grad.norm().clamp_min(1e-3)

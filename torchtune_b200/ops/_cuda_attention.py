@@ -107,17 +107,21 @@ class _FlashAttention(torch.autograd.Function):
             )
             return o
         lse = torch.empty(b, hq, s, dtype=torch.float32, device=q.device)
+        # The two-tile kernel takes the largest score before it is scaled, so its scale is positive: another sign (or 0) goes into the queries, which is exact.
+        queries, positive = q, scale
+        if scale <= 0 and softcap == 0.0:
+            queries, positive = (-q, -scale) if scale < 0 else (q * 0.0, 1.0)
         if mask is not None:
             lo, hi, solid = mask_row_bounds(mask)
             check(
-                lib().ttb_attn_fwd2_masked(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(), solid.data_ptr(),
-                                           s if lo.shape[0] > 1 else 0, mask.data_ptr(), mask.stride(0), mask.stride(1), b, s, sk, hq, hkv, d, float(scale),
+                lib().ttb_attn_fwd2_masked(queries.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), lo.data_ptr(), hi.data_ptr(), solid.data_ptr(),
+                                           s if lo.shape[0] > 1 else 0, mask.data_ptr(), mask.stride(0), mask.stride(1), b, s, sk, hq, hkv, d, float(positive),
                                            err_word(q.device).data_ptr(), stream_ptr()),
                 "attention forward (boolean mask)",
             )
         elif softcap == 0.0:  # structured (monotone) bounds
             check(
-                lib().ttb_attn_fwd2(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(lo), _p(hi), b, s, sk, hq, hkv, d, float(scale), int(causal),
+                lib().ttb_attn_fwd2(queries.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), _p(lo), _p(hi), b, s, sk, hq, hkv, d, float(positive), int(causal),
                                     err_word(q.device).data_ptr(), stream_ptr()),
                 "attention forward",
             )
