@@ -7,6 +7,7 @@ import torch
 
 from ..modules import TransformerDecoder
 from ..modules.attention import MaskLike
+from ..modules.kv_cache import counted_appends
 from ._rows import DecodeGraph, RowLayout, hidden_states
 from ._step_graph import StepGraph
 
@@ -104,6 +105,13 @@ def generate(
     ends only when every rank of the group has seen a stop token in every row, so ranks that hold shards of one model keep
     issuing the same number of forward passes (parity: torchtune/dev/rl/generation.py:29-190)."""
     prompt = prompt.view(1, -1) if prompt.ndim == 1 else prompt
+    # a plain decoder without hooks: nobody but the passes below writes to the caches until the last token
+    recorded = model.caches_are_enabled() and custom_generate_next_token is None and StepGraph.suits(model, prompt)
+    with counted_appends(model.plain_caches() if recorded else []):
+        return _generate(model, prompt, max_generated_tokens, pad_id, temperature, top_k, stop_tokens, rng, custom_generate_next_token, return_logits, stop_group, recorded)
+
+
+def _generate(model, prompt, max_generated_tokens, pad_id, temperature, top_k, stop_tokens, rng, custom_generate_next_token, return_logits, stop_group, recorded):
     bsz, prompt_len = prompt.shape
     total_len = prompt_len + max_generated_tokens
     device = prompt.device
@@ -161,7 +169,7 @@ def generate(
             logits = model.unembed_normed(graph(x))[:, -1]
             return sample(logits, temperature=temperature, top_k=top_k, q=q), logits.unsqueeze(1)
 
-    elif incremental and custom_generate_next_token is None and max_generated_tokens > 3 and StepGraph.suits(model, prompt):
+    elif recorded and max_generated_tokens > 3:
         graph_step = StepGraph(model, bsz)
 
         def step_fn(model, input_pos, x, q=None, *, mask=None, temperature=1.0, top_k=None):

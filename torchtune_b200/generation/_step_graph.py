@@ -87,14 +87,13 @@ class StepGraph:
         self.mask.copy_(mask)
         self.graph.replay()
         for cache in self.caches:
-            cache._note(cache.size + 1)
+            cache.advanced(1)
         return self.logits.clone()
 
     def _record(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> None:
         device = x.device
         for cache in self.caches:
             cache.reserve(self.batch, 1)
-        used = [cache.size for cache in self.caches]
         self.x, self.mask = torch.empty_like(x), torch.empty_like(mask)
         self.pos = torch.empty(self.batch, 1, dtype=torch.int32, device=device)
         if self.home.stream is None or self.home.stream.device != device:
@@ -112,8 +111,7 @@ class StepGraph:
                 finally:
                     graph.capture_end()
         finally:
-            for cache, n in zip(self.caches, used):
+            for cache in self.caches:
                 cache.recording = False
-                cache._note(n)  # nothing has run yet
         torch.cuda.current_stream(device).wait_stream(stream)
         self.graph = self.home.graph = graph

@@ -113,7 +113,7 @@ class MultiHeadAttention(nn.Module):
         if type(pe).forward is not RotaryPositionalEmbeddings.forward or has_hooks(pe) or has_hooks(cache):
             return None
         b, s = q.shape[:2]
-        out = ops.rope_append(q, k, v, pe.cache, input_pos, pe.interleaved, cache.k_cache[:b], cache.v_cache[:b], cache.reserve(b, s))
+        out = ops.rope_append(q, k, v, pe.cache, input_pos, pe.interleaved, cache.k_cache[:b], cache.v_cache[:b], lambda: cache.reserve(b, s))
         if out is not None:
             cache.advance(s)
         return out

@@ -5,6 +5,7 @@ attention kernels consume — rather than head-major.
 """
 from __future__ import annotations
 
+from contextlib import contextmanager
 from typing import Any, Iterator, List, Optional, Sequence, Tuple
 
 import torch
@@ -12,8 +13,8 @@ from torch import nn
 
 
 class KVCache(nn.Module):
-    # (cache_pos, its version, number of tokens at that version): spares the host a look at the device as long as nobody else wrote to it
-    _known: Optional[Tuple[torch.Tensor, int, int]] = None
+    # Tokens held, within counted_appends; None outside of it: cache_pos on the device alone knows, and whoever appends asks it.
+    _level: Optional[int] = None
     # True while a decode step is recorded: the recorded step moves cache_pos on for all layers at once
     recording = False
 
@@ -31,19 +32,12 @@ class KVCache(nn.Module):
         self.k_cache.zero_()
         self.v_cache.zero_()
         self.cache_pos -= self.cache_pos[0].clone()
-        self._note(0)
-
-    def _note(self, used: int) -> None:
-        self._known = None if self.cache_pos.is_inference() else (self.cache_pos, self.cache_pos._version, used)
+        if self._level is not None:
+            self._level = 0
 
     @property
     def size(self) -> int:
-        known, pos = self._known, self.cache_pos
-        if known is None or known[0] is not pos or known[1] != pos._version:
-            self._note(int(pos[0].item()))
-            if self._known is None:
-                return int(pos[0].item())
-        return self._known[2]
+        return int(self.cache_pos[0].item()) if self._level is None else self._level
 
     def reserve(self, bsz: int, seq_len: int) -> torch.Tensor:
         """Slots of the next ``seq_len`` tokens of ``bsz`` rows; :meth:`advance` follows once they are written."""
@@ -52,15 +46,19 @@ class KVCache(nn.Module):
                 f"The current cache has been setup with a batch size of {self.k_cache.shape[0]}"
                 f", but found new key tensors with batch size {bsz}!"
             )
-        if self.size + seq_len > self.max_seq_len:
+        if not self.recording and self.size + seq_len > self.max_seq_len:
             raise AssertionError("KV cache is full: cannot write past max_seq_len")
         return self.cache_pos[:seq_len]
 
     def advance(self, seq_len: int) -> None:
-        used = self.size + seq_len
         if not self.recording:
             self.cache_pos.add_(seq_len)
-        self._note(used)
+            self.advanced(seq_len)
+
+    def advanced(self, seq_len: int) -> None:
+        """Notes that ``cache_pos`` was moved on on the device."""
+        if self._level is not None:
+            self._level += seq_len
 
     def update(self, k_val: torch.Tensor, v_val: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """Append ``[b, s, n_kv, d]`` keys/values and return the full buffers."""
@@ -70,6 +68,23 @@ class KVCache(nn.Module):
         self.v_cache[:bsz].index_copy_(1, where, v_val)
         self.advance(seq_len)
         return self.k_cache[:bsz], self.v_cache[:bsz]
+
+
+@contextmanager
+def counted_appends(caches: Sequence[KVCache]) -> Iterator[None]:
+    """Asks the device once how many tokens the caches hold and counts their appends on the host until the block is left, for a caller that alone writes
+    to them meanwhile: one wait per block instead of one per layer and append."""
+    caches = [c for c in caches if c._level is None and not c.recording]
+    if len({c.cache_pos.device for c in caches}) > 1:
+        caches = []
+    if caches:
+        for c, level in zip(caches, torch.stack([c.cache_pos[0] for c in caches]).tolist()):
+            c._level = level
+    try:
+        yield
+    finally:
+        for c in caches:
+            c._level = None
 
 
 class RowCache(nn.Module):

@@ -12,6 +12,7 @@ from ..ops.mask import AttentionMask
 from .attention import MaskLike, MultiHeadAttention
 from .cached_mixer import CachedMixer
 from .hyper_connections import HyperConnection, LayerScale, StreamEntry
+from .kv_cache import KVCache, counted_appends
 from .rms_norm import StreamLayerNorm, StreamRMSNorm
 
 
@@ -338,6 +339,13 @@ class TransformerDecoder(nn.Module):
     def caches_are_enabled(self) -> bool:
         return self.layers[0].caches_are_enabled()
 
+    def plain_caches(self) -> List[KVCache]:
+        """The caches that the layers' attention appends to; none without enabled caches."""
+        if not self.caches_are_enabled():
+            return []
+        attns = [getattr(layer, "attn", None) for layer in self.layers]
+        return [a.kv_cache for a in attns if type(getattr(a, "kv_cache", None)) is KVCache and getattr(a, "cache_enabled", False)]
+
     def reset_caches(self) -> None:
         if not self.caches_are_enabled():
             raise RuntimeError("Key value caches are not setup. Call model.setup_caches first.")
@@ -381,21 +389,22 @@ class TransformerDecoder(nn.Module):
         hidden = []
         layer_state: dict = {}
         order = self.run_order()
-        for i, (idx, run) in enumerate(order):
-            layer = self.layers[idx]
-            if i in self.output_hidden_states:
-                hidden.append(_collapsed(h))
-            extra = {}
-            kind = getattr(layer, "inner_cls", type(layer))
-            after = self.layers[order[i + 1][0]] if i + 1 < len(order) else None
-            if kind is ResidualStreamLayer:
-                following = getattr(after, "sa_norm", None) if after is not None else self.norm
-                extra = {"layer_state": layer_state, "next_norm": following if isinstance(following, StreamRMSNorm) else None}
-            elif kind is HyperConnectionLayer:
-                layer_state["pass"] = run
-                last = StreamEntry(None, self.norm, keep=len(order) in self.output_hidden_states)
-                extra = {"layer_state": layer_state, "following": last if after is None else after.entry}
-            h = layer(h, mask=mask, encoder_input=encoder_input, encoder_mask=encoder_mask, input_pos=input_pos, **extra)
+        with counted_appends(self.plain_caches()):
+            for i, (idx, run) in enumerate(order):
+                layer = self.layers[idx]
+                if i in self.output_hidden_states:
+                    hidden.append(_collapsed(h))
+                extra = {}
+                kind = getattr(layer, "inner_cls", type(layer))
+                after = self.layers[order[i + 1][0]] if i + 1 < len(order) else None
+                if kind is ResidualStreamLayer:
+                    following = getattr(after, "sa_norm", None) if after is not None else self.norm
+                    extra = {"layer_state": layer_state, "next_norm": following if isinstance(following, StreamRMSNorm) else None}
+                elif kind is HyperConnectionLayer:
+                    layer_state["pass"] = run
+                    last = StreamEntry(None, self.norm, keep=len(order) in self.output_hidden_states)
+                    extra = {"layer_state": layer_state, "following": last if after is None else after.entry}
+                h = layer(h, mask=mask, encoder_input=encoder_input, encoder_mask=encoder_mask, input_pos=input_pos, **extra)
         if len(order) in self.output_hidden_states:
             hidden.append(_collapsed(h))
         h, normed = h if isinstance(h, tuple) else (h, None)

@@ -13,7 +13,7 @@ from __future__ import annotations
 
 import os
 import warnings
-from typing import Dict, List, Optional, Sequence, Tuple
+from typing import Callable, Dict, List, Optional, Sequence, Tuple, Union
 
 import torch
 import torch.nn.functional as F
@@ -326,9 +326,9 @@ def rope(
 
 
 def rope_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: torch.Tensor, input_pos: Optional[torch.Tensor], interleaved: bool, k_cache: torch.Tensor,
-                v_cache: torch.Tensor, slots: torch.Tensor) -> Optional[torch.Tensor]:
-    """:func:`rope` of ``q`` (returned) and of ``k``, the latter and ``v`` written to ``k_cache`` / ``v_cache`` ``[b, max_seq, heads, d]`` at ``slots`` (int64 ``[s]``), in one launch
-    outside autograd; ``None``, with nothing written, where that does not apply."""
+                v_cache: torch.Tensor, slots: Union[torch.Tensor, Callable[[], torch.Tensor]]) -> Optional[torch.Tensor]:
+    """:func:`rope` of ``q`` (returned) and of ``k``, the latter and ``v`` written to ``k_cache`` / ``v_cache`` ``[b, max_seq, heads, d]`` at ``slots`` (int64 ``[s]``, or what gives them once
+    nothing else stands in the way), in one launch outside autograd; ``None``, with nothing written, where that does not apply."""
     same = (torch.bfloat16,)
     if not (_native(q, same) and all(_native(t, same) for t in (k, v, k_cache, v_cache))) or _differentiated(q, k, v, k_cache, v_cache) or q.numel() == 0:
         return None
@@ -336,9 +336,10 @@ def rope_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cache: torch.
         return None
     if k.shape != v.shape or k.shape[:2] != q.shape[:2] or k_cache.shape != v_cache.shape or k_cache.shape[0] != k.shape[0] or k_cache.shape[2:] != k.shape[2:] or k.shape[3] != q.shape[3]:
         return None
-    if not (k_cache.is_contiguous() and v_cache.is_contiguous()) or slots.dtype != torch.int64 or not slots.is_contiguous() or slots.numel() != k.shape[1]:
+    if not (k_cache.is_contiguous() and v_cache.is_contiguous()) or any(t.data_ptr() % 16 for t in (cache, k_cache, v_cache)):
         return None
-    if any(t.data_ptr() % 16 for t in (cache, k_cache, v_cache)):
+    slots = slots() if callable(slots) else slots
+    if slots.dtype != torch.int64 or not slots.is_contiguous() or slots.numel() != k.shape[1]:
         return None
     from . import _cuda
 
