@@ -1,0 +1,36 @@
+"""When a projection may be joined with its surroundings instead of being called."""
+import pytest
+import torch
+from torch import nn
+
+from torchtune_b200.models.llama3_1 import llama3_1
+from torchtune_b200.modules.linear import Linear, has_hooks, is_plain_linear
+
+
+def _layer():
+    return llama3_1(vocab_size=64, num_layers=1, num_heads=4, num_kv_heads=2, embed_dim=32, max_seq_len=32, intermediate_dim=64).layers[0]
+
+
+def _watched(how, module):
+    if how == "forward hook":
+        module.register_forward_hook(lambda *a: None)
+    elif how == "forward pre-hook":
+        module.register_forward_pre_hook(lambda *a: None)
+    elif how == "backward hook":
+        module.register_full_backward_hook(lambda *a: None)
+    elif how == "replaced forward":
+        module.forward = module.forward
+    else:
+        module.compile(backend="eager")
+
+
+WAYS = ["forward hook", "forward pre-hook", "backward hook", "replaced forward", "compiled"]
+
+
+@pytest.mark.parametrize("how", WAYS)
+@pytest.mark.parametrize("kind", [Linear, nn.Linear])
+def test_watched_and_compiled_projections_are_called(kind, how):
+    lin = kind(8, 8)
+    assert is_plain_linear(lin) and not has_hooks(lin)
+    _watched(how, lin)
+    assert has_hooks(lin) and not is_plain_linear(lin)

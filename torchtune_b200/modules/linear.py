@@ -16,9 +16,11 @@ class Linear(nn.Linear):
 
 
 def has_hooks(module: nn.Module) -> bool:
-    """Whether calling ``module`` runs anything beside its class's ``forward``: hooks of its own, hooks on all modules, or a replaced ``forward``."""
+    """Whether calling ``module`` runs anything beside its class's ``forward``: hooks of its own, hooks on all modules, a replaced ``forward`` or a
+    compiled one (``module.compile()``)."""
     everywhere = nn.modules.module
     return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks or "forward" in module.__dict__
+                or module._compiled_call_impl is not None
                 or everywhere._global_forward_hooks or everywhere._global_forward_pre_hooks or everywhere._global_backward_hooks or everywhere._global_backward_pre_hooks)
 
 
