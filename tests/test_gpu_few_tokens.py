@@ -173,5 +173,19 @@ def test_observed_modules_are_called():
         generation.generate(model, torch.randint(1, 256, (1, 9), device="cuda"), max_generated_tokens=8)
     finally:
         handle.remove()
-    for m in (model.layers[0].attn.k_proj, model.layers[0].attn.output_proj, model.layers[0].mlp.w2, model.norm):
+    mlp = model.layers[0].mlp
+    for m in (model.layers[0].attn.k_proj, model.layers[0].attn.output_proj, mlp.w1, mlp.w2, mlp.w3, mlp.activation, model.norm):
         assert sum(x is m for x in seen) == 8
+
+
+@pytest.mark.parametrize("name", ["w1", "w3", "activation"])
+def test_a_hook_on_a_gate_changes_the_result(name):
+    from torchtune_b200.modules import FeedForward
+    from torchtune_b200.modules.linear import Linear
+
+    with torch.device("cuda"), torch.no_grad():
+        mlp = FeedForward(gate_proj=Linear(64, 128, bias=False), down_proj=Linear(128, 64, bias=False), up_proj=Linear(64, 128, bias=False)).bfloat16()
+        x = _rand(5, 64)
+        assert mlp(x).any()
+        getattr(mlp, name).register_forward_hook(lambda m, args, out: torch.zeros_like(out))
+        assert not mlp(x).any()

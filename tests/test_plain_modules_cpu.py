@@ -34,3 +34,15 @@ def test_watched_and_compiled_projections_are_called(kind, how):
     assert is_plain_linear(lin) and not has_hooks(lin)
     _watched(how, lin)
     assert has_hooks(lin) and not is_plain_linear(lin)
+
+
+@pytest.mark.parametrize("how", WAYS)
+@pytest.mark.parametrize("name", ["w1", "w3", "activation"])
+def test_watched_gates_are_called(name, how):
+    mlp = _layer().mlp
+    assert mlp._fusable()
+    _watched(how, getattr(mlp, name))
+    assert not mlp._fusable()
+    if how == "forward hook":  # and what it returns counts
+        getattr(mlp, name).register_forward_hook(lambda m, args, out: torch.zeros_like(out))
+        assert not mlp(torch.randn(3, 32)).any()

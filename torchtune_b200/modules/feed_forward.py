@@ -7,7 +7,7 @@ import torch
 from torch import nn
 
 from .. import ops
-from .linear import is_plain_linear
+from .linear import has_hooks, is_plain_linear
 
 
 class ClampedGLU(nn.Module):
@@ -46,9 +46,9 @@ class FeedForward(nn.Module):
             raise ValueError("a gate over two projections needs the up projection")
 
     def _fusable(self) -> bool:
-        """Plain bias-free bf16 linears on both sides of a SiLU or clamped gate: the gate / up projections and the activation run as one GEMM."""
-        lin = (type(self.w1), type(self.w3))
-        return (self._silu or self._glu is not None) and all(t.__name__ == "Linear" and issubclass(t, nn.Linear) for t in lin) and self.w1.bias is None and self.w3.bias is None
+        """Plain bias-free linears on both sides of a plain SiLU or clamped gate: the gate / up projections and the activation run as one GEMM."""
+        return ((self._silu or self._glu is not None) and is_plain_linear(self.w1) and is_plain_linear(self.w3) and self.w1.bias is None and self.w3.bias is None
+                and not has_hooks(self.activation))
 
     def _down(self, h: torch.Tensor, residual: Optional[torch.Tensor]) -> torch.Tensor:
         """Down projection; with ``residual`` the block's input stream is added in the projection's GEMM epilogue."""
@@ -72,5 +72,5 @@ class FeedForward(nn.Module):
         u = self.w3(x)
         if self._glu is not None:
             return self._down(self._glu(g, u), residual)
-        h = ops.swiglu(g, u) if self._silu else self.activation(g) * u
+        h = ops.swiglu(g, u) if self._silu and not has_hooks(self.activation) else self.activation(g) * u
         return self._down(h, residual)
