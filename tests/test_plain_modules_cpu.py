@@ -46,3 +46,32 @@ def test_watched_gates_are_called(name, how):
     if how == "forward hook":  # and what it returns counts
         getattr(mlp, name).register_forward_hook(lambda m, args, out: torch.zeros_like(out))
         assert not mlp(torch.randn(3, 32)).any()
+
+
+class _Wrapped(torch.Tensor):
+    """Stands for a weight that is held in another form and has no bytes of its own to point to."""
+
+
+@pytest.mark.parametrize("kind", [Linear, nn.Linear])
+@pytest.mark.parametrize("part", ["weight", "bias"])
+def test_projections_with_wrapped_parameters_are_called(kind, part):
+    lin = kind(8, 8)
+    setattr(lin, part, nn.Parameter(getattr(lin, part).detach().as_subclass(_Wrapped), requires_grad=False))
+    assert isinstance(getattr(lin, part), _Wrapped) and not is_plain_linear(lin)
+
+
+@pytest.mark.parametrize("kind", [Linear, nn.Linear])
+@pytest.mark.parametrize("grad", [False, True])
+def test_only_this_package_s_projections_are_joined_and_only_outside_autograd(kind, grad, monkeypatch):
+    """torch's own linear layers keep torch's own product: autocast, weights in other forms and modes that look at operations see it."""
+    from torchtune_b200 import ops
+    from torchtune_b200.modules import MultiHeadAttention
+
+    joined = []
+    plain = ops.linear_group
+    monkeypatch.setattr(ops, "linear_group", lambda *a: joined.append(a) or plain(*a))
+    attn = MultiHeadAttention(embed_dim=32, num_heads=4, num_kv_heads=2, head_dim=8, q_proj=kind(32, 32), k_proj=kind(32, 16), v_proj=kind(32, 16), output_proj=kind(32, 32))
+    x = torch.randn(1, 3, 32)
+    with torch.set_grad_enabled(grad):
+        attn(x, x)
+    assert len(joined) == (kind is Linear and not grad)

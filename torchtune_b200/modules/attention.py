@@ -10,7 +10,7 @@ from torch import nn
 from .. import ops
 from ..ops.mask import AttentionMask
 from .kv_cache import KVCache
-from .linear import has_hooks, is_plain_linear
+from .linear import Linear, has_hooks, is_plain_linear
 from .position_embeddings import RotaryPositionalEmbeddings
 
 logger = logging.getLogger(__name__)
@@ -132,7 +132,8 @@ class MultiHeadAttention(nn.Module):
         b, s_x, _ = x.shape
         k = v = None
         projections = (self.q_proj, self.k_proj, self.v_proj)
-        if y is x and all(is_plain_linear(m) for m in projections):
+        # torch's own linear layers keep torch's own product, which autocast, tensor subclasses and modes that look at operations know
+        if y is x and not torch.is_grad_enabled() and all(type(m) is Linear and is_plain_linear(m) for m in projections):
             q, k, v = ops.linear_group(x, [m.weight for m in projections], [m.bias for m in projections])
         else:
             q = self.q_proj(x)
