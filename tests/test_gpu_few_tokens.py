@@ -189,3 +189,30 @@ def test_a_hook_on_a_gate_changes_the_result(name):
         assert mlp(x).any()
         getattr(mlp, name).register_forward_hook(lambda m, args, out: torch.zeros_like(out))
         assert not mlp(x).any()
+
+
+@pytest.mark.parametrize("fresh", [True, False])
+@pytest.mark.parametrize("n", [2, 8])
+def test_padded_rows(n, fresh):
+    """Generation of left-padded prompts, with plain and with recorded steps, on fresh caches and on used ones, against one pass over each row without its padding."""
+    import copy
+
+    from torchtune_b200 import generation, training
+    from torchtune_b200.models.llama3_1 import llama3_1
+
+    torch.manual_seed(0)
+    with training.set_default_dtype(torch.bfloat16), torch.device("cuda"):
+        model = llama3_1(vocab_size=1024, num_layers=2, num_heads=8, num_kv_heads=2, embed_dim=512, max_seq_len=512, intermediate_dim=1024).eval()
+        plain = copy.deepcopy(model)
+        model.setup_caches(batch_size=3, dtype=torch.bfloat16, decoder_max_seq_len=40)
+    prompt = torch.randint(1, 1024, (3, 20), device="cuda")
+    if not fresh:
+        generation.generate(model, prompt, max_generated_tokens=8)
+        model.reset_caches()
+    prompt[0, :7], prompt[2, :1] = 0, 0
+    tokens, logits = generation.generate(model, prompt, max_generated_tokens=n, pad_id=0)
+    for row, got, pad in zip(tokens, logits, (7, 0, 1)):
+        with torch.no_grad():
+            want = plain(row[None, pad:])[0, 19 - pad : -1]
+        # bf16 activations through two layers
+        assert got.shape == want.shape and (got - want).norm() <= 0.03 * want.norm()

@@ -73,3 +73,13 @@ def test_residual_product_of_no_tokens(library, width):
     assert x.grad.shape == (0, width) and r.grad.shape == (0, 512) and w.grad.shape == (512, width) and not w.grad.any()
     assert _cuda.gemm_residual(_zeros(5, width), _zeros(0, width), _zeros(5, 0)).shape == (5, 0)
     assert library.calls == []
+
+
+def test_positions_of_single_tokens():
+    """Padded rows are stepped with one position each, as a vector: the rows', not the sequence's."""
+    assert torch.equal(_cuda._positions(torch.tensor([4, 7, 2]), 3, 1, "cpu"), torch.tensor([[4], [7], [2]], dtype=torch.int32))
+    assert torch.equal(_cuda._positions(torch.tensor([4, 7]), 3, 2, "cpu"), torch.tensor([[4, 7]] * 3, dtype=torch.int32))
+    assert torch.equal(_cuda._positions(torch.tensor([5]), 3, 1, "cpu"), torch.tensor([[5]] * 3, dtype=torch.int32))
+    assert torch.equal(_cuda._positions(torch.tensor([[4], [7], [2]]), 3, 1, "cpu"), torch.tensor([[4], [7], [2]], dtype=torch.int32))
+    with pytest.raises(RuntimeError):
+        _cuda._positions(torch.tensor([4, 7, 2]), 2, 1, "cpu")

@@ -1157,6 +1157,8 @@ def _positions(input_pos: Optional[torch.Tensor], b: int, s: int, device) -> Opt
     if input_pos is None:
         return None
     pos = input_pos.to(device=device, dtype=torch.int32)
+    if s == 1 and pos.shape == (b,):  # one token per row and a position for each
+        return pos.view(b, 1).contiguous()
     return pos.expand(b, s).contiguous() if pos.dim() == 2 else pos.view(1, s).expand(b, s).contiguous()
 
 
