@@ -3,7 +3,7 @@
 A step of a small model is a few hundred launches of a few microseconds each, and the host needs longer to issue one than the GPU to run it."""
 from __future__ import annotations
 
-from typing import Optional
+from typing import Optional, Set, Tuple
 
 import torch
 from torch import nn
@@ -28,6 +28,7 @@ class _LastGraph:
     def __init__(self) -> None:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.stream: Optional[torch.cuda.Stream] = None
+        self.stepped: Set[Tuple[int, ...]] = set()  # batch and mask shape of the steps that have run as they are
 
     def __deepcopy__(self, memo) -> "_LastGraph":
         return _LastGraph()
@@ -38,7 +39,8 @@ class _LastGraph:
 
 class StepGraph:
     """``model(x, input_pos, mask)[:, -1]`` for one token per row: a call is recorded, and it and all later ones replay the recording on the inputs
-    that they are given.  On caches that have not been stepped yet the first call runs as it is, so that one-time set-up stays out of the recording."""
+    that they are given.  The first step of a batch and mask shape on a set of caches runs as it is, so that the one-time set-up of the kernels that
+    these sizes choose stays out of the recording."""
 
     @staticmethod
     def suits(model: nn.Module, like: torch.Tensor) -> bool:
@@ -72,14 +74,15 @@ class StepGraph:
         self.caches = [layer.attn.kv_cache for layer in model.layers]
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.home: _LastGraph = self.caches[0].__dict__.setdefault("last_graph", _LastGraph())
-        self.ready = self.home.graph is not None
 
     def __call__(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
-        if self.graph is None and self.ready:
-            self._record(x, input_pos, mask)
         if self.graph is None:
-            self.ready = True
-            return self.model(x, input_pos=input_pos, mask=mask)[:, -1]
+            sizes = (self.batch, *mask.shape)
+            if sizes not in self.home.stepped:
+                logits = self.model(x, input_pos=input_pos, mask=mask)[:, -1]
+                self.home.stepped.add(sizes)
+                return logits
+            self._record(x, input_pos, mask)
         for cache in self.caches:
             cache.reserve(self.batch, 1)  # raises when the cache is full
         self.x.copy_(x)
