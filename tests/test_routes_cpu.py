@@ -83,3 +83,22 @@ def test_positions_of_single_tokens():
     assert torch.equal(_cuda._positions(torch.tensor([[4], [7], [2]]), 3, 1, "cpu"), torch.tensor([[4], [7], [2]], dtype=torch.int32))
     with pytest.raises(RuntimeError):
         _cuda._positions(torch.tensor([4, 7, 2]), 2, 1, "cpu")
+
+
+@pytest.mark.parametrize("bad", [-100, -1, 64, 2**40])
+def test_token_ids_out_of_range_are_refused(library, bad):
+    """Log-probabilities of ids that no column belongs to: refused by the same operation as in the plain statement."""
+    logits, tokens = torch.zeros(2, 3, 64), torch.zeros(2, 3, dtype=torch.int64)
+    assert _cuda.logits_logprobs_f32(logits, tokens, 1.0) is not None
+    tokens[1, 2] = bad
+    with pytest.raises(RuntimeError, match="out of bounds"):
+        _cuda.logits_logprobs_f32(logits, tokens, 1.0)
+    assert library.calls == ["ttb_token_logprobs_f32"]
+
+
+def test_log_probabilities_want_a_batch():
+    """As the plain statement does: rows of a batch, not a single sequence."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    with FakeTensorMode(), torch.no_grad():
+        assert ops.logits_logprobs(torch.zeros(3, 64, device="cuda"), torch.zeros(3, dtype=torch.int64, device="cuda")) is None

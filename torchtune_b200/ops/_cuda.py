@@ -1068,10 +1068,9 @@ def logits_logprobs(logits: torch.Tensor, tokens: torch.Tensor, temperature: flo
 def logits_logprobs_f32(logits: torch.Tensor, tokens: torch.Tensor, temperature: float) -> Optional[torch.Tensor]:
     """``log_softmax(logits / T)`` at ``tokens`` from fp32 logits ``[..., V]`` in one pass, outside autograd; rows may be a slice of a batch.  ``None`` for layouts that it does not cover."""
     V = logits.shape[-1]
-    if logits.dim() == 2:
-        logits = logits.unsqueeze(0)
     if logits.dim() != 3 or logits.stride(2) != 1 or V % 4 or logits.stride(0) % 4 or logits.stride(1) % 4 or logits.data_ptr() % 16 or logits.numel() // V >= 2**31:
         return None
+    logits.gather(2, tokens.unsqueeze(-1))  # refuses ids out of range, as the plain statement does; a few us
     out = torch.empty(tokens.shape, dtype=torch.float32, device=logits.device)
     tokens = tokens.contiguous()
     check(lib().ttb_token_logprobs_f32(logits.data_ptr(), logits.stride(0), logits.stride(1), logits.shape[1], tokens.data_ptr(), out.data_ptr(), tokens.numel(), V, float(temperature),
