@@ -102,3 +102,17 @@ def test_log_probabilities_want_a_batch():
 
     with FakeTensorMode(), torch.no_grad():
         assert ops.logits_logprobs(torch.zeros(3, 64, device="cuda"), torch.zeros(3, dtype=torch.int64, device="cuda")) is None
+
+
+def test_tensors_without_memory_take_the_plain_statements():
+    """Fake tensors of a trace and batched ones of vmap have no address to give to a kernel."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from torchtune_b200 import rlhf
+
+    with FakeTensorMode(), torch.no_grad():
+        logits, tokens = torch.zeros(2, 3, 64, device="cuda"), torch.zeros(2, 3, dtype=torch.int64, device="cuda")
+        assert rlhf.logits_to_logprobs(logits, tokens).shape == (2, 3)
+        assert ops.widen(torch.zeros(2**20, dtype=torch.bfloat16, device="cuda")).dtype == torch.float32
+        many = torch.vmap(rlhf.logits_to_logprobs)(torch.zeros(5, 2, 3, 64, device="cuda"), torch.zeros(5, 2, 3, dtype=torch.int64, device="cuda"))
+        assert many.shape == (5, 2, 3)

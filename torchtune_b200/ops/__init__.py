@@ -101,6 +101,11 @@ def _differentiated(*tensors: Optional[torch.Tensor]) -> bool:
     return (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)) or torch.autograd.forward_ad._current_level >= 0
 
 
+def _has_memory(*tensors: torch.Tensor) -> bool:
+    """Whether these are ordinary tensors, whose address a kernel can be given: not fake ones of a trace, batched ones of vmap or other subclasses."""
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t) for t in tensors)
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x @ weight.T (+ bias)``; bf16 CUDA inputs run the tcgen05 GEMM (fwd, dgrad, wgrad)."""
     if _native(x) and weight.dtype == torch.bfloat16:
@@ -148,7 +153,7 @@ def linear_wide(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 def widen(x: torch.Tensor) -> torch.Tensor:
     """``x.float()``; large contiguous bf16 CUDA tensors outside autograd in one vector pass."""
-    if _native(x) and x.numel() >= 2**20 and x.numel() % 8 == 0 and x.is_contiguous() and not _differentiated(x) and x.data_ptr() % 16 == 0:
+    if _native(x) and x.numel() >= 2**20 and x.numel() % 8 == 0 and x.is_contiguous() and not _differentiated(x) and _has_memory(x) and x.data_ptr() % 16 == 0:
         from ._lib import check, lib, stream_ptr
 
         y = torch.empty(x.shape, dtype=torch.float32, device=x.device)
@@ -441,7 +446,8 @@ def logits_logprobs(logits: torch.Tensor, tokens: torch.Tensor, temperature: flo
     from . import _cuda
 
     if logits.dtype == torch.float32:
-        return None if _differentiated(logits) or isinstance(temperature, torch.Tensor) else _cuda.logits_logprobs_f32(logits, tokens, temperature)
+        plain = _differentiated(logits) or isinstance(temperature, torch.Tensor) or not _has_memory(logits, tokens)
+        return None if plain else _cuda.logits_logprobs_f32(logits, tokens, temperature)
     return _cuda.logits_logprobs(logits, tokens, temperature) if logits.shape[-1] % 8 == 0 else None
 
 
