@@ -53,3 +53,19 @@ def test_widened_logits(n):
     with torch.no_grad():
         got = ops.widen(x)
     assert got.dtype == torch.float32 and torch.equal(got.view(torch.int32)[:, 1:], x.float().view(torch.int32)[:, 1:]) and got[0, 0].isnan()
+
+
+def test_loss_gradients_of_batched_and_differentiated_factors():
+    from torchtune_b200 import ops
+
+    h, w = (_logits(n, 64, torch.bfloat16, n).requires_grad_() for n in (16, 128))
+    loss, _ = ops.linear_cross_entropy(h, w, torch.randint(0, 128, (16,), device="cuda"))
+    once = torch.autograd.grad(loss, (h, w), retain_graph=True)
+    many = torch.autograd.grad(loss, (h, w), torch.tensor([1.0, 2.0, -4.0], device="cuda"), is_grads_batched=True, retain_graph=True)
+    for a, b in zip(once, many):
+        assert torch.equal(b, torch.stack([a, 2 * a, -4 * a]))
+    factor = torch.tensor(2.0, device="cuda", requires_grad=True)
+    g, = torch.autograd.grad(loss, h, factor, create_graph=True)
+    assert torch.equal(g, 2 * once[0])
+    d, = torch.autograd.grad(g.float().sum(), factor)
+    assert (d - once[0].float().sum()).abs() <= 2.0**-8 * once[0].float().abs().sum()

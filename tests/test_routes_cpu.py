@@ -116,3 +116,18 @@ def test_tensors_without_memory_take_the_plain_statements():
         assert ops.widen(torch.zeros(2**20, dtype=torch.bfloat16, device="cuda")).dtype == torch.float32
         many = torch.vmap(rlhf.logits_to_logprobs)(torch.zeros(5, 2, 3, 64, device="cuda"), torch.zeros(5, 2, 3, dtype=torch.int64, device="cuda"))
         assert many.shape == (5, 2, 3)
+
+
+def test_scaled_gradients_of_batched_and_differentiated_factors(library):
+    """The loss's stored gradients times an upstream factor: the kernel for a plain number, tensor operations where the factor is batched or its own gradient is wanted."""
+    t, many = torch.arange(16, dtype=torch.bfloat16), torch.tensor([1.0, 2.0, -4.0])
+    batched = torch.vmap(lambda f: _cuda._scaled(t, f))(many)
+    assert torch.equal(batched, t * many[:, None].bfloat16())
+    factor = torch.tensor(3.0, requires_grad=True)
+    g, = torch.autograd.grad(_cuda._scaled(t, factor).float().sum(), factor)
+    assert g == t.float().sum()
+    assert library.calls == []
+    with torch.no_grad():
+        _cuda._scaled(t, factor)
+    _cuda._scaled(t, factor.detach())
+    assert library.calls == ["ttb_scale_bf16"] * 2

@@ -1303,8 +1303,11 @@ def _ce_chunk_rows(T: int, num_chunks: int) -> int:
 
 
 def _scaled(t: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
-    """``t · factor`` for a contiguous gradient and a 0-dim fp32 tensor; one vector pass for bf16, with the factor unrounded."""
-    if t.dtype != _BF16 or factor.dtype != torch.float32 or t.numel() % 8 or t.data_ptr() % 16:
+    """``t · factor`` for a contiguous gradient and a 0-dim fp32 tensor; one vector pass for bf16, with the factor unrounded, unless the factor is batched
+    (``is_grads_batched``) or to be differentiated itself (``create_graph``)."""
+    from . import _differentiated, _has_memory
+
+    if t.dtype != _BF16 or factor.dtype != torch.float32 or not _has_memory(t, factor) or _differentiated(t, factor) or t.numel() % 8 or t.data_ptr() % 16:
         return t * factor.to(t.dtype)
     out = torch.empty_like(t)
     check(lib().ttb_scale_bf16(t.data_ptr(), out.data_ptr(), t.numel(), factor.data_ptr(), stream_ptr()), "scale")
