@@ -161,3 +161,14 @@ def test_scales_of_any_sign(s, sk, scale, d):
         assert ((got.double() - out).abs() <= bound).all() and ((alone.double() - out).abs() <= bound).all()
         for leaf, ref64 in zip(leaves, want):
             assert (leaf.grad.double() - ref64.grad).norm() <= 0.01 * ref64.grad.norm().clamp_min(1e-3)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_cap_below_zero_is_none(d):
+    q, k, v = (t.requires_grad_() for t in _qkv(2, 130, 130, 4, 2, d))
+    m = torch.rand(2, 130, 130, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)) < 0.5
+    for mask in (AttentionMask(causal=True), AttentionMask(causal=False, bool_mask=m)):
+        got, want = (ops.attention(q, k, v, mask, softcap=cap) for cap in (-5.0, 0.0))
+        assert torch.equal(got, want)
+        for a, b in zip(torch.autograd.grad(got, (k, v), torch.ones_like(got)), torch.autograd.grad(want, (k, v), torch.ones_like(want))):
+            assert torch.equal(a, b)

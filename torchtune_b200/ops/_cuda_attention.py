@@ -176,6 +176,7 @@ def attention(q, k, v, mask: AttentionMask, scale: Optional[float], softcap: flo
     b, s, hq, d = q.shape
     sk = k.shape[1]
     scale = (1.0 / math.sqrt(d)) if scale is None else scale
+    softcap = max(0.0, float(softcap or 0.0))  # 0 and below: no cap
     lo = hi = kmask = dense = None
     monotone, causal = 1, bool(mask.causal)
     if mask.key_start is not None:
@@ -204,4 +205,4 @@ def attention(q, k, v, mask: AttentionMask, scale: Optional[float], softcap: flo
         lo = lower_bounds(mask, b, s, q.device)
         if causal and s != sk:  # queries are the last s positions of the key sequence (bottom-right aligned causal mask)
             hi = (torch.arange(s, device=q.device, dtype=torch.int32) + (sk - s)).view(1, s).expand(b, s).contiguous()
-    return _FlashAttention.apply(q, k, v, lo, hi, kmask, monotone, scale, causal, float(softcap or 0.0), dense)
+    return _FlashAttention.apply(q, k, v, lo, hi, kmask, monotone, scale, causal, softcap, dense)
