@@ -172,3 +172,18 @@ def test_a_cap_below_zero_is_none(d):
         assert torch.equal(got, want)
         for a, b in zip(torch.autograd.grad(got, (k, v), torch.ones_like(got)), torch.autograd.grad(want, (k, v), torch.ones_like(want))):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("s", [3, 100, 129, 200, 255])
+def test_values_keep_clear_of_the_next_row(s, d):
+    """The last query tile of a batch row ends in the next one's queries: infinite scores there don't reach this row's values."""
+    q, k, v = _qkv(2, s, s, 4, 2, d, seed=s)
+    q[1] = float("inf")
+    k = k.abs() + 0.1
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    ops.attention(*leaves, AttentionMask(causal=True)).backward(torch.ones_like(q))
+    assert leaves[0].grad[0].isfinite().all() and leaves[2].grad[0].isfinite().all()
+    one = [t.detach()[:1].clone().requires_grad_() for t in leaves]
+    ops.attention(*one, AttentionMask(causal=True)).backward(torch.ones_like(one[0]))
+    assert torch.equal(one[2].grad, leaves[2].grad[:1])

@@ -310,6 +310,8 @@ attn_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
               const int lo_j = __shfl_sync(0xffffffffu, lo, j), hi_j = __shfl_sync(0xffffffffu, hi, j);  // by all lanes, whatever the first comparison says
               seen |= (key >= lo_j && key <= hi_j ? 1u : 0u) << j;
             }
+            const int left = p.s - first;  // queries of this batch row; behind them lie the next row's, whose scores may be infinite
+            if (left < 32) seen = left > 0 ? seen & ((1u << left) - 1) : 0;
             if (key >= p.sk) seen = 0;
           }
           uint32_t sv[32], pk[16];
