@@ -123,6 +123,18 @@ def test_scaled_gradients_of_batched_and_differentiated_factors(library):
     t, many = torch.arange(16, dtype=torch.bfloat16), torch.tensor([1.0, 2.0, -4.0])
     batched = torch.vmap(lambda f: _cuda._scaled(t, f))(many)
     assert torch.equal(batched, t * many[:, None].bfloat16())
+
+    class Stored(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.float().sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            return _cuda._scaled(t, g)
+
+    x = torch.zeros(16, dtype=torch.bfloat16, requires_grad=True)
+    assert torch.equal(torch.autograd.grad(Stored.apply(x), x, many, is_grads_batched=True)[0], batched)
     factor = torch.tensor(3.0, requires_grad=True)
     g, = torch.autograd.grad(_cuda._scaled(t, factor).float().sum(), factor)
     assert g == t.float().sum()

@@ -102,8 +102,8 @@ def _differentiated(*tensors: Optional[torch.Tensor]) -> bool:
 
 
 def _has_memory(*tensors: torch.Tensor) -> bool:
-    """Whether these are ordinary tensors, whose address a kernel can be given: not fake ones of a trace, batched ones of vmap or other subclasses."""
-    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t) for t in tensors)
+    """Whether these are ordinary tensors, whose address a kernel can be given: not fake ones of a trace, batched ones of vmap or of autograd, or other subclasses."""
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t) for t in tensors)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
