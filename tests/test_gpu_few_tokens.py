@@ -216,3 +216,53 @@ def test_padded_rows(n, fresh):
             want = plain(row[None, pad:])[0, 19 - pad : -1]
         # bf16 activations through two layers
         assert got.shape == want.shape and (got - want).norm() <= 0.03 * want.norm()
+
+
+def test_generation_beside_other_threads():
+    """Another thread waits for the device and draws random numbers all the while, and generates itself: nothing fails, and the results are those of a single thread."""
+    import threading
+
+    from torchtune_b200 import generation, training
+    from torchtune_b200.models.llama3_1 import llama3_1
+
+    def model(seed):
+        torch.manual_seed(seed)
+        with training.set_default_dtype(torch.bfloat16), torch.device("cuda"):
+            m = llama3_1(vocab_size=512, num_layers=2, num_heads=4, num_kv_heads=2, embed_dim=256, max_seq_len=128, intermediate_dim=512).eval()
+            m.setup_caches(batch_size=2, dtype=torch.bfloat16, decoder_max_seq_len=40)
+        return m
+
+    def run(m):
+        m.reset_caches()
+        rng = torch.Generator(device="cuda").manual_seed(1)
+        return generation.generate(m, torch.arange(1, 19, device="cuda").view(2, 9), max_generated_tokens=10, rng=rng)
+
+    models = model(1), model(2)
+    want = [run(m) for m in models]
+    errors, done = [], threading.Event()
+
+    def check(i):
+        for got, ref in zip(run(models[i]), want[i]):
+            assert torch.equal(got, ref)
+
+    def beside():
+        try:
+            for _ in range(2000):
+                if done.is_set():
+                    break
+                torch.rand(1000, device="cuda")
+                torch.cuda.synchronize()
+            check(1)
+        except BaseException as e:
+            errors.append(e)
+
+    other = threading.Thread(target=beside)
+    other.start()
+    try:
+        for _ in range(4):
+            check(0)
+    finally:
+        done.set()
+        other.join()
+    assert not errors, errors
+    check(0)

@@ -3,6 +3,7 @@
 A step of a small model is a few hundred launches of a few microseconds each, and the host needs longer to issue one than the GPU to run it."""
 from __future__ import annotations
 
+import threading
 from typing import Optional, Set, Tuple
 
 import torch
@@ -18,6 +19,13 @@ from ..modules.tied_linear import TiedLinear
 # Modules whose forward pass of one token is the same sequence of launches in every step and needs no look at the device.
 _PLAIN = (TransformerDecoder, TransformerSelfAttentionLayer, MultiHeadAttention, FeedForward, KVCache, RMSNorm, Linear, nn.Linear, nn.Embedding, nn.ModuleList, nn.Identity,
           nn.SiLU, nn.GELU, nn.ReLU)
+
+
+def _alone() -> bool:
+    """Whether no other thread of this program could get in the way of a recording or be hurt by it: until it ends, a thread that waits for the device or draws random
+    numbers on it fails, and the former breaks the recording.  Any other thread counts, except the one that keeps progress bars up to date."""
+    here = threading.current_thread()
+    return all(t is here or type(t).__module__ == "tqdm._monitor" for t in threading.enumerate())
 
 
 class _LastGraph:
@@ -40,7 +48,7 @@ class _LastGraph:
 class StepGraph:
     """``model(x, input_pos, mask)[:, -1]`` for one token per row: a call is recorded, and it and all later ones replay the recording on the inputs
     that they are given.  The first step of a batch and mask shape on a set of caches runs as it is, so that the one-time set-up of the kernels that
-    these sizes choose stays out of the recording."""
+    these sizes choose stays out of the recording.  While the program has other threads, all calls run as they are."""
 
     @staticmethod
     def suits(model: nn.Module, like: torch.Tensor) -> bool:
@@ -78,7 +86,7 @@ class StepGraph:
     def __call__(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         if self.graph is None:
             sizes = (self.batch, *mask.shape)
-            if sizes not in self.home.stepped:
+            if sizes not in self.home.stepped or not _alone():
                 logits = self.model(x, input_pos=input_pos, mask=mask)[:, -1]
                 self.home.stepped.add(sizes)
                 return logits
