@@ -386,27 +386,14 @@ class TransformerDecoder(nn.Module):
         seq_len = tokens.shape[1] if input_embeds is None else input_embeds.shape[1]
         self._validate_inputs(seq_len, mask=mask, encoder_input=encoder_input, encoder_mask=encoder_mask, input_pos=input_pos)
         h = self._embed(tokens, input_embeds, input_pos)
-        hidden = []
-        layer_state: dict = {}
-        order = self.run_order()
-        with counted_appends(self.plain_caches()):
-            for i, (idx, run) in enumerate(order):
-                layer = self.layers[idx]
-                if i in self.output_hidden_states:
-                    hidden.append(_collapsed(h))
-                extra = {}
-                kind = getattr(layer, "inner_cls", type(layer))
-                after = self.layers[order[i + 1][0]] if i + 1 < len(order) else None
-                if kind is ResidualStreamLayer:
-                    following = getattr(after, "sa_norm", None) if after is not None else self.norm
-                    extra = {"layer_state": layer_state, "next_norm": following if isinstance(following, StreamRMSNorm) else None}
-                elif kind is HyperConnectionLayer:
-                    layer_state["pass"] = run
-                    last = StreamEntry(None, self.norm, keep=len(order) in self.output_hidden_states)
-                    extra = {"layer_state": layer_state, "following": last if after is None else after.entry}
-                h = layer(h, mask=mask, encoder_input=encoder_input, encoder_mask=encoder_mask, input_pos=input_pos, **extra)
-        if len(order) in self.output_hidden_states:
-            hidden.append(_collapsed(h))
+        hidden: list = []
+        passed = dict(mask=mask, encoder_input=encoder_input, encoder_mask=encoder_mask, input_pos=input_pos)
+        caches = self.plain_caches()
+        if caches:
+            with counted_appends(caches):
+                h = self._run_layers(h, hidden, passed)
+        else:
+            h = self._run_layers(h, hidden, passed)
         h, normed = h if isinstance(h, tuple) else (h, None)
         h = self.norm(h) if normed is None else normed
         if self.skip_output_layer:
@@ -416,6 +403,29 @@ class TransformerDecoder(nn.Module):
         else:
             output = self.unembed_normed(h)
         return output if not hidden else [*hidden, output]
+
+    def _run_layers(self, h, hidden: list, passed: dict):
+        """All layers in their order; ``hidden`` takes the states that were asked for."""
+        layer_state: dict = {}
+        order = self.run_order()
+        for i, (idx, run) in enumerate(order):
+            layer = self.layers[idx]
+            if i in self.output_hidden_states:
+                hidden.append(_collapsed(h))
+            extra = {}
+            kind = getattr(layer, "inner_cls", type(layer))
+            after = self.layers[order[i + 1][0]] if i + 1 < len(order) else None
+            if kind is ResidualStreamLayer:
+                following = getattr(after, "sa_norm", None) if after is not None else self.norm
+                extra = {"layer_state": layer_state, "next_norm": following if isinstance(following, StreamRMSNorm) else None}
+            elif kind is HyperConnectionLayer:
+                layer_state["pass"] = run
+                last = StreamEntry(None, self.norm, keep=len(order) in self.output_hidden_states)
+                extra = {"layer_state": layer_state, "following": last if after is None else after.entry}
+            h = layer(h, **passed, **extra)
+        if len(order) in self.output_hidden_states:
+            hidden.append(_collapsed(h))
+        return h
 
     def _embed(self, tokens: Optional[torch.Tensor], input_embeds: Optional[torch.Tensor], input_pos: Optional[torch.Tensor]) -> torch.Tensor:
         if self.pos_embeddings is None:
