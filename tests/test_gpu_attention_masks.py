@@ -5,7 +5,6 @@ import torch
 pytestmark = pytest.mark.gpu
 
 from torchtune_b200 import ops
-from torchtune_b200.ops import reference as ref
 from torchtune_b200.ops.mask import AttentionMask
 
 
@@ -26,10 +25,60 @@ def _qkv(b, s, sk, hq, hkv, d, seed=0):
 def _check(q, k, v, mask, dense):
     with torch.no_grad():
         got = ops.attention(q, k, v, mask)
-    want = ref.span_attention(q.double(), k.double(), v.double(), dense, q.shape[-1] ** -0.5).double()
-    # probabilities are rounded to 8 bits once (2^-9 relative, weights sum to 1) and so is the result
-    bound = 2.0**-8 * (want.abs() + v.double().abs().amax())
+    b, s, hq, d = q.shape
+    group = q.double().view(b, s, k.shape[2], -1, d)
+    score = torch.einsum("bqgnd,bkgd->bgnqk", group, k.double()) * d**-0.5
+    p = torch.softmax(score.masked_fill(~dense[:, None, None], float("-inf")), -1).nan_to_num()  # a query without keys: 0
+    want, square = (torch.einsum("bgnqk,bkgd->bqgnd", w, t).reshape(b, s, hq, d) for w, t in ((p, v.double()), (p.square(), v.double().square())))
+    # The result is rounded to 8 bits (at most 2^-9 of it; twice that here), and so is every weight before it meets its value: errors of at most 2^-9 of
+    # the terms, without a common sign, so eight times 2^-9 of the terms' root of squares (14 standard deviations) bounds their sum.
+    bound = 2.0**-8 * want.abs() + 2.0**-6 * square.sqrt()
     assert ((got.double() - want).abs() <= bound).all(), float(((got.double() - want).abs() - bound).max())
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("sk", [1, 17, 64, 65, 333])
+def test_every_key_counts_for_few_queries(sk, d):
+    """One key holds all of the weight, another one in each batch row: the result is its value."""
+    u = _qkv(1, 1, 1, 1, 1, d, seed=1)[0].sign()
+    v = _qkv(sk, 1, sk, 1, 1, d, seed=2)[2]
+    k = torch.zeros_like(v)
+    at = torch.arange(sk, device="cuda")
+    k[at, at] = u[0, 0] * (40.0 / d**0.5)  # its score is 40, the others' 0
+    with torch.no_grad():
+        got = ops.attention(u.expand(sk, 1, 1, d).contiguous(), k, v, AttentionMask(causal=False))
+    assert ((got[:, 0].double() - v[at, at].double()).abs() <= 2.0**-8 * v[at, at].double().abs() + 1e-9).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("at", [0, 15, 16, 63, 64, 4095, 8191, 8192, 40000, 65535])
+def test_any_key_of_a_long_range_counts(at, d):
+    u = _qkv(1, 1, 1, 1, 1, d, seed=1)[0].sign()
+    v = _qkv(1, 1, 65536, 1, 1, d, seed=2)[2]
+    k = torch.zeros_like(v)
+    k[0, at] = u[0, 0] * (40.0 / d**0.5)
+    with torch.no_grad():
+        got = ops.attention(u, k, v, AttentionMask(causal=False, bool_mask=torch.ones(1, 1, 65536, dtype=torch.bool, device="cuda")))
+    assert ((got[0, 0].double() - v[0, at].double()).abs() <= 2.0**-8 * v[0, at].double().abs() + 1e-9).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("sk", [130, 300, 513])
+def test_every_key_counts_on_the_tiles(sk, d):
+    """Every query looks for one key, which a mask with gaps leaves visible; codes of random signs keep the other scores at least 20 below."""
+    code = _qkv(1, 1, sk, 1, 1, d, seed=3)[1].sign()
+    v = _qkv(1, 1, sk, 1, 1, d, seed=4)[2]
+    order = torch.randperm(sk, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    q = code[:, order] * 8
+    m = torch.rand(1, sk, sk, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)) < 0.5
+    m[0, torch.arange(sk, device="cuda"), order] = True
+    score = torch.einsum("qd,kd->qk", q[0, :, 0].double(), code[0, :, 0].double()) * d**-0.5
+    own = score.gather(1, order[:, None])
+    assert (score.scatter(1, order[:, None], float("-inf")).amax(1) <= own[:, 0] - 20).all()
+    with torch.no_grad():
+        got = ops.attention(q, code, v, AttentionMask(causal=False, bool_mask=m))
+    want = v[0, order].double()
+    assert ((got[0].double() - want).abs() <= 2.0**-8 * want.abs() + 1e-5).all()  # 513 others of weight e^-20
 
 
 @pytest.mark.parametrize("d", [64, 128])
