@@ -106,7 +106,7 @@ def generate(
     issuing the same number of forward passes (parity: torchtune/dev/rl/generation.py:29-190)."""
     prompt = prompt.view(1, -1) if prompt.ndim == 1 else prompt
     # a plain decoder without hooks: nobody but the passes below writes to the caches until the last token
-    recorded = model.caches_are_enabled() and custom_generate_next_token is None and StepGraph.suits(model, prompt)
+    recorded = model.caches_are_enabled() and custom_generate_next_token is None and max_generated_tokens > 3 and StepGraph.suits(model, prompt)
     with counted_appends(model.plain_caches() if recorded else []):
         return _generate(model, prompt, max_generated_tokens, pad_id, temperature, top_k, stop_tokens, rng, custom_generate_next_token, return_logits, stop_group, recorded)
 
@@ -169,7 +169,7 @@ def _generate(model, prompt, max_generated_tokens, pad_id, temperature, top_k, s
             logits = model.unembed_normed(graph(x))[:, -1]
             return sample(logits, temperature=temperature, top_k=top_k, q=q), logits.unsqueeze(1)
 
-    elif recorded and max_generated_tokens > 3:
+    elif recorded:
         graph_step = StepGraph(model, bsz)
 
         def step_fn(model, input_pos, x, q=None, *, mask=None, temperature=1.0, top_k=None):
