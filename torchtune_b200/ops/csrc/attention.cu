@@ -228,8 +228,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int lo_max = (p.lo == nullptr) ? 0 : (p.monotone ? p.lo[row_base + q_last] : p.sk);
     const int hi_min = (p.hi != nullptr) ? (p.monotone ? p.hi[row_base + q0] : -1) : (p.causal ? q0 : p.sk - 1);
     const uint8_t* mrow = (p.kmask != nullptr && row_valid) ? p.kmask + static_cast<long long>(row_base + q_idx) * p.sk : nullptr;
-    const float cap_in = p.softcap > 0.f ? p.scale / p.softcap : 0.f;  // score → tanh argument
-    const float cap_out = p.softcap * kLog2e;                           // tanh → log2-domain logit
+    const float cap_in = p.scale / p.softcap;    // score → tanh argument
+    const float cap_out = p.softcap * kLog2e;    // tanh → log2-domain logit
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int it = 0; it < n_blocks && !*abort_flag; ++it) {
