@@ -33,7 +33,12 @@ class KVCache(nn.Module):
         self.v_cache.zero_()
         self.cache_pos -= self.cache_pos[0].clone()
         if self._level is not None:
-            self._level = 0
+            self.__dict__["_level"] = 0  # nn.Module's own way to set an attribute takes longer than all the rest
+
+    @property
+    def counted(self) -> bool:
+        """Whether somebody up the call keeps count of the appends (or records them)."""
+        return self._level is not None or self.recording
 
     @property
     def size(self) -> int:
@@ -58,7 +63,7 @@ class KVCache(nn.Module):
     def advanced(self, seq_len: int) -> None:
         """Notes that ``cache_pos`` was moved on on the device."""
         if self._level is not None:
-            self._level += seq_len
+            self.__dict__["_level"] += seq_len
 
     def update(self, k_val: torch.Tensor, v_val: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """Append ``[b, s, n_kv, d]`` keys/values and return the full buffers."""
@@ -74,17 +79,17 @@ class KVCache(nn.Module):
 def counted_appends(caches: Sequence[KVCache]) -> Iterator[None]:
     """Asks the device once how many tokens the caches hold and counts their appends on the host until the block is left, for a caller that alone writes
     to them meanwhile: one wait per block instead of one per layer and append."""
-    caches = [c for c in caches if c._level is None and not c.recording]
+    caches = [c for c in caches if not c.counted]
     if len({c.cache_pos.device for c in caches}) > 1:
         caches = []
     if caches:
         for c, level in zip(caches, torch.stack([c.cache_pos[0] for c in caches]).tolist()):
-            c._level = level
+            c.__dict__["_level"] = level
     try:
         yield
     finally:
         for c in caches:
-            c._level = None
+            c.__dict__.pop("_level", None)
 
 
 class RowCache(nn.Module):

@@ -24,10 +24,10 @@ def has_hooks(module: nn.Module) -> bool:
                 or everywhere._global_forward_hooks or everywhere._global_forward_pre_hooks or everywhere._global_backward_hooks or everywhere._global_backward_pre_hooks)
 
 
-_PLAIN_TENSORS = (torch.Tensor, nn.Parameter, type(None))
-
-
 def is_plain_linear(module: nn.Module) -> bool:
     """Whether calling ``module`` is nothing but ``x @ weight.T (+ bias)`` on ordinary tensors: no derived class, no hooks, no parameter in another
     form (a quantised or sharded tensor subclass).  Callers may then take the weight and join the product with what surrounds it."""
-    return type(module) in (nn.Linear, Linear) and not has_hooks(module) and type(module.weight) in _PLAIN_TENSORS and type(module.bias) in _PLAIN_TENSORS
+    if type(module) not in (nn.Linear, Linear) or has_hooks(module):
+        return False
+    own = module._parameters
+    return type(own.get("weight")) is nn.Parameter and type(own.get("bias", module)) in (nn.Parameter, type(None))

@@ -340,11 +340,18 @@ class TransformerDecoder(nn.Module):
         return self.layers[0].caches_are_enabled()
 
     def plain_caches(self) -> List[KVCache]:
-        """The caches that the layers' attention appends to; none without enabled caches."""
+        """The caches that the layers' attention appends to; none without enabled caches or where their appends are counted already."""
         if not self.caches_are_enabled():
             return []
-        attns = [getattr(layer, "attn", None) for layer in self.layers]
-        return [a.kv_cache for a in attns if type(getattr(a, "kv_cache", None)) is KVCache and getattr(a, "cache_enabled", False)]
+        caches = []
+        for layer in self.layers:
+            attn = getattr(layer, "attn", None)
+            cache = getattr(attn, "kv_cache", None)
+            if type(cache) is KVCache and getattr(attn, "cache_enabled", False):
+                if cache.counted and not caches:
+                    return []
+                caches.append(cache)
+        return caches
 
     def reset_caches(self) -> None:
         if not self.caches_are_enabled():
