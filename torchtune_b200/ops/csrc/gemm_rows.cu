@@ -11,7 +11,7 @@
 // writes gate(x · W1ᵀ, x · W3ᵀ).
 // M is limited to 64 because one shared-memory read of a token fragment serves one 16-row tile: beyond about 32 tokens these reads and the
 // products, not the weights, set the pace.
-// us per launch in a graph, weights from HBM, before on the tile kernels -> here: 1 x 2048 x 2048 10.7 -> 4.5, 1 x 4096 x 4096 24.3 -> 9.7,
+// us per launch in a graph, weights from HBM, before on the tile kernels (whole contractions; cut into ranges since, 1 x 4096 x 14336 takes them 27) -> here: 1 x 2048 x 2048 10.7 -> 4.5, 1 x 4096 x 4096 24.3 -> 9.7,
 // 1 x 4096 x 14336 72 -> 23.8 (4.9 TB/s), 16 x 4096 x 14336 53 -> 25.6, 1 x 128256 x 4096 285 -> 181 (5.8 TB/s), 16 x (14336 + 14336) x 4096 gated 88 -> 48.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>

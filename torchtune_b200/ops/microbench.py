@@ -9,6 +9,7 @@
     python -m torchtune_b200.ops.microbench comm --world 8 --numel 268435456             (peer-memory kernels, ranks emulated on one GPU)
     python -m torchtune_b200.ops.microbench latent --heads 16 --rank 512       (latent attention beside grouped-query attention)
     python -m torchtune_b200.ops.microbench ragenex --heads 16 --streams 4     (lightning and span attention, stream steps)
+    python -m torchtune_b200.ops.microbench decode --shapes 4096x4096 6144x4096 --tokens 1 16 32   (few tokens: products, attention, sampling)
     python -m torchtune_b200.ops.microbench suite --tokens 8192      (norm, RoPE, SwiGLU, loss, embedding, LoRA, grouped GEMM, NF4, offload copies)
 
 Each command prints one JSON line: median milliseconds over ``--iters`` launches (an L2 flush
@@ -241,6 +242,55 @@ def bench_latent(args, flush):
             t = _time_captured(lambda i: lambda: linear(xq, wj[i % 8]), it, wj[0].numel() * 2.0)
             emit("linear_joined", t, rows=T, gbs=wj[0].numel() * 2.0 / t / 1e6)
     return {"op": "latent", "heads": H, "kernels": len(rows)}
+
+
+def bench_decode(args, flush):
+    """What a decode step of a plain decoder launches: products of a few tokens on the kernel for them and on the tile kernels, attention of one query per row under
+    a boolean mask, sampling.  Times are of one launch inside a CUDA graph, over inputs larger than L2."""
+    from . import _cuda
+    from ._cuda_attention import attention
+    from .mask import AttentionMask
+
+    bf = dict(device="cuda", dtype=torch.bfloat16)
+    rows = []
+
+    def emit(op, ms, **kw):
+        row = {"op": op, "us": round(ms * 1e3, 2), **{k: (round(v, 1) if isinstance(v, float) else v) for k, v in kw.items()}}
+        rows.append(row)
+        print(json.dumps(row), flush=True)
+
+    def on_tiles(make, nbytes):
+        plain = _cuda._runs_rows
+        _cuda._runs_rows = lambda *sizes: False
+        try:
+            return _time_captured(make, args.iters, nbytes)
+        finally:
+            _cuda._runs_rows = plain
+
+    with torch.no_grad():
+        for shape in args.shapes:
+            n, k = (int(t) for t in shape.split("x"))
+            nbytes = 2.0 * n * k
+            copies = int(max(4, min(64, 400e6 // nbytes + 1)))
+            w = [torch.randn(n, k, **bf) for _ in range(copies)]
+            for m in args.tokens:
+                x, out = torch.randn(m, k, **bf), torch.empty(m, n, **bf)
+                here = _time_captured(lambda i: lambda: _cuda._gemm_rows(x, [w[i % copies]], [out]), args.iters, nbytes) if m <= _cuda.ROWS_LIMIT else float("nan")
+                emit("linear", here, tokens=m, n=n, k=k, gbs=nbytes / here / 1e6, tiles_us=1e3 * on_tiles(lambda i: lambda: _cuda.gemm(x, w[i % copies], out=out), nbytes),
+                     taken="rows" if _cuda._runs_rows(m, n, k) else "tiles")
+            del w
+        for b, keys, d in (map(int, c.split("x")) for c in args.caches):
+            nbytes = 2.0 * 2 * b * keys * 8 * d
+            copies = int(max(4, min(64, 400e6 // nbytes + 1)))
+            kv = [torch.randn(2, b, keys, 8, d, **bf) for _ in range(copies)]
+            q, mask = torch.randn(b, 1, 32, d, **bf), torch.ones(1, 1, keys, dtype=torch.bool, device="cuda")
+            t = _time_captured(lambda i: lambda: attention(q, *kv[i % copies], AttentionMask(causal=False, bool_mask=mask), None, 0.0), args.iters, nbytes)
+            emit("attention of one query", t, rows=b, keys=keys, head_dim=d, gbs=nbytes / t / 1e6)
+            del kv
+        for b in (1, 16):
+            logits, q = torch.randn(b, 128256, device="cuda"), torch.rand(b, 128256, device="cuda") + 1e-3
+            emit("sample, top 300", _time_captured(lambda i: lambda: _cuda.sample(logits, q, 0.6, 300), args.iters, 8.0 * logits.numel()), rows=b, vocabulary=128256)
+    return {"op": "decode", "rows": len(rows)}
 
 
 def bench_ragenex(args, flush):
@@ -655,6 +705,10 @@ def main() -> None:
     la.add_argument("--rank", type=int, default=512)
     la.add_argument("--dim", type=int, default=2048)
     la.add_argument("--seq", type=int, default=8192)
+    de = sub.add_parser("decode")
+    de.add_argument("--shapes", nargs="+", default=["2048x2048", "4096x4096", "2048x8192", "4096x14336", "128256x4096"])
+    de.add_argument("--tokens", nargs="+", type=int, default=[1, 16, 64])
+    de.add_argument("--caches", nargs="*", default=["1x61x64", "16x732x128", "2x8012x128", "64x4096x128"], help="rows x keys x head dim, 32 query and 8 key heads")
     rx = sub.add_parser("ragenex")
     rx.add_argument("--heads", type=int, default=16)
     rx.add_argument("--head-dim", type=int, default=128)
@@ -667,7 +721,7 @@ def main() -> None:
     from ._lib import check_device_errors
 
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
-    fn = {"gemm": bench_gemm, "gemm_fp8": bench_gemm_fp8, "gemm_mxfp8": bench_gemm_mxfp8, "attention": bench_attention, "rmsnorm": bench_rmsnorm, "adamw": bench_adamw, "adamw8bit": bench_adamw8bit, "gate_up": bench_gate_up, "comm": bench_comm, "latent": bench_latent, "ragenex": bench_ragenex, "suite": bench_suite}[args.op]
+    fn = {"gemm": bench_gemm, "gemm_fp8": bench_gemm_fp8, "gemm_mxfp8": bench_gemm_mxfp8, "attention": bench_attention, "rmsnorm": bench_rmsnorm, "adamw": bench_adamw, "adamw8bit": bench_adamw8bit, "gate_up": bench_gate_up, "comm": bench_comm, "decode": bench_decode, "latent": bench_latent, "ragenex": bench_ragenex, "suite": bench_suite}[args.op]
     res = fn(args, flush)
     check_device_errors()
     print(json.dumps(res), flush=True)
