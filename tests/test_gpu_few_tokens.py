@@ -266,3 +266,45 @@ def test_generation_beside_other_threads():
         other.join()
     assert not errors, errors
     check(0)
+
+
+@pytest.mark.parametrize("how", ["inference mode", "checkpointed layers", "compiled projection", "three tokens"])
+def test_generation_of_models_that_are_not_recorded(how):
+    """The plain loop, with caches that live for one call as rollouts have them: the same tokens and logits as with recorded steps."""
+    import copy
+
+    from torchtune_b200 import generation, training
+    from torchtune_b200.models.llama3_1 import llama3_1
+    from torchtune_b200.modules import TransformerSelfAttentionLayer
+    from torchtune_b200.modules.common_utils import delete_kv_caches
+
+    torch.manual_seed(0)
+    with training.set_default_dtype(torch.bfloat16), torch.device("cuda"):
+        model = llama3_1(vocab_size=1024, num_layers=2, num_heads=8, num_kv_heads=2, embed_dim=512, max_seq_len=512, intermediate_dim=1024).eval()
+    other = copy.deepcopy(model)
+    if how == "checkpointed layers":
+        training.set_activation_checkpointing(other, auto_wrap_policy={TransformerSelfAttentionLayer})
+    elif how == "compiled projection":
+        attn = other.layers[0].attn
+        plain, attn.q_proj = attn.q_proj, torch.nn.Linear(512, 512, bias=False, device="cuda", dtype=torch.bfloat16)
+        attn.q_proj.weight = plain.weight
+        attn.q_proj.compile(backend="eager")
+    n = 3 if how == "three tokens" else 9
+    prompt = torch.randint(1, 1024, (3, 20), device="cuda")
+
+    def run(m):
+        with torch.device("cuda"):
+            m.setup_caches(batch_size=3, dtype=torch.bfloat16, decoder_max_seq_len=40)
+        out = generation.generate(m, prompt, max_generated_tokens=n, rng=torch.Generator(device="cuda").manual_seed(1))
+        assert [layer.attn.kv_cache.size for layer in m.layers] == [20 + n - 1] * 2
+        delete_kv_caches(m)
+        return out
+
+    want = run(model)
+    with torch.inference_mode(how == "inference mode"):
+        for _ in range(2):
+            got = run(other)
+            if how == "compiled projection":  # another product in another order: bf16 through two layers, before any draw
+                assert (got[1][:, 0] - want[1][:, 0]).norm() <= 0.03 * want[1][:, 0].norm()
+            else:
+                assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
