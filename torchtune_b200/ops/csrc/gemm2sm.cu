@@ -14,6 +14,10 @@
 // Barriers: `full` lives in the even CTA and counts the bytes of both CTAs' loads; `empty` and `tfull` exist in both
 // CTAs and are signalled by multicast commits; `tempty` lives in the even CTA and collects the eight epilogue warps.
 // Every wait is bounded (error word + abort flag), the two CTAs meet at a cluster barrier before TMEM is released.
+//
+// Large products run at the 1000 W limit, where instructions cost clock: producer and issuer are one elected thread each (no warp-wide loops, descriptors and
+// barrier addresses kept in registers) and waits with slack sleep between looks.  8192 x 4096 x 14336: 39.4 M -> 27.6 M warp instructions; TFLOP/s back to back for
+// a second: 8192 x 128256 x 4096 1303 -> 1345, 16384 x 14336 x 4096 1333 -> 1363, 14336 x 4096 x 8192 (weight gradient) 1250 -> 1259, 8192 x 4096 x 14336 1272 -> 1268.
 #include <cstdlib>
 #include <cstring>
 
@@ -187,29 +191,29 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs) {
-      int m_blk, n_blk;
-      tile_coords(p.tile_mult == 1 ? t : static_cast<int>((static_cast<long long>(t) * p.tile_mult) % num_tiles), num_m, num_n, p.group_m, m_blk, n_blk);
-      const int a_row = m_blk * PM + static_cast<int>(cta) * BM;
-      const int b_row = SWIGLU ? n_blk * (BN / 2) : n_blk * BN + static_cast<int>(cta) * (BN / 2);
-      const CUtensorMap* mapB = (SWIGLU && cta == 1) ? &tmB2 : &tmB;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(&empty[stage], phase ^ 1)) {
-          *abort_flag = 1;
-          if (lane == 0) atomicExch(p.err, 111);
-          break;
-        }
-        if (lane == 0) {
+    if (elect_one()) {
+      const uint32_t full0 = map_to_cta(&full[0], 0);
+      int stage = 0;
+      uint32_t phase = 1;
+      for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs) {
+        int m_blk, n_blk;
+        tile_coords(p.tile_mult == 1 ? t : static_cast<int>((static_cast<long long>(t) * p.tile_mult) % num_tiles), num_m, num_n, p.group_m, m_blk, n_blk);
+        const int a_row = m_blk * PM + static_cast<int>(cta) * BM;
+        const int b_row = SWIGLU ? n_blk * (BN / 2) : n_blk * BN + static_cast<int>(cta) * (BN / 2);
+        const CUtensorMap* mA = &tmA;
+        const CUtensorMap* mB = (SWIGLU && cta == 1) ? &tmB2 : &tmB;
+        int k0 = 0;
+        for (int kb = 0; kb < num_kb; ++kb, k0 += BK) {
+          if (!mbar_wait_idle(&empty[stage], phase, 64)) {
+            *abort_flag = 1;
+            atomicExch(p.err, 111);
+            break;
+          }
+          if (!SWIGLU && kb == num_kb1) mA = &tmA2, mB = &tmB2, k0 = 0;
           uint8_t* sa = smem + stage * kStageBytes;
           uint8_t* sb = sa + kABytes;
           if (cta == 0) mbar_arrive_expect_tx(&full[stage], 2 * kStageBytes);  // the bytes of both CTAs' loads
-          const uint32_t bar = map_to_cta(&full[stage], 0);
-          const bool second = !SWIGLU && kb >= num_kb1;
-          const CUtensorMap* mA = second ? &tmA2 : &tmA;
-          const CUtensorMap* mB = second ? &tmB2 : mapB;
-          const int k0 = (second ? kb - num_kb1 : kb) * BK;
+          const uint32_t bar = full0 + stage * 8;
           if (A_MN) {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, mA, bar, a_row + j * 64, k0);
@@ -222,65 +226,62 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           } else {
             tma_load_2d_pair(sb, mB, bar, k0, b_row);
           }
-        }
-        __syncwarp();
-        if (++stage == kNS) {
-          stage = 0;
-          phase ^= 1;
+          if (++stage == kNS) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1 && cta == 0) {
-    // ------------------------------------------------------------------ MMA issuer (even CTA)
+    // ------------------------------------------------------------------ MMA issuer (one thread of the even CTA)
     constexpr uint32_t idesc = make_idesc_bf16(PM, BN, A_MN, B_MN);
-    int stage = 0;
-    uint32_t phase = 0;
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs) {
-      if (!mbar_wait(&tempty[acc], acc_phase ^ 1)) {
-        *abort_flag = 1;
-        if (lane == 0) atomicExch(p.err, 112);
-        break;
-      }
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + acc * BN;
-      bool ok = true;
-      for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(&full[stage], phase)) {
-          ok = false;
+    if (elect_one()) {
+      const uint64_t desc_a = A_MN ? make_smem_desc_sw128(smem_u32(smem), 8192, 1024) : make_smem_desc_sw128(smem_u32(smem), 16, 1024);
+      const uint64_t desc_b = B_MN ? make_smem_desc_sw128(smem_u32(smem) + kABytes, 8192, 1024) : make_smem_desc_sw128(smem_u32(smem) + kABytes, 16, 1024);
+      int stage = 0;
+      uint32_t phase = 0;
+      int acc = 0;
+      uint32_t acc_phase = 1;
+      for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs) {
+        if (!mbar_wait(&tempty[acc], acc_phase)) {
+          *abort_flag = 1;
+          atomicExch(p.err, 112);
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t sa = smem_u32(smem + stage * kStageBytes);
-          const uint32_t sb = sa + kABytes;
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t da = A_MN ? make_smem_desc_sw128(sa + k * 2048, 8192, 1024) : make_smem_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(sb + k * 2048, 8192, 1024) : make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            umma_f16_pair(d_tmem, da, db, idesc, (kb | k) != 0);
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        bool ok = true;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(&full[stage], phase)) {
+            ok = false;
+            break;
           }
+          tc_fence_after();
+          const uint64_t at = static_cast<uint64_t>(stage * (kStageBytes >> 4));  // descriptors count 16-byte units; the address field does not overflow
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_f16_pair(d_tmem, desc_a + at + k * ((A_MN ? 2048 : 32) >> 4), desc_b + at + k * ((B_MN ? 2048 : 32) >> 4), idesc, (kb | k) != 0);
           umma_commit_pair(&empty[stage]);  // both CTAs' producers may refill the stage once these MMAs retire
+          if (++stage == kNS) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
-        __syncwarp();
-        if (++stage == kNS) {
-          stage = 0;
-          phase ^= 1;
+        if (!ok) {
+          *abort_flag = 1;
+          atomicExch(p.err, 113);
+          break;
         }
-      }
-      if (!ok) {
-        *abort_flag = 1;
-        if (lane == 0) atomicExch(p.err, 113);
-        break;
-      }
-      if (lane == 0) umma_commit_pair(&tfull[acc]);
-      __syncwarp();
-      if (++acc == 2) {
-        acc = 0;
-        acc_phase ^= 1;
+        umma_commit_pair(&tfull[acc]);
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
       }
     }
+    __syncwarp();
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ epilogue (both CTAs, own 128 rows)
     const int quarter = warp & 3;
@@ -291,7 +292,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int t = pair; t < num_tiles && !*abort_flag; t += num_pairs) {
       int m_blk, n_blk;
       tile_coords(p.tile_mult == 1 ? t : static_cast<int>((static_cast<long long>(t) * p.tile_mult) % num_tiles), num_m, num_n, p.group_m, m_blk, n_blk);
-      if (!mbar_wait(&tfull[acc], acc_phase)) {
+      if (!mbar_wait_idle(&tfull[acc], acc_phase, 256)) {
         *abort_flag = 1;
         if (lane == 0) atomicExch(p.err, 114);
         break;
