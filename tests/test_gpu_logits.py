@@ -55,6 +55,21 @@ def test_widened_logits(n):
     assert got.dtype == torch.float32 and torch.equal(got.view(torch.int32)[:, 1:], x.float().view(torch.int32)[:, 1:]) and got[0, 0].isnan()
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 64), (16, 9992, 4096), (17, 128256, 2048), (300, 19208, 136), (1031, 4136, 1024), (333, 520, 4096), (100, 24, 64), (0, 64, 64)])
+def test_widened_projection(M, N, K, bias):
+    """Kernel for few tokens, CTA pairs with ragged last tiles, sizes that are widened afterwards: the values of the bf16 projection in every case."""
+    from torchtune_b200 import ops
+
+    x, w = _logits(M, K, torch.bfloat16, 1) * 0.1, _logits(N, K, torch.bfloat16, 2)
+    b = _logits(1, N, torch.bfloat16, 3)[0] if bias else None
+    with torch.no_grad():
+        got, want = ops.linear_widened(x, w, b), ops.linear(x, w, b).float()
+    assert got.dtype == torch.float32 and torch.equal(got, want)
+    w.requires_grad_()
+    assert ops.linear_widened(x, w, b).requires_grad
+
+
 def test_loss_gradients_of_batched_and_differentiated_factors():
     from torchtune_b200 import ops
 

@@ -13,6 +13,7 @@ from .attention import MaskLike, MultiHeadAttention
 from .cached_mixer import CachedMixer
 from .hyper_connections import HyperConnection, LayerScale, StreamEntry
 from .kv_cache import KVCache, counted_appends
+from .linear import Linear, is_plain_linear
 from .rms_norm import StreamLayerNorm, StreamRMSNorm
 
 
@@ -452,6 +453,8 @@ class TransformerDecoder(nn.Module):
     def unembed_normed(self, h: torch.Tensor) -> torch.Tensor:
         if self.wide_logits and type(self.output).__name__ == "Linear" and self.output.bias is None:
             return self._cap(ops.linear_wide(h, self.output.weight))
+        if type(self.output) is Linear and is_plain_linear(self.output):
+            return self._cap(ops.linear_widened(h, self.output.weight, self.output.bias))
         return self._cap(ops.widen(self.output(h)))
 
     def unembed(self, h: torch.Tensor) -> torch.Tensor:

@@ -32,6 +32,7 @@ __all__ = [
     "linear_group",
     "linear_residual",
     "linear_wide",
+    "linear_widened",
     "residual_norm",
     "stream_step",
     "embed_positions",
@@ -149,6 +150,17 @@ def linear_wide(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         y = _cuda.gemm(x.reshape(-1, x.shape[-1]), weight, out_dtype=torch.float32)
         return y[:, :n].reshape(*x.shape[:-1], n)
     return linear(x, weight).float()
+
+
+def linear_widened(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``widen(linear(x, weight, bias))``, value for value; bf16 CUDA inputs outside autograd without a pass over the result."""
+    if _native(x) and weight.dtype == torch.bfloat16 and not _differentiated(x, weight, bias) and _has_memory(x, weight, *(() if bias is None else (bias,))):
+        from . import _cuda
+
+        y = _cuda.linear_widened(x, weight, bias)
+        if y is not None:
+            return y
+    return widen(linear(x, weight, bias))
 
 
 def widen(x: torch.Tensor) -> torch.Tensor:

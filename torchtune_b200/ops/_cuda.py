@@ -30,11 +30,15 @@ def _use_pair_kernel(M: int, N: int, K: int, out: torch.Tensor) -> bool:
     at least one 256 × 256 tile per SM pair; smaller ones keep 128-row tiles, which spread over more SMs, unless the contraction is so long that the
     pairs' faster products outweigh half of the SMs (us with 128-row tiles / with pairs: 1024 x 4096 x 4096 25.3 / 27.4, x 14336 92.6 / 86.7, and
     666 x 4096 x 14336 86.6 / 74.3)."""
+    return out.dtype == _BF16 and _fills_pairs(M, N, K, out.device)
+
+
+def _fills_pairs(M: int, N: int, K: int, device: torch.device) -> bool:
     global _SM_PAIRS
-    if not _PAIR_KERNEL or out.dtype != _BF16:
+    if not _PAIR_KERNEL:
         return False
     if _SM_PAIRS is None:
-        _SM_PAIRS = max(1, torch.cuda.get_device_properties(out.device).multi_processor_count // 2)
+        _SM_PAIRS = max(1, torch.cuda.get_device_properties(device).multi_processor_count // 2)
     tiles = (-(-M // 256)) * (-(-N // 256))
     return K >= 128 and (tiles >= _SM_PAIRS or (K >= 8192 and 2 * tiles > _SM_PAIRS and M > 128 and N > 128))
 
@@ -54,14 +58,15 @@ def _runs_rows(M: int, N: int, K: int) -> bool:
 
 
 def _gemm_rows(x: torch.Tensor, weights: Sequence[torch.Tensor], outs: Sequence[torch.Tensor], biases: Optional[Sequence[Optional[torch.Tensor]]] = None,
-               residual: Optional[torch.Tensor] = None, alpha: float = 1.0) -> None:
-    """``outs[i] = alpha · x · weights[i]ᵀ (+ biases[i]) (+ residual)`` for up to :data:`ROWS_LIMIT` tokens and three weights; rows 16-byte aligned."""
+               residual: Optional[torch.Tensor] = None, alpha: float = 1.0, rounded: bool = False) -> None:
+    """``outs[i] = alpha · x · weights[i]ᵀ (+ biases[i]) (+ residual)`` for up to :data:`ROWS_LIMIT` tokens and three weights; rows 16-byte aligned.  ``rounded``: fp32 outputs
+    hold the bf16 values."""
     n = len(weights)
     vps, lls = ctypes.c_void_p * n, ctypes.c_longlong * n
     rc = lib().ttb_gemm_rows(x.data_ptr(), x.stride(0), x.shape[0], x.shape[1], n, vps(*[w.data_ptr() for w in weights]), lls(*[w.stride(0) for w in weights]),
                              (ctypes.c_int * n)(*[w.shape[0] for w in weights]), vps(*[o.data_ptr() for o in outs]), lls(*[o.stride(0) for o in outs]),
                              None if biases is None else vps(*[_ptr(b) for b in biases]), _ptr(residual), 0 if residual is None else residual.stride(0),
-                             int(outs[0].dtype == torch.float32), float(alpha), stream_ptr())
+                             (1 + int(rounded)) * int(outs[0].dtype == torch.float32), float(alpha), stream_ptr())
     check(rc, f"gemm of few rows M={x.shape[0]} K={x.shape[1]}")
 
 
@@ -81,6 +86,30 @@ def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Seque
     outs = [torch.empty(M, w.shape[0], dtype=_BF16, device=x.device) for w in weights]
     _gemm_rows(x2, weights, outs, None if all(b is None for b in biases) else biases)
     return [o.view(*x.shape[:-1], o.shape[1]) for o in outs]
+
+
+def linear_widened(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """``float(bf16(x · weightᵀ (+ bias)))`` in one launch, outside autograd; ``None`` where neither the kernel for few tokens nor the one on CTA pairs takes the product
+    (then the result is widened by a pass of its own)."""
+    K = x.shape[-1]
+    M, N = x.numel() // K if K else 0, weight.shape[0]
+    if not M or not N or K % 8 or N % 8 or weight.shape[1] != K or weight.stride(1) != 1 or weight.stride(0) % 8 or weight.data_ptr() % 16:
+        return None
+    if bias is not None and (bias.dtype != _BF16 or bias.shape != (N,) or not bias.is_contiguous()):
+        return None
+    rows = _runs_rows(M, N, K)
+    if not rows and (_splits(M, N, K) > 1 or not _fills_pairs(M, N, K, x.device)):
+        return None
+    x2 = x.reshape(M, K)
+    if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+        x2 = x2.contiguous()
+    out = torch.empty(M, N, dtype=torch.float32, device=x.device)
+    if rows:
+        _gemm_rows(x2, [weight], [out], None if bias is None else [bias], rounded=True)
+    else:
+        check(lib().ttb_gemm_bf16_2sm_widened(x2.data_ptr(), weight.data_ptr(), out.data_ptr(), M, N, K, x2.stride(0), weight.stride(0), N, _ptr(bias), err_word(x.device).data_ptr(),
+                                              stream_ptr()), f"gemm (CTA pairs, widened) M={M} N={N} K={K}")
+    return out.view(*x.shape[:-1], N)
 
 
 def _check_contraction(K: int, Kb: int) -> None:

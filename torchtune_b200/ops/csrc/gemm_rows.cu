@@ -36,7 +36,7 @@ static constexpr int kPartPitch = 20;  // floats per token of a warp's 16 partia
 
 struct Segment {
   const __nv_bfloat16* w;
-  void* y;                    // [M, n] bf16, or fp32 with out_f32
+  void* y;                    // [M, n] bf16, or fp32 with out_f32 (2: rounded to bf16 first)
   const __nv_bfloat16* bias;  // [n] or nullptr
   long long ldw, ldy;
   int n, first_tile;
@@ -218,7 +218,7 @@ gemm_rows_kernel(const __grid_constant__ Params p, int splits) {
       if (p.residual != nullptr) v += __bfloat162float(p.residual[token * p.ldr + row]);
     }
     if (p.out_f32)
-      static_cast<float*>(sg.y)[token * sg.ldy + row] = v;
+      static_cast<float*>(sg.y)[token * sg.ldy + row] = p.out_f32 == 2 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
     else
       static_cast<__nv_bfloat16*>(sg.y)[token * sg.ldy + row] = __float2bfloat16_rn(v);
   }
@@ -290,7 +290,7 @@ static bool unaligned(const void* t, long long ld) { return (reinterpret_cast<ui
 }  // namespace ttb
 
 // Y_i[M, n_i] = alpha * X[M, K] · W_i[n_i, K]ᵀ (+ bias_i) (+ residual, first weight only) for up to three weights of one input, M <= 64, K a
-// multiple of 8, X and W rows 16-byte aligned.  bf16, or fp32 results with out_f32.
+// multiple of 8, X and W rows 16-byte aligned.  bf16 results; fp32 with out_f32 = 1, the bf16 ones widened with 2.
 extern "C" int ttb_gemm_rows(const void* x, long long ldx, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y, const long long* ldy,
                              const void* const* bias, const void* residual, long long ldr, int out_f32, float alpha, void* stream) {
   using namespace ttb;
