@@ -1,0 +1,85 @@
+"""All layers of a decoder issued by one native call: bit for bit what the modules give."""
+import pytest
+import torch
+from torch import nn
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(layers, dim, heads, kv, hidden, vocab, rows, slots, bias=False):
+    from torchtune_b200 import training
+    from torchtune_b200.models.llama3_1 import llama3_1
+    from torchtune_b200.modules.linear import Linear
+
+    torch.manual_seed(dim + hidden)
+    with training.set_default_dtype(torch.bfloat16), torch.device("cuda"):
+        model = llama3_1(vocab_size=vocab, num_layers=layers, num_heads=heads, num_kv_heads=kv, embed_dim=dim, max_seq_len=8192, intermediate_dim=hidden).eval()
+        if bias:
+            for layer in model.layers:
+                for name in ("q_proj", "k_proj", "v_proj"):
+                    old = getattr(layer.attn, name)
+                    setattr(layer.attn, name, Linear(old.in_features, old.out_features, bias=True))
+        model.setup_caches(batch_size=rows, dtype=torch.bfloat16, decoder_max_seq_len=slots)
+    return model
+
+
+SHAPES = [  # layers, dim, heads, key heads, hidden, rows, slots, tokens
+    (2, 512, 8, 2, 1024, 3, 60, 1),  # kernels for few tokens
+    (2, 2048, 32, 8, 8192, 1, 61, 37),  # gate and up projection apart, the rest for few tokens
+    (1, 1024, 8, 8, 4096, 2, 300, 4),  # several queries on the kernel for few queries
+    (1, 1024, 8, 8, 4096, 2, 300, 200),  # contraction in ranges, residual by itself
+    (1, 4096, 32, 8, 14336, 1, 700, 640),  # CTA pairs, alone and with ranges
+    (1, 2048, 32, 8, 8192, 3, 1100, 1030),  # CTA pairs throughout, ragged
+    (1, 192, 3, 3, 264, 5, 40, 33),
+]
+
+
+@pytest.mark.parametrize("padded,bias", [(False, False), (True, True)])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+@torch.no_grad()
+def test_results_and_caches_are_those_of_the_modules(shape, padded, bias):
+    from torchtune_b200 import generation
+    from torchtune_b200.generation._native_layers import NativeLayers
+    from torchtune_b200.generation._rows import hidden_states
+
+    layers, dim, heads, kv, hidden, rows, slots, n = shape
+    model = _model(layers, dim, heads, kv, hidden, 1024, rows, slots, bias)
+    native = NativeLayers.of(model, rows)
+    assert native is not None
+    x = torch.randint(1, 1024, (rows, n), device="cuda")
+    if padded:
+        real = torch.ones(rows, n, dtype=torch.bool, device="cuda")
+        for r in range(1, rows):
+            real[r, : min(n - 1, 3 * r)] = False
+        mask, pos = generation.get_causal_mask_from_padding_mask(real, target_seq_len=slots), generation.get_position_ids_from_padding_mask(real)
+    else:
+        mask, pos = torch.tril(torch.ones(n + 2, slots, dtype=torch.bool, device="cuda")).unsqueeze(0)[:, :n], torch.arange(n, device="cuda")
+    got = native(x, pos, mask)
+    caches = [(l.attn.kv_cache.k_cache.clone(), l.attn.kv_cache.v_cache.clone(), l.attn.kv_cache.cache_pos.clone()) for l in model.layers]
+    model.reset_caches()
+    want = hidden_states(model, x, input_pos=pos, mask=mask)
+    assert torch.equal(got, want)
+    for l, (k, v, at) in zip(model.layers, caches):
+        assert torch.equal(l.attn.kv_cache.k_cache, k) and torch.equal(l.attn.kv_cache.v_cache, v) and torch.equal(l.attn.kv_cache.cache_pos, at)
+    with pytest.raises(AssertionError, match="full"):
+        native(x.repeat(1, slots // n)[:, :slots], torch.arange(slots // n * n, device="cuda"), torch.ones(1, slots // n * n, slots, dtype=torch.bool, device="cuda"))
+
+
+@torch.no_grad()
+def test_what_the_call_does_not_do_is_left_to_the_modules():
+    from torchtune_b200.generation._native_layers import NativeLayers
+
+    for change in (lambda m: setattr(m.layers[1].mlp_norm, "eps", 1e-6), lambda m: setattr(m.layers[0].attn, "softcap", 50.0), lambda m: setattr(m.layers[1].mlp, "activation", nn.GELU()),
+                   lambda m: setattr(m.layers[0].attn, "q_proj", nn.Linear(512, 512, bias=False, dtype=torch.bfloat16, device="cuda")), lambda m: setattr(m.layers[0].attn, "scale", -1.0),
+                   lambda m: m.layers[1].attn.q_proj.register_forward_hook(lambda *a: None), lambda m: setattr(m.layers[0], "sa_scale", nn.Tanh()), lambda m: setattr(m.layers[0].mlp, "w3", None),
+                   lambda m: setattr(m.layers[1].attn.kv_cache, "k_cache", m.layers[1].attn.kv_cache.k_cache.float()), lambda m: setattr(m.layers[1].attn.pos_embeddings, "interleaved", False)):
+        model = _model(2, 512, 8, 2, 1024, 1024, 4, 60)
+        assert NativeLayers.of(model, 4) is not None and NativeLayers.of(model, 5) is None
+        model.layers[0].attn.pos_embeddings = type(model.layers[0].attn.pos_embeddings)(dim=64, max_seq_len=8192).to("cuda")  # layers share one module
+        change(model)
+        assert NativeLayers.of(model, 4) is None
+    model = _model(2, 512, 8, 2, 1024, 1024, 4, 60)
+    native = NativeLayers.of(model, 4)
+    x, pos, mask = torch.ones(4, 2, dtype=torch.int64, device="cuda"), torch.arange(2, device="cuda"), torch.ones(1, 2, 60, dtype=torch.bool, device="cuda")
+    assert native(x[:3], pos, mask) is None and native(x, pos, mask[:, :, :59]) is None and native(x, pos, mask.float()) is None
+    assert int(model.layers[0].attn.kv_cache.cache_pos[0]) == 0 and native(x, pos, mask) is not None

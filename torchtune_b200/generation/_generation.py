@@ -9,6 +9,7 @@ from ..modules import TransformerDecoder
 from ..modules.attention import MaskLike
 from ..modules.kv_cache import counted_appends
 from ._rows import DecodeGraph, RowLayout, hidden_states
+from ._native_layers import NativeLayers
 from ._step_graph import StepGraph
 
 
@@ -141,7 +142,12 @@ def _generate(model, prompt, max_generated_tokens, pad_id, temperature, top_k, s
     else:
         first_mask = masks[:, :prompt_len] if incremental else masks[:, :prompt_len, :prompt_len]
         first_pos = input_pos[:, :prompt_len].squeeze()
-    tokens, logits = generate_next_token(model, input_pos=first_pos, mask=first_mask, x=prompt, temperature=temperature, top_k=top_k, q=draw_q())
+    native = NativeLayers.of(model, bsz) if recorded else None
+    logits = None if native is None else native.last_logits(prompt, first_pos, first_mask)
+    if logits is None:
+        tokens, logits = generate_next_token(model, input_pos=first_pos, mask=first_mask, x=prompt, temperature=temperature, top_k=top_k, q=draw_q())
+    else:
+        tokens, logits = sample(logits, temperature=temperature, top_k=top_k, q=draw_q()), logits.unsqueeze(1)
     out_tokens = torch.cat([prompt, tokens], dim=-1)
     logit_steps = [logits] if return_logits else None  # joined once at the end: joining every step copies the whole history each time
     pos = prompt_len
@@ -170,7 +176,7 @@ def _generate(model, prompt, max_generated_tokens, pad_id, temperature, top_k, s
             return sample(logits, temperature=temperature, top_k=top_k, q=q), logits.unsqueeze(1)
 
     elif recorded:
-        graph_step = StepGraph(model, bsz)
+        graph_step = StepGraph(model, bsz, native)
 
         def step_fn(model, input_pos, x, q=None, *, mask=None, temperature=1.0, top_k=None):
             logits = graph_step(x, input_pos, mask)

@@ -15,6 +15,7 @@ from ..modules import FeedForward, KVCache, MultiHeadAttention, RMSNorm, Transfo
 from ..modules.linear import Linear, has_hooks
 from ..modules.position_embeddings import RotaryPositionalEmbeddings
 from ..modules.tied_linear import TiedLinear
+from ._native_layers import NativeLayers
 
 # Modules whose forward pass of one token is the same sequence of launches in every step and needs no look at the device.
 _PLAIN = (TransformerDecoder, TransformerSelfAttentionLayer, MultiHeadAttention, FeedForward, KVCache, RMSNorm, Linear, nn.Linear, nn.Embedding, nn.ModuleList, nn.Identity,
@@ -77,8 +78,8 @@ class StepGraph:
                 return False
         return all(p.device == like.device and p.dtype == torch.bfloat16 for p in model.parameters())
 
-    def __init__(self, model: TransformerDecoder, batch: int) -> None:
-        self.model, self.batch = model, batch
+    def __init__(self, model: TransformerDecoder, batch: int, native: Optional[NativeLayers] = None) -> None:
+        self.model, self.batch, self.native = model, batch, native
         self.caches = [layer.attn.kv_cache for layer in model.layers]
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.home: _LastGraph = self.caches[0].__dict__.setdefault("last_graph", _LastGraph())
@@ -87,7 +88,7 @@ class StepGraph:
         if self.graph is None:
             sizes = (self.batch, *mask.shape)
             if sizes not in self.home.stepped or not _alone():
-                logits = self.model(x, input_pos=input_pos, mask=mask)[:, -1]
+                logits = self._step(x, input_pos, mask)
                 self.home.stepped.add(sizes)
                 return logits
             self._record(x, input_pos, mask)
@@ -100,6 +101,10 @@ class StepGraph:
         for cache in self.caches:
             cache.advanced(1)
         return self.logits.clone()
+
+    def _step(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
+        logits = None if self.native is None else self.native.last_logits(x, input_pos, mask)
+        return self.model(x, input_pos=input_pos, mask=mask)[:, -1] if logits is None else logits
 
     def _record(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> None:
         device = x.device
@@ -117,7 +122,7 @@ class StepGraph:
             with torch.cuda.stream(stream):
                 graph.capture_begin(**({} if self.home.graph is None else {"pool": self.home.graph.pool()}), capture_error_mode="thread_local")
                 try:
-                    self.logits = self.model(self.x, input_pos=self.pos, mask=self.mask)[:, -1]
+                    self.logits = self._step(self.x, self.pos, self.mask)
                     torch._foreach_add_([cache.cache_pos for cache in self.caches], 1)
                 finally:
                     graph.capture_end()

@@ -94,6 +94,10 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_gemm_bf16_dual_2sm.restype = i32
     L.ttb_gemm_bf16_2sm_residual.argtypes = [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i64, vp, vp, vp]
     L.ttb_gemm_bf16_2sm_residual.restype = i32
+    L.ttb_decoder_layers_workspace.argtypes = [i32] * 9
+    L.ttb_decoder_layers_workspace.restype = i64
+    L.ttb_decoder_layers.argtypes = [vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32, i32, vp, vp, vp, vp, vp, i64, i64, vp, vp, vp]
+    L.ttb_decoder_layers.restype = i32
     L.ttb_gemm_bf16_2sm_widened.argtypes = [vp, vp, vp, i32, i32, i32, i64, i64, i64, vp, vp, vp]
     L.ttb_gemm_bf16_2sm_widened.restype = i32
     L.ttb_gemm_bf16_splitk.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, i64, i64, i64, i32, i32, vp, vp, i64, i32, f32, vp, vp]
@@ -169,8 +173,9 @@ def stream_ptr() -> int:
     """Handle of torch's current stream.  Also binds the calling thread (autograd workers
     included) to torch's current device inside the kernel library, whose CUDA runtime keeps
     its own per-thread device state."""
-    lib().ttb_ensure_device(torch.cuda.current_device())
-    return torch.cuda.current_stream().cuda_stream
+    device = torch.cuda.current_device()  # also initialises CUDA in the first call of a program
+    lib().ttb_ensure_device(device)
+    return torch._C._cuda_getCurrentRawStream(device)  # without the Python object around it, which takes longer to make than a launch does
 
 
 def err_word(device: torch.device) -> torch.Tensor:
