@@ -84,3 +84,38 @@ def test_loss_gradients_of_batched_and_differentiated_factors():
     assert torch.equal(g, 2 * once[0])
     d, = torch.autograd.grad(g.float().sum(), factor)
     assert (d - once[0].float().sum()).abs() <= 2.0**-8 * once[0].float().abs().sum()
+
+
+@pytest.mark.parametrize("T,D,V", [(1, 128, 128256), (257, 192, 9608), (700, 2048, 20000), (300, 1024, 128256), (4097, 64 * 3, 8448)])
+def test_softmax_statistics_of_the_logits_product(T, D, V):
+    """Losses and gradients where the product that makes the logits leaves the statistics of their softmax, against 64 bits on the same bf16 logits: ragged tiles, labels at both ends, ignored
+    rows and ids out of range, rows with one dominant logit."""
+    from torchtune_b200 import ops
+    from torchtune_b200.ops._cuda import _ce_stats
+    from torchtune_b200.ops._lib import index_violations
+
+    h, w = (_logits(T, D, torch.bfloat16, 1) * 0.25).requires_grad_(), (_logits(V, D, torch.bfloat16, 2) * 0.25 * D**-0.5).requires_grad_()
+    with torch.no_grad():
+        h[T // 2] *= 40
+    labels = torch.randint(0, V, (T,), device="cuda")
+    labels[-1], labels[0] = V - 1, 0
+    if T > 1:
+        labels[::5], labels[3::50] = -100, V + 3
+    with torch.no_grad():
+        logits = ops.linear(h, w)
+        assert _ce_stats(h, w, logits, 0.0) == (T > 16) and not _ce_stats(h, w, logits, 30.0)
+    index_violations()
+    total, count = ops.linear_cross_entropy(h, w, labels)
+    total.backward()
+    seen = (labels >= 0) & (labels < V)
+    assert int(count) == int((labels != -100).sum()) and index_violations() == int((labels >= V).sum())
+    z = logits.double()
+    lse = torch.logsumexp(z, -1)
+    want = torch.where(seen, lse - z.gather(1, labels.clamp(0, V - 1)[:, None])[:, 0], 0.0)
+    # fp32 sums of V terms (partials of 256 added pairwise) and one logarithm of a sum
+    assert abs(float(total) - float(want.sum())) <= 2.0**-19 * float((lse.abs() * seen).sum() + want.abs().sum()) + 1e-6
+    p = torch.softmax(z, -1)
+    p[torch.arange(T, device="cuda"), labels.clamp(0, V - 1)] -= 1
+    p *= seen[:, None]
+    for got, exact in ((h.grad, p @ w.double()), (w.grad, p.t() @ h.double())):
+        assert float((got.double() - exact).norm()) <= 2.0**-7 * float(exact.norm())  # p and the result are rounded to bf16

@@ -1350,6 +1350,14 @@ def _scaled(t: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
 _CE_SINGLE_PASS_BYTES = 6 * 2**30
 
 
+def _ce_stats(h: torch.Tensor, weight: torch.Tensor, logits: torch.Tensor, softcap: float) -> bool:
+    """Whether the product that makes these logits leaves the statistics of their softmax behind: the CTA-pair kernel does, unless the softmax runs over capped ones."""
+    (M, K), N = h.shape, weight.shape[0]
+    if softcap > 0.0 or K % 8 or weight.shape[1] != K or any(t.stride(1) != 1 or t.stride(0) % 8 or t.data_ptr() % 16 for t in (h, weight, logits)):
+        return False
+    return not _runs_rows(M, N, K) and _splits(M, N, K) == 1 and _fills_pairs(M, N, K, h.device)
+
+
 class _LinearCE(torch.autograd.Function):
     """Loss and both gradients in one forward sweep: logits = H·Wᵀ (bf16, as the unfused bf16
     projection produces), softmax-CE turns them into dlogits in place, then dH = dlogits·W and
@@ -1383,13 +1391,16 @@ class _LinearCE(torch.autograd.Function):
             n = min(rows, T - start)
             hc = h2[start : start + n]
             lg = buf[:n]
-            gemm(hc, weight, out=lg)
             mode = 0 if (need_h or need_w) else 1
-            if softcap > 0.0:  # Gemma-2: softmax over cap·tanh(logit/cap); the kernel writes the gradient w.r.t. the raw logit
-                check(L.ttb_softmax_ce_capped(lg.data_ptr(), y[start : start + n].data_ptr(), loss_rows[start : start + n].data_ptr(), None, n, V, lg.stride(0), int(ignore_index), mode,
-                                              float(softcap), stream_ptr()), "softmax_ce_capped")
+            if _ce_stats(hc, weight, lg, softcap):
+                stats, lse = torch.empty(-(-V // 256), n, 2, dtype=torch.float32, device=h2.device), torch.empty(n, dtype=torch.float32, device=h2.device)
+                check(L.ttb_gemm_bf16_2sm_stats(hc.data_ptr(), weight.data_ptr(), lg.data_ptr(), stats.data_ptr(), n, V, D, hc.stride(0), weight.stride(0), lg.stride(0),
+                                                err_word(h2.device).data_ptr(), stream_ptr()), f"logits and their statistics T={n} V={V} D={D}")
+                check(L.ttb_softmax_ce_stats(lg.data_ptr(), stats.data_ptr(), y[start : start + n].data_ptr(), loss_rows[start : start + n].data_ptr(), lse.data_ptr(), n, V, lg.stride(0),
+                                             int(ignore_index), 1 - mode, None, stream_ptr()), "softmax_ce_stats")
             else:
-                check(L.ttb_softmax_ce(lg.data_ptr(), y[start : start + n].data_ptr(), loss_rows[start : start + n].data_ptr(), None, n, V, lg.stride(0), int(ignore_index), mode, stream_ptr()), "softmax_ce")
+                gemm(hc, weight, out=lg)
+                _softmax_ce(lg, y[start : start + n], loss_rows[start : start + n], None, n, V, ignore_index, mode, softcap)
             if need_h:
                 gemm(lg, weight, b_mn=True, out=dh[start : start + n])
             if direct:

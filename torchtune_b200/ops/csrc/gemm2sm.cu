@@ -32,6 +32,7 @@ static constexpr int PM = 256;   // rows per CTA pair
 static constexpr int BN = 256;   // columns per pair tile (each CTA loads 128 of them)
 static constexpr int BK = 64;
 static constexpr int kThreads = 256;
+static constexpr float kLog2e = 1.4426950408889634f;
 static constexpr int kGroupM = 16;  // default number of pair-tiles in m per scheduling group (L2 reuse of the B panel)
 static constexpr int kABytes = BM * BK * 2;
 static constexpr int kBBytes = (BN / 2) * BK * 2;
@@ -58,6 +59,7 @@ struct Params {
   long long ldr;
   float alpha;
   int accumulate;
+  float2* stats;  // [n tiles, M]: maximum of a row's results in a tile and the sum of their exponentials relative to it (as stored, in bf16), or null
   int out_f32;  // C is fp32 and holds the results rounded to bf16 (vocabulary logits that callers want widened)
   int tma_store;
   int group_m;  // pair-tiles in m per scheduling group
@@ -136,6 +138,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmU,
                const __grid_constant__ CUtensorMap tmA2, Params p) {
   constexpr bool SWIGLU = GLU != kNoGate;
+  constexpr bool kStats = !A_MN && !B_MN && !SWIGLU;  // the form of a linear layer's forward pass
   constexpr int kNS = SWIGLU ? kStagesSwiglu : kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -391,6 +394,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           ++buf_toggle;
         }
       } else if (p.tma_store) {
+        float row_max = -INFINITY, row_sum = 0.f;
 #pragma unroll 1
         for (int c = 0; c < BN / 64; ++c) {
           const int col0 = n_blk * BN + c * 64;
@@ -433,6 +437,24 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               o.w = pack_bf16x2(f[6], f[7]);
               const int chunk = (h * 4 + j) ^ (lane & 7);
               *reinterpret_cast<uint4*>(buf + lane * 128 + chunk * 16) = o;
+              if (kStats) r[j * 4] = o.x, r[j * 4 + 1] = o.y, r[j * 4 + 2] = o.z, r[j * 4 + 3] = o.w;
+            }
+            if (kStats && p.stats != nullptr) {  // one row per thread: its 32 columns join the running maximum and sum
+              const int valid = min(4, (p.N - col0 - h * 32) / 8);
+              float mx = row_max;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r[i]));
+                if (i < valid * 4) mx = fmaxf(mx, fmaxf(t.x, t.y));
+              }
+              const float base = mx == -INFINITY ? 0.f : mx * kLog2e;
+              float sum = row_sum * fast_exp2(row_max * kLog2e - base);  // 0 before the first column: 0 * 2^-inf
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r[i]));
+                if (i < valid * 4) sum += fast_exp2(fmaf(t.x, kLog2e, -base)) + fast_exp2(fmaf(t.y, kLog2e, -base));
+              }
+              row_max = mx, row_sum = sum;
             }
           }
           fence_proxy_async_smem();
@@ -443,6 +465,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           ++buf_toggle;
         }
+        if (kStats && p.stats != nullptr && row < p.M) p.stats[static_cast<long long>(n_blk) * p.M + row] = make_float2(row_max, row_sum);
       } else {
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -697,6 +720,19 @@ extern "C" int ttb_gemm_bf16_2sm_widened(const void* A, const void* B, float* C,
   g2::Params p{};
   p.M = M, p.N = N, p.K = K, p.C = C, p.ldc = ldc, p.bias = static_cast<const __nv_bfloat16*>(bias), p.alpha = 1.f;
   p.out_f32 = 1, p.tile_mult = 1, p.err = err;
+  p.group_m = g2::group_setting();
+  return g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
+}
+
+// Logits C[M,N] = A[M,K] · B[N,K]ᵀ in bf16 and, per row and tile of 256 columns, the maximum and the sum of exponentials of what was stored: stats[ceil(N / 256), M].  The
+// softmax over them needs no pass of its own over the logits.  C 16-byte aligned.
+extern "C" int ttb_gemm_bf16_2sm_stats(const void* A, const void* B, void* C, float* stats, int M, int N, int K, long long lda, long long ldb, long long ldc, int* err, void* stream) {
+  using namespace ttb;
+  if (M <= 0 || N <= 0 || K <= 0 || stats == nullptr || (reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(stats) & 7)) return kErrBadShape;
+  if ((lda & 7) || (ldb & 7) || (ldc & 7) || (N & 7) || (K & 7)) return kErrBadShape;
+  g2::Params p{};
+  p.M = M, p.N = N, p.K = K, p.C = C, p.ldc = ldc, p.alpha = 1.f;
+  p.stats = reinterpret_cast<float2*>(stats), p.tile_mult = 1, p.err = err;
   p.group_m = g2::group_setting();
   return g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
 }
