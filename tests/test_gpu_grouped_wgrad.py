@@ -30,3 +30,31 @@ def test_ragged_contraction(counts, K, N):
             continue
         bound = 2.0**-8 * (a.t() @ b).abs() + 2.0**-19 * (a.abs().t() @ b.abs())  # one rounding to bf16, fp32 sums in any order
         assert ((w.grad[e].double() - a.t() @ b).abs() <= bound).all(), e
+
+
+@pytest.mark.parametrize("K,N", [(64, 256), (136, 264), (1024, 2056), (5120, 520)])
+@pytest.mark.parametrize("counts", [[1], [31, 32, 33], [0, 255, 256, 257, 0], [700, 1, 0, 513, 128, 64], [3] * 300, [2049, 5]])
+def test_grouped_products_on_cta_pairs(counts, K, N):
+    """Pieces of all sizes, ends inside a TMA box, experts without rows, ragged blocks of weight rows and contractions, rows that belong to nobody; a neighbour's infinities stay its own."""
+    g = torch.Generator(device="cuda").manual_seed(K + len(counts))
+    rows = sum(counts)
+    x = torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(len(counts), K, N, generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randn(rows, N, generator=g, device="cuda").to(torch.bfloat16)
+    bad = next((e for e, c in enumerate(counts) if e > 0 and c), None)
+    if bad is not None:
+        x[sum(counts[:bad])] = float("inf")
+    x.requires_grad_()
+    y = ops.grouped_matmul(x, w, torch.tensor(counts, device="cuda"))
+    y.backward(dy)
+    at = 0
+    for e, c in enumerate(counts):
+        a, d, we = x[at : at + c].detach().double(), dy[at : at + c].double(), w[e].double()
+        if e == bad:
+            assert not y[at].isfinite().all()
+            a, y_e = a[1:], y[at + 1 : at + c]
+        else:
+            y_e = y[at : at + c]
+        for got, want, bound in ((y_e, a @ we, a.abs() @ we.abs()), (x.grad[at : at + c], d @ we.t(), d.abs() @ we.abs().t())):
+            assert ((got.double() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-19 * bound).all(), e  # one rounding to bf16, fp32 sums in any order
+        at += c

@@ -450,13 +450,15 @@ def _grouped_gemm(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, b_mn: 
     E = w.shape[0]
     N = w.shape[2] if b_mn else w.shape[1]
     out = torch.empty(rows, N, dtype=_BF16, device=x.device)
-    max_tiles = -(-rows // 128) + E
-    scratch = torch.empty(3 * max_tiles + 1, dtype=torch.int32, device=x.device)
+    # CTA pairs (csrc/gemm_grouped2sm.cu) put 256 columns of the result on the rows of a tile; a narrower result would leave them empty
+    pairs = N >= 256 and _PAIR_KERNEL
+    launch = lib().ttb_gemm_grouped_bf16_2sm if pairs else lib().ttb_gemm_grouped_bf16
+    scratch = torch.empty(5 * (-(-rows // 256) + E) + 1 if pairs else 3 * (-(-rows // 128) + E) + 1, dtype=torch.int32, device=x.device)
     cnt = counts.to(torch.int64)
     cnt = cnt if cnt.is_contiguous() else cnt.contiguous()
     check(
-        lib().ttb_gemm_grouped_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), cnt.data_ptr(), scratch.data_ptr(), rows, E, N, K, int(b_mn), x.stride(0), w.stride(1), w.stride(0), N,
-                                    err_word(x.device).data_ptr(), stream_ptr()),
+        launch(x.data_ptr(), w.data_ptr(), out.data_ptr(), cnt.data_ptr(), scratch.data_ptr(), rows, E, N, K, int(b_mn), x.stride(0), w.stride(1), w.stride(0), N,
+               err_word(x.device).data_ptr(), stream_ptr()),
         "gemm_grouped",
     )
     return out

@@ -88,6 +88,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_ensure_device.argtypes = [i32]
     L.ttb_gemm_grouped_bf16.argtypes = [vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i64, i64, i64, i64, vp, vp]
     L.ttb_gemm_grouped_bf16.restype = i32
+    L.ttb_gemm_grouped_bf16_2sm.argtypes = L.ttb_gemm_grouped_bf16.argtypes
+    L.ttb_gemm_grouped_bf16_2sm.restype = i32
     L.ttb_gemm_bf16_dual.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i64, i64, i64, i64, i64, i32, i32, vp, f32, vp, vp]
     L.ttb_gemm_bf16_dual.restype = i32
     L.ttb_gemm_bf16_dual_2sm.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i64, i64, i64, i64, i64, vp, f32, vp, vp]
