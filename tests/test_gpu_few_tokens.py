@@ -308,3 +308,30 @@ def test_generation_of_models_that_are_not_recorded(how):
                 assert (got[1][:, 0] - want[1][:, 0]).norm() <= 0.03 * want[1][:, 0].norm()
             else:
                 assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("K", [1024, 1032, 2048, 4096])
+@pytest.mark.parametrize("M", [1, 2, 3, 7, 8])
+def test_products_of_normalised_tokens(M, K):
+    """Norms on the way into the products for few tokens: the values of the norm's kernel followed by the products', through every split of the contraction."""
+    import ctypes
+
+    from torchtune_b200 import ops
+    from torchtune_b200.ops import _cuda
+    from torchtune_b200.ops._lib import check, lib, stream_ptr
+
+    x, gain = _rand(M, K, seed=M) * 3, 1 + _rand(1, K, seed=4)[0] * 0.1
+    n = ops.rms_norm(x, gain, 1e-5)
+    for rows in ((16, 24), (520, 72), (4096, 1024), (20000, 8)):
+        ws = [_rand(r, K, seed=r) for r in rows]
+        want, got = [torch.empty(M, r, dtype=torch.bfloat16, device="cuda") for r in rows], [torch.empty(M, r, dtype=torch.bfloat16, device="cuda") for r in rows]
+        _cuda._gemm_rows(n, ws, want)
+        vps, lls = ctypes.c_void_p * 2, ctypes.c_longlong * 2
+        check(lib().ttb_gemm_rows_normed(x.data_ptr(), K, gain.data_ptr(), 1e-5, M, K, 2, vps(*[w.data_ptr() for w in ws]), lls(K, K), (ctypes.c_int * 2)(*rows), vps(*[o.data_ptr() for o in got]),
+                                         lls(*rows), None, stream_ptr()), "normed rows")
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        w1, w3 = _rand(rows[0], K, seed=5), _rand(rows[0], K, seed=6)
+        check(lib().ttb_gemm_rows_gated(n.data_ptr(), K, w1.data_ptr(), w3.data_ptr(), K, want[0].data_ptr(), rows[0], M, rows[0], K, 0.0, 0.0, stream_ptr()), "gated")
+        check(lib().ttb_gemm_rows_gated_normed(x.data_ptr(), K, gain.data_ptr(), 1e-5, w1.data_ptr(), w3.data_ptr(), K, got[0].data_ptr(), rows[0], M, rows[0], K, stream_ptr()), "gated, normed")
+        assert torch.equal(got[0], want[0])
+    assert not lib().ttb_gemm_rows_norms(9, 2048) and not lib().ttb_gemm_rows_norms(1, 1016) and not lib().ttb_gemm_rows_norms(1, 4104)

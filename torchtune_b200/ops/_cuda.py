@@ -49,8 +49,8 @@ ROWS_LIMIT = 64  # most tokens csrc/gemm_rows.cu takes
 def _runs_rows(M: int, N: int, K: int) -> bool:
     """Whether a linear layer streams its weights through registers (``csrc/gemm_rows.cu``) instead of running on a tile kernel.  The lines are drawn for the
     joined forms, which share them: there the tile kernels need several launches (us here / there: gated 32 x 14336 x 4096 55 / 88; one launch for query, key and value
-    of 64 tokens (4096 + 1024 + 1024 rows of 4096) 30 / three of about 40).  Products by themselves (weights from HBM): 16 x 4096 x 4096 11.2 / 13.8, 64 x 2048 x 2048 11.0 / 11.3, 16 x 18944 x 3584
-    29 / 35; with a vocabulary of rows the CTA-pair kernel streams as well: 16 x 128256 x 2048 100 / 116, x 4096 193 / 179, 8 x 128256 x 4096 185 / 203.
+    of 64 tokens (4096 + 1024 + 1024 rows of 4096) 30 / three of about 40).  Products by themselves (weights from HBM): 16 x 4096 x 4096 11.2 / 13.8, 64 x 2048 x 2048 11.0 / 11.3, 16 x 14336 x 4096
+    28 / 28; with a vocabulary of rows the CTA-pair kernel streams as well: 16 x 128256 x 2048 98 / 115, x 4096 198 / 186, 8 x 128256 x 4096 173 / 210.
     Since the tile kernels cut long contractions into ranges they win somewhat below these lines: 48 x 4096 x 4096 16.8 / 15.2, 64 x 4096 x 14336 43 / 31,
     16 x 5120 x 5120 18.4 / 17.1, 32 x 6144 x 4096 20.0 / 17.0, 24 x 28672 x 4096 57 / 53."""
     most = ROWS_LIMIT if N <= 4096 else 32 if N <= 32768 else 16 if K < 4096 else 8

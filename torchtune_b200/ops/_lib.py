@@ -85,6 +85,12 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_gemm_rows.restype = i32
     L.ttb_gemm_rows_gated.argtypes = [vp, i64, vp, vp, i64, vp, i64, i32, i32, i32, f32, f32, vp]
     L.ttb_gemm_rows_gated.restype = i32
+    L.ttb_gemm_rows_norms.argtypes = [i32, i32]
+    L.ttb_gemm_rows_norms.restype = i32
+    L.ttb_gemm_rows_normed.argtypes = [vp, i64, vp, f32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp]
+    L.ttb_gemm_rows_normed.restype = i32
+    L.ttb_gemm_rows_gated_normed.argtypes = [vp, i64, vp, f32, vp, vp, i64, vp, i64, i32, i32, i32, vp]
+    L.ttb_gemm_rows_gated_normed.restype = i32
     L.ttb_ensure_device.argtypes = [i32]
     L.ttb_gemm_grouped_bf16.argtypes = [vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i64, i64, i64, i64, vp, vp]
     L.ttb_gemm_grouped_bf16.restype = i32

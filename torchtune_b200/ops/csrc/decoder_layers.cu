@@ -23,6 +23,10 @@ int ttb_attn_fwd2_masked(const void* q, const void* k, const void* v, void* o, f
 int ttb_gemm_rows(const void* x, long long ldx, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y, const long long* ldy, const void* const* bias,
                   const void* residual, long long ldr, int out_f32, float alpha, void* stream);
 int ttb_gemm_rows_gated(const void* x, long long ldx, const void* w1, const void* w3, long long ldw, void* h, long long ldh, int M, int N, int K, float glu_limit, float glu_alpha, void* stream);
+int ttb_gemm_rows_norms(int M, int K);
+int ttb_gemm_rows_normed(const void* x, long long ldx, const void* norm, float eps, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y,
+                         const long long* ldy, const void* const* bias, void* stream);
+int ttb_gemm_rows_gated_normed(const void* x, long long ldx, const void* norm, float eps, const void* w1, const void* w3, long long ldw, void* h, long long ldh, int M, int N, int K, void* stream);
 int ttb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int out_fp32, int accumulate, const void* bias,
                   float alpha, int* err, void* stream);
 int ttb_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int accumulate, const void* bias, float alpha,
@@ -189,18 +193,20 @@ extern "C" int ttb_decoder_layers(const long long* words, int count, int b, int 
   float* rstd = static_cast<float*>(part(at.rstd));
   void *mid = part(at.mid), *xn = part(at.norm), *q = part(at.q), *k = part(at.k), *v = part(at.v), *rot = part(at.rot), *att = part(at.att), *act = part(at.act);
   int *lo = static_cast<int*>(part(at.lo)), *hi = static_cast<int*>(part(at.hi));
-  const bool few = decodes(z);
+  const bool few = decodes(z), norms = ttb_gemm_rows_norms(M, dim) != 0;
   if (!few) c.ok(ttb_mask_bounds(mask, mask_b, mask_r, mask_b != 0 ? b : 1, s, max_seq, lo, hi, part(at.solid), st));
   for (int i = 0; i < count && c.rc == kOk; ++i) {
     const Layer& l = reinterpret_cast<const Layer*>(words)[i];
-    c.ok(ttb_rmsnorm_fwd(h, l.sa_scale, xn, rstd, M, dim, eps, st));
-    if (c.rc == kOk && runs_rows(M, nq, dim) && runs_rows(M, nk, dim)) {
+    const bool joined = runs_rows(M, nq, dim) && runs_rows(M, nk, dim), gated = runs_rows(M, hidden, dim);
+    if (!(norms && joined)) c.ok(ttb_rmsnorm_fwd(h, l.sa_scale, xn, rstd, M, dim, eps, st));
+    if (c.rc == kOk && joined) {
       const void *w[] = {l.wq, l.wk, l.wv}, *bias[] = {l.bq, l.bk, l.bv};
       void* out[] = {q, k, v};
       const long long ldw[] = {dim, dim, dim}, ldy[] = {nq, nk, nk};
       const int n[] = {nq, nk, nk};
       const bool biased = l.bq != nullptr || l.bk != nullptr || l.bv != nullptr;
-      c.ok(ttb_gemm_rows(xn, dim, M, dim, 3, w, ldw, n, out, ldy, biased ? bias : nullptr, nullptr, 0, 0, 1.f, st));
+      c.ok(norms ? ttb_gemm_rows_normed(h, dim, l.sa_scale, eps, M, dim, 3, w, ldw, n, out, ldy, biased ? bias : nullptr, st)
+                 : ttb_gemm_rows(xn, dim, M, dim, 3, w, ldw, n, out, ldy, biased ? bias : nullptr, nullptr, 0, 0, 1.f, st));
     } else {
       c.product(xn, l.wq, l.bq, nullptr, q, M, nq, dim);
       c.product(xn, l.wk, l.bk, nullptr, k, M, nk, dim);
@@ -212,9 +218,11 @@ extern "C" int ttb_decoder_layers(const long long* words, int count, int b, int 
                : ttb_attn_fwd2_masked(rot, l.k_cache, l.v_cache, att, static_cast<float*>(part(at.lse)), lo, hi, part(at.solid), mask_b != 0 ? s : 0, mask, mask_b, mask_r, b, s, max_seq, hq,
                                       hkv, D, scale, err, st));
     c.product(att, l.wo, nullptr, h, mid, M, dim, nq);
-    if (c.rc == kOk) c.ok(ttb_rmsnorm_fwd(mid, l.mlp_scale, xn, rstd, M, dim, eps, st));
+    if (c.rc == kOk && !(norms && gated)) c.ok(ttb_rmsnorm_fwd(mid, l.mlp_scale, xn, rstd, M, dim, eps, st));
     if (c.rc != kOk) break;
-    if (runs_rows(M, hidden, dim)) {
+    if (norms && gated) {
+      c.ok(ttb_gemm_rows_gated_normed(mid, dim, l.mlp_scale, eps, l.w1, l.w3, dim, act, hidden, M, hidden, dim, st));
+    } else if (gated) {
       c.ok(ttb_gemm_rows_gated(xn, dim, l.w1, l.w3, dim, act, hidden, M, hidden, dim, 0.f, 0.f, st));
     } else if (gates_in_pairs(M, hidden, dim)) {
       c.ok(ttb_gemm_swiglu_bf16_2sm(xn, l.w1, l.w3, act, nullptr, nullptr, M, hidden, dim, dim, dim, hidden, 0.f, 0.f, err, st));

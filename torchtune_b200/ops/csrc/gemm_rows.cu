@@ -52,6 +52,8 @@ struct Params {
   int M, K, out_f32;
   float alpha;
   float glu_limit, glu_alpha;  // glu_limit > 0: the clamped gate
+  const __nv_bfloat16* norm;   // gain of an RMS norm of x, or nullptr
+  float eps;
 };
 
 __device__ __forceinline__ uint4 load_weight(const __nv_bfloat16* p) {
@@ -66,6 +68,15 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 }
 
 // MT: token tiles of 8.  WK: warps of a CTA that share 16 rows and split a chunk of WK * kChunk contraction steps.
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(b[i]);
+    f[2 * i] = t.x, f[2 * i + 1] = t.y;
+  }
+}
+
 template <int MT, int WK>
 struct Layout {
   static constexpr int kTokens = MT * 8;
@@ -76,6 +87,68 @@ struct Layout {
   static constexpr int kPartBytes = kWarps * kTokens * kPartPitch * 4;
   static constexpr int kSmem = kStages * kStageBytes > kPartBytes ? kStages * kStageBytes : kPartBytes;
 };
+
+// Partial sums of the warps and of the cluster's CTAs meet in (distributed) shared memory, in the order of warps and CTAs, and become results.  part: [warp][token][kPartPitch], 16 rows
+// of each token.
+template <int MT, int WK, bool GATED>
+__device__ __forceinline__ void finish(const Params& p, const Segment& sg, float* part, const float (&acc)[MT][4], int row0, int split, int splits) {
+  using L = Layout<MT, WK>;
+  constexpr int kOutWarps = GATED ? L::kRowWarps / 2 : L::kRowWarps;
+  constexpr int kOutRows = kOutWarps * 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  {
+    float* mine = part + warp * L::kTokens * kPartPitch;
+#pragma unroll
+    for (int n = 0; n < MT; ++n) {
+      float* at = mine + (n * 8 + t * 2) * kPartPitch + g;
+      at[0] = acc[n][0];
+      at[kPartPitch] = acc[n][1];
+      at[8] = acc[n][2];
+      at[kPartPitch + 8] = acc[n][3];
+    }
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  if (splits > 1)
+    cluster.sync();
+  else
+    __syncthreads();
+  for (int idx = split * kThreads + threadIdx.x; idx < kOutRows * p.M; idx += splits * kThreads) {
+    const int r = idx % kOutRows, token = idx / kOutRows, row = row0 + r;
+    const int at = ((r / 16) * WK * L::kTokens + token) * kPartPitch + r % 16;
+    constexpr int kNextWarp = L::kTokens * kPartPitch, kSecond = kOutWarps * WK * kNextWarp;
+    float v = 0.f, u = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) {
+      const float* from = splits > 1 ? cluster.map_shared_rank(part, s) : part;
+#pragma unroll
+      for (int k = 0; k < WK; ++k) {
+        v += from[at + k * kNextWarp];
+        if (GATED) u += from[at + kSecond + k * kNextWarp];
+      }
+    }
+    if (row >= sg.n) continue;
+    if (GATED) {
+      // pre-activations rounded to bf16, as the other gated kernels have them
+      const float a = __bfloat162float(__float2bfloat16_rn(v)), b = __bfloat162float(__float2bfloat16_rn(u));
+      if (p.glu_limit > 0.f) {
+        const float ac = fminf(a, p.glu_limit), bc = fminf(fmaxf(b, -p.glu_limit), p.glu_limit);
+        v = __fdividef(ac, 1.f + __expf(-p.glu_alpha * ac)) * (bc + 1.f);
+      } else {
+        v = a / (1.f + __expf(-a)) * b;
+      }
+    } else {
+      v *= p.alpha;
+      if (sg.bias != nullptr) v += __bfloat162float(sg.bias[row]);
+      if (p.residual != nullptr) v += __bfloat162float(p.residual[token * p.ldr + row]);
+    }
+    if (p.out_f32)
+      static_cast<float*>(sg.y)[token * sg.ldy + row] = p.out_f32 == 2 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+    else
+      static_cast<__nv_bfloat16*>(sg.y)[token * sg.ldy + row] = __float2bfloat16_rn(v);
+  }
+  if (splits > 1) cluster.sync();  // no CTA leaves while another reads its shared memory
+}
 
 // grid (tiles * splits), cluster (splits): consecutive CTAs split the contraction of one tile of kRowWarps * 16 weight rows.
 template <int MT, int WK, bool GATED>
@@ -171,67 +244,146 @@ gemm_rows_kernel(const __grid_constant__ Params p, int splits) {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
-  float* part = reinterpret_cast<float*>(smem);  // [warp][token][kPartPitch]: 16 rows of each token
-  {
-    float* mine = part + warp * L::kTokens * kPartPitch;
-#pragma unroll
-    for (int n = 0; n < MT; ++n) {
-      float* at = mine + (n * 8 + t * 2) * kPartPitch + g;
-      at[0] = acc[n][0];
-      at[kPartPitch] = acc[n][1];
-      at[8] = acc[n][2];
-      at[kPartPitch + 8] = acc[n][3];
-    }
-  }
-  cg::cluster_group cluster = cg::this_cluster();
-  if (splits > 1)
-    cluster.sync();
-  else
-    __syncthreads();
-  for (int idx = split * kThreads + threadIdx.x; idx < kOutRows * p.M; idx += splits * kThreads) {
-    const int r = idx % kOutRows, token = idx / kOutRows, row = row0 + r;
-    const int at = ((r / 16) * WK * L::kTokens + token) * kPartPitch + r % 16;
-    constexpr int kNextWarp = L::kTokens * kPartPitch, kSecond = kOutWarps * WK * kNextWarp;
-    float v = 0.f, u = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < splits; ++s) {
-      const float* from = splits > 1 ? cluster.map_shared_rank(part, s) : part;
-#pragma unroll
-      for (int k = 0; k < WK; ++k) {
-        v += from[at + k * kNextWarp];
-        if (GATED) u += from[at + kSecond + k * kNextWarp];
-      }
-    }
-    if (row >= sg.n) continue;
-    if (GATED) {
-      // pre-activations rounded to bf16, as the other gated kernels have them
-      const float a = __bfloat162float(__float2bfloat16_rn(v)), b = __bfloat162float(__float2bfloat16_rn(u));
-      if (p.glu_limit > 0.f) {
-        const float ac = fminf(a, p.glu_limit), bc = fminf(fmaxf(b, -p.glu_limit), p.glu_limit);
-        v = __fdividef(ac, 1.f + __expf(-p.glu_alpha * ac)) * (bc + 1.f);
-      } else {
-        v = a / (1.f + __expf(-a)) * b;
-      }
-    } else {
-      v *= p.alpha;
-      if (sg.bias != nullptr) v += __bfloat162float(sg.bias[row]);
-      if (p.residual != nullptr) v += __bfloat162float(p.residual[token * p.ldr + row]);
-    }
-    if (p.out_f32)
-      static_cast<float*>(sg.y)[token * sg.ldy + row] = p.out_f32 == 2 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
-    else
-      static_cast<__nv_bfloat16*>(sg.y)[token * sg.ldy + row] = __float2bfloat16_rn(v);
-  }
-  if (splits > 1) cluster.sync();  // no CTA leaves while another reads its shared memory
+  finish<MT, WK, GATED>(p, sg, reinterpret_cast<float*>(smem), acc, row0, split, splits);
 }
 
-template <int MT, int WK, bool GATED>
-static int launch(Params& p, int tiles, int splits, cudaStream_t st) {
-  constexpr int smem = Layout<MT, WK>::kSmem;
-  auto kernel = gemm_rows_kernel<MT, WK, GATED>;
-  static bool attr = false;
+// Up to 16 tokens whose share of a CTA's contraction fits shared memory as a whole: they are staged once, and the warps stream their weights without meeting until the end.  With NORM, x is normalised on
+// the way in (the sums of squares in the order of the norm's own kernel, so the values are the same ones): a norm by itself is a launch of 2 us in a decode step, and here its reads
+// hide behind the first weights.
+// us in a graph, weights from HBM, with the ring above -> here, 1 / 16 tokens: 6144 x 4096 14.9 / 16.7 -> 13.3 / 15.7, 4096 x 14336 24.7 / 27.3 -> 22.1 / 24.7 (5.3 TB/s), 128256 x 2048
+// 94.8 / 104.5 -> 83.0 / 98.2 (6.3 TB/s), 128256 x 4096 186 -> 163 (6.4 TB/s).  A chat turn of the 16-layer 1B model, with the norms, 25.1 -> 23.0 ms.
+template <int MT, int WK, bool GATED, bool NORM>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_rows_resident_kernel(const __grid_constant__ Params p, int splits) {
+  using L = Layout<MT, WK>;
+  constexpr int kOutWarps = GATED ? L::kRowWarps / 2 : L::kRowWarps;
+  constexpr int kOutRows = kOutWarps * 16;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ float sums[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / splits, split = blockIdx.x % splits;
+  int si = 0;
+  if (p.segments > 1 && tile >= p.seg[1].first_tile) si = 1;
+  if (p.segments > 2 && tile >= p.seg[2].first_tile) si = 2;
+  const Segment& sg = p.seg[si];
+  const int row0 = (tile - sg.first_tile) * kOutRows;
+  const int wr = warp / WK, wk = warp % WK;
+  const bool second = GATED && wr >= kOutWarps;
+  const int wrow = row0 + (second ? wr - kOutWarps : wr) * 16;
+  const int g = lane >> 2, t = lane & 3;
+  const __nv_bfloat16* w = second ? p.up : sg.w;
+  const __nv_bfloat16* w0 = w + static_cast<long long>(min(wrow + g, sg.n - 1)) * sg.ldw;
+  const __nv_bfloat16* w1 = w + static_cast<long long>(min(wrow + g + 8, sg.n - 1)) * sg.ldw;
+  const int chunks = (p.K + L::kStep - 1) / L::kStep;
+  const int own = chunks > split ? (chunks - split + splits - 1) / splits : 0;
+  auto load_w = [&](int i, uint4 (&a)[4], uint4 (&b)[4]) {
+    const int k0 = (split + i * splits) * L::kStep + wk * kChunk + t * 8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int k = k0 + j * 32;
+      if (i < own && k < p.K) {
+        a[j] = load_weight(w0 + k);
+        b[j] = load_weight(w1 + k);
+      } else {
+        a[j] = make_uint4(0, 0, 0, 0);
+        b[j] = make_uint4(0, 0, 0, 0);
+      }
+    }
+  };
+  uint4 a0[4], b0[4], a1[4], b1[4];
+  load_w(0, a0, b0);
+  load_w(1, a1, b1);
+
+  // the own chunks of a token, one after the other; the two tokens of a quarter warp read different halves of the 32 banks
+  const int pitch = (chunks + splits - 1) / splits * L::kStep * 2 + 64;
+  if (NORM) {
+    // half of the CTA takes a token, as the norm's kernel of 128 threads does
+    for (int m0 = 0; m0 < p.M; m0 += 2) {
+      const int m = m0 + (threadIdx.x >> 7), at = threadIdx.x & 127;
+      float ss = 0.f;
+      uint4 u[4];
+      if (m < p.M) {
+        const uint4* xr = reinterpret_cast<const uint4*>(p.x + m * p.ldx);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          u[k] = at + k * 128 < p.K / 8 ? xr[at + k * 128] : make_uint4(0, 0, 0, 0);
+          float f[8];
+          unpack8(u[k], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (m0 > 0) __syncthreads();  // the last pair's sums are read
+      if (lane == 0) sums[warp] = ss;
+      __syncthreads();
+      if (m < p.M) {
+        const float* four = sums + (warp & 4);
+        const float rstd = rsqrtf(((four[0] + four[2]) + (four[1] + four[3])) / p.K + p.eps);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int i = at + k * 128, chunk = i / (L::kStep / 8);
+          if (i < p.K / 8 && chunk % splits == split) {
+            float f[8], s[8];
+            unpack8(u[k], f);
+            unpack8(__ldg(reinterpret_cast<const uint4*>(p.norm) + i), s);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = __bfloat162float(__float2bfloat16_rn(f[j] * rstd)) * s[j];
+            *reinterpret_cast<uint4*>(smem + m * pitch + (chunk / splits * (L::kStep / 8) + i % (L::kStep / 8)) * 16) =
+                make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+          }
+        }
+      }
+    }
+  } else {
+    constexpr int kPieces = L::kStep / 8;
+    for (int c = threadIdx.x; c < own * kPieces; c += kThreads) {
+      const int k = (split + c / kPieces * splits) * L::kStep + c % kPieces * 8;
+      if (k < p.K) {
+        for (int m = 0; m < p.M; ++m)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem) + m * pitch + c * 16), "l"(p.x + m * p.ldx + k) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+  __syncthreads();
+
+  float acc[MT][4];
+#pragma unroll
+  for (int n = 0; n < MT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  auto products = [&](int i, const uint4 (&a)[4], const uint4 (&b)[4]) {
+    const int at = wk * kChunk + t * 8, k0 = (split + i * splits) * L::kStep + at;
+    const uint8_t* xs = smem + g * pitch + (i * L::kStep + at) * 2;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+      for (int n = 0; n < MT; ++n) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (g + n * 8 < p.M && k0 + j * 32 < p.K) v = *reinterpret_cast<const uint4*>(xs + n * 8 * pitch + j * 64);
+        mma16816(acc[n], a[j].x, b[j].x, a[j].y, b[j].y, v.x, v.y);
+        mma16816(acc[n], a[j].z, b[j].z, a[j].w, b[j].w, v.z, v.w);
+      }
+    }
+  };
+  for (int i = 0; i < own; i += 2) {
+    products(i, a0, b0);
+    load_w(i + 2, a0, b0);
+    if (i + 1 >= own) break;
+    products(i + 1, a1, b1);
+    load_w(i + 3, a1, b1);
+  }
+  __syncthreads();
+  finish<MT, WK, GATED>(p, sg, reinterpret_cast<float*>(smem), acc, row0, split, splits);
+}
+
+static constexpr int kMaxResident = 96 * 1024;  // two CTAs per SM
+
+template <typename Kernel>
+static int start(Kernel kernel, bool& attr, int most, int smem, const Params& p, int tiles, int splits, cudaStream_t st) {
   if (!attr) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kErrDriver;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return kErrDriver;
     attr = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -244,7 +396,26 @@ static int launch(Params& p, int tiles, int splits, cudaStream_t st) {
   at[0].val.clusterDim.x = splits, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
   cfg.attrs = at, cfg.numAttrs = 1;
   TTB_COUNT_LAUNCH(1);
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<const Params&>(p), splits) == cudaSuccess ? kOk : kErrDriver;
+  return cudaLaunchKernelEx(&cfg, kernel, p, splits) == cudaSuccess ? kOk : kErrDriver;
+}
+
+template <int MT, int WK, bool GATED>
+static int launch(Params& p, int tiles, int splits, cudaStream_t st) {
+  static bool attr[3] = {false, false, false};
+  if constexpr (MT <= 2) {
+    using L = Layout<MT, WK>;
+    const int chunks = (p.K + L::kStep - 1) / L::kStep;
+    long long bytes = p.M * ((chunks + splits - 1) / splits * L::kStep * 2ll + 64);
+    bytes = bytes > L::kPartBytes ? bytes : L::kPartBytes;
+    // with fewer than four chunks to a CTA the staging in front is what counts (16 x 3072 x 2048: 7.0 us with the ring, 7.5 with all of it first)
+    if (bytes <= kMaxResident && (p.norm != nullptr || chunks >= 4 * splits)) {
+      if (p.norm == nullptr) return start(gemm_rows_resident_kernel<MT, WK, GATED, false>, attr[0], kMaxResident, static_cast<int>(bytes), p, tiles, splits, st);
+      if constexpr (MT == 1) return start(gemm_rows_resident_kernel<MT, WK, GATED, true>, attr[1], kMaxResident, static_cast<int>(bytes), p, tiles, splits, st);
+    }
+  }
+  if (p.norm != nullptr) return kErrBadShape;
+  constexpr int smem = Layout<MT, WK>::kSmem;
+  return start(gemm_rows_kernel<MT, WK, GATED>, attr[2], smem, smem, p, tiles, splits, st);
 }
 
 // Rows per CTA: the most (fewest re-reads of the tokens, longest loads per row) that can still fill more than half of the two CTA places per SM; the
@@ -291,13 +462,13 @@ static bool unaligned(const void* t, long long ld) { return (reinterpret_cast<ui
 
 // Y_i[M, n_i] = alpha * X[M, K] · W_i[n_i, K]ᵀ (+ bias_i) (+ residual, first weight only) for up to three weights of one input, M <= 64, K a
 // multiple of 8, X and W rows 16-byte aligned.  bf16 results; fp32 with out_f32 = 1, the bf16 ones widened with 2.
-extern "C" int ttb_gemm_rows(const void* x, long long ldx, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y, const long long* ldy,
-                             const void* const* bias, const void* residual, long long ldr, int out_f32, float alpha, void* stream) {
+static int rows_product(const void* x, long long ldx, const void* norm, float eps, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y,
+                        const long long* ldy, const void* const* bias, const void* residual, long long ldr, int out_f32, float alpha, void* stream) {
   using namespace ttb;
   if (M <= 0 || M > 64 || K <= 0 || (K & 7) || count < 1 || count > rows::kMaxSegments || rows::unaligned(x, ldx)) return kErrBadShape;
   rows::Params p{};
   p.segments = count, p.M = M, p.K = K, p.out_f32 = out_f32, p.alpha = alpha;
-  p.x = static_cast<const __nv_bfloat16*>(x), p.ldx = ldx;
+  p.x = static_cast<const __nv_bfloat16*>(x), p.ldx = ldx, p.norm = static_cast<const __nv_bfloat16*>(norm), p.eps = eps;
   p.residual = static_cast<const __nv_bfloat16*>(residual), p.ldr = ldr;
   for (int i = 0; i < count; ++i) {
     if (n[i] <= 0 || rows::unaligned(w[i], ldw[i])) return kErrBadShape;
@@ -306,16 +477,40 @@ extern "C" int ttb_gemm_rows(const void* x, long long ldx, int M, int K, int cou
   }
   return rows::by_tokens<false>(p, static_cast<cudaStream_t>(stream));
 }
-
-// H[M, N] = silu(X · W1ᵀ) ⊙ (X · W3ᵀ), or the clamped gate with glu_limit > 0 (as ttb_gemm_swiglu_bf16_2sm), M <= 64; both weights [N, K] with pitch ldw.
-extern "C" int ttb_gemm_rows_gated(const void* x, long long ldx, const void* w1, const void* w3, long long ldw, void* h, long long ldh, int M, int N, int K, float glu_limit,
-                                   float glu_alpha, void* stream) {
+static int rows_gated(const void* x, long long ldx, const void* norm, float eps, const void* w1, const void* w3, long long ldw, void* h, long long ldh, int M, int N, int K, float glu_limit,
+                      float glu_alpha, void* stream) {
   using namespace ttb;
   if (M <= 0 || M > 64 || N <= 0 || K <= 0 || (K & 7) || rows::unaligned(x, ldx) || rows::unaligned(w1, ldw) || rows::unaligned(w3, ldw)) return kErrBadShape;
   rows::Params p{};
   p.segments = 1, p.M = M, p.K = K, p.alpha = 1.f, p.glu_limit = glu_limit, p.glu_alpha = glu_alpha;
-  p.x = static_cast<const __nv_bfloat16*>(x), p.ldx = ldx;
+  p.x = static_cast<const __nv_bfloat16*>(x), p.ldx = ldx, p.norm = static_cast<const __nv_bfloat16*>(norm), p.eps = eps;
   p.up = static_cast<const __nv_bfloat16*>(w3);
   p.seg[0].w = static_cast<const __nv_bfloat16*>(w1), p.seg[0].y = h, p.seg[0].ldw = ldw, p.seg[0].ldy = ldh, p.seg[0].n = N;
   return rows::by_tokens<true>(p, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ttb_gemm_rows(const void* x, long long ldx, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y, const long long* ldy,
+                             const void* const* bias, const void* residual, long long ldr, int out_f32, float alpha, void* stream) {
+  return rows_product(x, ldx, nullptr, 0.f, M, K, count, w, ldw, n, y, ldy, bias, residual, ldr, out_f32, alpha, stream);
+}
+
+// H[M, N] = silu(X · W1ᵀ) ⊙ (X · W3ᵀ), or the clamped gate with glu_limit > 0 (as ttb_gemm_swiglu_bf16_2sm), M <= 64; both weights [N, K] with pitch ldw.
+extern "C" int ttb_gemm_rows_gated(const void* x, long long ldx, const void* w1, const void* w3, long long ldw, void* h, long long ldh, int M, int N, int K, float glu_limit,
+                                   float glu_alpha, void* stream) {
+  return rows_gated(x, ldx, nullptr, 0.f, w1, w3, ldw, h, ldh, M, N, K, glu_limit, glu_alpha, stream);
+}
+
+// Whether the two below take rows of these sizes: tokens that fit shared memory, widths whose norm has a kernel of 128 threads per row.
+extern "C" int ttb_gemm_rows_norms(int M, int K) { return M > 0 && M <= 8 && K >= 1024 && K <= 4096 && K % 8 == 0 && M * (K * 2ll + 64) <= ttb::rows::kMaxResident; }
+
+// ttb_gemm_rows and ttb_gemm_rows_gated on rmsnorm(X) = bf16(X · rsqrt(mean(X²) + eps)) · norm, value for value what ttb_rmsnorm_fwd gives.
+extern "C" int ttb_gemm_rows_normed(const void* x, long long ldx, const void* norm, float eps, int M, int K, int count, const void* const* w, const long long* ldw, const int* n, void* const* y,
+                                    const long long* ldy, const void* const* bias, void* stream) {
+  if (!ttb_gemm_rows_norms(M, K) || norm == nullptr || (reinterpret_cast<uintptr_t>(norm) & 15)) return ttb::kErrBadShape;
+  return rows_product(x, ldx, norm, eps, M, K, count, w, ldw, n, y, ldy, bias, nullptr, 0, 0, 1.f, stream);
+}
+extern "C" int ttb_gemm_rows_gated_normed(const void* x, long long ldx, const void* norm, float eps, const void* w1, const void* w3, long long ldw, void* h, long long ldh, int M, int N, int K,
+                                          void* stream) {
+  if (!ttb_gemm_rows_norms(M, K) || norm == nullptr || (reinterpret_cast<uintptr_t>(norm) & 15)) return ttb::kErrBadShape;
+  return rows_gated(x, ldx, norm, eps, w1, w3, ldw, h, ldh, M, N, K, 0.f, 0.f, stream);
 }
