@@ -25,6 +25,8 @@ def _model(layers, dim, heads, kv, hidden, vocab, rows, slots, bias=False):
 
 SHAPES = [  # layers, dim, heads, key heads, hidden, rows, slots, tokens
     (2, 512, 8, 2, 1024, 3, 60, 1),  # kernels for few tokens
+    (2, 1024, 16, 1, 1024, 5, 1030, 1),  # one token: 16 query heads to a key head, ranges of keys
+    (1, 1024, 8, 4, 512, 9, 65, 1),  # head dimension 128
     (2, 2048, 32, 8, 8192, 1, 61, 37),  # gate and up projection apart, the rest for few tokens
     (1, 1024, 8, 8, 4096, 2, 300, 4),  # several queries on the kernel for few queries
     (1, 1024, 8, 8, 4096, 2, 300, 200),  # contraction in ranges, residual by itself
@@ -34,10 +36,10 @@ SHAPES = [  # layers, dim, heads, key heads, hidden, rows, slots, tokens
 ]
 
 
-@pytest.mark.parametrize("padded,bias", [(False, False), (True, True)])
+@pytest.mark.parametrize("padded,bias,start", [(False, False, 0), (True, True, 0), (True, False, 5)])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
 @torch.no_grad()
-def test_results_and_caches_are_those_of_the_modules(shape, padded, bias):
+def test_results_and_caches_are_those_of_the_modules(shape, padded, bias, start):
     from torchtune_b200 import generation
     from torchtune_b200.generation._native_layers import NativeLayers
     from torchtune_b200.generation._rows import hidden_states
@@ -47,22 +49,36 @@ def test_results_and_caches_are_those_of_the_modules(shape, padded, bias):
     native = NativeLayers.of(model, rows)
     assert native is not None
     x = torch.randint(1, 1024, (rows, n), device="cuda")
+
+    def restart():  # caches that hold `start` tokens
+        model.reset_caches()
+        for i, layer in enumerate(model.layers):
+            cache = layer.attn.kv_cache
+            g = torch.Generator(device="cuda").manual_seed(i)
+            cache.k_cache[:, :start].normal_(generator=g), cache.v_cache[:, :start].normal_(generator=g)
+            cache.cache_pos.add_(start)
+            layer.attn.pos_embeddings.interleaved = start == 0
+
+    restart()
+    native = NativeLayers.of(model, rows)
     if padded:
         real = torch.ones(rows, n, dtype=torch.bool, device="cuda")
         for r in range(1, rows):
             real[r, : min(n - 1, 3 * r)] = False
-        mask, pos = generation.get_causal_mask_from_padding_mask(real, target_seq_len=slots), generation.get_position_ids_from_padding_mask(real)
+        real = torch.nn.functional.pad(real, (start, 0), value=True)
+        mask, pos = generation.get_causal_mask_from_padding_mask(real, target_seq_len=slots)[:, start:], generation.get_position_ids_from_padding_mask(real)[:, start:]
     else:
         mask, pos = torch.tril(torch.ones(n + 2, slots, dtype=torch.bool, device="cuda")).unsqueeze(0)[:, :n], torch.arange(n, device="cuda")
     got = native(x, pos, mask)
     caches = [(l.attn.kv_cache.k_cache.clone(), l.attn.kv_cache.v_cache.clone(), l.attn.kv_cache.cache_pos.clone()) for l in model.layers]
-    model.reset_caches()
+    restart()
     want = hidden_states(model, x, input_pos=pos, mask=mask)
     assert torch.equal(got, want)
     for l, (k, v, at) in zip(model.layers, caches):
         assert torch.equal(l.attn.kv_cache.k_cache, k) and torch.equal(l.attn.kv_cache.v_cache, v) and torch.equal(l.attn.kv_cache.cache_pos, at)
     with pytest.raises(AssertionError, match="full"):
-        native(x.repeat(1, slots // n)[:, :slots], torch.arange(slots // n * n, device="cuda"), torch.ones(1, slots // n * n, slots, dtype=torch.bool, device="cuda"))
+        more = slots - n - start + 1
+        native(x[:, :1].repeat(1, more), torch.arange(more, device="cuda"), torch.ones(1, more, slots, dtype=torch.bool, device="cuda"))
 
 
 @torch.no_grad()

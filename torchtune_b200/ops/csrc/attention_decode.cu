@@ -19,6 +19,8 @@
 #include "common/ptx.cuh"
 #include "common/tmap.h"
 
+TTB_DEFINE_VIOLATION_COUNTER(decode)
+
 namespace ttb {
 namespace dec {
 
@@ -43,6 +45,12 @@ struct Params {
   const int* hi;
   int s, sk, hq, hkv;
   float scale;
+  // APPEND: one query per row; q is still to be rotated, and the new key (to be rotated as well) and value go to slot slots[0] of the caches k and v first
+  const __nv_bfloat16 *k_new, *v_new;  // [b, hkv, D]
+  const float* rope;                   // [rope_len, D / 2, 2] cosine and sine
+  const int* pos;                      // [b]
+  const long long* slots;
+  int rope_len, interleaved;
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool keep) {
@@ -68,16 +76,20 @@ struct Layout {
   static constexpr int kPart = kMaxRows * D * 4;              // fp32 output of one warp; reuses the warp's ring
   static_assert(kPart <= kWarpBytes, "a warp's partial output fits its ring");
   static constexpr int kStats = (kWarps + 1) * kMaxRows * 2 * 4;  // maximum and sum per warp, and of the CTA
+  static constexpr int kQueryPitch = D * 2 + 16;
+  static constexpr int kQueries = kMaxRows * kQueryPitch;         // APPEND: the rotated queries
 };
 
 // grid (splits = cluster, key heads, batch)
-template <int D>
+// With APPEND the step between the projections and the cache, a launch of 2 - 5 us that moved a few KB, happens here: the queries are rotated into shared memory, and the CTA whose
+// blocks hold the new slot writes the cache before it reads.
+template <int D, bool APPEND>
 __global__ void __launch_bounds__(kWarps * 32)
 decode_kernel(Params p) {
   using L = Layout<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   float* stats = reinterpret_cast<float*>(smem + L::kRing);
-  uint64_t* bits = reinterpret_cast<uint64_t*>(smem + L::kRing + L::kStats);  // [own blocks][s + 1]: one word per query, then their union
+  uint64_t* bits = reinterpret_cast<uint64_t*>(smem + L::kRing + L::kStats + (APPEND ? L::kQueries : 0));  // [own blocks][s + 1]: one word per query, then their union
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x, splits = gridDim.x, hk = blockIdx.y, bi = blockIdx.z;
   const int group = p.hq / p.hkv, rows = p.s * group;
@@ -112,16 +124,53 @@ decode_kernel(Params p) {
   uint32_t qf[D / 16][4];
   const int r0 = lane >> 2, r1 = r0 + 8;
   const int q0 = r0 / group, q1 = r1 / group;  // query of the two rows of this lane
-  auto qrow = [&](int r) { return p.q + ((static_cast<long long>(bi) * p.s + r / group) * p.hq + hk * group + r % group) * D; };
+  if constexpr (APPEND) {
+    uint8_t* queries = smem + L::kRing + L::kStats;
+    const long long slot = p.slots[0];
+    const bool mine = slot >= 0 && slot < p.sk && static_cast<int>(slot / kKeys) % splits == split;  // the host has checked the cache's own counter; nothing is written outside it
+    int at = p.pos[bi];
+    if (at < 0 || at >= p.rope_len) {
+      if (threadIdx.x == 0 && hk == 0 && split == 0) TTB_NOTE_VIOLATION(decode);
+      at = 0;
+    }
+    const float2* table = reinterpret_cast<const float2*>(p.rope + static_cast<long long>(at) * D);
+    const __nv_bfloat16* q = p.q + (static_cast<long long>(bi) * p.hq + hk * group) * D;
+    const long long new_at = (static_cast<long long>(bi) * p.hkv + hk) * D;
+    const long long cache_at = ((static_cast<long long>(bi) * p.sk + slot) * p.hkv + hk) * D;
+    for (int idx = threadIdx.x; idx < (kMaxRows + 1) * (D / 2); idx += kWarps * 32) {
+      const int r = idx / (D / 2), e = idx % (D / 2);
+      const int c0 = p.interleaved ? 2 * e : e, c1 = p.interleaved ? 2 * e + 1 : e + D / 2;
+      __nv_bfloat16 o0 = __float2bfloat16_rn(0.f), o1 = o0;  // unused rows of the tile are zeros
+      if (r < group || (r == kMaxRows && mine)) {
+        const __nv_bfloat16* src = r < kMaxRows ? q + r * D : p.k_new + new_at;
+        const float x = __bfloat162float(src[c0]), y = __bfloat162float(src[c1]);
+        const float2 cs = table[e];
+        o0 = __float2bfloat16_rn(x * cs.x - y * cs.y), o1 = __float2bfloat16_rn(y * cs.x + x * cs.y);
+      }
+      if (r < kMaxRows) {
+        __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(queries + r * L::kQueryPitch);
+        to[c0] = o0, to[c1] = o1;
+      } else if (mine) {
+        const_cast<__nv_bfloat16*>(p.k)[cache_at + c0] = o0, const_cast<__nv_bfloat16*>(p.k)[cache_at + c1] = o1;
+      }
+    }
+    if (mine && threadIdx.x < D / 8)
+      *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(p.v) + cache_at + threadIdx.x * 8) = *reinterpret_cast<const uint4*>(p.v_new + new_at + threadIdx.x * 8);
+    __syncthreads();
 #pragma unroll
-  for (int kk = 0; kk < D / 16; ++kk) {
-    const int c = kk * 16 + (lane & 3) * 2;
-    qf[kk][0] = r0 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r0) + c) : 0u;
-    qf[kk][1] = r1 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r1) + c) : 0u;
-    qf[kk][2] = r0 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r0) + c + 8) : 0u;
-    qf[kk][3] = r1 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r1) + c + 8) : 0u;
+    for (int kk = 0; kk < D / 16; ++kk) ldsm4(smem_u32(queries) + (((lane >> 3) & 1) * 8 + (lane & 7)) * L::kQueryPitch + kk * 32 + (lane >> 4) * 16, qf[kk]);
+  } else {
+    auto qrow = [&](int r) { return p.q + ((static_cast<long long>(bi) * p.s + r / group) * p.hq + hk * group + r % group) * D; };
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      const int c = kk * 16 + (lane & 3) * 2;
+      qf[kk][0] = r0 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r0) + c) : 0u;
+      qf[kk][1] = r1 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r1) + c) : 0u;
+      qf[kk][2] = r0 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r0) + c + 8) : 0u;
+      qf[kk][3] = r1 < rows ? *reinterpret_cast<const uint32_t*>(qrow(r1) + c + 8) : 0u;
+    }
+    __syncthreads();
   }
-  __syncthreads();
 
   const uint32_t ring = smem_u32(smem) + warp * L::kWarpBytes;
   const int shift = warp * 16;
@@ -287,7 +336,7 @@ decode_kernel(Params p) {
   cluster.sync();  // no CTA leaves while another reads its shared memory
 }
 
-template <int D>
+template <int D, bool APPEND>
 static int launch(const Params& p, int b, cudaStream_t st) {
   const int blocks = (p.sk + kKeys - 1) / kKeys;
   int splits = 1;  // fill the SMs twice over as long as every CTA has a block of its own
@@ -295,10 +344,11 @@ static int launch(const Params& p, int b, cudaStream_t st) {
   const int own = (blocks + splits - 1) / splits;
   const long long bit_bytes = static_cast<long long>(own) * (p.s + 1) * 8;
   if (bit_bytes > kMaxBitBytes) return kErrTooLarge;
-  const int smem = Layout<D>::kRing + Layout<D>::kStats + static_cast<int>(bit_bytes);
+  constexpr int fixed = Layout<D>::kRing + Layout<D>::kStats + (APPEND ? Layout<D>::kQueries : 0);
+  const int smem = fixed + static_cast<int>(bit_bytes);
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<D>::kRing + Layout<D>::kStats + kMaxBitBytes) != cudaSuccess) return kErrDriver;
+    if (cudaFuncSetAttribute(decode_kernel<D, APPEND>, cudaFuncAttributeMaxDynamicSharedMemorySize, fixed + kMaxBitBytes) != cudaSuccess) return kErrDriver;
     attr = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -311,7 +361,7 @@ static int launch(const Params& p, int b, cudaStream_t st) {
   at[0].val.clusterDim.x = splits, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
   cfg.attrs = at, cfg.numAttrs = 1;
   TTB_COUNT_LAUNCH(1);
-  return cudaLaunchKernelEx(&cfg, decode_kernel<D>, p) == cudaSuccess ? kOk : kErrDriver;
+  return cudaLaunchKernelEx(&cfg, decode_kernel<D, APPEND>, p) == cudaSuccess ? kOk : kErrDriver;
 }
 
 // First and last visible key of every mask row and whether all keys between them are visible; one warp per row, 16 bytes per lane and
@@ -376,7 +426,25 @@ extern "C" int ttb_attn_decode(const void* q, const void* k, const void* v, void
   p.mask = static_cast<const uint8_t*>(mask), p.mask_b = mask_b, p.mask_r = mask_r, p.lo = lo, p.hi = hi;
   p.s = s, p.sk = sk, p.hq = hq, p.hkv = hkv, p.scale = scale;
   auto st = static_cast<cudaStream_t>(stream);
-  return d == 128 ? dec::launch<128>(p, b, st) : dec::launch<64>(p, b, st);
+  return d == 128 ? dec::launch<128, false>(p, b, st) : dec::launch<64, false>(p, b, st);
+}
+
+// ttb_rope_append for one token per row followed by ttb_attn_decode on the caches, in one launch and with the same values: q, o [b, hq, d], k, v [b, hkv, d] before the rotation, caches [b, max_seq,
+// hkv, d], rope [rope_len, d / 2, 2] fp32, pos int32 [b], slots[0] the slot of the new tokens; mask as above, max_seq bytes a row (mask_b 0: the same for all rows).
+extern "C" int ttb_attn_decode_append(const void* q, const void* k, const void* v, void* o, void* k_cache, void* v_cache, const float* rope, const int* pos, const long long* slots, const void* mask,
+                                      long long mask_b, int b, int max_seq, int hq, int hkv, int d, int interleaved, int rope_len, float scale, void* stream) {
+  using namespace ttb;
+  if ((d != 64 && d != 128) || b <= 0 || max_seq <= 0 || hkv <= 0 || hq % hkv || hq / hkv > dec::kMaxRows || b > 65535 || hkv > 65535 || rope_len <= 0) return kErrBadShape;
+  for (const void* t : {q, k, v, static_cast<const void*>(o), static_cast<const void*>(k_cache), static_cast<const void*>(v_cache), static_cast<const void*>(rope)})
+    if (reinterpret_cast<uintptr_t>(t) & 15) return kErrBadShape;
+  dec::Params p{};
+  p.q = static_cast<const __nv_bfloat16*>(q), p.k = static_cast<const __nv_bfloat16*>(k_cache), p.v = static_cast<const __nv_bfloat16*>(v_cache), p.o = static_cast<__nv_bfloat16*>(o);
+  p.mask = static_cast<const uint8_t*>(mask), p.mask_b = mask_b;
+  p.s = 1, p.sk = max_seq, p.hq = hq, p.hkv = hkv, p.scale = scale;
+  p.k_new = static_cast<const __nv_bfloat16*>(k), p.v_new = static_cast<const __nv_bfloat16*>(v), p.rope = rope, p.pos = pos, p.slots = slots;
+  p.rope_len = rope_len, p.interleaved = interleaved;
+  auto st = static_cast<cudaStream_t>(stream);
+  return d == 128 ? dec::launch<128, true>(p, b, st) : dec::launch<64, true>(p, b, st);
 }
 
 // lo / hi int32 [b, s]: first / last nonzero byte of every mask row (sk / -1 for rows without one); solid uint8 [b, s]: 1 if all bytes between are nonzero.

@@ -17,6 +17,8 @@ int ttb_rope_append(const void* q, const void* k, const void* v, void* q_out, vo
                     int hkv, int d, int seq_len, int max_seq, int interleaved, int cache_len, void* stream);
 int ttb_attn_decode(const void* q, const void* k, const void* v, void* o, const void* mask, long long mask_b, long long mask_r, const int* lo, const int* hi, int b, int s, int sk, int hq, int hkv,
                     int d, float scale, void* stream);
+int ttb_attn_decode_append(const void* q, const void* k, const void* v, void* o, void* k_cache, void* v_cache, const float* rope, const int* pos, const long long* slots, const void* mask,
+                           long long mask_b, int b, int max_seq, int hq, int hkv, int d, int interleaved, int rope_len, float scale, void* stream);
 int ttb_mask_bounds(const void* mask, long long stride_b, long long stride_r, int b, int s, int sk, int* lo, int* hi, void* solid, void* stream);
 int ttb_attn_fwd2_masked(const void* q, const void* k, const void* v, void* o, float* lse, const int* lo, const int* hi, const void* solid, long long bound_b, const void* mask, long long mask_b,
                          long long mask_r, int b, int s, int sk, int hq, int hkv, int d, float scale, int* err, void* stream);
@@ -212,11 +214,14 @@ extern "C" int ttb_decoder_layers(const long long* words, int count, int b, int 
       c.product(xn, l.wk, l.bk, nullptr, k, M, nk, dim);
       c.product(xn, l.wv, l.bv, nullptr, v, M, nk, dim);
     }
-    if (c.rc == kOk) c.ok(ttb_rope_append(q, k, v, rot, l.k_cache, l.v_cache, l.rope, pos, l.slots, M, hq, hkv, D, s, max_seq, interleaved, static_cast<int>(l.rope_len), st));
-    if (c.rc == kOk)
+    const int rope_len = static_cast<int>(l.rope_len);
+    if (c.rc == kOk && few && s == 1) {
+      c.ok(ttb_attn_decode_append(q, k, v, att, l.k_cache, l.v_cache, l.rope, pos, l.slots, mask, mask_b, b, max_seq, hq, hkv, D, interleaved, rope_len, scale, st));
+    } else if (c.rc == kOk && c.ok(ttb_rope_append(q, k, v, rot, l.k_cache, l.v_cache, l.rope, pos, l.slots, M, hq, hkv, D, s, max_seq, interleaved, rope_len, st))) {
       c.ok(few ? ttb_attn_decode(rot, l.k_cache, l.v_cache, att, mask, mask_b, mask_r, nullptr, nullptr, b, s, max_seq, hq, hkv, D, scale, st)
                : ttb_attn_fwd2_masked(rot, l.k_cache, l.v_cache, att, static_cast<float*>(part(at.lse)), lo, hi, part(at.solid), mask_b != 0 ? s : 0, mask, mask_b, mask_r, b, s, max_seq, hq,
                                       hkv, D, scale, err, st));
+    }
     c.product(att, l.wo, nullptr, h, mid, M, dim, nq);
     if (c.rc == kOk && !(norms && gated)) c.ok(ttb_rmsnorm_fwd(mid, l.mlp_scale, xn, rstd, M, dim, eps, st));
     if (c.rc != kOk) break;
