@@ -99,3 +99,33 @@ def test_what_the_call_does_not_do_is_left_to_the_modules():
     x, pos, mask = torch.ones(4, 2, dtype=torch.int64, device="cuda"), torch.arange(2, device="cuda"), torch.ones(1, 2, 60, dtype=torch.bool, device="cuda")
     assert native(x[:3], pos, mask) is None and native(x, pos, mask[:, :, :59]) is None and native(x, pos, mask.float()) is None
     assert int(model.layers[0].attn.kv_cache.cache_pos[0]) == 0 and native(x, pos, mask) is not None
+
+
+@pytest.mark.parametrize("M,N,Ks", [(40, 64, (64, 24)), (300, 520, (512, 128, 128)), (8200, 1032, (1024, 136, 264)), (4100, 2048, (2048, 512, 512)), (700, 2048, (8192, 4096)), (9000, 520, (200, 8192))])
+def test_linear_layers_of_one_input(M, N, Ks):
+    """Values of joined layers are those of single ones; the input gradient, summed by its products, against 64 bits; outputs that nobody uses, frozen weights, biases."""
+    from torchtune_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    x, ws, bs = rand(2, M // 2, N).requires_grad_(), [(rand(K, N) * N**-0.5).requires_grad_() for K in Ks], [rand(K).requires_grad_() if i != 1 else None for i, K in enumerate(Ks)]
+    ws[-1].requires_grad_(False)
+    assert ops.joins_gradients(x)
+    ys = ops.linear_group(x, ws, bs)
+    dys = [rand(*y.shape) for y in ys]
+    single = [ops.linear(x, w, b) for w, b in zip(ws, bs)]
+    assert all(torch.equal(a, b) for a, b in zip(ys, single))
+    leaves = [x, *ws[:-1], *(b for b in bs if b is not None)]
+    got = torch.autograd.grad(ys, leaves, dys)
+    want = torch.autograd.grad(single, leaves, dys)
+    assert all(torch.equal(a, b) for a, b in zip(got[1:], want[1:]))
+    terms = [d.view(-1, d.shape[-1]).double() @ w.double() for d, w in zip(dys, ws)]
+    exact = sum(terms).view_as(x)
+    # a rounding to bf16 errs by at most 2^-8 of what it rounds: the result, and for each further product the sum so far or the product
+    bound = 2.0**-8 * (exact.abs() + sum(t.abs() for t in terms).view_as(x) * (len(Ks) - 1)) + 1e-4
+    assert ((got[0].double() - exact).abs() <= bound).all()
+    assert float((got[0].double() - exact).norm()) <= 1.02 * float((want[0].double() - exact).norm())
+    first = torch.autograd.grad(ops.linear_group(x, ws, bs)[0], x, dys[0])[0]
+    assert torch.equal(first, torch.autograd.grad(ops.linear(x, ws[0], bs[0]), x, dys[0])[0])
+    with torch.no_grad():
+        assert all(torch.equal(a, b) for a, b in zip(ops.linear_group(x, ws, bs), [ops.linear(x, w, b) for w, b in zip(ws, bs)]))

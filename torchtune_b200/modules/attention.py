@@ -133,7 +133,8 @@ class MultiHeadAttention(nn.Module):
         k = v = None
         projections = (self.q_proj, self.k_proj, self.v_proj)
         # torch's own linear layers keep torch's own product, which autocast, tensor subclasses and modes that look at operations know
-        if y is x and not torch.is_grad_enabled() and all(type(m) is Linear and is_plain_linear(m) for m in projections):
+        # (inside autograd where the joined form has a gradient of its own)
+        if y is x and (not torch.is_grad_enabled() or ops.joins_gradients(x)) and all(type(m) is Linear and is_plain_linear(m) for m in projections):
             q, k, v = ops.linear_group(x, [m.weight for m in projections], [m.bias for m in projections])
         else:
             q = self.q_proj(x)

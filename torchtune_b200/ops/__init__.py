@@ -128,14 +128,24 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return F.linear(x, weight, bias)
 
 
-def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Sequence[Optional[torch.Tensor]]) -> List[torch.Tensor]:
-    """``[linear(x, w, b) for w, b in zip(weights, biases)]``; a few bf16 CUDA tokens outside autograd take all of them in one launch."""
-    if _native(x) and not _differentiated(x, *weights, *biases):
+def joins_gradients(x: torch.Tensor) -> bool:
+    """Whether :func:`linear_group` of this input has a gradient of its own."""
+    return type(x) is torch.Tensor and _native(x) and _has_memory(x) and torch.autograd.forward_ad._current_level < 0
+
+
+def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Sequence[Optional[torch.Tensor]]) -> Sequence[torch.Tensor]:
+    """``[linear(x, w, b) for w, b in zip(weights, biases)]``; a few bf16 CUDA tokens outside autograd take all of them in one launch, and inside autograd
+    the products of their input gradients add up without a pass of their own."""
+    if _native(x):
         from . import _cuda
 
-        ys = _cuda.linear_group(x, weights, biases)
-        if ys is not None:
-            return ys
+        if not _differentiated(x, *weights, *biases):
+            ys = _cuda.linear_group(x, weights, biases)
+            if ys is not None:
+                return ys
+        elif (len(weights) > 1 and joins_gradients(x) and _has_memory(*weights, *(b for b in biases if b is not None)) and x.shape[-1] % 8 == 0 and x.numel() > 0
+              and all(w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[1] == x.shape[-1] and w.shape[0] % 8 == 0 for w in weights)):
+            return _cuda.linear_group_differentiated(x, weights, biases)
     return [linear(x, w, b) for w, b in zip(weights, biases)]
 
 

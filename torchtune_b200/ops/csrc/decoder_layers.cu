@@ -33,7 +33,7 @@ int ttb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, in
                   float alpha, int* err, void* stream);
 int ttb_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int accumulate, const void* bias, float alpha,
                       int* err, void* stream);
-int ttb_gemm_bf16_2sm_residual(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb, long long ldc, long long ldr, const void* bias, int* err,
+int ttb_gemm_bf16_2sm_residual(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int b_mn, long long lda, long long ldb, long long ldc, long long ldr, const void* bias, int* err,
                                void* stream);
 int ttb_gemm_bf16_splitk(const void* A, const void* B, float* work, void* C, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int out_fp32, int accumulate,
                          const void* bias, const void* residual, long long ldr, int splits, float alpha, int* err, void* stream);
@@ -152,7 +152,7 @@ struct Call {
       ok(ttb_gemm_bf16_splitk(x, w, split, y, M, N, K, 0, 0, K, K, N, 0, 0, bias, residual, residual == nullptr ? 0 : N, splits, 1.f, err, st));
     } else if (fills_pairs(M, N, K)) {
       ok(residual == nullptr ? ttb_gemm_bf16_2sm(x, w, y, M, N, K, 0, 0, K, K, N, 0, bias, 1.f, err, st)
-                             : ttb_gemm_bf16_2sm_residual(x, w, y, residual, M, N, K, K, K, N, N, bias, err, st));
+                             : ttb_gemm_bf16_2sm_residual(x, w, y, residual, M, N, K, 0, K, K, N, N, bias, err, st));
     } else if (ok(ttb_gemm_bf16(x, w, y, M, N, K, 0, 0, K, K, N, 0, 0, bias, 1.f, err, st)) && residual != nullptr) {
       const long long n = static_cast<long long>(M) * N / 8, blocks = (n + 255) / 256;
       TTB_COUNT_LAUNCH(1);

@@ -648,10 +648,10 @@ extern "C" int ttb_gemm_swiglu_bf16_2sm(const void* X, const void* W1, const voi
 }
 
 
-// C[M,N] = A[M,K] · B[N,K]ᵀ (+ bias) + R[M,N]: a linear layer whose output is added to the residual stream in the GEMM epilogue (the
+// C[M,N] = A[M,K] · op(B) (+ bias) + R[M,N] (b_mn = 0: B [N, K], 1: [K, N]): a linear layer whose output is added to the residual stream in the GEMM epilogue (the
 // attention output projection and the MLP down projection of a decoder layer, torchtune/modules/transformer.py:119-135), so the separate
 // element-wise add and its re-read of both tensors disappear.  R: bf16, row pitch ldr (multiple of 8), 16-byte aligned; R may not alias C.
-extern "C" int ttb_gemm_bf16_2sm_residual(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb, long long ldc,
+extern "C" int ttb_gemm_bf16_2sm_residual(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int b_mn, long long lda, long long ldb, long long ldc,
                                           long long ldr, const void* bias, int* err, void* stream) {
   using namespace ttb;
   if (M <= 0 || N <= 0 || K <= 0 || R == nullptr) return kErrBadShape;
@@ -661,7 +661,8 @@ extern "C" int ttb_gemm_bf16_2sm_residual(const void* A, const void* B, void* C,
   p.residual = static_cast<const __nv_bfloat16*>(R), p.ldr = ldr;
   p.accumulate = 0, p.tma_store = 0, p.save_gate_up = 0, p.tile_mult = 1, p.err = err;
   p.group_m = g2::group_setting();
-  return g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
+  auto s = static_cast<cudaStream_t>(stream);
+  return b_mn ? g2::launch<false, true, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, s) : g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, s);
 }
 
 // C[M,N] = float(bf16(A[M,K] · B[N,K]ᵀ (+ bias))): fp32 logits with the values of a bf16 output projection, without a pass of its own that widens them.
