@@ -119,3 +119,47 @@ def test_softmax_statistics_of_the_logits_product(T, D, V):
     p *= seen[:, None]
     for got, exact in ((h.grad, p @ w.double()), (w.grad, p.t() @ h.double())):
         assert float((got.double() - exact).norm()) <= 2.0**-7 * float(exact.norm())  # p and the result are rounded to bf16
+
+
+@pytest.mark.parametrize("T,V", [(16, 128), (700, 20000)])
+def test_mean_loss(T, V):
+    """The mean's gradients with and without statistics of the softmax, for factors of one and others, kept graphs, hooks on saved tensors, batched factors, and no valid token."""
+    from torchtune_b200 import ops
+    from torchtune_b200.modules.loss import LinearCrossEntropyLoss
+
+    h, w = _logits(T, 64, torch.bfloat16, T).requires_grad_(), (_logits(V, 64, torch.bfloat16, V) * 0.1).requires_grad_()
+    labels = torch.randint(0, V, (T,), device="cuda")
+    labels[::3] = -100
+    total, count = ops.linear_cross_entropy(h, w, labels)
+    sums = torch.autograd.grad(total, (h, w))
+    mean = lambda: ops.linear_cross_entropy_mean(h, w, labels)
+    exact = [g.double() / int(count) for g in sums]
+    assert abs(float(mean().detach()) - float(total.detach()) / int(count)) <= 2.0**-20 * abs(float(total.detach()))
+
+    def near(got, factor=1.0):
+        for a, e in zip(got, exact):
+            assert float((a.double() - factor * e).norm()) <= 2.0**-7 * abs(factor) * float(e.norm())  # a rounding to bf16 on each side, and one more of a rescaled result
+
+    near(torch.autograd.grad(mean(), (h, w)))
+    near(torch.autograd.grad(mean() * -2.5, (h, w)), -2.5)
+    loss = mean()
+    kept = torch.autograd.grad(loss, (h, w), retain_graph=True)
+    again = torch.autograd.grad(loss, (h, w), torch.tensor(4.0, device="cuda"), retain_graph=True)
+    once_more = torch.autograd.grad(loss, (h, w))
+    assert all(torch.equal(a, c) and torch.equal(4 * a, b) for a, b, c in zip(kept, again, once_more))
+    many = torch.autograd.grad(mean(), (h, w), torch.tensor([1.0, -2.0], device="cuda"), is_grads_batched=True)
+    assert all(torch.equal(m, torch.stack([a, -2 * a])) for m, a in zip(many, kept))
+    held = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: held.append(t) or t, lambda t: t):
+        loss = mean()
+    before = [t.clone() for t in held]
+    near(torch.autograd.grad(loss * 3, (h, w)), 3.0)
+    assert all(torch.equal(a, b) for a, b in zip(held, before))
+    labels.fill_(-100)
+    loss = mean()
+    assert float(loss.detach()) == 0.0 and all(not g.any() for g in torch.autograd.grad(loss, (h, w)))
+    module = LinearCrossEntropyLoss()
+    module.linear_projection = torch.nn.Linear(64, V, bias=False, device="cuda", dtype=torch.bfloat16)
+    labels[1::3] = 5
+    got, want = module(h, labels), torch.nn.functional.cross_entropy((h.double() @ module.linear_projection.weight.double().t()), labels)
+    assert abs(float(got.detach()) - float(want.detach())) <= 0.02 * abs(float(want.detach()))

@@ -62,6 +62,11 @@ class LinearCrossEntropyLoss(nn.Module, SFTLoss):
         return ops.linear_cross_entropy(outputs, self._weight(), targets, self.ignore_index, self.num_output_chunks)
 
     def forward(self, outputs: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        plain = type(self).compute_sum is LinearCrossEntropyLoss.compute_sum and "compute_sum" not in self.__dict__
+        if plain and self.logit_softcap <= 0.0 and not hasattr(self.linear_projection, "linear_cross_entropy"):
+            mean = ops.linear_cross_entropy_mean(outputs, self._weight(), targets, self.ignore_index, self.num_output_chunks)
+            if mean is not None:
+                return mean
         total, n_valid = self.compute_sum(outputs, targets)
         if isinstance(n_valid, torch.Tensor):
             return total / n_valid.clamp_min(1).to(total.dtype)

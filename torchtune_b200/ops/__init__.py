@@ -45,6 +45,7 @@ __all__ = [
     "swiglu",
     "attention",
     "linear_cross_entropy",
+    "linear_cross_entropy_mean",
     "token_logprobs",
     "embedding",
     "embed_tokens",
@@ -440,6 +441,15 @@ def linear_cross_entropy(
 
         return _cuda.linear_cross_entropy(hidden, weight, labels, ignore_index, num_chunks, softcap)
     return reference.linear_cross_entropy(hidden, weight, labels, ignore_index, num_chunks, softcap=softcap)
+
+
+def linear_cross_entropy_mean(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, ignore_index: int = -100, num_chunks: int = 8) -> Optional[torch.Tensor]:
+    """``total / max(count, 1)`` of :func:`linear_cross_entropy`, with gradients that are formed for the mean; ``None`` where that has no kernel."""
+    if _native(hidden) and weight.dtype == torch.bfloat16 and _has_memory(hidden, weight, labels):
+        from . import _cuda
+
+        return _cuda.linear_cross_entropy_mean(hidden, weight, labels, ignore_index, num_chunks)
+    return None
 
 
 def token_logprobs(

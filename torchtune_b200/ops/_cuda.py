@@ -1412,9 +1412,32 @@ def _scaled(t: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def _rescaled(t: torch.Tensor, factor: torch.Tensor, mine: bool) -> torch.Tensor:
+    """:func:`_scaled`, in place where the gradient is ``mine`` (nobody keeps it after this backward pass): a factor of one then costs a launch."""
+    from . import _differentiated, _has_memory
+
+    if not mine or t.dtype != _BF16 or factor.dtype != torch.float32 or not _has_memory(t, factor) or _differentiated(t, factor) or t.numel() % 8 or t.data_ptr() % 16:
+        return _scaled(t, factor)
+    check(lib().ttb_scale_bf16(t.data_ptr(), t.data_ptr(), t.numel(), factor.data_ptr(), stream_ptr()), "scale")
+    return t
+
+
 # Above this many bytes of bf16 logits the token dimension is processed in chunks; below it the
 # whole batch is one pass (one logits GEMM, one dgrad, one wgrad written once in bf16).
 _CE_SINGLE_PASS_BYTES = 6 * 2**30
+
+
+def _gemm_scaled(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, factor: torch.Tensor, *, a_mn: bool) -> None:
+    """``out = factor · op(a) · b`` (``b`` ``[K, N]``) with a factor on the device, in the epilogue of the CTA-pair kernel or in a pass over a (then small) result."""
+    M, K = (a.shape[1], a.shape[0]) if a_mn else a.shape
+    N = b.shape[1]
+    fit = all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (a, b, out))
+    if fit and (M if a_mn else K) % 8 == 0 and N % 8 == 0 and _splits(M, N, K) == 1 and _use_pair_kernel(M, N, K, out):
+        check(lib().ttb_gemm_bf16_2sm_scaled(a.data_ptr(), b.data_ptr(), out.data_ptr(), factor.data_ptr(), M, N, K, int(a_mn), 1, a.stride(0), b.stride(0), out.stride(0),
+                                             err_word(a.device).data_ptr(), stream_ptr()), f"gemm (CTA pairs, scaled) M={M} N={N} K={K}")
+        return
+    gemm(a, b, a_mn=a_mn, b_mn=True, out=out)
+    check(lib().ttb_scale_bf16(out.data_ptr(), out.data_ptr(), out.numel(), factor.data_ptr(), stream_ptr()), "scale")
 
 
 def _ce_stats(h: torch.Tensor, weight: torch.Tensor, logits: torch.Tensor, softcap: float) -> bool:
@@ -1432,7 +1455,10 @@ class _LinearCE(torch.autograd.Function):
     only used when the full logits buffer would exceed ``_CE_SINGLE_PASS_BYTES``."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0):
+    def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0, mean=False):
+        """``mean``: the loss is the mean over the valid tokens, and so are, in a single pass, the gradients: 1 / count multiplies the sums of the products that make them, before they are rounded,
+        instead of both results in a pass of its own (1 GB of weight gradient for a vocabulary of 128256 x 4096: 0.33 ms).  It may not go into the gradient of the logits: that is nearly -1, which bf16
+        holds exactly, at every label."""
         D = hidden.shape[-1]
         h2 = hidden.reshape(-1, D)
         if not h2.is_contiguous():
@@ -1453,6 +1479,9 @@ class _LinearCE(torch.autograd.Function):
         if need_w and not direct:
             dw = torch.empty(V, D, dtype=_BF16, device=h2.device) if single else torch.zeros(V, D, dtype=torch.float32, device=h2.device)
         buf = torch.empty(min(rows, T), V, dtype=_BF16, device=h2.device)
+        n_valid = (y != ignore_index).sum()
+        share = n_valid.clamp_min(1).to(torch.float32).reciprocal() if mean else None
+        folded = mean and single and not direct
         L = lib()
         for start in range(0, T, rows):
             n = min(rows, T - start)
@@ -1464,10 +1493,16 @@ class _LinearCE(torch.autograd.Function):
                 check(L.ttb_gemm_bf16_2sm_stats(hc.data_ptr(), weight.data_ptr(), lg.data_ptr(), stats.data_ptr(), n, V, D, hc.stride(0), weight.stride(0), lg.stride(0),
                                                 err_word(h2.device).data_ptr(), stream_ptr()), f"logits and their statistics T={n} V={V} D={D}")
                 check(L.ttb_softmax_ce_stats(lg.data_ptr(), stats.data_ptr(), y[start : start + n].data_ptr(), loss_rows[start : start + n].data_ptr(), lse.data_ptr(), n, V, lg.stride(0),
-                                             int(ignore_index), 1 - mode, None, stream_ptr()), "softmax_ce_stats")
+                                             int(ignore_index), 1 - mode, stream_ptr()), "softmax_ce_stats")
             else:
                 gemm(hc, weight, out=lg)
                 _softmax_ce(lg, y[start : start + n], loss_rows[start : start + n], None, n, V, ignore_index, mode, softcap)
+            if folded:
+                if need_h:
+                    _gemm_scaled(lg, weight, dh, share, a_mn=False)
+                if need_w:
+                    _gemm_scaled(lg, hc, dw, share, a_mn=True)
+                break
             if need_h:
                 gemm(lg, weight, b_mn=True, out=dh[start : start + n])
             if direct:
@@ -1475,23 +1510,27 @@ class _LinearCE(torch.autograd.Function):
                 owner._grad_written = True
             elif need_w:
                 gemm(lg, hc, a_mn=True, b_mn=True, out=dw, accumulate=not single)
-        ctx.save_for_backward(dh, dw)
+        ctx.save_for_backward(dh, dw, None if folded else share)
+        ctx.hooked = torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
         ctx.h_shape = hidden.shape
         ctx.w_dtype = weight.dtype
         ctx.direct = direct
-        n_valid = (y != ignore_index).sum()
         ctx.mark_non_differentiable(n_valid)
-        return loss_rows.sum(), n_valid
+        total = loss_rows.sum()
+        return (total / n_valid.clamp_min(1).to(total.dtype) if mean else total), n_valid
 
     @staticmethod
     def backward(ctx, g_loss, _g_count):
-        dh, dw = ctx.saved_tensors
-        # The gradients were formed for d(loss_sum) = 1; an upstream factor multiplies them.
+        dh, dw, share = ctx.saved_tensors
+        # The gradients were formed for d(loss) = 1 (of the sum, with `share`); an upstream factor multiplies them.
         # With direct delivery the weight gradient already sits in the flat buffer, which is
         # only valid for an upstream factor of one (the recipes back-propagate the sum itself).
-        gh = _scaled(dh, g_loss).view(ctx.h_shape) if dh is not None else None
-        gw = _scaled(dw, g_loss).to(ctx.w_dtype) if dw is not None else None
-        return gh, gw, None, None, None, None
+        if share is not None:
+            g_loss = g_loss * share
+        mine = not (ctx.hooked or torch._C._autograd._get_current_graph_task_keep_graph())
+        gh = _rescaled(dh, g_loss, mine).view(ctx.h_shape) if dh is not None else None
+        gw = _rescaled(dw, g_loss, mine).to(ctx.w_dtype) if dw is not None else None
+        return gh, gw, None, None, None, None, None
 
 
 def linear_cross_entropy(hidden, weight, labels, ignore_index: int, num_chunks: int, softcap: float = 0.0):
@@ -1501,6 +1540,12 @@ def linear_cross_entropy(hidden, weight, labels, ignore_index: int, num_chunks: 
         _fallback("linear_cross_entropy", f"width {hidden.shape[-1]} or vocabulary {weight.shape[0]} is not a multiple of 8", hidden)
         return reference.linear_cross_entropy(hidden, weight, labels, ignore_index, num_chunks, softcap=softcap)
     return _LinearCE.apply(hidden, weight, labels, ignore_index, num_chunks, float(softcap))
+
+
+def linear_cross_entropy_mean(hidden, weight, labels, ignore_index: int, num_chunks: int) -> Optional[torch.Tensor]:
+    if hidden.shape[-1] % 8 or weight.shape[0] % 8:
+        return None
+    return _LinearCE.apply(hidden, weight, labels, ignore_index, num_chunks, 0.0, True)[0]
 
 
 def _softmax_ce(buf, labels, loss_out, row_scale, n, V, ignore_index, mode, softcap=0.0):
@@ -1517,7 +1562,10 @@ class _TokenLogprobs(torch.autograd.Function):
     chunk and scales the in-place softmax gradient by the incoming per-token gradient."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0):
+    def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0, mean=False):
+        """``mean``: the loss is the mean over the valid tokens, and so are, in a single pass, the gradients: 1 / count multiplies the sums of the products that make them, before they are rounded,
+        instead of both results in a pass of its own (1 GB of weight gradient for a vocabulary of 128256 x 4096: 0.33 ms).  It may not go into the gradient of the logits: that is nearly -1, which bf16
+        holds exactly, at every label."""
         D = hidden.shape[-1]
         h2 = hidden.reshape(-1, D).contiguous()
         y = labels.reshape(-1).to(torch.int64).contiguous()

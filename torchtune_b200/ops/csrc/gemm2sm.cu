@@ -58,6 +58,7 @@ struct Params {
   const __nv_bfloat16* residual;  // [M, N] (row pitch ldr) added to the product in the epilogue (the residual stream of a decoder layer), or null
   long long ldr;
   float alpha;
+  const float* factor;  // another one, on the device, or null
   int accumulate;
   float2* stats;  // [n tiles, M]: maximum of a row's results in a tile and the sum of their exponentials relative to it (as stored, in bf16), or null
   int out_f32;  // C is fp32 and holds the results rounded to bf16 (vocabulary logits that callers want widened)
@@ -241,6 +242,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ epilogue (both CTAs, own 128 rows)
     const int quarter = warp & 3;
+    const float alpha = p.factor != nullptr ? p.alpha * __ldg(p.factor) : p.alpha;
     int acc = 0;
     uint32_t acc_phase = 0;
     int buf_toggle = 0;
@@ -331,7 +333,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             float f[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              f[i] = __uint_as_float(r[j * 4 + i]) * p.alpha;
+              f[i] = __uint_as_float(r[j * 4 + i]) * alpha;
               if (p.bias != nullptr && col0 + j * 4 + i < p.N) f[i] += __bfloat162float(__ldg(p.bias + col0 + j * 4 + i));
               f[i] = __bfloat162float(__float2bfloat16_rn(f[i]));
             }
@@ -363,7 +365,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int j = 0; j < 4; ++j) {
               float f[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[j * 8 + i]) * p.alpha;
+              for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[j * 8 + i]) * alpha;
               if (p.bias != nullptr) {
                 const int cb = col0 + h * 32 + j * 8;
 #pragma unroll
@@ -428,7 +430,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (row < p.M && col0 < p.N) {
             float v[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * alpha;
             if (p.bias != nullptr) {
 #pragma unroll
               for (int i = 0; i < 32; ++i)
@@ -688,4 +690,18 @@ extern "C" int ttb_gemm_bf16_2sm_stats(const void* A, const void* B, void* C, fl
   p.stats = reinterpret_cast<float2*>(stats), p.tile_mult = 1, p.err = err;
   p.group_m = g2::group_setting();
   return g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
+}
+
+// ttb_gemm_bf16_2sm without bias or accumulation, times a factor that lies on the device: gradients of a mean need no pass that divides them.
+extern "C" int ttb_gemm_bf16_2sm_scaled(const void* A, const void* B, void* C, const float* factor, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int* err,
+                                        void* stream) {
+  using namespace ttb;
+  if (M <= 0 || N <= 0 || K <= 0 || factor == nullptr || !b_mn) return kErrBadShape;
+  if ((lda & 7) || (ldb & 7) || (ldc & 7) || (N & 7) || (a_mn ? (M & 7) : (K & 7))) return kErrBadShape;
+  g2::Params p{};
+  p.M = M, p.N = N, p.K = K, p.C = C, p.ldc = ldc, p.alpha = 1.f, p.factor = factor;
+  p.tile_mult = 1, p.err = err;
+  p.group_m = g2::group_setting();
+  auto s = static_cast<cudaStream_t>(stream);
+  return a_mn ? g2::launch<true, true, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, s) : g2::launch<false, true, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, s);
 }

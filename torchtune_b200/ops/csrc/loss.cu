@@ -174,9 +174,9 @@ ce_merge_kernel(const float2* __restrict__ stats, const __nv_bfloat16* __restric
   loss_out[row] = ignored ? 0.f : lse - __bfloat162float(logits[row * ld + label]);
 }
 
-// logits <- (softmax - onehot) * scale, rows with lse = inf <- 0.  blockIdx.y: row.
+// logits <- softmax - onehot, rows with lse = inf <- 0.  blockIdx.y: row.
 __global__ void __launch_bounds__(256)
-ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ lse, int V, long long ld, const float* __restrict__ scale) {
+ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ lse, int V, long long ld) {
   const long long row = blockIdx.y;
   uint4* lr = reinterpret_cast<uint4*>(logits + row * ld);
   const int nvec = V >> 3, first = blockIdx.x * 1024 + threadIdx.x;
@@ -188,7 +188,6 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__
     return;
   }
   const int label = static_cast<int>(labels[row]);
-  const float f = scale != nullptr ? *scale : 1.f;
   uint4 u[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -204,7 +203,7 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__
       float g0 = __expf(t.x - z), g1 = __expf(t.y - z);
       if (i * 8 + 2 * k == label) g0 -= 1.f;
       if (i * 8 + 2 * k + 1 == label) g1 -= 1.f;
-      b[k] = __floats2bfloat162_rn(g0 * f, g1 * f);
+      b[k] = __floats2bfloat162_rn(g0, g1);
     }
     lr[i] = u[j];
   }
@@ -288,9 +287,11 @@ token_logprob_kernel(const float* __restrict__ x, long long stride_outer, long l
 // ----------------------------------------------------------------------------- gradient times a scalar on the device
 // y = bf16(x · *factor); 16 bytes per lane and load, bound by memory: 128 256 x 2048 in 174 us (6.0 TB/s), where
 // the broadcast multiplication of tensors, two bytes at a time, took 859 us.
+// In place a factor of one, that of a loss that is differentiated by itself, needs no pass at all.
 __global__ void __launch_bounds__(256)
-scale_bf16_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, long long nvec, const float* __restrict__ factor) {
+scale_bf16_kernel(const uint4* x, uint4* y, long long nvec, const float* __restrict__ factor) {
   const float f = *factor;
+  if (f == 1.f && x == y) return;
   const long long step = static_cast<long long>(gridDim.x) * 256;
   auto scaled = [&](uint4 u) {
     __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&u);
@@ -465,9 +466,9 @@ extern "C" int ttb_softmax_ce(void* logits, const long long* labels, float* loss
 }
 
 // Loss of every row (0 where the label is ignore_index) from the statistics that ttb_gemm_bf16_2sm_stats left; lse [rows] is scratch.  With grad the logits become the gradient
-// (softmax - onehot) * scale[0] (scale nullable: 1), in place.
+// softmax - onehot, in place.
 extern "C" int ttb_softmax_ce_stats(void* logits, const float* stats, const long long* labels, float* loss_out, float* lse, int rows, int V, long long ld, long long ignore_index, int grad,
-                                    const float* scale, void* stream) {
+                                    void* stream) {
   if ((V & 7) || (ld & 7) || (reinterpret_cast<uintptr_t>(logits) & 15) || V <= 0) return kErrBadShape;
   if (rows <= 0) return kOk;
   auto st = static_cast<cudaStream_t>(stream);
@@ -478,7 +479,7 @@ extern "C" int ttb_softmax_ce_stats(void* logits, const float* stats, const long
     for (int r = 0; r < rows; r += 65535) {  // rows of one launch: the grid's second dimension
       const int n = rows - r < 65535 ? rows - r : 65535;
       TTB_COUNT_LAUNCH(1);
-      ce_grad_kernel<<<dim3((V / 8 + 1023) / 1024, n), 256, 0, st>>>(lg + r * ld, labels + r, lse + r, V, ld, scale);
+      ce_grad_kernel<<<dim3((V / 8 + 1023) / 1024, n), 256, 0, st>>>(lg + r * ld, labels + r, lse + r, V, ld);
     }
   }
   return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
@@ -509,7 +510,7 @@ extern "C" int ttb_token_logprobs_f32(const float* x, long long stride_outer, lo
   return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
 }
 
-// y = bf16(x * factor[0]) for n bf16 values (a multiple of 8, 16-byte aligned).
+// y = bf16(x * factor[0]) for n bf16 values (a multiple of 8, 16-byte aligned); y may be x.
 extern "C" int ttb_scale_bf16(const void* x, void* y, long long n, const float* factor, void* stream) {
   if (n <= 0) return kOk;
   if ((n & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(y) & 15)) return kErrBadShape;
