@@ -129,3 +129,49 @@ def test_linear_layers_of_one_input(M, N, Ks):
     assert torch.equal(first, torch.autograd.grad(ops.linear(x, ws[0], bs[0]), x, dys[0])[0])
     with torch.no_grad():
         assert all(torch.equal(a, b) for a, b in zip(ops.linear_group(x, ws, bs), [ops.linear(x, w, b) for w, b in zip(ws, bs)]))
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (9, 264), (592, 1024), (3001, 4096), (31, 2056)])
+def test_gain_gradient(rows, D):
+    from torchtune_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, dy = (torch.randn(rows, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    gain = torch.ones(D, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    got, = torch.autograd.grad(ops.rms_norm(x, gain, 1e-5), gain, dy)
+    terms = dy.double() * x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5)
+    assert ((got.double() - terms.sum(0)).abs() <= 2.0**-8 * terms.sum(0).abs() + 2.0**-18 * terms.abs().sum(0)).all()  # one rounding, fp32 sums
+
+
+@pytest.mark.parametrize("n,dim,run", [(1, 8, 1), (7, 64, 7), (8, 264, 8), (9, 2056, 9), (666, 2048, 300), (5000, 128, 4097)])
+def test_embedding_gradient_of_long_runs(n, dim, run):
+    """One id for `run` tokens, the end of a run inside and on a group of eight: sums in the order of the tokens."""
+    from torchtune_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = torch.randint(0, 50, (n,), generator=g, device="cuda")
+    ids[torch.randperm(n, generator=g, device="cuda")[:run]] = 3
+    table = torch.zeros(64, dim, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    dy = torch.randn(n, dim, generator=g, device="cuda").to(torch.bfloat16)
+    got, = torch.autograd.grad(ops.embedding(ids, table), table, dy)
+    want, size = (torch.zeros(64, dim, device="cuda", dtype=torch.float64).index_add_(0, ids, t) for t in (dy.double(), dy.double().abs()))
+    assert ((got.double() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-23 * run * size).all()  # one rounding, fp32 sums one after the other
+
+
+@pytest.mark.parametrize("b,s,hq,hkv,D", [(1, 1, 1, 1, 64), (3, 7, 3, 1, 128), (2, 333, 32, 8, 64), (1, 129, 20, 4, 128)])
+def test_attention_gradient_of_ragged_tokens(b, s, hq, hkv, D):
+    """The products of outputs and their gradients, eight tokens at a time, where tokens and heads fill no group."""
+    from torchtune_b200 import ops
+    from torchtune_b200.ops import AttentionMask
+
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randn(b, s, h, D, generator=g, device="cuda").to(torch.bfloat16).requires_grad_() for h in (hq, hkv, hkv))
+    dy = torch.randn(b, s, hq, D, generator=g, device="cuda").to(torch.bfloat16)
+    got = torch.autograd.grad(ops.attention(q, k, v, AttentionMask(causal=True)), (q, k, v), dy)
+    leaves = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    kk, vv = (t.repeat_interleave(hq // hkv, 2) for t in leaves[1:])
+    scores = torch.einsum("bqhd,bkhd->bhqk", leaves[0], kk) * D**-0.5
+    p = torch.softmax(scores.masked_fill(~torch.ones(s, s, dtype=torch.bool, device="cuda").tril(), float("-inf")), -1)
+    want = torch.autograd.grad(torch.einsum("bhqk,bkhd->bqhd", p, vv), leaves, dy.double())
+    for a, e in zip(got, want):
+        assert float((a.double() - e).norm()) <= 0.01 * float(e.norm()) + 1e-3  # probabilities and their gradients are rounded to bf16 once each

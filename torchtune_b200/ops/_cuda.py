@@ -1120,7 +1120,10 @@ class _RMSNorm(torch.autograd.Function):
             n_part = lib().ttb_rmsnorm_bwd_partials(rows)
             partial = torch.empty(n_part, D, dtype=torch.float32, device=x2.device)
         check(lib().ttb_rmsnorm_bwd(dy2.data_ptr(), x2.data_ptr(), _ptr(scale), rstd.data_ptr(), dx.data_ptr(), _ptr(partial), rows, D, stream_ptr()), "rmsnorm_bwd")
-        dscale = partial.sum(0).to(scale.dtype) if partial is not None else None
+        dscale = None
+        if partial is not None:
+            dscale = torch.empty_like(scale)
+            check(lib().ttb_column_sum(partial.data_ptr(), dscale.data_ptr(), partial.shape[0], D, stream_ptr()), "gain gradient")
         return dx.view(dy.shape), dscale, None
 
 

@@ -45,6 +45,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_rmsnorm_fwd.argtypes = [vp, vp, vp, vp, i32, i32, f32, vp]
     L.ttb_rmsnorm_bwd_partials.argtypes = [i32]
     L.ttb_rmsnorm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, vp]
+    L.ttb_column_sum.argtypes = [vp, vp, i32, i32, vp]
+    L.ttb_column_sum.restype = i32
     L.ttb_rope.argtypes = [vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, vp]
     L.ttb_kd_divergence.argtypes = [vp, vp, vp, vp, vp, i32, i32, i64, i64, i64, i64, f32, f32, vp]
     L.ttb_kd_divergence.restype = i32

@@ -446,6 +446,40 @@ extern "C" int ttb_rmsnorm_fwd(const void* x, const void* scale, void* y, float*
   return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
 }
 
+namespace ttb {
+// out[D] = bf16(sum over n rows of part): 32 columns per CTA, rows dealt to eight warps with four loads in flight each.  The norm's gain gradient of 592 x 4096 partial sums: 26 us and a
+// launch that converts with the general reduction, 12 us here; of 592 x 2048 17.7 -> 6.8 us.
+__global__ void __launch_bounds__(256) column_sum_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int n, int D) {
+  __shared__ float sums[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  if (col < D) {
+    int r = warp;
+    for (; r + 24 < n; r += 32) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] += part[static_cast<long long>(r + 8 * j) * D + col];
+    }
+    for (; r < n; r += 8) acc[0] += part[static_cast<long long>(r) * D + col];
+  }
+  sums[warp][lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+  __syncthreads();
+  if (warp == 0 && col < D) {
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) total += sums[w][lane];
+    out[col] = __float2bfloat16_rn(total);
+  }
+}
+}  // namespace ttb
+
+// out[D] bf16 = sum over dim 0 of part [n, D] fp32.
+extern "C" int ttb_column_sum(const float* part, void* out, int n, int D, void* stream) {
+  if (n <= 0 || D <= 0) return kErrBadShape;
+  TTB_COUNT_LAUNCH(1);
+  column_sum_kernel<<<(D + 31) / 32, 256, 0, static_cast<cudaStream_t>(stream)>>>(part, static_cast<__nv_bfloat16*>(out), n, D);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrDriver;
+}
+
 // dscale_partial: [*n_partials_out rows, D] fp32, caller sums over dim 0.  The caller sizes it
 // with ttb_rmsnorm_bwd_partials().
 extern "C" int ttb_rmsnorm_bwd_partials(int rows) {
