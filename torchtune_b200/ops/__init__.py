@@ -145,7 +145,7 @@ def linear_group(x: torch.Tensor, weights: Sequence[torch.Tensor], biases: Seque
             if ys is not None:
                 return ys
         elif (len(weights) > 1 and joins_gradients(x) and _has_memory(*weights, *(b for b in biases if b is not None)) and x.shape[-1] % 8 == 0 and x.numel() > 0
-              and all(w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[1] == x.shape[-1] and w.shape[0] % 8 == 0 for w in weights)):
+              and all(w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[1] == x.shape[-1] and w.shape[0] > 0 and w.shape[0] % 8 == 0 for w in weights)):
             return _cuda.linear_group_differentiated(x, weights, biases)
     return [linear(x, w, b) for w, b in zip(weights, biases)]
 

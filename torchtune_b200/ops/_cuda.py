@@ -1122,7 +1122,7 @@ class _RMSNorm(torch.autograd.Function):
         check(lib().ttb_rmsnorm_bwd(dy2.data_ptr(), x2.data_ptr(), _ptr(scale), rstd.data_ptr(), dx.data_ptr(), _ptr(partial), rows, D, stream_ptr()), "rmsnorm_bwd")
         dscale = None
         if partial is not None:
-            dscale = torch.empty_like(scale)
+            dscale = torch.empty(D, dtype=_BF16, device=x2.device)
             check(lib().ttb_column_sum(partial.data_ptr(), dscale.data_ptr(), partial.shape[0], D, stream_ptr()), "gain gradient")
         return dx.view(dy.shape), dscale, None
 
@@ -1565,10 +1565,7 @@ class _TokenLogprobs(torch.autograd.Function):
     chunk and scales the in-place softmax gradient by the incoming per-token gradient."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0, mean=False):
-        """``mean``: the loss is the mean over the valid tokens, and so are, in a single pass, the gradients: 1 / count multiplies the sums of the products that make them, before they are rounded,
-        instead of both results in a pass of its own (1 GB of weight gradient for a vocabulary of 128256 x 4096: 0.33 ms).  It may not go into the gradient of the logits: that is nearly -1, which bf16
-        holds exactly, at every label."""
+    def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0):
         D = hidden.shape[-1]
         h2 = hidden.reshape(-1, D).contiguous()
         y = labels.reshape(-1).to(torch.int64).contiguous()

@@ -143,6 +143,8 @@ class _FlashAttention(torch.autograd.Function):
         b, s, hq, d = q.shape
         sk, hkv = k.shape[1], k.shape[2]
         d_o = d_o.contiguous()
+        if o.data_ptr() % 16:  # handed back by a saved-tensor hook
+            o = o.clone()
         delta = torch.empty(b, hq, s, dtype=torch.float32, device=q.device)
         dq_acc = torch.zeros(b, s, hq, d, dtype=torch.float32, device=q.device)
         dk = torch.empty_like(k)

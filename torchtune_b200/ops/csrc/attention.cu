@@ -375,8 +375,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 static constexpr int kDeltaTokens = 8;
 template <int D>
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta, long long tokens, int s, int hq) {
-  extern __shared__ float sums[];  // [hq][kDeltaTokens]
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta, long long tokens, int s, int hq, bool staged) {
+  extern __shared__ float sums[];  // [hq][kDeltaTokens]; without `staged`, for more heads than fit, results leave one by one
   constexpr int kLanes = D / 8, kItems = 256 / kLanes;
   const long long tok0 = blockIdx.x * static_cast<long long>(kDeltaTokens);
   const int count = static_cast<int>(min(static_cast<long long>(kDeltaTokens), tokens - tok0)) * hq;
@@ -404,9 +404,16 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 #pragma unroll
       for (int off = kLanes / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
       const int item = first + j * kItems;
-      if (lane == 0 && item < count) sums[item % hq * kDeltaTokens + item / hq] = acc;
+      if (lane == 0 && item < count) {
+        const long long tok = tok0 + item / hq;
+        if (staged)
+          sums[item % hq * kDeltaTokens + item / hq] = acc;
+        else
+          delta[(tok / s * hq + item % hq) * s + tok % s] = acc;
+      }
     }
   }
+  if (!staged) return;
   __syncthreads();
   for (int i = threadIdx.x; i < hq * kDeltaTokens; i += 256) {
     const long long tok = tok0 + i % kDeltaTokens;
@@ -781,11 +788,12 @@ extern "C" int ttb_attn_bwd(const void* q, const void* k, const void* v, const v
   if (causal && hi == nullptr && s != sk) return kErrBadShape;
   auto st = static_cast<cudaStream_t>(stream);
   const long long tokens = static_cast<long long>(b) * s;
-  const int smem = hq * kDeltaTokens * 4;
-  if (smem > 48 * 1024) return kErrTooLarge;
+  if ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o)) & 15) return kErrBadShape;  // both are read 16 bytes at a time
+  const bool staged = hq <= 48 * 1024 / (kDeltaTokens * 4);
+  const int smem = staged ? hq * kDeltaTokens * 4 : 0;
   TTB_COUNT_LAUNCH(1);
   auto delta_kernel = d == 128 ? attn_delta_kernel<128> : attn_delta_kernel<64>;
-  delta_kernel<<<static_cast<unsigned>((tokens + kDeltaTokens - 1) / kDeltaTokens), 256, smem, st>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, tokens, s, hq);
+  delta_kernel<<<static_cast<unsigned>((tokens + kDeltaTokens - 1) / kDeltaTokens), 256, smem, st>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, tokens, s, hq, staged);
   AttnParams p{};
   p.b = b, p.s = s, p.sk = sk, p.hq = hq, p.hkv = hkv, p.d = d, p.scale = scale, p.causal = causal, p.lo = lo, p.hi = hi;
   p.kmask = static_cast<const uint8_t*>(kmask), p.monotone = monotone, p.softcap = softcap;

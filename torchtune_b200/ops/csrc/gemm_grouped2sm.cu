@@ -249,13 +249,13 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 
 // One block: first row and pieces of every expert; `table` is Params' five arrays of max_pieces entries each and the total.  Few experts are listed by the size of their pieces, so
 // that the tiles that the pairs take in turn are of one size and all pairs get the same work; with many it averages out.
-__global__ void __launch_bounds__(256) piece_table_kernel(const long long* __restrict__ counts, int num_experts, int max_pieces, int* __restrict__ table) {
+__global__ void __launch_bounds__(256) piece_table_kernel(const long long* __restrict__ counts, int num_experts, int max_pieces, long long rows, int* __restrict__ table) {
   __shared__ int row0[1025], piece0[1024];
   if (threadIdx.x == 0) {
     long long r = 0;
     for (int e = 0; e < num_experts; ++e) {
       row0[e] = static_cast<int>(r);
-      r += counts[e];
+      r += min(max(counts[e], 0ll), rows - r);  // no row outside the result, whatever the counts say
     }
     row0[num_experts] = static_cast<int>(r);
     const bool sorted = num_experts <= 64;
@@ -318,7 +318,7 @@ extern "C" int ttb_gemm_grouped_bf16_2sm(const void* X, const void* W, void* C, 
   int* t = static_cast<int*>(table);
   auto st = static_cast<cudaStream_t>(stream);
   TTB_COUNT_LAUNCH(1);
-  gg::piece_table_kernel<<<1, 256, 0, st>>>(static_cast<const long long*>(counts), num_experts, max_pieces, t);
+  gg::piece_table_kernel<<<1, 256, 0, st>>>(static_cast<const long long*>(counts), num_experts, max_pieces, rows, t);
   if (cudaGetLastError() != cudaSuccess) return kErrDriver;
   gg::Params p{};
   p.N = N, p.K = K, p.C = static_cast<__nv_bfloat16*>(C), p.ldc = ldc, p.err = err;
