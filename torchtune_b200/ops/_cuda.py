@@ -510,6 +510,13 @@ def lora_linear_nf4(x, xd, nf4, bias, a, b, scale):
     return _LoRANF4Linear.apply(x, xd, nf4, bias, a, b, scale)
 
 
+def _groups_on_pairs(rows: int, E: int, N: int, K: int) -> bool:
+    """Whether grouped products run on CTA pairs (``csrc/gemm_grouped2sm.cu``), which put 256 columns of the result on the rows of a tile (a narrower result would leave them empty) and need work for many tiles to
+    hide that pairs start later and come in half the number: us with 128-row tiles / with pairs for up to 128 rows per expert 16 x 2048 x 1536 36 / 42, 64 x 2048 x 1536 93 / 101,
+    64 x 2880 x 2880 202 / 198, 128 x 2048 x 1536 161 / 151; 512 rows per expert 8 x 512 x 256 19.5 / 23.5, 16 x 768 x 2048 42 / 44, 16 x 2048 x 1536 64 / 60, 64 x 2048 x 768 116 / 106."""
+    return N >= 256 and (E * K * N >= 2**28 or (rows >= 256 * E and E * K * N >= 2**25))
+
+
 def _grouped_gemm(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, b_mn: bool) -> torch.Tensor:
     """One launch over all experts: ``x`` ``[rows, K]`` sorted by expert, ``w`` ``[E, K, N]`` (``b_mn``) or ``[E, N, K]``, ``counts`` int64 ``[E]``
     on the device.  The tile → expert table is built on the device, so the call never synchronises with the host."""
@@ -517,8 +524,7 @@ def _grouped_gemm(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, b_mn: 
     E = w.shape[0]
     N = w.shape[2] if b_mn else w.shape[1]
     out = torch.empty(rows, N, dtype=_BF16, device=x.device)
-    # CTA pairs (csrc/gemm_grouped2sm.cu) put 256 columns of the result on the rows of a tile; a narrower result would leave them empty
-    pairs = N >= 256 and _PAIR_KERNEL
+    pairs = _PAIR_KERNEL and _groups_on_pairs(rows, E, N, K)
     launch = lib().ttb_gemm_grouped_bf16_2sm if pairs else lib().ttb_gemm_grouped_bf16
     scratch = torch.empty(5 * (-(-rows // 256) + E) + 1 if pairs else 3 * (-(-rows // 128) + E) + 1, dtype=torch.int32, device=x.device)
     cnt = counts.to(torch.int64)
