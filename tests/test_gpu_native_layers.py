@@ -101,6 +101,34 @@ def test_what_the_call_does_not_do_is_left_to_the_modules():
     assert int(model.layers[0].attn.kv_cache.cache_pos[0]) == 0 and native(x, pos, mask) is not None
 
 
+@pytest.mark.parametrize("how", ["context", "default"])
+def test_generation_where_tensors_are_made_on_the_device(how):
+    """Inside a device context and with a default device: tokens and logits of a plain call, recorded steps included."""
+    from torchtune_b200 import generation
+    from torchtune_b200.generation._native_layers import NativeLayers
+
+    model = _model(2, 512, 8, 2, 1024, 1024, 3, 60)
+    prompt = torch.randint(1, 1024, (3, 9), device="cuda")
+    prompt[0, :4] = 0
+
+    def run():
+        model.reset_caches()
+        return generation.generate(model, prompt, max_generated_tokens=8, temperature=0.7, top_k=20, rng=torch.Generator(device="cuda").manual_seed(1))
+
+    want = run()
+    if how == "context":
+        with torch.device("cuda"):
+            assert NativeLayers.of(model, 3) is not None
+            got = run()
+    else:
+        torch.set_default_device("cuda")
+        try:
+            got = run()
+        finally:
+            torch.set_default_device(None)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("M,N,Ks", [(40, 64, (64, 24)), (300, 520, (512, 128, 128)), (8200, 1032, (1024, 136, 264)), (4100, 2048, (2048, 512, 512)), (700, 2048, (8192, 4096)), (9000, 520, (200, 8192))])
 def test_linear_layers_of_one_input(M, N, Ks):
     """Values of joined layers are those of single ones; the input gradient, summed by its products, against 64 bits; outputs that nobody uses, frozen weights, biases."""

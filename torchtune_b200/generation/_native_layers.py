@@ -1,6 +1,7 @@
 """Forward passes of a plain decoder on its KV caches with all layers issued by one native call (``ops/csrc/decoder_layers.cu``)."""
 from __future__ import annotations
 
+import ctypes
 import os
 from typing import List, Optional
 
@@ -77,7 +78,7 @@ class NativeLayers:
         self.model, self.batch, self.sizes, self.eps, self.scale, self.interleaved = model, batch, sizes, eps, scale, interleaved
         self.caches = [layer.attn.kv_cache for layer in model.layers]
         self.positions = [cache.cache_pos for cache in self.caches]
-        self.words = torch.tensor(words, dtype=torch.int64)
+        self.words = (ctypes.c_longlong * len(words))(*words)  # read by the host, so not a tensor, which would lie wherever the program makes tensors
 
     def __call__(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> Optional[torch.Tensor]:
         """Normalised hidden states ``[b, s, dim]`` of new tokens ``x`` ``[b, s]``, whose keys and values are appended; ``None``, with nothing done, for a mask or sizes that the call
@@ -100,7 +101,7 @@ class NativeLayers:
         h = ops.embed_tokens(self.model.tok_embeddings, x)
         y, work = torch.empty_like(h), torch.empty(need, dtype=torch.uint8, device=h.device)
         pos = _positions(input_pos, b, s, h.device)
-        check(lib().ttb_decoder_layers(self.words.data_ptr(), count, b, s, *self.sizes, self.eps, self.scale, self.interleaved, h.data_ptr(), y.data_ptr(), self.model.norm.scale.data_ptr(),
+        check(lib().ttb_decoder_layers(self.words, count, b, s, *self.sizes, self.eps, self.scale, self.interleaved, h.data_ptr(), y.data_ptr(), self.model.norm.scale.data_ptr(),
                                        pos.data_ptr(), mask.data_ptr(), mask.stride(0) if mask.shape[0] > 1 else 0, mask.stride(1), work.data_ptr(), err_word(h.device).data_ptr(),
                                        stream_ptr()), f"decoder layers for {b} x {s} tokens")
         if not self.caches[0].recording:  # a recorded step moves the positions on itself
