@@ -121,6 +121,45 @@ def test_softmax_statistics_of_the_logits_product(T, D, V):
         assert float((got.double() - exact).norm()) <= 2.0**-7 * float(exact.norm())  # p and the result are rounded to bf16
 
 
+@pytest.mark.parametrize("V", [19208, 18944])
+def test_softmax_statistics_of_shifted_and_extreme_logits(V):
+    """Maximum and sum of exponentials of every tile against 64 bits: rows with a common offset, all or every other tile at either end of bf16's range; and the losses from them."""
+    from torchtune_b200 import ops
+    from torchtune_b200.ops._cuda import _ce_stats
+    from torchtune_b200.ops._lib import check, err_word, lib, stream_ptr
+
+    T, D, big = 300, 192, torch.finfo(torch.bfloat16).max
+    w, h = torch.zeros(V, D, device="cuda"), torch.zeros(T, D, device="cuda")
+    w[:, 0], w[:, 1], w[:, 2] = 1, _logits(1, V, torch.float32)[0], (torch.arange(V, device="cuda") // 256 + 1) % 2  # ones, noise, every other tile
+    offsets = torch.tensor([0.0, 100.0, -1000.0, 1000.0, 3e4, -1e6, 1e6, big, -big], device="cuda")
+    h[:, 0], h[:, 1] = offsets.repeat(T // 9 + 1)[:T], 1
+    h[-2:, 0] = 0
+    h[-2, 2], h[-1, 2] = big, -big  # every other tile masked, the first one with them
+    h, w = h.to(torch.bfloat16), w.to(torch.bfloat16)
+    logits = torch.empty(T, V, dtype=torch.bfloat16, device="cuda")
+    assert _ce_stats(h, w, logits, 0.0)
+    stats = torch.empty(-(-V // 256), T, 2, device="cuda")
+    check(lib().ttb_gemm_bf16_2sm_stats(h.data_ptr(), w.data_ptr(), logits.data_ptr(), stats.data_ptr(), T, V, D, D, D, V, err_word(h.device).data_ptr(), stream_ptr()), "statistics")
+    with torch.no_grad():
+        assert torch.equal(logits, ops.linear(h, w))
+    z = logits.double()
+    for tile in range(stats.shape[0]):
+        part = z[:, tile * 256 : (tile + 1) * 256]
+        top = part.amax(1)
+        assert torch.equal(stats[tile, :, 0].double(), top)
+        # differences and products of fp32, exponentials good to 2^-22 and eight rescaled partial sums: 2^-18 of a sum that is at least 1
+        assert ((stats[tile, :, 1].double() / (part - top[:, None]).exp().sum(1) - 1).abs() <= 2.0**-18).all(), tile
+    lse, labels = torch.logsumexp(z, -1), torch.randint(0, V, (T,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    want = lse - z.gather(1, labels[:, None])[:, 0]
+    half_ulp = (torch.nextafter(lse.float().abs(), torch.full_like(lse, float("inf"), dtype=torch.float32)).double() - lse.float().abs().double()) / 2
+    for i in (*range(9), T - 2, T - 1):
+        alone = torch.full_like(labels, -100)
+        alone[i] = labels[i]
+        got = float(ops.linear_cross_entropy(h, w, alone)[0])
+        # the logarithm's 2^-19, one rounding of its sum with the maximum, and one of the difference with the label's logit
+        assert abs(got - float(want[i])) <= 2.0**-19 * 20 + float(half_ulp[i]) + 2.0**-24 * abs(float(want[i])), (i, got, float(want[i]))
+
+
 @pytest.mark.parametrize("T,V", [(16, 128), (700, 20000)])
 def test_mean_loss(T, V):
     """The mean's gradients with and without statistics of the softmax, for factors of one and others, kept graphs, hooks on saved tensors, batched factors, and no valid token."""

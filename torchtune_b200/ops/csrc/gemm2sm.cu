@@ -401,12 +401,13 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r[i]));
                 if (i < valid * 4) mx = fmaxf(mx, fmaxf(t.x, t.y));
               }
-              const float base = mx == -INFINITY ? 0.f : mx * kLog2e;
-              float sum = row_sum * fast_exp2(row_max * kLog2e - base);  // 0 before the first column: 0 * 2^-inf
+              // the difference first, which is exact between near values: a product that is rounded first costs |max| 2^-24 in every term and overflows at the ends of the range
+              const float base = mx == -INFINITY ? 0.f : mx;
+              float sum = row_sum * fast_exp2((row_max - base) * kLog2e);  // 0 before the first column: 0 * 2^-inf
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
                 const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r[i]));
-                if (i < valid * 4) sum += fast_exp2(fmaf(t.x, kLog2e, -base)) + fast_exp2(fmaf(t.y, kLog2e, -base));
+                if (i < valid * 4) sum += fast_exp2((t.x - base) * kLog2e) + fast_exp2((t.y - base) * kLog2e);
               }
               row_max = mx, row_sum = sum;
             }
