@@ -194,6 +194,16 @@ def test_mean_loss(T, V):
     before = [t.clone() for t in held]
     near(torch.autograd.grad(loss * 3, (h, w)), 3.0)
     assert all(torch.equal(a, b) for a, b in zip(held, before))
+    for keep in (lambda t: t, lambda t: t.detach(), torch.clone):  # hooks on the node's own saved tensors, which come later
+        loss, held = mean(), []
+        for saved in loss.grad_fn._raw_saved_tensors[:2]:
+            saved.register_hooks(lambda t: held.append(keep(t)) or len(held) - 1, lambda i: held[i])
+        before = [t.clone() for t in held]
+        near(torch.autograd.grad(loss * 3, (h, w)), 3.0)
+        assert len(held) == 2 and all(torch.equal(a, b) for a, b in zip(held, before))
+    loss = mean()
+    places = [t.data_ptr() for t in loss.grad_fn.saved_tensors[:2]]
+    assert [g.data_ptr() for g in torch.autograd.grad(loss, (h, w))] == places  # nobody else has them: no copies
     labels.fill_(-100)
     loss = mean()
     assert float(loss.detach()) == 0.0 and all(not g.any() for g in torch.autograd.grad(loss, (h, w)))

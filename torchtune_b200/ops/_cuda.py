@@ -5,6 +5,7 @@ from __future__ import annotations
 import ctypes
 import os
 import math
+import weakref
 from typing import Any, Dict, List, Optional, Sequence, Tuple, Union
 
 import torch
@@ -1520,7 +1521,9 @@ class _LinearCE(torch.autograd.Function):
             elif need_w:
                 gemm(lg, hc, a_mn=True, b_mn=True, out=dw, accumulate=not single)
         ctx.save_for_backward(dh, dw, None if folded else share)
-        ctx.hooked = torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+        # what hooks on saved tensors hand back may be kept by them: backward writes only to the very tensors that were made here
+        hooked = torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+        ctx.formed = () if hooked else tuple(weakref.ref(t) for t in (dh, dw) if t is not None)
         ctx.h_shape = hidden.shape
         ctx.w_dtype = weight.dtype
         ctx.direct = direct
@@ -1536,9 +1539,10 @@ class _LinearCE(torch.autograd.Function):
         # only valid for an upstream factor of one (the recipes back-propagate the sum itself).
         if share is not None:
             g_loss = g_loss * share
-        mine = not (ctx.hooked or torch._C._autograd._get_current_graph_task_keep_graph())
-        gh = _rescaled(dh, g_loss, mine).view(ctx.h_shape) if dh is not None else None
-        gw = _rescaled(dw, g_loss, mine).to(ctx.w_dtype) if dw is not None else None
+        formed = () if torch._C._autograd._get_current_graph_task_keep_graph() else tuple(r() for r in ctx.formed)
+        mine = lambda t: any(t is f for f in formed)
+        gh = _rescaled(dh, g_loss, mine(dh)).view(ctx.h_shape) if dh is not None else None
+        gw = _rescaled(dw, g_loss, mine(dw)).to(ctx.w_dtype) if dw is not None else None
         return gh, gw, None, None, None, None, None
 
 
