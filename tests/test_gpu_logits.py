@@ -212,3 +212,36 @@ def test_mean_loss(T, V):
     labels[1::3] = 5
     got, want = module(h, labels), torch.nn.functional.cross_entropy((h.double() @ module.linear_projection.weight.double().t()), labels)
     assert abs(float(got.detach()) - float(want.detach())) <= 0.02 * abs(float(want.detach()))
+
+
+@pytest.mark.parametrize("written", [False, True])
+@pytest.mark.parametrize("T,V", [(16, 128), (700, 20000)])
+def test_mean_loss_of_a_weight_with_a_gradient_window(T, V, written):
+    """A weight whose gradients are delivered straight to a flat buffer: the mean's arrives as that of the mean, whatever multiplies it and whatever was there before; the sum's
+    goes straight to the buffer."""
+    from types import SimpleNamespace
+
+    from torchtune_b200 import ops
+    from torchtune_b200.ops import _cuda
+    from torchtune_b200.parallel.dp import FlatLayout
+
+    h, w = _logits(T, 64, torch.bfloat16, T).requires_grad_(), torch.nn.Parameter(_logits(V, 64, torch.bfloat16, V) * 0.1)
+    labels = torch.randint(0, V, (T,), device="cuda")
+    labels[::3] = -100
+    total, count = ops.linear_cross_entropy(h, w, labels)
+    want_h, want_w = (g.double() / int(count) for g in torch.autograd.grad(total, (h, w)))
+    w._grad_buffer, w._grad_written = torch.full_like(w, 0.25 if written else float("nan")), written
+    _cuda.enable_direct_wgrad(True, use_side_stream=False)
+    _cuda.register_grad_window(w)
+    try:
+        (ops.linear_cross_entropy_mean(h, w, labels) * 0.5).backward()
+        FlatLayout.collect_autograd_grads(SimpleNamespace(params=[w]))
+        for got, want in ((h.grad.double(), want_h), (w._grad_buffer.double() - 0.25 * written, want_w)):
+            # roundings to bf16 of the gradient on both sides and of a sum with 0.25
+            assert float((got - 0.5 * want).norm()) <= 2.0**-7 * 0.5 * float(want.norm()) + written * 2.0**-9 * want.numel() ** 0.5
+        w._grad_written = False
+        ops.linear_cross_entropy(h, w, labels)[0].backward()
+        assert w.grad is None and w._grad_written and float((w._grad_buffer.double() - int(count) * want_w).norm()) <= 2.0**-7 * int(count) * float(want_w.norm())
+    finally:
+        _cuda.enable_direct_wgrad(False)
+        _cuda.unregister_grad_window(w.data_ptr())

@@ -1483,7 +1483,9 @@ class _LinearCE(torch.autograd.Function):
         single = rows >= T
         loss_rows = torch.empty(T, dtype=torch.float32, device=h2.device)
         dh = torch.empty_like(h2) if need_h else None
-        owner = grad_window_owner(weight) if (need_w and single) else None
+        # A window takes what is written now for good, so it suits the sum, which the recipes differentiate by itself.  The mean's weight gradient goes through autograd, whose
+        # factor it gets, and which the owner of the window collects.
+        owner = grad_window_owner(weight) if (need_w and single and not mean) else None
         direct = owner is not None
         dw = None
         if need_w and not direct:
@@ -1491,7 +1493,7 @@ class _LinearCE(torch.autograd.Function):
         buf = torch.empty(min(rows, T), V, dtype=_BF16, device=h2.device)
         n_valid = (y != ignore_index).sum()
         share = n_valid.clamp_min(1).to(torch.float32).reciprocal() if mean else None
-        folded = mean and single and not direct
+        folded = mean and single
         L = lib()
         for start in range(0, T, rows):
             n = min(rows, T - start)
