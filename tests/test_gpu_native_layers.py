@@ -129,6 +129,24 @@ def test_generation_where_tensors_are_made_on_the_device(how):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@torch.no_grad()
+@pytest.mark.parametrize("first", [False, True])
+def test_a_step_is_recorded_once_its_own_kernels_have_run(first):
+    """Caches that were stepped by the modules, then by the native call, and the other way round: the first step of either way runs as it is."""
+    from torchtune_b200.generation._native_layers import NativeLayers
+    from torchtune_b200.generation._step_graph import StepGraph, _alone
+
+    model = _model(1, 512, 8, 2, 1024, 1024, 2, 60)
+    x, mask = torch.randint(1, 1024, (2, 1), device="cuda"), torch.tril(torch.ones(60, 60, dtype=torch.bool, device="cuda")).unsqueeze(0)
+    at = 0
+    for native in (first, not first):
+        step = StepGraph(model, 2, NativeLayers.of(model, 2) if native else None)
+        for recorded in (False, _alone()):
+            step(x, torch.full((2,), at, device="cuda"), mask[:, at : at + 1].contiguous())
+            at += 1
+            assert (step.graph is not None) == recorded
+
+
 @pytest.mark.parametrize("M,N,Ks", [(40, 64, (64, 24)), (300, 520, (512, 128, 128)), (8200, 1032, (1024, 136, 264)), (4100, 2048, (2048, 512, 512)), (700, 2048, (8192, 4096)), (9000, 520, (200, 8192))])
 def test_linear_layers_of_one_input(M, N, Ks):
     """Values of joined layers are those of single ones; the input gradient, summed by its products, against 64 bits; outputs that nobody uses, frozen weights, biases."""

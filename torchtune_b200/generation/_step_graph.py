@@ -37,7 +37,7 @@ class _LastGraph:
     def __init__(self) -> None:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.stream: Optional[torch.cuda.Stream] = None
-        self.stepped: Set[Tuple[int, ...]] = set()  # batch and mask shape of the steps that have run as they are
+        self.stepped: Set[Tuple[int, ...]] = set()  # the way (native or not), batch and mask shape of the steps that have run as they are
 
     def __deepcopy__(self, memo) -> "_LastGraph":
         return _LastGraph()
@@ -48,7 +48,7 @@ class _LastGraph:
 
 class StepGraph:
     """``model(x, input_pos, mask)[:, -1]`` for one token per row: a call is recorded, and it and all later ones replay the recording on the inputs
-    that they are given.  The first step of a batch and mask shape on a set of caches runs as it is, so that the one-time set-up of the kernels that
+    that they are given.  The first step of a batch and mask shape on a set of caches, by the modules and by the native call, runs as it is, so that the one-time set-up of the kernels that
     these sizes choose stays out of the recording.  While the program has other threads, all calls run as they are."""
 
     @staticmethod
@@ -86,7 +86,7 @@ class StepGraph:
 
     def __call__(self, x: torch.Tensor, input_pos: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         if self.graph is None:
-            sizes = (self.batch, *mask.shape)
+            sizes = (self.native is not None, self.batch, *mask.shape)  # the native call runs kernels of its own
             if sizes not in self.home.stepped or not _alone():
                 logits = self._step(x, input_pos, mask)
                 self.home.stepped.add(sizes)
