@@ -82,7 +82,7 @@ def test_results_and_caches_are_those_of_the_modules(shape, padded, bias, start)
 
 
 @torch.no_grad()
-def test_what_the_call_does_not_do_is_left_to_the_modules():
+def test_what_the_call_does_not_do_is_left_to_the_modules(monkeypatch):
     from torchtune_b200.generation._native_layers import NativeLayers
 
     for change in (lambda m: setattr(m.layers[1].mlp_norm, "eps", 1e-6), lambda m: setattr(m.layers[0].attn, "softcap", 50.0), lambda m: setattr(m.layers[1].mlp, "activation", nn.GELU()),
@@ -95,6 +95,10 @@ def test_what_the_call_does_not_do_is_left_to_the_modules():
         change(model)
         assert NativeLayers.of(model, 4) is None
     model = _model(2, 512, 8, 2, 1024, 1024, 4, 60)
+    for name in ("TTB_FUSE_RESIDUAL", "TTB_FUSE_SWIGLU"):
+        with monkeypatch.context() as m:
+            m.setenv(name, "0")
+            assert NativeLayers.of(model, 4) is None
     native = NativeLayers.of(model, 4)
     x, pos, mask = torch.ones(4, 2, dtype=torch.int64, device="cuda"), torch.arange(2, device="cuda"), torch.ones(1, 2, 60, dtype=torch.bool, device="cuda")
     assert native(x[:3], pos, mask) is None and native(x, pos, mask[:, :, :59]) is None and native(x, pos, mask.float()) is None

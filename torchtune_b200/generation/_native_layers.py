@@ -34,7 +34,9 @@ class NativeLayers:
         from ..ops._cuda import _PAIR_KERNEL
 
         emb = model.tok_embeddings.weight
-        if not emb.is_cuda or not ops.cuda_ops_enabled(emb) or not _PAIR_KERNEL or os.environ.get("TTB_FUSE_RESIDUAL", "1") == "0" or not len(model.layers):
+        if not emb.is_cuda or not ops.cuda_ops_enabled(emb) or not len(model.layers):
+            return None
+        if not _PAIR_KERNEL or any(os.environ.get(name, "1") == "0" for name in ("TTB_FUSE_RESIDUAL", "TTB_FUSE_SWIGLU")):  # switches that the modules follow
             return None
         if type(model.norm) is not RMSNorm or not _plain(model.norm.scale, emb.shape[1:]):
             return None
