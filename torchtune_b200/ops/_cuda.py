@@ -34,14 +34,23 @@ def _use_pair_kernel(M: int, N: int, K: int, out: torch.Tensor) -> bool:
     return out.dtype == _BF16 and _fills_pairs(M, N, K, out.device)
 
 
-def _fills_pairs(M: int, N: int, K: int, device: torch.device) -> bool:
+def _sm_pairs(device: torch.device) -> int:
     global _SM_PAIRS
-    if not _PAIR_KERNEL:
-        return False
     if _SM_PAIRS is None:
         _SM_PAIRS = max(1, torch.cuda.get_device_properties(device).multi_processor_count // 2)
-    tiles = (-(-M // 256)) * (-(-N // 256))
-    return K >= 128 and (tiles >= _SM_PAIRS or (K >= 8192 and 2 * tiles > _SM_PAIRS and M > 128 and N > 128))
+    return _SM_PAIRS
+
+
+def _fills_pairs(M: int, N: int, K: int, device: torch.device) -> bool:
+    if not _PAIR_KERNEL:
+        return False
+    pairs, tiles = _sm_pairs(device), (-(-M // 256)) * (-(-N // 256))
+    return K >= 128 and (tiles >= pairs or (K >= 8192 and 2 * tiles > pairs and M > 128 and N > 128))
+
+
+def _gates_in_pairs(M: int, N: int, K: int, device: torch.device) -> bool:
+    """Whether gate and up projection of these sizes fill the SM pairs with tiles of 256 rows and 128 columns of each."""
+    return _PAIR_KERNEL and K >= 128 and (-(-M // 256)) * (-(-N // 128)) >= _sm_pairs(device)
 
 
 ROWS_LIMIT = 64  # most tokens csrc/gemm_rows.cu takes
@@ -1382,10 +1391,7 @@ def gate_up_swiglu(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, clamp: O
         check(lib().ttb_gemm_rows_gated(x2.data_ptr(), x2.stride(0), w1.data_ptr(), w3.data_ptr(), K, h.data_ptr(), N, M, N, K, *(clamp or (0.0, 0.0)), stream_ptr()),
               f"gate/up GEMM of few rows M={M} N={N} K={K}")
         return h.view(*x.shape[:-1], N)
-    global _SM_PAIRS
-    if _SM_PAIRS is None:
-        _SM_PAIRS = max(1, torch.cuda.get_device_properties(x.device).multi_processor_count // 2)
-    if K < 128 or (-(-M // 256)) * (-(-N // 128)) < _SM_PAIRS:
+    if not _gates_in_pairs(M, N, K, x.device):
         return None
     return _GateUpSwiGLU.apply(x, w1, w3, clamp)
 

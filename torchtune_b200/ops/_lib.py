@@ -106,6 +106,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_gemm_bf16_2sm_residual.restype = i32
     L.ttb_decoder_layers_workspace.argtypes = [i32] * 9
     L.ttb_decoder_layers_workspace.restype = i64
+    L.ttb_product_rules.argtypes = [i32, i32, i32, i32, c.POINTER(i32)]
+    L.ttb_product_rules.restype = None
     L.ttb_decoder_layers.argtypes = [vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32, i32, vp, vp, vp, vp, vp, i64, i64, vp, vp, vp]
     L.ttb_decoder_layers.restype = i32
     L.ttb_gemm_bf16_2sm_stats.argtypes = [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, vp, vp]

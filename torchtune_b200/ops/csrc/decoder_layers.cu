@@ -75,7 +75,7 @@ struct Sizes {
 
 static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// ---- which kernel takes a product: the rules of ops._cuda (_runs_rows, _splits, _fills_pairs, gate_up_swiglu), where their reasons stand
+// ---- which kernel takes a product: the rules of ops._cuda (_runs_rows, _splits, _fills_pairs, _gates_in_pairs), where their reasons stand; ttb_product_rules lets a test compare the two
 static bool runs_rows(int M, int N, int K) {
   const int most = N <= 4096 ? 64 : N <= 32768 ? 32 : K < 4096 ? 16 : 8;
   return M > 0 && M <= most && K > 0 && K % 8 == 0;
@@ -89,11 +89,11 @@ static int splits_of(int M, int N, int K) {
   return s > 1 ? s : 1;
 }
 static int sm_pairs() { return sm_count() / 2 > 1 ? sm_count() / 2 : 1; }
-static bool fills_pairs(int M, int N, int K) {
+static bool fills_pairs(int M, int N, int K, int pairs) {
   const long long tiles = static_cast<long long>(ceil_div(M, 256)) * ceil_div(N, 256);
-  return K >= 128 && (tiles >= sm_pairs() || (K >= 8192 && 2 * tiles > sm_pairs() && M > 128 && N > 128));
+  return K >= 128 && (tiles >= pairs || (K >= 8192 && 2 * tiles > pairs && M > 128 && N > 128));
 }
-static bool gates_in_pairs(int M, int N, int K) { return K >= 128 && static_cast<long long>(ceil_div(M, 256)) * ceil_div(N, 128) >= sm_pairs(); }
+static bool gates_in_pairs(int M, int N, int K, int pairs) { return K >= 128 && static_cast<long long>(ceil_div(M, 256)) * ceil_div(N, 128) >= pairs; }
 static bool decodes(const Sizes& z) { return z.s * (z.hq / z.hkv) <= 16 && static_cast<long long>(ceil_div(z.max_seq, 64)) * (z.s + 1) * 8 <= 16384; }
 
 static long long split_bytes(int M, int N, int K) {
@@ -116,7 +116,7 @@ struct Work {
     const int nq = z.hq * z.D, nk = z.hkv * z.D;
     mid = take(2 * M * z.dim), norm = take(2 * M * z.dim);
     q = take(2 * M * nq), k = take(2 * M * nk), v = take(2 * M * nk), rot = take(2 * M * nq), att = take(2 * M * nq);
-    const bool fused = runs_rows(z.M(), z.hidden, z.dim) || gates_in_pairs(z.M(), z.hidden, z.dim);
+    const bool fused = runs_rows(z.M(), z.hidden, z.dim) || gates_in_pairs(z.M(), z.hidden, z.dim, sm_pairs());
     gate = take(fused ? 0 : 2 * M * z.hidden), up = take(fused ? 0 : 2 * M * z.hidden), act = take(2 * M * z.hidden);
     rstd = take(4 * M);
     const bool tiles = !decodes(z);
@@ -150,7 +150,7 @@ struct Call {
       ok(ttb_gemm_rows(x, K, M, K, 1, &w, &ldw, &N, &y, &ldy, bias == nullptr ? nullptr : &bias, residual, residual == nullptr ? 0 : N, 0, 1.f, st));
     } else if (const int splits = splits_of(M, N, K); splits > 1) {
       ok(ttb_gemm_bf16_splitk(x, w, split, y, M, N, K, 0, 0, K, K, N, 0, 0, bias, residual, residual == nullptr ? 0 : N, splits, 1.f, err, st));
-    } else if (fills_pairs(M, N, K)) {
+    } else if (fills_pairs(M, N, K, sm_pairs())) {
       ok(residual == nullptr ? ttb_gemm_bf16_2sm(x, w, y, M, N, K, 0, 0, K, K, N, 0, bias, 1.f, err, st)
                              : ttb_gemm_bf16_2sm_residual(x, w, y, residual, M, N, K, 0, K, K, N, N, bias, err, st));
     } else if (ok(ttb_gemm_bf16(x, w, y, M, N, K, 0, 0, K, K, N, 0, 0, bias, 1.f, err, st)) && residual != nullptr) {
@@ -170,6 +170,12 @@ static bool takes(const Sizes& z) {
 
 }  // namespace layers
 }  // namespace ttb
+
+// What the rules above say of a product on a device of `pairs` SM pairs: rows, ranges, pairs, gated pairs.  No device is needed.
+extern "C" void ttb_product_rules(int M, int N, int K, int pairs, int* out) {
+  using namespace ttb::layers;
+  out[0] = runs_rows(M, N, K), out[1] = splits_of(M, N, K), out[2] = fills_pairs(M, N, K, pairs), out[3] = gates_in_pairs(M, N, K, pairs);
+}
 
 // Bytes of workspace of a pass over b rows of s new tokens; 0 for sizes that it does not take.
 extern "C" long long ttb_decoder_layers_workspace(int count, int b, int s, int dim, int hq, int hkv, int D, int hidden, int max_seq) {
@@ -229,7 +235,7 @@ extern "C" int ttb_decoder_layers(const long long* words, int count, int b, int 
       c.ok(ttb_gemm_rows_gated_normed(mid, dim, l.mlp_scale, eps, l.w1, l.w3, dim, act, hidden, M, hidden, dim, st));
     } else if (gated) {
       c.ok(ttb_gemm_rows_gated(xn, dim, l.w1, l.w3, dim, act, hidden, M, hidden, dim, 0.f, 0.f, st));
-    } else if (gates_in_pairs(M, hidden, dim)) {
+    } else if (gates_in_pairs(M, hidden, dim, sm_pairs())) {
       c.ok(ttb_gemm_swiglu_bf16_2sm(xn, l.w1, l.w3, act, nullptr, nullptr, M, hidden, dim, dim, dim, hidden, 0.f, 0.f, err, st));
     } else {
       c.product(xn, l.w1, nullptr, nullptr, part(at.gate), M, hidden, dim);
