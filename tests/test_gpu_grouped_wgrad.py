@@ -59,3 +59,26 @@ def test_grouped_products_on_cta_pairs(counts, K, N, monkeypatch):
         for got, want, bound in ((y_e, a @ we, a.abs() @ we.abs()), (x.grad[at : at + c], d @ we.t(), d.abs() @ we.abs().t())):
             assert ((got.double() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-19 * bound).all(), e  # one rounding to bf16, fp32 sums in any order
         at += c
+
+
+@pytest.mark.parametrize("w_mn", [0, 1])
+@pytest.mark.parametrize("counts", [[0, 0], [100, 0, 33], [300, -5, 257, 1], [700, 1], [600, 90, 400], [2**40, 3]])
+def test_rows_of_no_expert_on_cta_pairs(counts, w_mn):
+    """Counts that add up to fewer rows than there are leave the rest of the result alone, and no counts reach past it."""
+    from torchtune_b200.ops._lib import check, check_device_errors, err_word, lib, stream_ptr
+
+    rows, K, N, E = 700, 136, 264, len(counts)
+    g = torch.Generator(device="cuda").manual_seed(E)
+    x, w = torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16), torch.randn(E, *((K, N) if w_mn else (N, K)), generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((rows + 300, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    table, held = torch.empty(5 * (-(-rows // 256) + E) + 1, dtype=torch.int32, device="cuda"), torch.tensor(counts, device="cuda")
+    check(lib().ttb_gemm_grouped_bf16_2sm(x.data_ptr(), w.data_ptr(), out.data_ptr(), held.data_ptr(), table.data_ptr(), rows, E, N, K, w_mn, K, w.stride(1),
+                                          w.stride(0), N, err_word(x.device).data_ptr(), stream_ptr()), "grouped product")
+    check_device_errors()
+    at = 0
+    for e, c in enumerate(counts):
+        c = min(max(c, 0), rows - at)
+        a, b = x[at : at + c].double(), w[e].double() if w_mn else w[e].double().t()
+        assert ((out[at : at + c].double() - a @ b).abs() <= 2.0**-8 * (a @ b).abs() + 2.0**-19 * (a.abs() @ b.abs())).all(), e  # one rounding to bf16, fp32 sums in any order
+        at += c
+    assert (out[at:] == 7).all()

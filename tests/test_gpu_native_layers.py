@@ -225,3 +225,57 @@ def test_attention_gradient_of_ragged_tokens(b, s, hq, hkv, D):
     want = torch.autograd.grad(torch.einsum("bhqk,bkhd->bqhd", p, vv), leaves, dy.double())
     for a, e in zip(got, want):
         assert float((a.double() - e).norm()) <= 0.01 * float(e.norm()) + 1e-3  # probabilities and their gradients are rounded to bf16 once each
+
+
+def test_attention_gradient_of_a_saved_output_at_an_odd_address():
+    """A hook on saved tensors hands the output back where 16-byte loads can't read it: the same gradients."""
+    from torchtune_b200 import ops
+    from torchtune_b200.ops import AttentionMask
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, dy = (torch.randn(2, 77, h, 64, generator=g, device="cuda").to(torch.bfloat16) for h in (8, 2, 2, 8))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    want = torch.autograd.grad(ops.attention(q, k, v, AttentionMask(causal=True)), leaves, dy)
+    moved = []
+
+    def unpack(t):
+        if t.dtype != torch.bfloat16 or t.shape != q.shape or torch.equal(t, q):
+            return t
+        moved.append(torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t))
+        return moved[-1]
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        y = ops.attention(q, k, v, AttentionMask(causal=True))
+    got = torch.autograd.grad(y, leaves, dy)
+    assert len(moved) == 1 and moved[0].data_ptr() % 16 and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("b,hq,hkv,D,slots", [(1, 4, 1, 64, 40), (3, 8, 2, 128, 700)])
+@pytest.mark.parametrize("interleaved", [0, 1])
+def test_decode_step_with_indices_out_of_range(b, hq, hkv, D, slots, interleaved):
+    """Positions outside the table count as position 0 and are noted; a slot outside the cache is not written.  Caches lie between guards."""
+    from torchtune_b200.ops._lib import check, index_violations, lib, stream_ptr
+
+    g = torch.Generator(device="cuda").manual_seed(slots)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    q, k, v, size, table_len = rand(b, hq, D), rand(b, hkv, D), rand(b, hkv, D), b * slots * hkv * D, 50
+    angles = torch.rand(table_len, D // 2, generator=g, device="cuda")
+    table, mask = torch.stack([angles.cos(), angles.sin()], -1).contiguous(), torch.ones(slots, dtype=torch.bool, device="cuda")
+    guarded = [rand(size + 2 * 4096) for _ in range(2)]
+
+    def step(pos, slot):
+        buffers, o = [t.clone() for t in guarded], torch.empty_like(q)
+        at, to = torch.tensor(pos[:b], dtype=torch.int32, device="cuda"), torch.tensor([slot], device="cuda")
+        caches = [t[4096 : 4096 + size] for t in buffers]
+        check(lib().ttb_attn_decode_append(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), caches[0].data_ptr(), caches[1].data_ptr(), table.data_ptr(), at.data_ptr(),
+                                           to.data_ptr(), mask.data_ptr(), 0, b, slots, hq, hkv, D, interleaved, table_len, D**-0.5, stream_ptr()), "step")
+        return o, buffers
+
+    index_violations()
+    want, kept = step([0, 0, 0], slots - 1)
+    assert index_violations() == 0 and not torch.equal(kept[0], guarded[0]) and not torch.equal(kept[1], guarded[1])
+    got, buffers = step([-1, table_len, 2**31 - 1], slots - 1)
+    assert index_violations() == b and torch.equal(got, want) and all(torch.equal(x, y) for x, y in zip(buffers, kept))
+    for slot in (slots, -1, 2**40):
+        got, buffers = step([3, 1, 2], slot)
+        assert index_violations() == 0 and got.isfinite().all() and all(torch.equal(x, y) for x, y in zip(buffers, guarded))

@@ -104,6 +104,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_gemm_bf16_dual_2sm.restype = i32
     L.ttb_gemm_bf16_2sm_residual.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i64, i64, i64, i64, vp, vp, vp]
     L.ttb_gemm_bf16_2sm_residual.restype = i32
+    L.ttb_attn_decode_append.argtypes = [vp] * 10 + [i64] + [i32] * 7 + [f32, vp]
+    L.ttb_attn_decode_append.restype = i32
     L.ttb_decoder_layers_workspace.argtypes = [i32] * 9
     L.ttb_decoder_layers_workspace.restype = i64
     L.ttb_product_rules.argtypes = [i32, i32, i32, i32, c.POINTER(i32)]
