@@ -1449,7 +1449,7 @@ def _gemm_scaled(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, factor: to
     N = b.shape[1]
     fit = all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (a, b, out))
     if fit and (M if a_mn else K) % 8 == 0 and N % 8 == 0 and _splits(M, N, K) == 1 and _use_pair_kernel(M, N, K, out):
-        check(lib().ttb_gemm_bf16_2sm_scaled(a.data_ptr(), b.data_ptr(), out.data_ptr(), factor.data_ptr(), M, N, K, int(a_mn), 1, a.stride(0), b.stride(0), out.stride(0),
+        check(lib().ttb_gemm_bf16_2sm_scaled(a.data_ptr(), b.data_ptr(), out.data_ptr(), factor.data_ptr(), M, N, K, int(a_mn), a.stride(0), b.stride(0), out.stride(0),
                                              err_word(a.device).data_ptr(), stream_ptr()), f"gemm (CTA pairs, scaled) M={M} N={N} K={K}")
         return
     gemm(a, b, a_mn=a_mn, b_mn=True, out=out)

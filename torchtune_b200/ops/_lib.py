@@ -115,7 +115,7 @@ def _declare(L: ctypes.CDLL) -> None:
     L.ttb_gemm_bf16_2sm_stats.argtypes = [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, vp, vp]
     L.ttb_gemm_bf16_2sm_stats.restype = i32
     L.ttb_softmax_ce_stats.argtypes = [vp, vp, vp, vp, vp, i32, i32, i64, i64, i32, vp]
-    L.ttb_gemm_bf16_2sm_scaled.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, i64, i64, i64, vp, vp]
+    L.ttb_gemm_bf16_2sm_scaled.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i64, i64, i64, vp, vp]
     L.ttb_gemm_bf16_2sm_scaled.restype = i32
     L.ttb_softmax_ce_stats.restype = i32
     L.ttb_gemm_bf16_2sm_widened.argtypes = [vp, vp, vp, i32, i32, i32, i64, i64, i64, vp, vp, vp]

@@ -693,11 +693,11 @@ extern "C" int ttb_gemm_bf16_2sm_stats(const void* A, const void* B, void* C, fl
   return g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
 }
 
-// ttb_gemm_bf16_2sm without bias or accumulation, times a factor that lies on the device: gradients of a mean need no pass that divides them.
-extern "C" int ttb_gemm_bf16_2sm_scaled(const void* A, const void* B, void* C, const float* factor, int M, int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int* err,
+// C[M,N] = factor · op(A) · B[K,N] (a_mn = 0: A [M, K], 1: [K, M]) with a factor that lies on the device: gradients of a mean need no pass that divides them.
+extern "C" int ttb_gemm_bf16_2sm_scaled(const void* A, const void* B, void* C, const float* factor, int M, int N, int K, int a_mn, long long lda, long long ldb, long long ldc, int* err,
                                         void* stream) {
   using namespace ttb;
-  if (M <= 0 || N <= 0 || K <= 0 || factor == nullptr || !b_mn) return kErrBadShape;
+  if (M <= 0 || N <= 0 || K <= 0 || factor == nullptr) return kErrBadShape;
   if ((lda & 7) || (ldb & 7) || (ldc & 7) || (N & 7) || (a_mn ? (M & 7) : (K & 7))) return kErrBadShape;
   g2::Params p{};
   p.M = M, p.N = N, p.K = K, p.C = C, p.ldc = ldc, p.alpha = 1.f, p.factor = factor;

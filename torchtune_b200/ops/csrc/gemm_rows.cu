@@ -67,7 +67,6 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// MT: token tiles of 8.  WK: warps of a CTA that share 16 rows and split a chunk of WK * kChunk contraction steps.
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
@@ -77,6 +76,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   }
 }
 
+// MT: token tiles of 8.  WK: warps of a CTA that share 16 rows and split a chunk of WK * kChunk contraction steps.
 template <int MT, int WK>
 struct Layout {
   static constexpr int kTokens = MT * 8;

@@ -10,6 +10,7 @@
     python -m torchtune_b200.ops.microbench latent --heads 16 --rank 512       (latent attention beside grouped-query attention)
     python -m torchtune_b200.ops.microbench ragenex --heads 16 --streams 4     (lightning and span attention, stream steps)
     python -m torchtune_b200.ops.microbench decode --shapes 4096x4096 6144x4096 --tokens 1 16 32   (few tokens: products, attention, sampling)
+    python -m torchtune_b200.ops.microbench joined      (epilogues that take a pass along, sums of input gradients, grouped products)
     python -m torchtune_b200.ops.microbench suite --tokens 8192      (norm, RoPE, SwiGLU, loss, embedding, LoRA, grouped GEMM, NF4, offload copies)
 
 Each command prints one JSON line: median milliseconds over ``--iters`` launches (an L2 flush
@@ -291,6 +292,64 @@ def bench_decode(args, flush):
             logits, q = torch.randn(b, 128256, device="cuda"), torch.rand(b, 128256, device="cuda") + 1e-3
             emit("sample, top 300", _time_captured(lambda i: lambda: _cuda.sample(logits, q, 0.6, 300), args.iters, 8.0 * logits.numel()), rows=b, vocabulary=128256)
     return {"op": "decode", "rows": len(rows)}
+
+
+def bench_joined(args, flush):
+    """Operations that take a pass along beside the same ones apart: logits widened in the epilogue, the mean's gradients out of the products, input gradients of joined
+    projections, and by themselves the backward passes of norm and attention and the grouped products of an expert layer.  One JSON line per operation."""
+    from . import attention, grouped_matmul, linear, linear_cross_entropy, linear_cross_entropy_mean, linear_group, linear_widened, rms_norm, widen
+    from .mask import AttentionMask
+
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    rand = lambda *s, std=1.0: torch.empty(*s, dtype=torch.bfloat16, device="cuda").normal_(0, std, generator=gen)
+    rows = []
+
+    def emit(op, joined, apart=None, **kw):
+        fns = [joined] if apart is None else [joined, apart]
+        times = [[] for _ in fns]
+        for i in range(args.warmup + args.iters):  # in turn: what ran before decides how far the clock is from the power limit
+            for fn, t in zip(fns, times):
+                ms = _time(fn, 1, 0, flush)
+                if i >= args.warmup:
+                    t.append(ms)
+        row = {"op": op, **kw, **{name: round(1e3 * sorted(t)[len(t) // 2], 1) for name, t in zip(("us", "apart_us"), times)}}
+        rows.append(row)
+        print(json.dumps(row), flush=True)
+
+    def back(y, leaves, dy):
+        return lambda: torch.autograd.grad(y, leaves, dy, retain_graph=True)
+
+    x, w = rand(6144, 4096), rand(128256, 4096, std=0.02)
+    with torch.no_grad():
+        emit("widened logits", lambda: linear_widened(x, w), lambda: widen(linear(x, w)), tokens=6144, vocabulary=128256, dim=4096)
+    for n, dim in ((8192, 4096), (16384, 2048), (1332, 2048)):
+        h, w, labels = rand(n, dim).requires_grad_(), rand(128256, dim, std=0.02).requires_grad_(), torch.randint(0, 128256, (n,), device="cuda", generator=gen)
+
+        def apart():
+            total, count = linear_cross_entropy(h, w, labels)
+            torch.autograd.grad(total / count, (h, w))
+
+        emit("mean cross-entropy with both gradients", lambda: torch.autograd.grad(linear_cross_entropy_mean(h, w, labels), (h, w)), apart, tokens=n, vocabulary=128256, dim=dim)
+    del h, w
+    for n, dim, outs in ((8192, 4096, (4096, 1024, 1024)), (16384, 2048, (2048, 512, 512)), (16384, 2048, (8192, 8192))):
+        x, ws = rand(n, dim).requires_grad_(), [rand(o, dim, std=0.02) for o in outs]
+        dys = [rand(n, o) for o in outs]
+        emit("input gradient", back(list(linear_group(x, ws, [None] * len(ws))), x, dys), back([linear(x, w) for w in ws], x, dys), tokens=n, dim=dim, outputs=outs)
+    for n, dim in ((8192, 4096), (16384, 2048)):
+        x, gain = rand(n, dim).requires_grad_(), rand(dim).requires_grad_()
+        emit("norm backward", back(rms_norm(x, gain, 1e-5), (x, gain), rand(n, dim)), tokens=n, dim=dim)
+    for heads, kv, d in ((32, 8, 128), (32, 8, 64)):
+        q, k, v = (rand(1, 16384, n, d).requires_grad_() for n in (heads, kv, kv))
+        emit("attention backward", back(attention(q, k, v, AttentionMask(causal=True)), (q, k, v), rand(1, 16384, heads, d)), tokens=16384, heads=heads, key_heads=kv, head_dim=d)
+    del q, k, v
+    for experts, n, k, out in ((16, 300, 5120, 8192), (16, 1024, 5120, 8192), (16, 1024, 8192, 5120), (16, 4096, 5120, 8192), (16, 8192, 5120, 8192), (16, 12000, 5120, 8192),
+                               (16, 16384, 2048, 8192), (8, 2048, 4096, 14336), (64, 8192, 2048, 768), (16, 2048, 2048, 1536)):
+        x, w = rand(n, k).requires_grad_(), rand(experts, k, out, std=0.02)
+        counts = torch.bincount(torch.randint(0, experts, (n,), device="cuda", generator=gen), minlength=experts)
+        with torch.no_grad():
+            emit("grouped product", lambda: grouped_matmul(x, w, counts), experts=experts, rows=n, contraction=k, outputs=out)
+        emit("grouped input gradient", back(grouped_matmul(x, w, counts), x, rand(n, out)), experts=experts, rows=n, contraction=out, outputs=k)
+    return {"op": "joined", "rows": len(rows)}
 
 
 def bench_ragenex(args, flush):
@@ -715,13 +774,14 @@ def main() -> None:
     rx.add_argument("--dim", type=int, default=2048)
     rx.add_argument("--streams", type=int, default=4)
     rx.add_argument("--seq", type=int, default=8192)
+    sub.add_parser("joined")
     su = sub.add_parser("suite")
     su.add_argument("--tokens", type=int, default=8192)
     args = ap.parse_args()
     from ._lib import check_device_errors
 
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
-    fn = {"gemm": bench_gemm, "gemm_fp8": bench_gemm_fp8, "gemm_mxfp8": bench_gemm_mxfp8, "attention": bench_attention, "rmsnorm": bench_rmsnorm, "adamw": bench_adamw, "adamw8bit": bench_adamw8bit, "gate_up": bench_gate_up, "comm": bench_comm, "decode": bench_decode, "latent": bench_latent, "ragenex": bench_ragenex, "suite": bench_suite}[args.op]
+    fn = {"gemm": bench_gemm, "gemm_fp8": bench_gemm_fp8, "gemm_mxfp8": bench_gemm_mxfp8, "attention": bench_attention, "rmsnorm": bench_rmsnorm, "adamw": bench_adamw, "adamw8bit": bench_adamw8bit, "gate_up": bench_gate_up, "comm": bench_comm, "decode": bench_decode, "joined": bench_joined, "latent": bench_latent, "ragenex": bench_ragenex, "suite": bench_suite}[args.op]
     res = fn(args, flush)
     check_device_errors()
     print(json.dumps(res), flush=True)
