@@ -208,9 +208,9 @@ def test_embedding_gradient_of_long_runs(n, dim, run):
     assert ((got.double() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-23 * run * size).all()  # one rounding, fp32 sums one after the other
 
 
-@pytest.mark.parametrize("b,s,hq,hkv,D", [(1, 1, 1, 1, 64), (3, 7, 3, 1, 128), (2, 333, 32, 8, 64), (1, 129, 20, 4, 128), (1, 9, 1600, 1600, 64)])
+@pytest.mark.parametrize("b,s,hq,hkv,D", [(1, 1, 1, 1, 64), (3, 7, 3, 1, 128), (2, 333, 32, 8, 64), (1, 129, 20, 4, 128), (1, 9, 1600, 1600, 64), (1, 333, 3, 1, 128), (2, 601, 4, 2, 64), (1, 3, 12400, 12400, 64)])
 def test_attention_gradient_of_ragged_tokens(b, s, hq, hkv, D):
-    """The products of outputs and their gradients, eight tokens at a time, where tokens and heads fill no group, and for more heads than are staged."""
+    """The products of outputs and their gradients, one to eight tokens at a time, where tokens and heads fill no group, and for more heads than are staged."""
     from torchtune_b200 import ops
     from torchtune_b200.ops import AttentionMask
 

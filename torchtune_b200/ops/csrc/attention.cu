@@ -369,17 +369,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // ===================================================================================== backward
-// delta[b, h, q] = sum_d dO * O (fp32).  A CTA takes kDeltaTokens tokens of all heads, which lie one after the other: 16 bytes per lane and load, four pairs of loads in
+// delta[b, h, q] = sum_d dO * O (fp32).  A CTA takes up to kDeltaTokens tokens of all heads, which lie one after the other: 16 bytes per lane and load, four pairs of loads in
 // flight, bound by them; the results turn in shared memory and leave as full sectors.  With a warp per (token, head), 4 bytes per lane and single stores 32 heads of 16384 tokens took 131 us
-// at head dim 128 and 125 us at 64, here 59 and 34 us.
+// at head dim 128 and 125 us at 64, here 59 and 34 us.  Fewer tokens to a CTA where eight would leave SMs without one (the launcher's rule): a backward pass of 128 tokens, 32 heads of 128, took 38.0 us with
+// eight and takes 33.9 us, one of 512 69.8 and 65.7 us.
 static constexpr int kDeltaTokens = 8;
 template <int D>
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta, long long tokens, int s, int hq, bool staged) {
-  extern __shared__ float sums[];  // [hq][kDeltaTokens]; without `staged`, for more heads than fit, results leave one by one
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta, long long tokens, int s, int hq, int log_per, bool staged) {
+  extern __shared__ float sums[];  // [hq][2^log_per], a column for each token; without `staged`, for more heads than fit, results leave one by one
   constexpr int kLanes = D / 8, kItems = 256 / kLanes;
-  const long long tok0 = blockIdx.x * static_cast<long long>(kDeltaTokens);
-  const int count = static_cast<int>(min(static_cast<long long>(kDeltaTokens), tokens - tok0)) * hq;
+  const int per = 1 << log_per;
+  const long long tok0 = blockIdx.x * static_cast<long long>(per);
+  const int count = static_cast<int>(min(static_cast<long long>(per), tokens - tok0)) * hq;
   const int lane = threadIdx.x % kLanes;
   const uint4* po = reinterpret_cast<const uint4*>(o + tok0 * hq * D) + lane;
   const uint4* pd = reinterpret_cast<const uint4*>(d_o + tok0 * hq * D) + lane;
@@ -407,7 +409,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
       if (lane == 0 && item < count) {
         const long long tok = tok0 + item / hq;
         if (staged)
-          sums[item % hq * kDeltaTokens + item / hq] = acc;
+          sums[item % hq * per + item / hq] = acc;
         else
           delta[(tok / s * hq + item % hq) * s + tok % s] = acc;
       }
@@ -415,9 +417,9 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   }
   if (!staged) return;
   __syncthreads();
-  for (int i = threadIdx.x; i < hq * kDeltaTokens; i += 256) {
-    const long long tok = tok0 + i % kDeltaTokens;
-    if (tok < tokens) delta[(tok / s * hq + i / kDeltaTokens) * s + tok % s] = sums[i];
+  for (int i = threadIdx.x; i < hq * per; i += 256) {
+    const long long tok = tok0 + (i & (per - 1));
+    if (tok < tokens) delta[(tok / s * hq + (i >> log_per)) * s + tok % s] = sums[i];
   }
 }
 
@@ -789,11 +791,15 @@ extern "C" int ttb_attn_bwd(const void* q, const void* k, const void* v, const v
   auto st = static_cast<cudaStream_t>(stream);
   const long long tokens = static_cast<long long>(b) * s;
   if ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o)) & 15) return kErrBadShape;  // both are read 16 bytes at a time
-  const bool staged = hq <= 48 * 1024 / (kDeltaTokens * 4);
-  const int smem = staged ? hq * kDeltaTokens * 4 : 0;
+  int log_per = 3;
+  static_assert(kDeltaTokens == 1 << 3, "eight tokens, halved below");
+  while (log_per > 0 && (tokens >> log_per) < sm_count()) --log_per;
+  const int per = 1 << log_per;
+  const bool staged = hq <= 48 * 1024 / (per * 4);
+  const int smem = staged ? hq * per * 4 : 0;
   TTB_COUNT_LAUNCH(1);
   auto delta_kernel = d == 128 ? attn_delta_kernel<128> : attn_delta_kernel<64>;
-  delta_kernel<<<static_cast<unsigned>((tokens + kDeltaTokens - 1) / kDeltaTokens), 256, smem, st>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, tokens, s, hq, staged);
+  delta_kernel<<<static_cast<unsigned>((tokens + per - 1) / per), 256, smem, st>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, tokens, s, hq, log_per, staged);
   AttnParams p{};
   p.b = b, p.s = s, p.sk = sk, p.hq = hq, p.hkv = hkv, p.d = d, p.scale = scale, p.causal = causal, p.lo = lo, p.hi = hi;
   p.kmask = static_cast<const uint8_t*>(kmask), p.monotone = monotone, p.softcap = softcap;
