@@ -60,7 +60,7 @@ struct Params {
   float alpha;
   const float* factor;  // another one, on the device, or null
   int accumulate;
-  float2* stats;  // [n tiles, M]: maximum of a row's results in a tile and the sum of their exponentials relative to it (as stored, in bf16), or null
+  float2* stats;  // [n tiles, M]: maximum of a row's results in a tile and the sum of their exponentials relative to it (as stored, in bf16); STATS only
   int out_f32;  // C is fp32 and holds the results rounded to bf16 (vocabulary logits that callers want widened)
   int tma_store;
   int group_m;  // pair-tiles in m per scheduling group
@@ -85,13 +85,14 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int gro
 // of the same 128 hidden units, in both CTAs' tensor memory.  The epilogue writes h = silu(gate) · up ([M, N], N = hidden width; tmC) and,
 // when the backward pass will need them, gate and up as well (tmG, tmU).  The separate SwiGLU kernel and its re-read of both
 // pre-activations disappear; in a gradient-free forward pass the pre-activations never reach HBM at all.
-template <bool A_MN, bool B_MN, int GLU>
+// STATS: the epilogue leaves the statistics of a softmax over the result's rows.  A kernel of its own, since the registers and moves that they take cost every product of the form, X · Wᵀ of
+// short contractions most (2432 x 2048 x 128 12.4 us without, 14.5 with; x 2048 no difference).
+template <bool A_MN, bool B_MN, int GLU, bool STATS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmU,
                const __grid_constant__ CUtensorMap tmA2, Params p) {
   constexpr bool SWIGLU = GLU != kNoGate;
-  constexpr bool kStats = !A_MN && !B_MN && !SWIGLU;  // the form of a linear layer's forward pass
   constexpr int kNS = SWIGLU ? kStagesSwiglu : kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -391,9 +392,9 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               o.w = pack_bf16x2(f[6], f[7]);
               const int chunk = (h * 4 + j) ^ (lane & 7);
               *reinterpret_cast<uint4*>(buf + lane * 128 + chunk * 16) = o;
-              if (kStats) r[j * 4] = o.x, r[j * 4 + 1] = o.y, r[j * 4 + 2] = o.z, r[j * 4 + 3] = o.w;
+              if (STATS) r[j * 4] = o.x, r[j * 4 + 1] = o.y, r[j * 4 + 2] = o.z, r[j * 4 + 3] = o.w;
             }
-            if (kStats && p.stats != nullptr) {  // one row per thread: its 32 columns join the running maximum and sum
+            if (STATS) {  // one row per thread: its 32 columns join the running maximum and sum
               const int valid = min(4, (p.N - col0 - h * 32) / 8);
               float mx = row_max;
 #pragma unroll
@@ -420,7 +421,7 @@ gemm2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           ++buf_toggle;
         }
-        if (kStats && p.stats != nullptr && row < p.M) p.stats[static_cast<long long>(n_blk) * p.M + row] = make_float2(row_max, row_sum);
+        if (STATS && row < p.M) p.stats[static_cast<long long>(n_blk) * p.M + row] = make_float2(row_max, row_sum);
       } else {
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -518,7 +519,7 @@ static int shuffle_multiplier(int num_tiles) {
   return m;
 }
 
-template <bool A_MN, bool B_MN, int GLU>
+template <bool A_MN, bool B_MN, int GLU, bool STATS = false>
 static int launch(const void* A, const void* B, const void* B2, void* G, void* U, const Params& p, long long lda, long long ldb, cudaStream_t stream,
                   const void* A2 = nullptr, long long lda2 = 0, long long ldb2 = 0) {
   constexpr bool SWIGLU = GLU != kNoGate;
@@ -564,7 +565,8 @@ static int launch(const void* A, const void* B, const void* B2, void* G, void* U
   } else {
     q.tma_store = (!p.accumulate && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && map_c(&tmC, p.C) == kOk) ? 1 : 0;
   }
-  auto kern = gemm2sm_kernel<A_MN, B_MN, GLU>;
+  if (STATS && q.tma_store == 0) return kErrBadShape;  // they are taken from what goes to the staging tiles
+  auto kern = gemm2sm_kernel<A_MN, B_MN, GLU, STATS>;
   constexpr int smem = SWIGLU ? kSmemBytesSwiglu : kSmemBytes;
   static bool attr_set = false;
   if (!attr_set) {
@@ -690,7 +692,7 @@ extern "C" int ttb_gemm_bf16_2sm_stats(const void* A, const void* B, void* C, fl
   p.M = M, p.N = N, p.K = K, p.C = C, p.ldc = ldc, p.alpha = 1.f;
   p.stats = reinterpret_cast<float2*>(stats), p.tile_mult = 1, p.err = err;
   p.group_m = g2::group_setting();
-  return g2::launch<false, false, g2::kNoGate>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
+  return g2::launch<false, false, g2::kNoGate, true>(A, B, nullptr, nullptr, nullptr, p, lda, ldb, static_cast<cudaStream_t>(stream));
 }
 
 // C[M,N] = factor · op(A) · B[K,N] (a_mn = 0: A [M, K], 1: [K, M]) with a factor that lies on the device: gradients of a mean need no pass that divides them.
