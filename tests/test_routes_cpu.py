@@ -143,3 +143,8 @@ def test_scaled_gradients_of_batched_and_differentiated_factors(library):
         _cuda._scaled(t, factor)
     _cuda._scaled(t, factor.detach())
     assert library.calls == ["ttb_scale_bf16"] * 2
+
+
+@pytest.mark.parametrize("M,N,K,pays", [(64, 32000, 2048, False), (1000, 32000, 2048, True), (20, 128256, 2048, True), (300, 128256, 1024, False), (4096, 128256, 512, False), (8192, 128256, 4096, True)])
+def test_softmax_statistics_are_taken_where_they_were_measured_to_pay(library, M, N, K, pays):
+    assert _cuda._stats_pay(M, N, K, None) is pays

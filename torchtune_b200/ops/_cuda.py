@@ -1457,11 +1457,18 @@ def _gemm_scaled(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, factor: to
 
 
 def _ce_stats(h: torch.Tensor, weight: torch.Tensor, logits: torch.Tensor, softcap: float) -> bool:
-    """Whether the product that makes these logits leaves the statistics of their softmax behind: the CTA-pair kernel does, unless the softmax runs over capped ones."""
+    """Whether the product that makes these logits can leave the statistics of their softmax behind: the CTA-pair kernel can, unless the softmax runs over capped ones."""
     (M, K), N = h.shape, weight.shape[0]
     if softcap > 0.0 or K % 8 or weight.shape[1] != K or any(t.stride(1) != 1 or t.stride(0) % 8 or t.data_ptr() % 16 for t in (h, weight, logits)):
         return False
     return not _runs_rows(M, N, K) and _splits(M, N, K) == 1 and _fills_pairs(M, N, K, h.device)
+
+
+def _stats_pay(M: int, N: int, K: int, device: torch.device) -> bool:
+    """Whether those statistics cost less than the pass over the logits that they save: the epilogue that takes them hides behind the products of the next tile, so there has to be one, and
+    its contraction has to be as long.  Loss and both gradients, us without / with: 64 tokens of 32000 x 2048 143.1 / 146.7, 300 220.2 / 221.5, 1000 365.8 / 355.6; 20 of 128256 x 2048
+    382.1 / 378.0, 4096 4730 / 4568; 300 of 128256 x 1024 388 / 401, x 512 292 / 322.  Loss alone: 300 of 128256 x 2048 214.7 / 202.4, x 1024 138.1 / 159.6."""
+    return K >= 2048 and (-(-M // 256)) * (-(-N // 256)) >= 3 * _sm_pairs(device)
 
 
 class _LinearCE(torch.autograd.Function):
@@ -1506,7 +1513,7 @@ class _LinearCE(torch.autograd.Function):
             hc = h2[start : start + n]
             lg = buf[:n]
             mode = 0 if (need_h or need_w) else 1
-            if _ce_stats(hc, weight, lg, softcap):
+            if _stats_pay(n, V, D, h2.device) and _ce_stats(hc, weight, lg, softcap):
                 stats, lse = torch.empty(-(-V // 256), n, 2, dtype=torch.float32, device=h2.device), torch.empty(n, dtype=torch.float32, device=h2.device)
                 check(L.ttb_gemm_bf16_2sm_stats(hc.data_ptr(), weight.data_ptr(), lg.data_ptr(), stats.data_ptr(), n, V, D, hc.stride(0), weight.stride(0), lg.stride(0),
                                                 err_word(h2.device).data_ptr(), stream_ptr()), f"logits and their statistics T={n} V={V} D={D}")
