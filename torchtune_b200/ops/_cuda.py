@@ -521,10 +521,20 @@ def lora_linear_nf4(x, xd, nf4, bias, a, b, scale):
 
 
 def _groups_on_pairs(rows: int, E: int, N: int, K: int) -> bool:
-    """Whether grouped products run on CTA pairs (``csrc/gemm_grouped2sm.cu``), which put 256 columns of the result on the rows of a tile (a narrower result would leave them empty) and need work for many tiles to
-    hide that pairs start later and come in half the number: us with 128-row tiles / with pairs for up to 128 rows per expert 16 x 2048 x 1536 36 / 42, 64 x 2048 x 1536 93 / 101,
-    64 x 2880 x 2880 202 / 198, 128 x 2048 x 1536 161 / 151; 512 rows per expert 8 x 512 x 256 19.5 / 23.5, 16 x 768 x 2048 42 / 44, 16 x 2048 x 1536 64 / 60, 64 x 2048 x 768 116 / 106."""
-    return N >= 256 and (E * K * N >= 2**28 or (rows >= 256 * E and E * K * N >= 2**25))
+    """Whether grouped products run on CTA pairs (``csrc/gemm_grouped2sm.cu``), which put 256 columns of the result on the rows of a tile (a narrower result would leave them empty), start later and come in
+    half the number, so that few tiles leave more of them idle.  us with 128-row tiles / with pairs, 60 launches in a row over more weights than the L2 holds:
+
+    * from 256 rows per expert on it takes enough products and tiles: 8 x 2048 x 2048 (contraction, result) of 4096 rows 39 / 45, 6144 53 / 57, 8192 67 / 61; 32 x 2048 x 768 of 8192 rows 44 / 49,
+      of 16384 60 / 62, the other way round 66 / 63; 64 x 768 x 1024 of 16384 rows 46 / 53, of 49152 96 / 90; 16 x 2048 x 1280 of 10000 rows 55 / 58, the other way round 59 / 57;
+    * from 128 rows per expert on large weights are loaded half as often: 4 x 8192 x 8192 of 600 rows 126 / 102, 16 x 4096 x 4096 of 2048 115 / 105, 128 x 2048 x 1536 of 19200 209 / 162;
+    * fewer rows only stream the weights.  64 rows per expert: 8 x 8192 x 4096 97 / 104, 16 x 4096 x 4096 95 / 100, 64 x 2048 x 2048 103 / 105, but 16 x 5120 x 8192 228 / 220,
+      32 x 4096 x 4096 186 / 180, 128 x 2048 x 1024 110 / 101, 256 x 1024 x 1024 115 / 105."""
+    size = E * N * K
+    if N < 256 or size < 2**25:
+        return False
+    if size >= 2**28:
+        return rows >= 128 * E or E >= 128 or (E >= 16 and size >= 2**29)
+    return rows >= 256 * E and rows * N * K >= 3 * 2**33 and E * -(-rows // (256 * E)) * -(-N // 256) >= 256
 
 
 def _grouped_gemm(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor, b_mn: bool) -> torch.Tensor:
