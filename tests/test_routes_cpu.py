@@ -145,7 +145,7 @@ def test_scaled_gradients_of_batched_and_differentiated_factors(library):
     assert library.calls == ["ttb_scale_bf16"] * 2
 
 
-@pytest.mark.parametrize("M,N,K,pays", [(64, 32000, 2048, False), (1000, 32000, 2048, True), (20, 128256, 2048, True), (300, 128256, 1024, False), (4096, 128256, 512, False), (8192, 128256, 4096, True)])
+@pytest.mark.parametrize("M,N,K,pays", [(64, 32000, 2048, False), (300, 32000, 2048, False), (1000, 32000, 2048, True), (20, 128256, 2048, True), (300, 128256, 1024, False), (4096, 128256, 512, False), (8192, 128256, 4096, True)])
 def test_softmax_statistics_are_taken_where_they_were_measured_to_pay(library, M, N, K, pays):
     assert _cuda._stats_pay(M, N, K, None) is pays
 
@@ -153,6 +153,6 @@ def test_softmax_statistics_are_taken_where_they_were_measured_to_pay(library, M
 @pytest.mark.parametrize("rows,E,K,N,pairs", [
     (4096, 8, 2048, 2048, False), (6144, 8, 2048, 2048, False), (8192, 32, 2048, 768, False), (16384, 32, 1024, 1024, False), (16384, 64, 768, 1024, False), (4096, 8, 4096, 2048, False), (4096, 8, 2048, 4096, True), (10000, 16, 2048, 1280, False), (10000, 16, 1280, 2048, True),
     (8192, 16, 2048, 2048, True), (32768, 64, 768, 2048, True), (5000, 8, 8192, 8192, True), (600, 4, 8192, 8192, True), (2048, 16, 4096, 4096, True), (256, 4, 8192, 14336, False),
-    (512, 8, 8192, 4096, False), (1024, 16, 4096, 4096, False), (4096, 64, 2048, 2048, False), (300, 16, 5120, 8192, True), (8192, 128, 2048, 1024, True), (40000, 16, 8192, 200, False)])
+    (512, 8, 8192, 4096, False), (1024, 16, 4096, 4096, False), (4096, 64, 2048, 2048, False), (2048, 32, 4096, 4096, False), (300, 16, 5120, 8192, True), (8192, 128, 2048, 1024, True), (40000, 16, 8192, 200, False)])
 def test_grouped_products_run_where_they_were_measured_to_be_faster(rows, E, K, N, pairs):
     assert _cuda._groups_on_pairs(rows, E, N, K) is pairs

@@ -522,18 +522,18 @@ def lora_linear_nf4(x, xd, nf4, bias, a, b, scale):
 
 def _groups_on_pairs(rows: int, E: int, N: int, K: int) -> bool:
     """Whether grouped products run on CTA pairs (``csrc/gemm_grouped2sm.cu``), which put 256 columns of the result on the rows of a tile (a narrower result would leave them empty), start later and come in
-    half the number, so that few tiles leave more of them idle.  us with 128-row tiles / with pairs, 60 launches in a row over more weights than the L2 holds:
+    half the number, so that few tiles leave more of them idle.  us with 128-row tiles / with pairs, out of a graph over more weights than the L2 holds (``microbench joined``):
 
-    * from 256 rows per expert on it takes enough products and tiles: 8 x 2048 x 2048 (contraction, result) of 4096 rows 39 / 45, 6144 53 / 57, 8192 67 / 61; 32 x 2048 x 768 of 8192 rows 44 / 49,
-      of 16384 60 / 62, the other way round 66 / 63; 64 x 768 x 1024 of 16384 rows 46 / 53, of 49152 96 / 90; 16 x 2048 x 1280 of 10000 rows 55 / 58, the other way round 59 / 57;
-    * from 128 rows per expert on large weights are loaded half as often: 4 x 8192 x 8192 of 600 rows 126 / 102, 16 x 4096 x 4096 of 2048 115 / 105, 128 x 2048 x 1536 of 19200 209 / 162;
-    * fewer rows only stream the weights.  64 rows per expert: 8 x 8192 x 4096 97 / 104, 16 x 4096 x 4096 95 / 100, 64 x 2048 x 2048 103 / 105, but 16 x 5120 x 8192 228 / 220,
-      32 x 4096 x 4096 186 / 180, 128 x 2048 x 1024 110 / 101, 256 x 1024 x 1024 115 / 105."""
+    * from 256 rows per expert on it takes enough products and tiles: 8 x 2048 x 2048 (contraction, result) of 4096 rows 36 / 42, 8192 63 / 57; 32 x 2048 x 768 of 16384 rows 55 / 60, the other way
+      round 60 / 59; 64 x 768 x 1024 of 16384 rows 45 / 48, of 49152 88 / 85; 16 x 2048 x 1280 of 10000 rows 52 / 55, the other way round 56 / 53; 64 x 768 x 2048 of 32768 119 / 107;
+    * from 128 rows per expert on large weights are loaded half as often: 4 x 8192 x 8192 of 600 rows 122 / 97, 16 x 4096 x 4096 of 2048 112 / 101, 128 x 2048 x 1536 of 19200 197 / 155;
+    * fewer rows only stream the weights.  64 rows per expert: 8 x 8192 x 4096 95 / 102, 16 x 4096 x 4096 93 / 97, 64 x 2048 x 2048 98 / 103, 32 x 4096 x 4096 178 / 175 and as an input
+      gradient 182 / 190, but 16 x 5120 x 8192 220 / 211, 128 x 2048 x 1024 105 / 98, 256 x 1024 x 1024 117 / 103."""
     size = E * N * K
     if N < 256 or size < 2**25:
         return False
     if size >= 2**28:
-        return rows >= 128 * E or E >= 128 or (E >= 16 and size >= 2**29)
+        return rows >= 128 * E or E >= 128 or (E >= 16 and size > 2**29)
     return rows >= 256 * E and rows * N * K >= 3 * 2**33 and E * -(-rows // (256 * E)) * -(-N // 256) >= 256
 
 
@@ -1476,9 +1476,9 @@ def _ce_stats(h: torch.Tensor, weight: torch.Tensor, logits: torch.Tensor, softc
 
 def _stats_pay(M: int, N: int, K: int, device: torch.device) -> bool:
     """Whether those statistics cost less than the pass over the logits that they save: the epilogue that takes them hides behind the products of the next tile, so there has to be one, and
-    its contraction has to be as long.  Loss and both gradients, us without / with: 64 tokens of 32000 x 2048 143.1 / 146.7, 300 220.2 / 221.5, 1000 365.8 / 355.6; 20 of 128256 x 2048
-    382.1 / 378.0, 4096 4730 / 4568; 300 of 128256 x 1024 388 / 401, x 512 292 / 322.  Loss alone: 300 of 128256 x 2048 214.7 / 202.4, x 1024 138.1 / 159.6."""
-    return K >= 2048 and (-(-M // 256)) * (-(-N // 256)) >= 3 * _sm_pairs(device)
+    its contraction has to be as long.  Loss and both gradients, us without / with (``microbench joined``): 64 tokens of 32000 x 2048 144 / 149, 300 218 / 220, 1000 361 / 351; 20 of 128256 x 2048
+    384 / 380, 300 642 / 620, 4096 5319 / 4995; 300 of 128256 x 1024 445 / 468, x 512 294 / 321."""
+    return K >= 2048 and (-(-M // 256)) * (-(-N // 256)) >= 4 * _sm_pairs(device)
 
 
 class _LinearCE(torch.autograd.Function):

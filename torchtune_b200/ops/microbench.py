@@ -296,20 +296,30 @@ def bench_decode(args, flush):
 
 def bench_joined(args, flush):
     """Operations that take a pass along beside the same ones apart: logits widened in the epilogue, the mean's gradients out of the products, input gradients of joined
-    projections, and by themselves the backward passes of norm and attention and the grouped products of an expert layer.  One JSON line per operation."""
-    from . import attention, grouped_matmul, linear, linear_cross_entropy, linear_cross_entropy_mean, linear_group, linear_widened, rms_norm, widen
+    projections, softmax statistics; the backward passes of norm and attention by themselves; grouped products on CTA pairs beside one CTA to a tile.  One JSON line per operation."""
+    from . import _cuda, attention, linear, linear_cross_entropy, linear_cross_entropy_mean, linear_group, linear_widened, rms_norm, widen
     from .mask import AttentionMask
 
     gen = torch.Generator(device="cuda").manual_seed(0)
     rand = lambda *s, std=1.0: torch.empty(*s, dtype=torch.bfloat16, device="cuda").normal_(0, std, generator=gen)
     rows = []
 
+    def once(fn) -> float:
+        for _ in range(4):  # also the time in which the host gets ahead, so that only the device's counts
+            flush.zero_()
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        fn()
+        e1.record()
+        torch.cuda.synchronize()
+        return e0.elapsed_time(e1)
+
     def emit(op, joined, apart=None, **kw):
         fns = [joined] if apart is None else [joined, apart]
         times = [[] for _ in fns]
         for i in range(args.warmup + args.iters):  # in turn: what ran before decides how far the clock is from the power limit
             for fn, t in zip(fns, times):
-                ms = _time(fn, 1, 0, flush)
+                ms = once(fn)
                 if i >= args.warmup:
                     t.append(ms)
         row = {"op": op, **kw, **{name: round(1e3 * sorted(t)[len(t) // 2], 1) for name, t in zip(("us", "apart_us"), times)}}
@@ -342,13 +352,47 @@ def bench_joined(args, flush):
         q, k, v = (rand(1, 16384, n, d).requires_grad_() for n in (heads, kv, kv))
         emit("attention backward", back(attention(q, k, v, AttentionMask(causal=True)), (q, k, v), rand(1, 16384, heads, d)), tokens=16384, heads=heads, key_heads=kv, head_dim=d)
     del q, k, v
-    for experts, n, k, out in ((16, 300, 5120, 8192), (16, 1024, 5120, 8192), (16, 1024, 8192, 5120), (16, 4096, 5120, 8192), (16, 8192, 5120, 8192), (16, 12000, 5120, 8192),
-                               (16, 16384, 2048, 8192), (8, 2048, 4096, 14336), (64, 8192, 2048, 768), (16, 2048, 2048, 1536)):
-        x, w = rand(n, k).requires_grad_(), rand(experts, k, out, std=0.02)
+    # statistics of the softmax out of the logits' product, or a pass over the logits
+    for n, vocab, dim in ((64, 32000, 2048), (300, 32000, 2048), (1000, 32000, 2048), (20, 128256, 2048), (300, 128256, 2048), (4096, 128256, 2048), (300, 128256, 1024), (300, 128256, 512)):
+        h, w, labels = rand(n, dim).requires_grad_(), rand(vocab, dim, std=0.02).requires_grad_(), torch.randint(0, vocab, (n,), device="cuda", generator=gen)
+
+        def loss(stats, grads):
+            def run():
+                rule, _cuda._stats_pay = _cuda._stats_pay, lambda *sizes: stats
+                try:
+                    if grads:
+                        torch.autograd.grad(linear_cross_entropy(h, w, labels)[0], (h, w))
+                    else:
+                        linear_cross_entropy(h.detach(), w.detach(), labels)
+                finally:
+                    _cuda._stats_pay = rule
+            return run
+
+        for grads in (False, True):
+            emit("cross-entropy and both gradients, statistics" if grads else "cross-entropy, statistics", loss(True, grads), loss(False, grads), tokens=n, vocabulary=vocab, dim=dim,
+                 taken=_cuda._stats_pay(n, vocab, dim, h.device))
+    # grouped products on CTA pairs or one CTA to a tile: launches in a graph, over more weights than the L2 holds
+    for experts, n, k, out in ((16, 300, 5120, 8192), (16, 1024, 5120, 8192), (16, 4096, 5120, 8192), (16, 12000, 5120, 8192), (8, 2048, 4096, 14336), (4, 600, 8192, 8192), (4, 256, 8192, 14336),
+                               (8, 512, 4096, 8192), (16, 1024, 4096, 4096), (16, 2048, 4096, 4096), (32, 2048, 4096, 4096), (64, 4096, 2048, 2048), (128, 8192, 2048, 1024), (128, 19200, 2048, 1536),
+                               (256, 16384, 1024, 1024), (8, 4096, 2048, 2048), (8, 6144, 2048, 2048), (8, 8192, 2048, 2048), (32, 8192, 2048, 768), (32, 16384, 2048, 768),
+                               (64, 16384, 768, 1024), (64, 49152, 768, 1024), (16, 10000, 2048, 1280), (64, 32768, 2048, 768)):
+        copies = int(400e6 // (experts * k * out * 2)) + 2
+        ws = [rand(experts, k, out, std=0.02) for _ in range(copies)]
         counts = torch.bincount(torch.randint(0, experts, (n,), device="cuda", generator=gen), minlength=experts)
-        with torch.no_grad():
-            emit("grouped product", lambda: grouped_matmul(x, w, counts), experts=experts, rows=n, contraction=k, outputs=out)
-        emit("grouped input gradient", back(grouped_matmul(x, w, counts), x, rand(n, out)), experts=experts, rows=n, contraction=out, outputs=k)
+        for forward in (True, False):
+            x, size, result = rand(n, k if forward else out), *((k, out) if forward else (out, k))
+            rule, us = _cuda._groups_on_pairs, {}
+            for pairs in (True, False):
+                _cuda._groups_on_pairs = lambda *sizes: pairs
+                try:
+                    us[pairs] = 1e3 * _time_captured(lambda i: lambda: _cuda._grouped_gemm(x, ws[i % copies], counts, forward), args.iters, 2.0 * experts * k * out)
+                finally:
+                    _cuda._groups_on_pairs = rule
+            row = {"op": "grouped product on CTA pairs" if forward else "grouped input gradient on CTA pairs", "experts": experts, "rows": n, "contraction": size, "outputs": result,
+                   "taken": rule(n, experts, result, size), "us": round(us[True], 1), "apart_us": round(us[False], 1)}
+            rows.append(row)
+            print(json.dumps(row), flush=True)
+        del ws
     return {"op": "joined", "rows": len(rows)}
 
 
