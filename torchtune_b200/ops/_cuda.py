@@ -59,8 +59,8 @@ ROWS_LIMIT = 64  # most tokens csrc/gemm_rows.cu takes
 def _runs_rows(M: int, N: int, K: int) -> bool:
     """Whether a linear layer streams its weights through registers (``csrc/gemm_rows.cu``) instead of running on a tile kernel.  The lines are drawn for the
     joined forms, which share them: there the tile kernels need several launches (us here / there: gated 32 x 14336 x 4096 55 / 88; one launch for query, key and value
-    of 64 tokens (4096 + 1024 + 1024 rows of 4096) 30 / three of about 40).  Products by themselves (weights from HBM): 16 x 4096 x 4096 11.2 / 13.8, 64 x 2048 x 2048 11.0 / 11.3, 16 x 14336 x 4096
-    28 / 28; with a vocabulary of rows the CTA-pair kernel streams as well: 16 x 128256 x 2048 98 / 115, x 4096 198 / 186, 8 x 128256 x 4096 173 / 210.
+    of 64 tokens (4096 + 1024 + 1024 rows of 4096) 30 / three of about 40).  Products by themselves (weights from HBM): 16 x 4096 x 4096 11.3 / 14.0, 64 x 2048 x 2048 11.0 / 11.3, 16 x 14336 x 4096
+    28 / 28; with a vocabulary of rows the CTA-pair kernel streams as well: 16 x 128256 x 2048 97 / 123, x 4096 201 / 185, 8 x 128256 x 4096 171 / 205.
     Since the tile kernels cut long contractions into ranges they win somewhat below these lines: 48 x 4096 x 4096 16.8 / 15.2, 64 x 4096 x 14336 43 / 31,
     16 x 5120 x 5120 18.4 / 17.1, 32 x 6144 x 4096 20.0 / 17.0, 24 x 28672 x 4096 57 / 53."""
     most = ROWS_LIMIT if N <= 4096 else 32 if N <= 32768 else 16 if K < 4096 else 8
@@ -277,8 +277,8 @@ def gemm_residual(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, bias
 
 def gemm_sum(dys: Sequence[torch.Tensor], ws: Sequence[torch.Tensor]) -> torch.Tensor:
     """``Σ dys[i] · ws[i]`` (``[M, K_i] · [K_i, N]``): the input gradient of several linear layers of one input.  Two products share an accumulator, unless their contractions are cut into ranges,
-    and on CTA pairs a further one adds the sum so far in its epilogue: fewer passes over ``[M, N]`` and fewer roundings than products that autograd adds up (us before -> here: 8192 x 4096 of
-    4096 + 1024 + 1024 332 -> 291, 16384 x 2048 of 2048 + 512 + 512 291 -> 222, of 8192 + 8192 740 -> 722; error against 64 bits 2.9e-3 -> 2.2e-3)."""
+    and on CTA pairs a further one adds the sum so far in its epilogue: fewer passes over ``[M, N]`` and fewer roundings than products that autograd adds up (us of those / here, ``microbench joined``:
+    8192 x 4096 of 4096 + 1024 + 1024 329 / 282, 16384 x 2048 of 2048 + 512 + 512 232 / 177, of 8192 + 8192 746 / 729; error against 64 bits 2.9e-3 / 2.2e-3)."""
     M, N = dys[0].shape[0], ws[0].shape[1]
     sizes = [w.shape[0] for w in ws]
     fit = lambda t: t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
@@ -524,11 +524,11 @@ def _groups_on_pairs(rows: int, E: int, N: int, K: int) -> bool:
     """Whether grouped products run on CTA pairs (``csrc/gemm_grouped2sm.cu``), which put 256 columns of the result on the rows of a tile (a narrower result would leave them empty), start later and come in
     half the number, so that few tiles leave more of them idle.  us with 128-row tiles / with pairs, out of a graph over more weights than the L2 holds (``microbench joined``):
 
-    * from 256 rows per expert on it takes enough products and tiles: 8 x 2048 x 2048 (contraction, result) of 4096 rows 36 / 42, 8192 63 / 57; 32 x 2048 x 768 of 16384 rows 55 / 60, the other way
-      round 60 / 59; 64 x 768 x 1024 of 16384 rows 45 / 48, of 49152 88 / 85; 16 x 2048 x 1280 of 10000 rows 52 / 55, the other way round 56 / 53; 64 x 768 x 2048 of 32768 119 / 107;
-    * from 128 rows per expert on large weights are loaded half as often: 4 x 8192 x 8192 of 600 rows 122 / 97, 16 x 4096 x 4096 of 2048 112 / 101, 128 x 2048 x 1536 of 19200 197 / 155;
-    * fewer rows only stream the weights.  64 rows per expert: 8 x 8192 x 4096 95 / 102, 16 x 4096 x 4096 93 / 97, 64 x 2048 x 2048 98 / 103, 32 x 4096 x 4096 178 / 175 and as an input
-      gradient 182 / 190, but 16 x 5120 x 8192 220 / 211, 128 x 2048 x 1024 105 / 98, 256 x 1024 x 1024 117 / 103."""
+    * from 256 rows per expert on it takes enough products and tiles: 8 x 2048 x 2048 (contraction, result) of 4096 rows 37 / 43, 8192 63 / 57; 32 x 2048 x 768 of 16384 rows 56 / 60, the other way
+      round 62 / 60; 64 x 768 x 1024 of 16384 rows 46 / 49, of 49152 90 / 86; 16 x 2048 x 1280 of 10000 rows 52 / 56, the other way round 56 / 55; 64 x 768 x 2048 of 32768 122 / 109;
+    * from 128 rows per expert on large weights are loaded half as often: 4 x 8192 x 8192 of 600 rows 124 / 99, 16 x 4096 x 4096 of 2048 114 / 102, 128 x 2048 x 1536 of 19200 206 / 159;
+    * fewer rows only stream the weights.  64 rows per expert: 8 x 8192 x 4096 97 / 104, 16 x 4096 x 4096 93 / 98, 64 x 2048 x 2048 100 / 104, 32 x 4096 x 4096 183 / 176 and as an input
+      gradient 186 / 193, but 16 x 5120 x 8192 225 / 213, 128 x 2048 x 1024 106 / 98, 256 x 1024 x 1024 114 / 103."""
     size = E * N * K
     if N < 256 or size < 2**25:
         return False
@@ -1476,8 +1476,8 @@ def _ce_stats(h: torch.Tensor, weight: torch.Tensor, logits: torch.Tensor, softc
 
 def _stats_pay(M: int, N: int, K: int, device: torch.device) -> bool:
     """Whether those statistics cost less than the pass over the logits that they save: the epilogue that takes them hides behind the products of the next tile, so there has to be one, and
-    its contraction has to be as long.  Loss and both gradients, us without / with (``microbench joined``): 64 tokens of 32000 x 2048 144 / 149, 300 218 / 220, 1000 361 / 351; 20 of 128256 x 2048
-    384 / 380, 300 642 / 620, 4096 5319 / 4995; 300 of 128256 x 1024 445 / 468, x 512 294 / 321."""
+    its contraction has to be as long.  Loss and both gradients, us without / with (``microbench joined``): 64 tokens of 32000 x 2048 144 / 148, 300 220 / 222, 1000 361 / 351; 20 of 128256 x 2048
+    386 / 380, 300 632 / 616, 4096 5687 / 5344; 300 of 128256 x 1024 544 / 571, x 512 300 / 327."""
     return K >= 2048 and (-(-M // 256)) * (-(-N // 256)) >= 4 * _sm_pairs(device)
 
 
@@ -1489,8 +1489,8 @@ class _LinearCE(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, weight, labels, ignore_index, num_chunks, softcap=0.0, mean=False):
-        """``mean``: the loss is the mean over the valid tokens, and so are, in a single pass, the gradients: 1 / count multiplies the sums of the products that make them, before they are rounded,
-        instead of both results in a pass of its own (1 GB of weight gradient for a vocabulary of 128256 x 4096: 0.33 ms).  It may not go into the gradient of the logits: that is nearly -1, which bf16
+        """``mean``: the loss is the mean over the valid tokens, and so are, in a single pass, the gradients: 1 / count multiplies what the products that make them add up, on CTA pairs before it is
+        rounded, instead of both results in a pass of its own (1 GB of weight gradient for a vocabulary of 128256 x 4096: 0.33 ms).  It may not go into the gradient of the logits: that is nearly -1, which bf16
         holds exactly, at every label."""
         D = hidden.shape[-1]
         h2 = hidden.reshape(-1, D)

@@ -7,9 +7,9 @@
 // which also leave out the rows of the next expert that a last piece has computed.
 // Pipeline, barriers and failure handling are those of gemm2sm.cu; the piece's size travels with the tile through the table that a small kernel builds from the row counts on the
 // device, so no host read is needed.
-// 16 experts of 5120 x 8192, us forward / input gradient with one CTA per 128 x 256 tile -> here: 300 rows 225 / 254 -> 219 / 243 (6.1 TB/s of weights), 4096 rows 391 / 399 -> 326 / 326, 12000 rows
-// 841 / 850 -> 760 / 778 (1324 TFLOP/s).  At 4096 rows the pieces of few tokens wait for weights and those of many for products; mixing them (all experts at a block of weight rows) read
-// the tokens again for each block and took 371 / 369.
+// 16 experts of 5120 x 8192, us forward / input gradient with one CTA per 128 x 256 tile -> here, out of a graph over more weights than the L2 holds: 300 rows 217 / 245 -> 207 / 230 (6.5 TB/s of
+// weights), 4096 rows 372 / 404 -> 338 / 360, 12000 rows 846 / 894 -> 751 / 808 (1340 TFLOP/s).  Where products of this kernel are slower, see ops._cuda._groups_on_pairs.  At 4096 rows the pieces of
+// few tokens wait for weights and those of many for products; mixing them (all experts at a block of weight rows) read the tokens again for each block and took 14 % longer.
 #include <cstring>
 
 #include "common/pair.cuh"

@@ -250,8 +250,8 @@ gemm_rows_kernel(const __grid_constant__ Params p, int splits) {
 // Up to 16 tokens whose share of a CTA's contraction fits shared memory as a whole: they are staged once, and the warps stream their weights without meeting until the end.  With NORM, x is normalised on
 // the way in (the sums of squares in the order of the norm's own kernel, so the values are the same ones): a norm by itself is a launch of 2 us in a decode step, and here its reads
 // hide behind the first weights.
-// us in a graph, weights from HBM, with the ring above -> here, 1 / 16 tokens: 6144 x 4096 14.9 / 16.7 -> 13.3 / 15.7, 4096 x 14336 24.7 / 27.3 -> 22.1 / 24.7 (5.3 TB/s), 128256 x 2048
-// 94.8 / 104.5 -> 83.0 / 98.2 (6.3 TB/s), 128256 x 4096 186 -> 163 (6.4 TB/s).  A chat turn of the 16-layer 1B model, with the norms, 25.1 -> 23.0 ms.
+// us in a graph, weights from HBM, with the ring above -> here, 1 / 16 tokens: 6144 x 4096 14.6 / 16.9 -> 13.2 / 15.8, 4096 x 14336 25.1 / 27.6 -> 23.0 / 25.2 (5.1 TB/s), 128256 x 2048
+// 94.8 / 104 -> 82.4 / 97.2 (6.4 TB/s), 128256 x 4096 186 -> 163 (6.4 TB/s).  A chat turn of the 16-layer 1B model, with the norms, 25.1 -> 23.0 ms.
 template <int MT, int WK, bool GATED, bool NORM>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_rows_resident_kernel(const __grid_constant__ Params p, int splits) {

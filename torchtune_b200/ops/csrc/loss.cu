@@ -134,7 +134,7 @@ softmax_ce_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restric
 // Where the product that made the logits left each row's maximum and sum of exponentials per tile of 256 columns (gemm2sm.cu), the softmax needs no pass over the logits: one kernel
 // merges a row's partials in their order (rows next to each other in a warp, the tiles dealt to eight warps), and the gradient is one element-wise pass, 64 bytes in flight per
 // thread and no reduction, bound by its reads and writes.  8192 x 128256: 1.0 - 1.55 ms with the kernel above, 0.65 ms here (6.5 TB/s); the
-// GEMM's epilogue hides behind its products.
+// GEMM's epilogue hides behind the products of its next tile where their contraction is long (ops._cuda._stats_pay).
 static constexpr int kStatTile = 256;
 
 __global__ void __launch_bounds__(256)
