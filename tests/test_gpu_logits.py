@@ -220,7 +220,7 @@ def test_mean_loss(T, V):
 @pytest.mark.parametrize("T,V", [(16, 128), (700, 20000)])
 def test_mean_loss_of_a_weight_with_a_gradient_window(T, V, written):
     """A weight whose gradients are delivered straight to a flat buffer: the mean's arrives as that of the mean, whatever multiplies it and whatever was there before; the sum's
-    goes straight to the buffer."""
+    goes straight to the buffer, and that of a loss without autograd nowhere."""
     from types import SimpleNamespace
 
     from torchtune_b200 import ops
@@ -244,6 +244,13 @@ def test_mean_loss_of_a_weight_with_a_gradient_window(T, V, written):
         w._grad_written = False
         ops.linear_cross_entropy(h, w, labels)[0].backward()
         assert w.grad is None and w._grad_written and float((w._grad_buffer.double() - int(count) * want_w).norm()) <= 2.0**-7 * int(count) * float(want_w.norm())
+        before = w._grad_buffer.clone()
+        with torch.no_grad():  # a validation loss between two steps
+            for w._grad_written in (True, False):
+                again, mean = ops.linear_cross_entropy(h, w, labels)[0], ops.linear_cross_entropy_mean(h, w, labels)
+                assert torch.equal(w._grad_buffer, before) and not again.requires_grad and not mean.requires_grad
+                assert abs(float(again) - float(total)) <= 2.0**-20 * float(total) and abs(float(mean) * int(count) - float(total)) <= 2.0**-19 * float(total)
+            assert w._grad_written is False
     finally:
         _cuda.enable_direct_wgrad(False)
         _cuda.unregister_grad_window(w.data_ptr())

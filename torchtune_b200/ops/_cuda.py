@@ -1571,19 +1571,25 @@ class _LinearCE(torch.autograd.Function):
         return gh, gw, None, None, None, None, None
 
 
+def _undifferentiated(*tensors: torch.Tensor) -> Tuple[torch.Tensor, ...]:
+    """``tensors`` as they are, detached where autograd is off: a function that forms gradients in forward is told of parameters alone, not of the mode, and a validation loss must not
+    write to the window of its weight."""
+    return tensors if torch.is_grad_enabled() else tuple(t.detach() for t in tensors)
+
+
 def linear_cross_entropy(hidden, weight, labels, ignore_index: int, num_chunks: int, softcap: float = 0.0):
     if hidden.shape[-1] % 8 or weight.shape[0] % 8:
         from . import _fallback, reference
 
         _fallback("linear_cross_entropy", f"width {hidden.shape[-1]} or vocabulary {weight.shape[0]} is not a multiple of 8", hidden)
         return reference.linear_cross_entropy(hidden, weight, labels, ignore_index, num_chunks, softcap=softcap)
-    return _LinearCE.apply(hidden, weight, labels, ignore_index, num_chunks, float(softcap))
+    return _LinearCE.apply(*_undifferentiated(hidden, weight), labels, ignore_index, num_chunks, float(softcap))
 
 
 def linear_cross_entropy_mean(hidden, weight, labels, ignore_index: int, num_chunks: int) -> Optional[torch.Tensor]:
     if hidden.shape[-1] % 8 or weight.shape[0] % 8:
         return None
-    return _LinearCE.apply(hidden, weight, labels, ignore_index, num_chunks, 0.0, True)[0]
+    return _LinearCE.apply(*_undifferentiated(hidden, weight), labels, ignore_index, num_chunks, 0.0, True)[0]
 
 
 def _softmax_ce(buf, labels, loss_out, row_scale, n, V, ignore_index, mode, softcap=0.0):
